@@ -397,6 +397,38 @@ def test_gemm(dtype, out_dtype, m, n, k) -> None:
     torch.testing.assert_close(out.float(), want.float(), **t)
 
 
+@pytest.mark.parametrize("m", [1, 2, 5, 9, 17, 33, 65, 130])
+@pytest.mark.parametrize("n,k", [(1, 4), (301, 72), (64, 64), (1000, 132), (1024, 3072), (129, 1028)])
+def test_gemm_f32_forms_agree_bit_for_bit(m, n, k) -> None:
+    """Every form of the 32-bit product keeps one order of summation: 16 chains over K and 15 additions, so an
+    output is off by at most (K / 16 + 4 + 15) roundings of the sum of its terms' sizes."""
+    x, w = rnd(m, k, seed=1), rnd(n, k, seed=2)
+    out = torch.full((m, n), float("nan"), device="cuda")
+    ops.gemm(x, w, out)
+    wide = x.double() @ w.double().T
+    bound = (k / 16 + 4 + 15 + 1) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    assert bool(((out.double() - wide).abs() <= bound).all())
+    for form in range(1, 6):
+        other = torch.full((m, n), float("nan"), device="cuda")
+        ops._check(ops._fn("ts_gemm_f32")(x.data_ptr(), w.data_ptr(), other.data_ptr(), m, n, k, form, ops._stream()), "gemm")
+        assert torch.equal(out, other), form
+    row = torch.empty(1, n, device="cuda")
+    ops.gemm(x[m - 1:].contiguous(), w, row)
+    assert torch.equal(row[0], out[m - 1])
+
+
+def test_gemm_f32_rows_off_the_16_byte_grid_take_the_general_kernel() -> None:
+    x, w = rnd(7, 33, seed=1), rnd(20, 33, seed=2)
+    out = torch.empty(7, 20, device="cuda")
+    ops.gemm(x, w, out)
+    torch.testing.assert_close(out, x @ w.T, atol=1e-4, rtol=1e-5)
+    base = rnd(1, 7 * 32 + 1, seed=3).flatten()
+    out2, want2 = torch.empty(7, 20, device="cuda"), torch.empty(7, 20, device="cuda")
+    ops.gemm(base[1:].view(7, 32), w[:, :32].contiguous(), out2)
+    ops.gemm_simt(base[1:].clone().view(7, 32), w[:, :32].contiguous(), want2)
+    assert torch.equal(out2, want2)
+
+
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("m", [1, 3, 8, 9, 16, 31, 64])
 @pytest.mark.parametrize("n,k", [(16, 32), (48, 96), (1024, 2048), (4096, 1024), (151936, 1024), (1040, 3072)])

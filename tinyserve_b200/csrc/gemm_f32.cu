@@ -1,0 +1,330 @@
+// out[M, N] = x[M, K] * w[N, K]^T, all 32-bit floats, on CUDA cores (no tensor cores, no reduced precision).
+// Two kernels for two regimes, one order of summation. K % 4 == 0 and 16-byte aligned pointers.
+//
+// Order of the sums. K is cut into 16 equal parts (4 * ceil(K / 64) long; the last ones may be shorter or empty). A
+// part is one chain of fused multiply-adds in index order; four neighbouring parts make a group, added left to right;
+// the four groups are added left to right. Both kernels, every tile and every split keep that order bit for bit, so a
+// row's result depends neither on M nor on the rows beside it. (One chain over all of K, which this replaces, has the
+// larger error: 16 short chains and 15 additions against K dependent roundings.)
+//
+// A few rows (M <= 16): bound by the stream of the weights. A CTA takes 8 rows of w; thread = (row, part), the 16
+// parts of a row side by side, so 128 threads add up 128 chains and 1,024 weight rows already give 128 CTAs. Slabs of
+// 32 k per part (16 KB of w) come through a ring of cp.async stages, the first ones in front of the wait for the
+// kernels before this one. Every weight is read from shared memory once for up to 8 rows of x; from three rows and
+// 2,048 columns on a thread owns two weight rows, because a broadcast word of x costs the shared memory as much as a
+// word of w (8 rows of the 151,936 x 1,024 head: 207 us with one, 165 us with two). Measured back to back on B200, one
+// row, 64 x 64 tiles of all K before / now: 4,096 x 1,024 70 / 11 us, 1,024 x 3,072 205 / 8 us, the head 92 us (6.8 TB/s).
+//
+// More rows: bound by the multiply-adds and, below some hundred rows, by the latency of the chains. Register tiles of
+// 4 x 4 outputs a thread, 32 x 64 a CTA, operands in shared memory as [row][16 k] read in 16-byte words (rows a thread owns lie a stride apart, so that eight neighbouring threads read
+// eight different groups of banks), three cp.async stages. Where the tiles are too few for the machine, the four
+// groups of K go to the two or four CTAs of a cluster, which leave their sums in shared memory; each then adds up its
+// share of the tile through distributed shared memory. Measured, before / now: 45 rows of 4,096 x 1,024 76 / 25 us,
+// of 1,024 x 3,072 221 / 29 us; 190 rows of 6,144 x 1,024 115 / 80 us. Tiles of 64 x 64 and 128 x 128 (8 outputs a
+// thread and side) were no faster at any of 1 to 600 rows: they leave too few warps on an SM.
+#define TS_PDL_CLASS PDL_OTHER
+#include <cooperative_groups.h>
+
+#include "common.cuh"
+
+namespace ts {
+namespace cg = cooperative_groups;
+
+__device__ __forceinline__ void f32_copy16(float* dst, const float* src, bool ok) {
+  const unsigned int d = (unsigned int)__cvta_generic_to_shared(dst);
+  const int n = ok ? 16 : 0;     // zero-filled beyond the matrix
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void f32_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT> __device__ __forceinline__ void f32_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+
+constexpr int FP_PARTS = 16;
+__host__ __device__ __forceinline__ int f32_part_length(int K) { return 4 * ((K + 63) / 64); }
+
+// ------------------------------------------------------------------------------------------------- a few rows
+constexpr int FR_THREADS = 128, FR_SLAB = 32, FR_STRIDE = FR_SLAB + 4, FR_STAGES = 4;
+
+// MT rows of x; a thread owns R rows of w (8 R a CTA).
+template <int MT, int R>
+struct F32Rows {
+  static constexpr int ROWS = 8 * R;
+  static constexpr int STAGE = FP_PARTS * ROWS * FR_STRIDE + MT * FP_PARTS * FR_SLAB;     // floats
+};
+
+template <int MT, int R>
+__global__ void __launch_bounds__(FR_THREADS) gemm_f32_rows_kernel(const float* x, const float* __restrict__ w, float* out,
+                                                                  int M, int N, int K) {
+  using Rows = F32Rows<MT, R>;
+  constexpr int ROWS = Rows::ROWS;
+  extern __shared__ float smem[];
+  __shared__ float sums[4][ROWS][MT];
+  pdl_trigger();
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int row = lane & 7, part = (tid >> 5) * 4 + (lane >> 3);     // a warp holds one group of four parts
+  const int n0 = blockIdx.x * ROWS, m0 = blockIdx.y * MT;
+  const int len = f32_part_length(K), slabs = (len + FR_SLAB - 1) / FR_SLAB;
+
+  auto load_w = [&](int slab, int stage) {
+    float* dst = smem + stage * Rows::STAGE;
+    // 16 parts x ROWS rows x 8 words of 16 bytes; eight neighbouring threads copy 128 bytes of a row
+#pragma unroll
+    for (int i = 0; i < FP_PARTS * ROWS * (FR_SLAB / 4) / FR_THREADS; ++i) {
+      const int c = i * FR_THREADS + tid;
+      const int word = c & 7, r = (c >> 3) % ROWS, p = (c >> 3) / ROWS;
+      const int in_part = slab * FR_SLAB + word * 4, k = p * len + in_part;
+      const bool ok = in_part < len && k < K && n0 + r < N;
+      f32_copy16(dst + (p * ROWS + r) * FR_STRIDE + word * 4, w + (ok ? (size_t)(n0 + r) * K + k : 0), ok);
+    }
+  };
+  auto load_x = [&](int slab, int stage) {
+    float* dst = smem + stage * Rows::STAGE + FP_PARTS * ROWS * FR_STRIDE;
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      const int word = tid & 7, p = tid >> 3;
+      const int in_part = slab * FR_SLAB + word * 4, k = p * len + in_part;
+      const bool ok = in_part < len && k < K && m0 + m < M;
+      f32_copy16(dst + (m * FP_PARTS + p) * FR_SLAB + word * 4, x + (ok ? (size_t)(m0 + m) * K + k : 0), ok);
+    }
+  };
+
+  // Weights do not depend on the kernels before this one: as many slabs as the ring takes are asked for before the wait.
+  const int first = slabs < FR_STAGES - 1 ? slabs : FR_STAGES - 1;
+  for (int s = 0; s < first; ++s) load_w(s, s);
+  pdl_wait();
+  for (int s = 0; s < FR_STAGES - 1; ++s) {
+    if (s < first) load_x(s, s);
+    f32_commit();          // the first of these groups also holds the weights of all of them
+  }
+
+  float acc[R][MT];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int m = 0; m < MT; ++m) acc[r][m] = 0.f;
+  for (int s = 0; s < slabs; ++s) {
+    f32_wait<FR_STAGES - 2>();
+    __syncthreads();       // slab s has arrived for everyone, and slab s - 1 has been read by everyone
+    const int ahead = s + FR_STAGES - 1;
+    if (ahead < slabs) {
+      load_w(ahead, ahead % FR_STAGES);
+      load_x(ahead, ahead % FR_STAGES);
+    }
+    f32_commit();
+    const float* stage = smem + (s % FR_STAGES) * Rows::STAGE;
+    const float* ws = stage + (part * ROWS + row) * FR_STRIDE;
+    const float* xs = stage + FP_PARTS * ROWS * FR_STRIDE + part * FR_SLAB;
+#pragma unroll
+    for (int i = 0; i < FR_SLAB; i += 4) {
+      float4 b[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) b[r] = *reinterpret_cast<const float4*>(ws + r * 8 * FR_STRIDE + i);
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        const float4 a = *reinterpret_cast<const float4*>(xs + m * FP_PARTS * FR_SLAB + i);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          acc[r][m] = fmaf(a.x, b[r].x, acc[r][m]);
+          acc[r][m] = fmaf(a.y, b[r].y, acc[r][m]);
+          acc[r][m] = fmaf(a.z, b[r].z, acc[r][m]);
+          acc[r][m] = fmaf(a.w, b[r].w, acc[r][m]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      const float p1 = __shfl_sync(0xffffffffu, acc[r][m], row + 8), p2 = __shfl_sync(0xffffffffu, acc[r][m], row + 16),
+                  p3 = __shfl_sync(0xffffffffu, acc[r][m], row + 24);
+      if (lane < 8) sums[tid >> 5][r * 8 + row][m] = ((acc[r][m] + p1) + p2) + p3;
+    }
+  __syncthreads();
+  for (int o = tid; o < ROWS * MT; o += FR_THREADS) {
+    const int r = o % ROWS, m = o / ROWS;
+    if (n0 + r < N && m0 + m < M)
+      out[(size_t)(m0 + m) * N + n0 + r] = ((sums[0][r][m] + sums[1][r][m]) + sums[2][r][m]) + sums[3][r][m];
+  }
+}
+
+template <int MT, int R>
+static int launch_rows(const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
+  using Rows = F32Rows<MT, R>;
+  const int most = FR_STAGES * Rows::STAGE * (int)sizeof(float);
+  static bool ready[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !ready[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<MT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 64) ready[dev] = true;
+  }
+  // fewer slabs than stages: room for those alone, so that more CTAs fit an SM
+  const int slabs = (f32_part_length(K) + FR_SLAB - 1) / FR_SLAB, smem = slabs < FR_STAGES ? most / FR_STAGES * slabs : most;
+  const dim3 grid((N + Rows::ROWS - 1) / Rows::ROWS, (M + MT - 1) / MT);
+  return launch(gemm_f32_rows_kernel<MT, R>, grid, FR_THREADS, smem, stream, x, w, out, M, N, K);
+}
+
+// -------------------------------------------------------------------------------------------------- more rows
+constexpr int FT_M = 32, FT_N = 64, FT_OWN = 4, FT_K = 16, FT_STRIDE = FT_K + 4, FT_STAGES = 3;
+constexpr int FT_THREADS = (FT_M / FT_OWN) * (FT_N / FT_OWN), FT_STAGE = (FT_M + FT_N) * FT_STRIDE;     // floats
+
+template <int SPLIT>
+__global__ void __launch_bounds__(FT_THREADS) gemm_f32_tile_kernel(const float* x, const float* __restrict__ w, float* out,
+                                                                   int M, int N, int K) {
+  constexpr int BM = FT_M, BN = FT_N, TM = FT_OWN, TN = FT_OWN;
+  constexpr int THREADS = FT_THREADS, GROUPS = 4 / SPLIT, OUTS = TM * TN;
+  extern __shared__ float smem[];
+  float* kept = smem + FT_STAGES * FT_STAGE;           // [group of this CTA][output of a thread][thread]
+  pdl_trigger();
+  const int tid = threadIdx.x;
+  const int tx = tid % (BN / TN), ty = tid / (BN / TN);
+  const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
+  const int len = f32_part_length(K), steps = (len + FT_K - 1) / FT_K;    // steps of a part
+  const int first_part = blockIdx.z * GROUPS * 4, total = GROUPS * 4 * steps;
+
+  auto load = [&](int step, int stage, bool a_side, bool b_side) {
+    float* dst = smem + stage * FT_STAGE;
+    const int part = first_part + step / steps, base = (step % steps) * FT_K;
+    if (a_side) {
+#pragma unroll
+      for (int c = tid; c < BM * (FT_K / 4); c += THREADS) {
+        const int word = c & 3, r = c >> 2, in_part = base + word * 4, k = part * len + in_part;
+        const bool ok = in_part < len && k < K && m0 + r < M;
+        f32_copy16(dst + r * FT_STRIDE + word * 4, x + (ok ? (size_t)(m0 + r) * K + k : 0), ok);
+      }
+    }
+    if (b_side) {
+#pragma unroll
+      for (int c = tid; c < BN * (FT_K / 4); c += THREADS) {
+        const int word = c & 3, r = c >> 2, in_part = base + word * 4, k = part * len + in_part;
+        const bool ok = in_part < len && k < K && n0 + r < N;
+        f32_copy16(dst + (BM + r) * FT_STRIDE + word * 4, w + (ok ? (size_t)(n0 + r) * K + k : 0), ok);
+      }
+    }
+  };
+#pragma unroll
+  for (int s = 0; s < FT_STAGES - 1; ++s) load(s, s, false, true);        // weights first (total is at least four steps)
+  pdl_wait();
+#pragma unroll
+  for (int s = 0; s < FT_STAGES - 1; ++s) { load(s, s, true, false); f32_commit(); }
+
+  float acc[TM][TN], group[TM][TN];
+  int step = 0;
+  for (int g = 0; g < GROUPS; ++g) {
+    for (int p = 0; p < 4; ++p) {
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+      for (int b = 0; b < steps; ++b, ++step) {
+        f32_wait<FT_STAGES - 2>();
+        __syncthreads();
+        if (step + FT_STAGES - 1 < total) load(step + FT_STAGES - 1, (step + FT_STAGES - 1) % FT_STAGES, true, true);
+        f32_commit();
+        const float* as = smem + (step % FT_STAGES) * FT_STAGE + ty * FT_STRIDE;
+        const float* bs = smem + (step % FT_STAGES) * FT_STAGE + (BM + tx) * FT_STRIDE;
+#pragma unroll
+        for (int k = 0; k < FT_K; k += 4) {
+          float4 a[TM];
+#pragma unroll
+          for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(as + i * (BM / TM) * FT_STRIDE + k);
+#pragma unroll
+          for (int j = 0; j < TN; ++j) {
+            const float4 v = *reinterpret_cast<const float4*>(bs + j * (BN / TN) * FT_STRIDE + k);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].x, v.x, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].y, v.y, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].z, v.z, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].w, v.w, acc[i][j]);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) group[i][j] = p == 0 ? acc[i][j] : group[i][j] + acc[i][j];
+    }
+    // SPLIT 1: the sum of the groups so far; else one group beside the other (a thread's own words: no barrier)
+    float* mine = kept + (SPLIT == 1 ? 0 : g * OUTS * THREADS) + tid;
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) {
+        float* o = mine + (i * TN + j) * THREADS;
+        *o = (SPLIT == 1 && g > 0) ? *o + group[i][j] : group[i][j];
+      }
+  }
+  f32_wait<0>();
+  auto store = [&](int o, float v) {
+    const int r = m0 + ty + (o / TN) * (BM / TM), c = n0 + tx + (o % TN) * (BN / TN);
+    if (r < M && c < N) out[(size_t)r * N + c] = v;
+  };
+  if (SPLIT == 1) {
+#pragma unroll 4
+    for (int o = 0; o < OUTS; ++o) store(o, kept[o * THREADS + tid]);
+  } else {
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    const float* of_group[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) of_group[g] = cluster.map_shared_rank(kept, g / GROUPS) + (g % GROUPS) * OUTS * THREADS + tid;
+    constexpr int SHARE = OUTS / SPLIT;
+#pragma unroll 4
+    for (int o = (int)blockIdx.z * SHARE; o < ((int)blockIdx.z + 1) * SHARE; ++o)
+      store(o, ((of_group[0][o * THREADS] + of_group[1][o * THREADS]) + of_group[2][o * THREADS]) + of_group[3][o * THREADS]);
+    cluster.sync();        // nobody leaves while its sums are still read
+  }
+}
+
+template <int SPLIT>
+static int launch_tile(const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
+  auto kernel = gemm_f32_tile_kernel<SPLIT>;
+  // the ring, and the sums of the CTA's groups
+  const int smem = (FT_STAGES * FT_STAGE + (SPLIT == 2 ? 2 : 1) * FT_M * FT_N) * (int)sizeof(float);
+  static bool ready[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !ready[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 64) ready[dev] = true;
+  }
+  if ((M + FT_M - 1) / FT_M > 65535) return TS_ERR_BAD_ARGUMENT;
+  const dim3 grid((N + FT_N - 1) / FT_N, (M + FT_M - 1) / FT_M, SPLIT);
+  if (SPLIT == 1) return launch(kernel, grid, FT_THREADS, smem, stream, x, w, out, M, N, K);
+  return launch_cluster(kernel, grid, FT_THREADS, smem, stream, dim3(1, 1, SPLIT), x, w, out, M, N, K);
+}
+
+}  // namespace ts
+
+using namespace ts;
+
+// `form`: 0 = chosen here; 1, 2 = a few rows, one or two weight rows a thread; 3, 4, 5 = tiles, K over 1, 2, 4 CTAs.
+extern "C" int ts_gemm_f32(const float* x, const float* w, float* out, int M, int N, int K, int form, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (K <= 0 || form < 0 || form > 5) return TS_ERR_BAD_ARGUMENT;
+  if (K % 4 != 0 || (((uintptr_t)x | (uintptr_t)w) & 15) != 0) return TS_ERR_UNSUPPORTED;
+  if (form == 0) {
+    const long long tiles = (long long)((M + FT_M - 1) / FT_M) * ((N + FT_N - 1) / FT_N);
+    // (tiles: 150 rows of 1,024 x 2,048, 80 tiles: 64 / 47 / 35 us over 1 / 2 / 4 CTAs; 600 of 4,096 x 1,024, 1,216 tiles:
+    // 164 / 158 / 165 us; 17 rows of the head, 2,374 tiles: 301 / 295 / 309 us)
+    if (M <= 16) form = M > 2 && N >= 2048 ? 2 : 1;
+    else form = tiles <= 400 ? 5 : tiles <= 1300 ? 4 : 3;
+  }
+  if (form <= 2) {
+    if ((M + 7) / 8 > 65535) return TS_ERR_BAD_ARGUMENT;
+    if (form == 1) {
+      if (M == 1) return launch_rows<1, 1>(x, w, out, M, N, K, stream);
+      if (M == 2) return launch_rows<2, 1>(x, w, out, M, N, K, stream);
+      if (M <= 4) return launch_rows<4, 1>(x, w, out, M, N, K, stream);
+      return launch_rows<8, 1>(x, w, out, M, N, K, stream);
+    }
+    return M <= 4 ? launch_rows<4, 2>(x, w, out, M, N, K, stream) : launch_rows<8, 2>(x, w, out, M, N, K, stream);
+  }
+  if (form == 3) return launch_tile<1>(x, w, out, M, N, K, stream);
+  return form == 4 ? launch_tile<2>(x, w, out, M, N, K, stream) : launch_tile<4>(x, w, out, M, N, K, stream);
+}

@@ -88,6 +88,7 @@ _SIGNATURES: dict[str, list[Any]] = {
     "ts_gemm_skinny_to_stream_parts": [_i, _i, _i],
     "ts_prefetch_l2": [_vp, _vp, _i, _i, _vp],
     "ts_prefetch_pages": [_vp, _vp, _c.c_ulonglong, _vp, _i, _vp, _i, _i, _i, _vp],
+    "ts_gemm_f32": [_vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "ts_gemm_simt": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _vp],
     "ts_gemm_skinny": [_vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "ts_gemm_skinny_swiglu": [_vp, _vp, _vp, _i, _i, _i, _vp],
@@ -713,8 +714,11 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     if m == 0:
         return
     if x.dtype == torch.float32:
-        _check(_fn("ts_gemm_simt")(_dev(x, "x"), _dev(w, "w"), _dev(out, "out"), m, n, k, _F32, _F32, _stream()),
-               "gemm")
+        px, pw = _dev(x, "x"), _dev(w, "w")
+        if k % 4 == 0 and (px | pw) % 16 == 0:
+            _check(_fn("ts_gemm_f32")(px, pw, _dev(out, "out"), m, n, k, 0, _stream()), "gemm")
+        else:       # rows that do not start on a 16-byte boundary
+            _check(_fn("ts_gemm_simt")(px, pw, _dev(out, "out"), m, n, k, _F32, _F32, _stream()), "gemm")
         return
     if m <= SKINNY_MAX_ROWS and k % 32 == 0 and n % 16 == 0 and (n * k <= SKINNY_MAX_WEIGHTS or out.dtype != x.dtype):
         gemm_skinny(x, w, out)
