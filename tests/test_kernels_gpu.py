@@ -601,6 +601,33 @@ def test_sample_temperature_and_top_p_match_reference(vocab) -> None:
         assert out.tolist() == want.tolist()
 
 
+@pytest.mark.parametrize("vocab", [3, 31, 32768, 151936, 163841])
+def test_sample_nucleus_of_wide_rows(vocab) -> None:
+    """The eight chunks of a row (some empty at the smallest vocabularies; weights held in registers up to 163,840
+    tokens, read again beyond) find the same nucleus as a sort does: with the temperature low and the noise removed
+    by comparing eligibility, every drawn token's more likely tokens hold less than top_p, and the most likely token
+    is always eligible. A row of -inf but one token, and greedy rows beside it."""
+    r = 12
+    logits = rnd(r, vocab, seed=6, scale=3.0)
+    logits[5, :] = float("-inf")
+    logits[5, vocab // 2] = -7.0
+    temps = torch.tensor([0.7, 1.0, 1.6, 0.0] * 3, device="cuda")
+    top_p = torch.tensor([0.9, 0.5, 0.05, 0.9] * 2 + [1.0, 0.999, 0.3, 1.0], device="cuda")
+    seeds = torch.arange(r, device="cuda", dtype=torch.int64) + 77
+    z = logits.double() / torch.where(temps > 0, temps, torch.ones_like(temps)).double()[:, None]
+    p = torch.softmax(z, -1)
+    for draw in range(6):
+        out = torch.empty(r, device="cuda", dtype=torch.int32)
+        ops.sample(logits, out, temps, top_p, seeds, torch.full((r,), draw, device="cuda", dtype=torch.int64))
+        for b, tok in enumerate(out.tolist()):
+            assert 0 <= tok < vocab
+            if temps[b] == 0:
+                assert tok == int(logits[b].argmax())
+            else:           # 32-bit sums of up to 163,841 weights: 1e-5 of slack
+                assert float(p[b][p[b] > p[b][tok]].sum()) < float(top_p[b]) + 1e-5
+        assert out[5].item() == vocab // 2
+
+
 def test_sample_frequencies_follow_softmax() -> None:
     vocab, n = 8, 4096
     row = torch.tensor([2.0, 1.0, 0.0, -1.0, 0.5, -3.0, 1.5, 0.2], device="cuda")
