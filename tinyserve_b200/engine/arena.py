@@ -5,6 +5,10 @@ tables, logits); two ``frames`` alternate from layer to layer, so that the outpu
 leaves pending on the residual stream is still intact while the next layer, working in the
 other frame, reads it. Nothing is allocated from the device allocator in steady state; a
 region grows (once, outside any graph capture) when a step needs more than it has.
+
+The layers of a step ask for the same shapes at the same offsets, so a region keeps the views it
+has made of its buffer (slicing and viewing took a quarter of the host's time for a step that is
+launched kernel by kernel: 1.2 of 4.4 ms for 28 dense layers).
 """
 
 from __future__ import annotations
@@ -12,6 +16,7 @@ from __future__ import annotations
 import torch
 
 _ALIGN = 256
+_MOST_VIEWS = 1024      # kept per region; prompts of ever new lengths ask for ever new shapes
 _ELEMENT_SIZE: dict[torch.dtype, int] = {}
 
 
@@ -27,6 +32,8 @@ class _Region:
         self.device = device
         self.buf = torch.empty(0, dtype=torch.uint8, device=device)
         self._typed: dict[torch.dtype, torch.Tensor] = {}     # ``buf`` seen as each dtype asked for so far
+        # (offset, shape, dtype) -> (the view of ``buf`` handed out for it, its bytes)
+        self._views: dict[tuple[int, tuple[int, ...], torch.dtype], tuple[torch.Tensor, int]] = {}
         self.used = 0          # offset in ``buf`` of the next take
         self.demand = 0        # bytes taken since the last reset, wherever they came from
         self.high_water = 0    # the largest demand of any step so far
@@ -37,10 +44,21 @@ class _Region:
             # holds a whole step, so that from now on nothing moves.
             self.buf = torch.empty(self.high_water // _ALIGN * _ALIGN + _ALIGN, dtype=torch.uint8, device=self.device)
             self._typed = {}
+            self._views = {}
+        elif len(self._views) > _MOST_VIEWS:
+            self._views = {}
         self.used = 0
         self.demand = 0
 
     def take(self, shape: tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
+        start = (self.used + _ALIGN - 1) // _ALIGN * _ALIGN
+        made = self._views.get((start, shape, dtype))
+        if made is not None:
+            self.demand = (self.demand + _ALIGN - 1) // _ALIGN * _ALIGN + made[1]
+            if self.demand > self.high_water:
+                self.high_water = self.demand
+            self.used = start + made[1]
+            return made[0]
         numel = 1
         for s in shape:
             numel *= int(s)
@@ -48,13 +66,13 @@ class _Region:
         nbytes = numel * size
         self.demand = (self.demand + _ALIGN - 1) // _ALIGN * _ALIGN + nbytes
         self.high_water = max(self.high_water, self.demand)
-        start = (self.used + _ALIGN - 1) // _ALIGN * _ALIGN
         end = start + nbytes
         if end > self.buf.numel():
             # Grow: views handed out earlier keep the old buffer alive until they die.
             grow = max(nbytes, 2 * self.buf.numel(), 1 << 16)
             self.buf = torch.empty((grow + _ALIGN - 1) // _ALIGN * _ALIGN, dtype=torch.uint8, device=self.device)
             self._typed = {}
+            self._views = {}
             start, end = 0, nbytes
         self.used = end
         if numel == 0:
@@ -62,7 +80,9 @@ class _Region:
         typed = self._typed.get(dtype)
         if typed is None:
             typed = self._typed[dtype] = self.buf.view(dtype)     # buffer sizes are multiples of 256 bytes
-        return typed[start // size: end // size].view(shape)
+        view = typed[start // size: end // size].view(shape)
+        self._views[(start, shape, dtype)] = (view, nbytes)
+        return view
 
 
 class Arena:
