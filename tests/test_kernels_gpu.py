@@ -541,6 +541,26 @@ def test_gemm_skinny_streaming_form_with_wide_rows(m) -> None:
     torch.testing.assert_close(out, want, atol=2e-4, rtol=1e-4)
 
 
+@pytest.mark.parametrize("slices", [1, 3, 8])
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("m", [1, 15, 16, 17, 33, 64])
+@pytest.mark.parametrize("n,k", [(128, 512), (127, 520), (200, 1000), (4098, 4096)])
+def test_gemm_rows_tcgen05(m, n, k, swiglu, slices) -> None:
+    """Weight tiles as the A operand: partly filled tiles of weight rows and of x rows, a K that ends inside a block, and
+    slices of K that the CTAs of a cluster add up."""
+    x = rnd(m, k, dtype=torch.bfloat16, seed=1)
+    w = rnd(2 * n if swiglu else n, k, dtype=torch.bfloat16, seed=2, scale=0.05)
+    out = torch.full((m, n), float("nan"), device="cuda", dtype=torch.bfloat16)
+    want = torch.empty_like(out)
+    ops.gemm_rows_tcgen05(x, w, out, swiglu=swiglu, slices=slices)
+    ops.check_device_errors()
+    (ref.gemm_swiglu if swiglu else ref.gemm)(x, w, want)
+    # 32-bit sums in another order, then the roundings of the output: one unit (2^-8 relative); with SwiGLU three
+    # roundings on either side, where those of gate and up grow by at most the slope of silu (1.1)
+    rtol = 2 ** -7 if not swiglu else 2 ** -5
+    torch.testing.assert_close(out.float(), want.float(), atol=rtol * want.float().abs().mean().item(), rtol=rtol)
+
+
 def test_gemm_skinny_refuses_what_it_cannot_take() -> None:
     x, w = rnd(4, 80, dtype=torch.bfloat16), rnd(32, 80, dtype=torch.bfloat16)
     with pytest.raises(ops.KernelError, match="not supported"):

@@ -91,6 +91,7 @@ _SIGNATURES: dict[str, list[Any]] = {
     "ts_gemm_f32": [_vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "ts_gemm_simt": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _vp],
     "ts_gemm_skinny": [_vp, _vp, _vp, _i, _i, _i, _i, _vp],
+    "ts_gemm_rows_tcgen05": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp],
     "ts_gemm_skinny_swiglu": [_vp, _vp, _vp, _i, _i, _i, _vp],
     "ts_gemm_tcgen05": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp],
     "ts_gemm_tcgen05_swiglu": [_vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp],
@@ -720,6 +721,9 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
         else:       # rows that do not start on a 16-byte boundary
             _check(_fn("ts_gemm_simt")(px, pw, _dev(out, "out"), m, n, k, _F32, _F32, _stream()), "gemm")
         return
+    if takes_rows_tcgen05(m, n * k, k) and out.dtype == x.dtype:
+        gemm_rows_tcgen05(x, w, out)
+        return
     if m <= SKINNY_MAX_ROWS and k % 32 == 0 and n % 16 == 0 and (n * k <= SKINNY_MAX_WEIGHTS or out.dtype != x.dtype):
         gemm_skinny(x, w, out)
         return
@@ -737,10 +741,40 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
 
 # Up to this many rows a bf16 product streams the weights through the skinny kernel ...
 SKINNY_MAX_ROWS = 16
-# ... if the matrix is not larger than this (measured on B200: at the Qwen3-8B and 32B layer
-# shapes the vendor library streams 15-35% faster; at the 0.6B shapes and for the output head
-# the skinny kernel is level or ahead).
+# ... if the matrix is smaller than this (or the output head's): larger ones go to the tcgen05 kernel that streams the
+# weights by TMA. Measured on B200 in a chain of products, one row, skinny / vendor library / that kernel: 4,096 x 4,096
+# 12.5 / 12.5 / 8.8 us, 4,096 x 12,288 36 / 30 / 19 us, 5,120 x 25,600 138 / 47 / 43 us, 2 x 12,288 x 4,096 with SwiGLU
+# 46 / 37.5 / 36.3 us; 16 rows 13.3 / 9.6 / 9.4, 38 / 22 / 20, 145 / 46 / 44, 54 / 38.0 / 37.4 us. At the 0.6B shapes
+# (4,096 x 1,024) the skinny kernel is ahead, 3.3 / 5.4 / 4.5 us.
 SKINNY_MAX_WEIGHTS = 1 << 24
+# Up to this many rows: at 64 rows the library is level or ahead (4,096 x 12,288 22 / 23 us, 4,096 x 4,096 10 / 12 us).
+ROWS_TCGEN05_MAX_ROWS = 16
+
+
+def takes_rows_tcgen05(m: int, weights: int, k: int) -> bool:
+    """Whether a bf16 product of ``m`` rows with a matrix of so many ``weights`` goes to :func:`gemm_rows_tcgen05`."""
+    return m <= ROWS_TCGEN05_MAX_ROWS and weights >= SKINNY_MAX_WEIGHTS and k % 8 == 0
+
+
+def rows_tcgen05_slices(tiles: int, k: int) -> int:
+    """Slices of K (the CTAs of a cluster) for ``tiles`` tiles of 128 weight rows: as many as let all CTAs run at once, two
+    an SM with room for clusters to be placed (measured on B200: 4,096 x 4,096, 32 tiles, 9.9 us with 4 slices, 8.8 with 8;
+    6,144 x 4,096, 48 tiles, 12.3 us with 4, 11.5 with 5 = 240 CTAs, 17.7 with 6 = 288 CTAs)."""
+    return max(1, min(8, 256 // tiles, -(-k // 64)))
+
+
+def gemm_rows_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, swiglu: bool = False, slices: int = 0) -> None:
+    """bf16 ``out[M, N] = x[M, K] @ w[N, K]^T`` (``swiglu``: ``silu(x Wgate^T) * (x Wup^T)``, ``w`` = ``2 N`` rows) for
+    ``M <= 64`` and ``K % 8 == 0``: weight tiles as the A operand of tcgen05.mma (``csrc/gemm_rows_tcgen05.cu``).
+    ``slices``: CTAs that share K (0: chosen by the size)."""
+    m, k = x.shape
+    n = out.shape[1]
+    if (tuple(w.shape) != ((2 * n if swiglu else n), k) or out.shape[0] != m or x.dtype != torch.bfloat16
+            or w.dtype != torch.bfloat16 or out.dtype != torch.bfloat16):
+        raise KernelError("gemm_rows_tcgen05: shape or dtype mismatch")
+    slices = slices or rows_tcgen05_slices(-(-n // (64 if swiglu else 128)), k)
+    _check(_fn("ts_gemm_rows_tcgen05")(_dev(x, "x"), _dev(w, "w"), _dev(out, "out"), m, n, k, int(bool(swiglu)), slices,
+                                       _error_word(x.device).data_ptr(), _stream()), "gemm_rows_tcgen05")
 
 
 def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
@@ -878,6 +912,9 @@ def gemm_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, are
             and 2 * inter * k <= SKINNY_MAX_WEIGHTS):
         _check(_fn("ts_gemm_skinny_swiglu")(_dev(x, "x"), _dev(w_gate_up, "w_gate_up"), _dev(out, "out"), m, inter, k,
                                             _stream()), "gemm_swiglu")
+        return
+    if x.dtype == torch.bfloat16 and takes_rows_tcgen05(m, 2 * inter * k, k):
+        gemm_rows_tcgen05(x, w_gate_up, out, swiglu=True)
         return
     tiles = tcgen05_tiles(m, inter, 128)
     if x.dtype == torch.bfloat16 and m >= TCGEN05_MIN_ROWS and 2 * inter >= TCGEN05_MIN_COLS and k % 8 == 0 and tiles:
