@@ -7,7 +7,7 @@
 // softmax in 32-bit (online, base 2), o = sum p v in 32-bit, cast once to the output type.
 // Query head h reads kv head h / (num_heads / num_kv_heads).
 //
-//  * prefill kernel: one CTA per (tile of 32 queries of one request, query head); keys and
+//  * prefill kernel: one CTA per (tile of 16 or 32 queries of one request, query head); keys and
 //    values are staged through shared memory in tiles of 32 (after upstream
 //    src/tinyserve/triton_prefill.py:50-125, which tiles the same way over the paged cache).
 //  * decode kernel: one CTA per (request, kv head, split of the keys); a group of lanes reads
@@ -24,23 +24,45 @@ namespace ts {
 constexpr float NEG_INF = -INFINITY;
 
 // =============================================================== prefill (tiled)
-constexpr int PF_TQ = 32;       // queries per CTA
+// What bounds it at the sizes it serves (the 32-bit path's prompts, odd head sizes): the serial chain of a CTA's key tiles.
+// So the operands lie in shared memory in rows of whole 16-byte words and are read four elements at a time (scalar reads
+// cost six shared-memory instructions for eight multiply-adds), float tiles come by cp.async into the second buffer
+// while the first one is worked on, and a step with few CTAs is cut into tiles of 16 queries instead of 32. Whatever the
+// cut, a row's scores are one chain over the head's elements, its sums go over the keys in order and are rescaled every
+// 32 keys, so its result does not depend on the batch. B200, float, 16 / 8 heads of 128: see launch_prefill_dj.
 constexpr int PF_TK = 32;       // keys per tile
 constexpr int PF_THREADS = 128;
 
-template <typename T, int DJMAX>
-__global__ void __launch_bounds__(PF_THREADS) prefill_attn_kernel(AttnArgs a) {
-  extern __shared__ float smem[];
+__device__ __forceinline__ void pf_copy16(float* dst, const void* src, bool ok) {
+  const unsigned int d = (unsigned int)__cvta_generic_to_shared(dst);
+  const int n = ok ? 16 : 0;     // zeros where the key is not visible
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+
+// Shared memory in floats: queries [TQ][DS], `buffers` x (keys [TK][DS], values [TK][VS]), scores [TQ][TK + 4], 3 row arrays.
+// DS, VS: the head sizes up to a multiple of 4, plus one 16-byte word (rows that eight neighbouring threads read start in
+// eight different groups of banks).
+__host__ __device__ __forceinline__ int pf_stride(int d) { return (d + 3) / 4 * 4 + 4; }
+constexpr int PF_SS = PF_TK + 4;
+static inline size_t pf_smem(int tq, int D, int DV, int buffers) {
+  return sizeof(float) * ((size_t)tq * pf_stride(D) + (size_t)buffers * PF_TK * (pf_stride(D) + pf_stride(DV)) + (size_t)tq * PF_SS + 3 * tq);
+}
+
+// TQ = queries per CTA (16 or 32); QJ = groups of 64 value columns (a thread owns four neighbouring ones of each).
+template <typename T, int TQ, int QJ>
+__global__ void __launch_bounds__(PF_THREADS) prefill_attn_kernel(AttnArgs a, int buffers) {
+  constexpr int RT = TQ / 8;                    // rows a thread owns
+  extern __shared__ __align__(16) float smem[];
   const int D = a.head_dim;
   const int DV = a.v_head_dim ? a.v_head_dim : D;   // values may have a head size of their own
-  const int DS = D + 1;                         // padded row stride
+  const int DS = pf_stride(D), VS = pf_stride(DV);
   float* Qs = smem;                             // [TQ][DS]  pre-scaled queries
-  float* Ks = Qs + PF_TQ * DS;                  // [TK][DS]
-  float* Vs = Ks + PF_TK * DS;                  // [TK][DV]
-  float* Ss = Vs + PF_TK * DV;                  // [TQ][TK + 1]
-  float* row_m = Ss + PF_TQ * (PF_TK + 1);      // [TQ]
-  float* row_l = row_m + PF_TQ;                 // [TQ]
-  float* row_c = row_l + PF_TQ;                 // [TQ] correction factor of this tile
+  float* tiles = Qs + TQ * DS;
+  const int tile_floats = PF_TK * (DS + VS);
+  float* Ss = tiles + buffers * tile_floats;    // [TQ][PF_SS]
+  float* row_m = Ss + TQ * PF_SS;               // [TQ]
+  float* row_l = row_m + TQ;                    // [TQ]
+  float* row_c = row_l + TQ;                    // [TQ] correction factor of this tile
 
   pdl_trigger();
   pdl_wait();
@@ -49,32 +71,16 @@ __global__ void __launch_bounds__(PF_THREADS) prefill_attn_kernel(AttnArgs a) {
   const int kvh = head / (a.num_heads / a.num_kv_heads);
   const int row0 = a.cu_q[seq];
   const int n = a.cu_q[seq + 1] - row0;
-  const int q0 = blockIdx.x * PF_TQ;
+  const int q0 = blockIdx.x * TQ;
   if (q0 >= n) return;
   const int ctx = a.ctx_lens[seq];
   const int first_pos = ctx - n;                // position of the request's first new token
-  const int nq = min(PF_TQ, n - q0);
+  const int nq = min(TQ, n - q0);
   const int* table = a.block_tables + (size_t)seq * a.table_width;
   const T* q = (const T*)a.q;
   const T* kc = (const T*)a.k_cache;
   const T* vc = (const T*)a.v_cache;
   const int tid = threadIdx.x;
-
-  for (int idx = tid; idx < PF_TQ * D; idx += PF_THREADS) {
-    const int r = idx / D, d = idx - r * D;
-    float v = 0.f;
-    if (r < nq && q_col_lives(head, d, D, a)) v = to_float(q[q_row_of(row0 + q0 + r, head, a) * D + d]) * a.scale_log2;
-    Qs[r * DS + d] = v;
-  }
-  if (tid < PF_TQ) { row_m[tid] = NEG_INF; row_l[tid] = 0.f; }
-
-  const int ty = tid >> 4, tx = tid & 15;       // 8 row groups x 16 column groups
-  float acc[4][DJMAX];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < DJMAX; ++j) acc[i][j] = 0.f;
-  const int dj = (DV + 15) >> 4;
 
   const int qpos_first = first_pos + q0;
   const int qpos_last = first_pos + q0 + nq - 1;
@@ -84,78 +90,112 @@ __global__ void __launch_bounds__(PF_THREADS) prefill_attn_kernel(AttnArgs a) {
   const int kept = (a.window > 0) ? min(a.keep_first, k_lo) : 0;
   const int kept_end = min(k_begin, ((kept + PF_TK - 1) / PF_TK) * PF_TK);
   constexpr int VEC = Vec<T>::N;
-  const int chunks = D / VEC, vchunks = DV / VEC;
   const bool vec_ok = (D % VEC == 0) && (DV % VEC == 0);
 
-  for (int k0 = kept_end > 0 ? 0 : k_begin; k0 <= qpos_last; k0 = (k0 + PF_TK == kept_end) ? k_begin : k0 + PF_TK) {
-    __syncthreads();   // previous tile fully consumed (and Qs/row state initialised)
-    // ---- stage keys and values k0 .. k0+TK-1 (zeros outside the request's visible range)
-    if (vec_ok) {
-      for (int idx = tid; idx < PF_TK * (chunks + vchunks); idx += PF_THREADS) {
-        const int kk = idx / (chunks + vchunks), c = idx - kk * (chunks + vchunks);
-        const bool is_key = c < chunks;
-        const int cc = is_key ? c : c - chunks;
-        const int kpos = k0 + kk;
-        float f[VEC];
-        if ((kpos >= k_lo || kpos < kept) && kpos <= qpos_last) {
-          const size_t row = kv_row_of(table, kpos, kvh, a);
-          Vec<T> raw;
-          raw.load(is_key ? kc + row * D + (size_t)cc * VEC : vc + row * DV + (size_t)cc * VEC);
-          raw.unpack(f);
-        } else {
+  // Keys and values k0 .. k0 + TK - 1 into a buffer (zeros outside the request's visible range and in the padding columns).
+  // Four threads a key: one look-up in the block table each, then nothing but copies.
+  const int skey = tid >> 2, spart = tid & 3;
+  auto stage = [&](int k0, float* Ks) {
+    const int kpos = k0 + skey;
+    const bool ok = (kpos >= k_lo || kpos < kept) && kpos <= qpos_last;
+    const size_t row = ok ? kv_row_of(table, kpos, kvh, a) : 0;
+    auto copy = [&](const T* src, float* dst, int n) {      // n elements of a row; the thread's share of it
+      if (vec_ok) {
+#pragma unroll 4
+        for (int c = spart * VEC; c < n; c += 4 * VEC) {
+          if constexpr (VEC == 4) {
+            pf_copy16(dst + c, src + c, ok);
+          } else {
+            float f[VEC];
+            Vec<T> raw;
+            if (ok) raw.load(src + c); else raw.zero();
+            raw.unpack(f);
 #pragma unroll
-          for (int e = 0; e < VEC; ++e) f[e] = 0.f;
+            for (int e = 0; e < VEC; e += 4) *reinterpret_cast<float4*>(dst + c + e) = make_float4(f[e], f[e + 1], f[e + 2], f[e + 3]);
+          }
         }
-        float* dst = is_key ? Ks + kk * DS + cc * VEC : Vs + kk * DV + cc * VEC;
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) dst[e] = f[e];
+      } else {
+        // head sizes that are no multiple of a 16-byte vector: element by element, the padding included
+        for (int c = spart; c < pf_stride(n) - 4; c += 4) dst[c] = ok && c < n ? to_float(src[c]) : 0.f;
       }
+    };
+    copy(kc + row * D, Ks + skey * DS, D);
+    copy(vc + row * DV, Ks + PF_TK * DS + skey * VS, DV);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto next_tile = [&](int k0) { return (k0 + PF_TK == kept_end) ? k_begin : k0 + PF_TK; };
+
+  int k0 = kept_end > 0 ? 0 : k_begin, turn = 0;
+  stage(k0, tiles);
+  {
+    constexpr int TPR = PF_THREADS / TQ;        // threads per query row
+    const int r = tid / TPR;
+    const T* src = q + q_row_of(row0 + q0 + (r < nq ? r : 0), head, a) * D;
+#pragma unroll 4
+    for (int c = tid % TPR * 4; c < DS - 4; c += 4 * TPR) {
+      float f[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int d = c + e;
+        f[e] = r < nq && d < D && q_col_lives(head, d, D, a) ? to_float(src[d]) * a.scale_log2 : 0.f;
+      }
+      *reinterpret_cast<float4*>(Qs + r * DS + c) = make_float4(f[0], f[1], f[2], f[3]);
+    }
+  }
+  if (tid < TQ) { row_m[tid] = NEG_INF; row_l[tid] = 0.f; }
+
+  const int ty = tid >> 4, tx = tid & 15;       // 8 row groups x 16 column groups
+  float4 acc[RT][QJ];
+#pragma unroll
+  for (int i = 0; i < RT; ++i)
+#pragma unroll
+    for (int j = 0; j < QJ; ++j) acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+
+  while (true) {
+    const int k_next = next_tile(k0);
+    const bool more = k_next <= qpos_last;
+    const float* Ks = tiles + turn * tile_floats;
+    const float* Vs = Ks + PF_TK * DS;
+    // with two buffers the next tile is asked for now: its buffer was read before the barrier at the end of the last tile
+    if (buffers == 2 && more) {
+      stage(k_next, tiles + (turn ^ 1) * tile_floats);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
     } else {
-      // head sizes that are no multiple of a 16-byte vector: element by element
-      for (int idx = tid; idx < PF_TK * (D + DV); idx += PF_THREADS) {
-        const int kk = idx / (D + DV), c = idx - kk * (D + DV);
-        const bool is_key = c < D;
-        const int cc = is_key ? c : c - D;
-        const int kpos = k0 + kk;
-        float f = 0.f;
-        if ((kpos >= k_lo || kpos < kept) && kpos <= qpos_last) {
-          const size_t row = kv_row_of(table, kpos, kvh, a);
-          f = is_key ? to_float(kc[row * D + cc]) : to_float(vc[row * DV + cc]);
-        }
-        if (is_key) Ks[kk * DS + cc] = f; else Vs[kk * DV + cc] = f;
-      }
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     __syncthreads();
-    // ---- scores: thread (ty, tx) owns rows ty*4..+3, keys tx*2..+1
-    float s[4][2];
+    // ---- scores: thread (ty, tx) owns RT rows from ty * RT, keys tx and tx + 16
+    float s[RT][2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { s[i][0] = 0.f; s[i][1] = 0.f; }
-    for (int d = 0; d < D; ++d) {
-      const float kv0 = Ks[(tx * 2) * DS + d], kv1 = Ks[(tx * 2 + 1) * DS + d];
+    for (int i = 0; i < RT; ++i) { s[i][0] = 0.f; s[i][1] = 0.f; }
+#pragma unroll 4
+    for (int d = 0; d < DS - 4; d += 4) {
+      const float4 u = *reinterpret_cast<const float4*>(Ks + tx * DS + d);
+      const float4 v = *reinterpret_cast<const float4*>(Ks + (tx + 16) * DS + d);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float qv = Qs[(ty * 4 + i) * DS + d];
-        s[i][0] = fmaf(qv, kv0, s[i][0]);
-        s[i][1] = fmaf(qv, kv1, s[i][1]);
+      for (int i = 0; i < RT; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(Qs + (ty * RT + i) * DS + d);
+        s[i][0] = fmaf(x.w, u.w, fmaf(x.z, u.z, fmaf(x.y, u.y, fmaf(x.x, u.x, s[i][0]))));
+        s[i][1] = fmaf(x.w, v.w, fmaf(x.z, v.z, fmaf(x.y, v.y, fmaf(x.x, v.x, s[i][1]))));
       }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = ty * 4 + i;
+    for (int i = 0; i < RT; ++i) {
+      const int r = ty * RT + i;
       const int qpos = first_pos + q0 + r;
       const int first = first_visible(qpos, a);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const int kpos = k0 + tx * 2 + j;
+        const int kpos = k0 + tx + 16 * j;
         const bool ok = (r < nq) && (kpos <= qpos) && (kpos >= first || kpos < a.keep_first);
-        Ss[r * (PF_TK + 1) + tx * 2 + j] = ok ? s[i][j] : NEG_INF;
+        Ss[r * PF_SS + tx + 16 * j] = ok ? s[i][j] : NEG_INF;
       }
     }
     __syncthreads();
     // ---- online softmax per row: 4 threads per row
-    {
+    if (tid < 4 * TQ) {
       const int r = tid >> 2, part = tid & 3;
-      float* srow = Ss + r * (PF_TK + 1);
+      float* srow = Ss + r * PF_SS;
       float mx = NEG_INF;
 #pragma unroll
       for (int j = 0; j < PF_TK / 4; ++j) mx = fmaxf(mx, srow[part * (PF_TK / 4) + j]);
@@ -183,44 +223,64 @@ __global__ void __launch_bounds__(PF_THREADS) prefill_attn_kernel(AttnArgs a) {
       }
     }
     __syncthreads();
-    // ---- acc = acc * corr + P V: thread owns rows ty*4..+3, columns tx + 16 j
+    // ---- acc = acc * corr + P V: thread owns RT rows, columns 4 tx .. + 3 of every 64
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float corr = row_c[ty * 4 + i];
+    for (int i = 0; i < RT; ++i) {
+      const float corr = row_c[ty * RT + i];
 #pragma unroll
-      for (int j = 0; j < DJMAX; ++j) acc[i][j] *= corr;
+      for (int j = 0; j < QJ; ++j) { acc[i][j].x *= corr; acc[i][j].y *= corr; acc[i][j].z *= corr; acc[i][j].w *= corr; }
     }
-    for (int kk = 0; kk < PF_TK; ++kk) {
-      float p[4];
+#pragma unroll 2
+    for (int kk = 0; kk < PF_TK; kk += 4) {
+      float p[RT][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) p[i] = Ss[(ty * 4 + i) * (PF_TK + 1) + kk];
-#pragma unroll
-      for (int j = 0; j < DJMAX; ++j) {
-        if (j < dj && tx + 16 * j < DV) {
-          const float vv = Vs[kk * DV + tx + 16 * j];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) acc[i][j] = fmaf(p[i], vv, acc[i][j]);
-        }
+      for (int i = 0; i < RT; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(Ss + (ty * RT + i) * PF_SS + kk);
+        p[i][0] = v.x; p[i][1] = v.y; p[i][2] = v.z; p[i][3] = v.w;
       }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int j = 0; j < QJ; ++j) {
+          if (4 * tx + 64 * j < DV) {
+            const float4 vv = *reinterpret_cast<const float4*>(Vs + (kk + e) * VS + 4 * tx + 64 * j);
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+              acc[i][j].x = fmaf(p[i][e], vv.x, acc[i][j].x);
+              acc[i][j].y = fmaf(p[i][e], vv.y, acc[i][j].y);
+              acc[i][j].z = fmaf(p[i][e], vv.z, acc[i][j].z);
+              acc[i][j].w = fmaf(p[i][e], vv.w, acc[i][j].w);
+            }
+          }
+        }
     }
+    if (!more) break;
+    __syncthreads();       // this tile's keys, values and scores have been read by everyone
+    if (buffers == 1) stage(k_next, tiles);
+    else turn ^= 1;
+    k0 = k_next;
   }
-  __syncthreads();
   T* out = (T*)a.out;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = ty * 4 + i;
+  for (int i = 0; i < RT; ++i) {
+    const int r = ty * RT + i;
     if (r < nq) {
 #pragma unroll
-      for (int j = 0; j < DJMAX; ++j)
-        if (j < dj && tx + 16 * j < DV)
-          out[((size_t)(row0 + q0 + r) * a.num_heads + head) * DV + tx + 16 * j] =
-              from_float<T>(finish_row(acc[i][j], row_l[r], row_m[r], a.sinks, head));
+      for (int j = 0; j < QJ; ++j) {
+        const float v[4] = {acc[i][j].x, acc[i][j].y, acc[i][j].z, acc[i][j].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int c = 4 * tx + 64 * j + e;
+          if (c < DV)
+            out[((size_t)(row0 + q0 + r) * a.num_heads + head) * DV + c] = from_float<T>(finish_row(v[e], row_l[r], row_m[r], a.sinks, head));
+        }
+      }
     }
   }
 }
 
 // ================================================================ decode (split-K)
-constexpr int DC_WARPS = 4;
+constexpr int DC_WARPS = 8;
 constexpr int DC_THREADS = DC_WARPS * 32;
 constexpr int DC_MAX_COUNTERS = 1 << 16;
 
@@ -230,9 +290,12 @@ constexpr int DC_MAX_COUNTERS = 1 << 16;
 static __device__ unsigned int g_decode_counters[DC_MAX_COUNTERS];
 
 // GT = query heads handled per CTA (a kv group is covered by ceil(G / GT) CTAs);
-// CPL = 16-byte chunks of a key per lane; U = keys per lane group whose loads are in flight.
-template <typename T, int GT, int CPL, int U>
-__global__ void __launch_bounds__(DC_THREADS) decode_attn_kernel(AttnArgs a, int lanes_per_key, int passes) {
+// LPK = lanes that share a key; CPL = 16-byte chunks of a key per lane; U = keys per lane group whose loads are in flight.
+// Bound by its chain of latencies: block table, keys, the sums over the lanes of a key, the exponentials. Few lanes a key
+// make few exchanges (three steps for four keys at once with LPK = 8, five for one with 32), and the number of lanes is
+// known to the compiler so that the exchanges of all keys and heads overlap.
+template <typename T, int GT, int CPL, int LPK, int U>
+__global__ void __launch_bounds__(DC_THREADS) decode_attn_kernel(AttnArgs a, int passes) {
   constexpr int VEC = Vec<T>::N;
   constexpr int EPL = VEC * CPL;                 // elements of a key per lane
   extern __shared__ float smem[];                // [DC_WARPS][GT][D + 2]
@@ -246,9 +309,8 @@ __global__ void __launch_bounds__(DC_THREADS) decode_attn_kernel(AttnArgs a, int
   const int ng = min(GT, G - g0);
   const int split = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int LPK = lanes_per_key;
   const int sub = lane / LPK, lk = lane - sub * LPK;  // which key of the warp's batch, which lane of it
-  const int KPW = 32 / LPK;                           // keys per warp per batch
+  constexpr int KPW = 32 / LPK;                       // keys per warp per batch
   const int chunks = D / VEC;
   pdl_wait();
 
@@ -339,6 +401,7 @@ __global__ void __launch_bounds__(DC_THREADS) decode_attn_kernel(AttnArgs a, int
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         float d = s[g][u];
+#pragma unroll
         for (int o = LPK >> 1; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
         s[g][u] = valid[u] ? d : NEG_INF;
       }
@@ -375,6 +438,7 @@ __global__ void __launch_bounds__(DC_THREADS) decode_attn_kernel(AttnArgs a, int
   }
 
   // ---- merge the lane groups of a warp (lanes with equal lk hold the same elements)
+#pragma unroll
   for (int o = LPK; o < 32; o <<= 1) {
 #pragma unroll
     for (int g = 0; g < GT; ++g) {
@@ -439,61 +503,83 @@ __global__ void __launch_bounds__(DC_THREADS) decode_attn_kernel(AttnArgs a, int
   merge_splits<T>(a, si, qrow, kvh * G + g0, ng, smem);
 }
 
-template <typename T, int DJMAX>
-static int launch_prefill_dj(const AttnArgs& a, int max_query_len, cudaStream_t stream) {
+template <typename T, int TQ, int QJ>
+static int launch_prefill_tq(const AttnArgs& a, int max_query_len, cudaStream_t stream) {
   const int D = a.head_dim, DV = a.v_head_dim ? a.v_head_dim : D;
-  const size_t smem = sizeof(float) * ((size_t)PF_TQ * (D + 1) + (size_t)PF_TK * (D + 1) + (size_t)PF_TK * DV +
-                                       (size_t)PF_TQ * (PF_TK + 1) + 3 * PF_TQ);
-  auto kern = prefill_attn_kernel<T, DJMAX>;
+  int buffers = sizeof(T) == 4 ? 2 : 1;       // only float tiles come asynchronously
+  if (pf_smem(TQ, D, DV, buffers) > 200 * 1024) buffers = 1;
+  const size_t smem = pf_smem(TQ, D, DV, buffers);
+  auto kern = prefill_attn_kernel<T, TQ, QJ>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  dim3 grid((max_query_len + PF_TQ - 1) / PF_TQ, a.num_seqs, a.num_heads);
-  return launch(kern, grid, PF_THREADS, smem, stream, a);
+  dim3 grid((max_query_len + TQ - 1) / TQ, a.num_seqs, a.num_heads);
+  return launch(kern, grid, PF_THREADS, smem, stream, a, buffers);
+}
+
+template <typename T, int QJ>
+static int launch_prefill_qj(const AttnArgs& a, int max_query_len, cudaStream_t stream) {
+  // tiles of 16 queries while those of 32 leave SMs without a CTA (the work per query is then larger, but more of it at once)
+  const long long ctas = (long long)((max_query_len + 31) / 32) * a.num_seqs * a.num_heads;
+  return ctas < 148 ? launch_prefill_tq<T, 16, QJ>(a, max_query_len, stream) : launch_prefill_tq<T, 32, QJ>(a, max_query_len, stream);
 }
 
 template <typename T>
 static int launch_prefill(const AttnArgs& a, int max_query_len, cudaStream_t stream) {
-  const int dj = ((a.v_head_dim ? a.v_head_dim : a.head_dim) + 15) / 16;
-  if (dj <= 2) return launch_prefill_dj<T, 2>(a, max_query_len, stream);
-  if (dj <= 4) return launch_prefill_dj<T, 4>(a, max_query_len, stream);
-  if (dj <= 8) return launch_prefill_dj<T, 8>(a, max_query_len, stream);
-  return launch_prefill_dj<T, 16>(a, max_query_len, stream);
+  const int qj = ((a.v_head_dim ? a.v_head_dim : a.head_dim) + 63) / 64;
+  if (qj <= 1) return launch_prefill_qj<T, 1>(a, max_query_len, stream);
+  if (qj <= 2) return launch_prefill_qj<T, 2>(a, max_query_len, stream);
+  return launch_prefill_qj<T, 4>(a, max_query_len, stream);
 }
 
-template <typename T, int GT, int CPL>
-static int launch_decode_gc(const AttnArgs& a, int lpk, cudaStream_t stream) {
-  constexpr int U = (CPL == 1 && GT <= 4) ? 8 : 4;
+template <typename T, int GT, int CPL, int LPK>
+static int launch_decode_gc(const AttnArgs& a, cudaStream_t stream) {
+  constexpr int U = CPL >= 8 ? 1 : CPL >= 4 ? 2 : (CPL == 1 && GT <= 4) ? 8 : 4;
   const int G = a.num_heads / a.num_kv_heads;
   const int passes = (G + GT - 1) / GT;
   if ((long long)a.num_seqs * a.num_kv_heads * passes > DC_MAX_COUNTERS && a.num_splits > 1) return TS_ERR_UNSUPPORTED;
-  const size_t smem = sizeof(float) * (size_t)DC_WARPS * GT * (a.head_dim + 2);
-  auto kern = decode_attn_kernel<T, GT, CPL, U>;
+  // the warps' sums; the merge of the ranges keeps its (max, sum) pairs in the same memory
+  const size_t sums = (size_t)DC_WARPS * GT * (a.head_dim + 2), pairs = (size_t)GT * a.num_splits * 2;
+  const size_t smem = sizeof(float) * (sums > pairs ? sums : pairs);
+  auto kern = decode_attn_kernel<T, GT, CPL, LPK, U>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
   dim3 grid(a.num_seqs, a.num_kv_heads * passes, a.num_splits);
-  return launch(kern, grid, DC_THREADS, smem, stream, a, lpk, passes);
+  return launch(kern, grid, DC_THREADS, smem, stream, a, passes);
 }
 
 template <typename T>
 static int launch_decode(const AttnArgs& a, cudaStream_t stream) {
   constexpr int VEC = Vec<T>::N;
   const int chunks = a.head_dim / VEC;
-  int lpk = 1;
-  while (lpk < chunks && lpk < 32) lpk <<= 1;
-  const int cpl = (chunks + lpk - 1) / lpk;
   const int G = a.num_heads / a.num_kv_heads;
-  if (cpl > 2) return TS_ERR_UNSUPPORTED;
+  if (chunks > 64) return TS_ERR_UNSUPPORTED;
+  if (G <= 2) {
+    // up to eight lanes a key: the heads' queries and sums still fit the registers
 #define TS_DECODE_CASE(GT_)                                                   \
-  return cpl == 1 ? launch_decode_gc<T, GT_, 1>(a, lpk, stream) : launch_decode_gc<T, GT_, 2>(a, lpk, stream)
-  if (G == 1) { TS_DECODE_CASE(1); }
-  if (G == 2) { TS_DECODE_CASE(2); }
-  if (G <= 4) { TS_DECODE_CASE(4); }
+    if (chunks <= 4) return launch_decode_gc<T, GT_, 1, 4>(a, stream);        \
+    if (chunks <= 8) return launch_decode_gc<T, GT_, 1, 8>(a, stream);        \
+    if (chunks <= 16) return launch_decode_gc<T, GT_, 2, 8>(a, stream);       \
+    if (chunks <= 32) return launch_decode_gc<T, GT_, 4, 8>(a, stream);       \
+    if constexpr (VEC == 4) return launch_decode_gc<T, GT_, 8, 8>(a, stream)
+    if (G == 1) { TS_DECODE_CASE(1); return TS_ERR_UNSUPPORTED; }
+    TS_DECODE_CASE(2);
+    return TS_ERR_UNSUPPORTED;
+#undef TS_DECODE_CASE
+  }
+#define TS_DECODE_CASE(GT_)                                                   \
+  if (chunks <= 4) return launch_decode_gc<T, GT_, 1, 4>(a, stream);          \
+  if (chunks <= 8) return launch_decode_gc<T, GT_, 1, 8>(a, stream);          \
+  if (chunks <= 16) return launch_decode_gc<T, GT_, 1, 16>(a, stream);        \
+  if (chunks <= 32) return launch_decode_gc<T, GT_, 1, 32>(a, stream);        \
+  if constexpr (VEC == 4) return launch_decode_gc<T, GT_, 2, 32>(a, stream)
+  if (G <= 4) { TS_DECODE_CASE(4); return TS_ERR_UNSUPPORTED; }
   TS_DECODE_CASE(8);
 #undef TS_DECODE_CASE
+  return TS_ERR_UNSUPPORTED;
 }
 
 }  // namespace ts

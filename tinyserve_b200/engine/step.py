@@ -115,7 +115,7 @@ class DecodeGraph:
             context_lens_dev=dev[self.s_ctx], decode_seqs=dev[self.s_dec], prefill_seqs=dev[self.s_pre],
             num_decode=n, num_prefill=0, max_query_len=1, max_context_len=cap, kv=kv,
             state_slots=dev[self.s_state] if cache.has_state else None, state_slots_host=[0] * n,
-            arena=self.arena, dtype=runner.model.dtype)
+            arena=self.arena, dtype=runner.model.dtype, recorded=True)
 
     def record(self, runner: "ModelRunner") -> None:
         model, caches = runner.model, runner.cache.entries
@@ -230,7 +230,7 @@ class PrefillGraph:
             context_lens_dev=dev[self.s_ctx], decode_seqs=dev[self.s_dec], prefill_seqs=dev[self.s_pre],
             num_decode=0, num_prefill=1, max_query_len=t, max_context_len=cap, kv=kv,
             state_slots=dev[self.s_state] if cache.has_state else None, state_slots_host=[0],
-            arena=self.arena, dtype=runner.model.dtype)
+            arena=self.arena, dtype=runner.model.dtype, recorded=True)
 
     def record(self, runner: "ModelRunner") -> None:
         model, caches = runner.model, runner.cache.entries

@@ -87,7 +87,7 @@ class GQAAttention(Mixer):
         interleaved = False if rot is None else rot.interleaved
         attn = arena.take((t, self.q_size), ctx.dtype)
         join = None
-        if ops.PREFETCH_WEIGHTS and ctx.num_prefill == 0 and ctx.num_decode <= ops.PREFETCH_MAX_ROWS and x_device.type == "cuda":
+        if ops.PREFETCH_WEIGHTS and ctx.recorded and ctx.num_prefill == 0 and ctx.num_decode <= ops.PREFETCH_MAX_ROWS and x_device.type == "cuda":
             # decode: attention streams the cache and leaves bandwidth idle; the weights of the
             # products after it (output projection, feed-forward) come into L2 meanwhile
             ahead = [w for w in [self.w_o, *ctx.upcoming_weights] if w is not None][:8]
