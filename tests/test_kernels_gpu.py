@@ -408,7 +408,7 @@ def test_gemm_f32_forms_agree_bit_for_bit(m, n, k) -> None:
     wide = x.double() @ w.double().T
     bound = (k / 16 + 4 + 15 + 1) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
     assert bool(((out.double() - wide).abs() <= bound).all())
-    for form in range(1, 6):
+    for form in range(1, 5):
         other = torch.full((m, n), float("nan"), device="cuda")
         ops._check(ops._fn("ts_gemm_f32")(x.data_ptr(), w.data_ptr(), other.data_ptr(), m, n, k, form, ops._stream()), "gemm")
         assert torch.equal(out, other), form

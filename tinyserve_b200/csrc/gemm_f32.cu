@@ -16,12 +16,13 @@
 // row, 64 x 64 tiles of all K before / now: 4,096 x 1,024 70 / 11 us, 1,024 x 3,072 205 / 8 us, the head 92 us (6.8 TB/s).
 //
 // More rows: bound by the multiply-adds and, below some hundred rows, by the latency of the chains. Register tiles of
-// 4 x 4 outputs a thread, 32 x 64 a CTA, operands in shared memory as [row][16 k] read in 16-byte words (rows a thread owns lie a stride apart, so that eight neighbouring threads read
+// 4 x 4 outputs a thread, 32 x 64 a CTA, operands in shared memory as [row][32 k] read in 16-byte words (rows a thread owns lie a stride apart, so that eight neighbouring threads read
 // eight different groups of banks), three cp.async stages. Where the tiles are too few for the machine, the four
-// groups of K go to the two or four CTAs of a cluster, which leave their sums in shared memory; each then adds up its
-// share of the tile through distributed shared memory. Measured, before / now: 45 rows of 4,096 x 1,024 76 / 25 us,
-// of 1,024 x 3,072 221 / 29 us; 190 rows of 6,144 x 1,024 115 / 80 us. Tiles of 64 x 64 and 128 x 128 (8 outputs a
-// thread and side) were no faster at any of 1 to 600 rows: they leave too few warps on an SM.
+// groups of K go to the four CTAs of a cluster, which leave their sums in shared memory; each then adds up its
+// share of the tile through distributed shared memory. Measured, one kernel of 64 x 64 tiles for all sizes (which these
+// replace) / now: 45 rows of 4,096 x 1,024 76 / 20 us, 64 rows of 1,024 x 3,072 221 / 24 us, 190 rows of 6,144 x 1,024 115 /
+// 67 us; many rows reach 38 TFLOP/s. Steps of 16 k, with a division per copy, took 25, 40 and 80 us. Tiles of 64 x 64 and
+// 128 x 128 (8 outputs a thread and side) were no faster at any of 1 to 600 rows: they leave too few warps on an SM.
 #define TS_PDL_CLASS PDL_OTHER
 #include <cooperative_groups.h>
 
@@ -166,16 +167,17 @@ static int launch_rows(const float* x, const float* w, float* out, int M, int N,
 }
 
 // -------------------------------------------------------------------------------------------------- more rows
-constexpr int FT_M = 32, FT_N = 64, FT_OWN = 4, FT_K = 16, FT_STRIDE = FT_K + 4, FT_STAGES = 3;
+constexpr int FT_M = 32, FT_N = 64, FT_OWN = 4, FT_K = 32, FT_STRIDE = FT_K + 4, FT_STAGES = 3;
 constexpr int FT_THREADS = (FT_M / FT_OWN) * (FT_N / FT_OWN), FT_STAGE = (FT_M + FT_N) * FT_STRIDE;     // floats
 
 template <int SPLIT>
 __global__ void __launch_bounds__(FT_THREADS) gemm_f32_tile_kernel(const float* x, const float* __restrict__ w, float* out,
                                                                    int M, int N, int K) {
+  static_assert(SPLIT == 1 || SPLIT == 4, "all groups of K in one CTA, or one in each");
   constexpr int BM = FT_M, BN = FT_N, TM = FT_OWN, TN = FT_OWN;
   constexpr int THREADS = FT_THREADS, GROUPS = 4 / SPLIT, OUTS = TM * TN;
   extern __shared__ float smem[];
-  float* kept = smem + FT_STAGES * FT_STAGE;           // [group of this CTA][output of a thread][thread]
+  float* kept = smem + FT_STAGES * FT_STAGE;           // [output of a thread][thread]
   pdl_trigger();
   const int tid = threadIdx.x;
   const int tx = tid % (BN / TN), ty = tid / (BN / TN);
@@ -183,34 +185,31 @@ __global__ void __launch_bounds__(FT_THREADS) gemm_f32_tile_kernel(const float* 
   const int len = f32_part_length(K), steps = (len + FT_K - 1) / FT_K;    // steps of a part
   const int first_part = blockIdx.z * GROUPS * 4, total = GROUPS * 4 * steps;
 
-  auto load = [&](int step, int stage, bool a_side, bool b_side) {
-    float* dst = smem + stage * FT_STAGE;
-    const int part = first_part + step / steps, base = (step % steps) * FT_K;
-    if (a_side) {
+  // Step by step in order: `at` is the place of the next step inside its part, `from` the part's first k. Either side (x or
+  // w) keeps its own, because the first steps of w are asked for before x may be read.
+  constexpr int WORDS = FT_K / 4;
+  struct Place { int at, from; };
+  auto load = [&](Place& p, int rows, int r0, int limit, const float* src, float* dst) {
 #pragma unroll
-      for (int c = tid; c < BM * (FT_K / 4); c += THREADS) {
-        const int word = c & 3, r = c >> 2, in_part = base + word * 4, k = part * len + in_part;
-        const bool ok = in_part < len && k < K && m0 + r < M;
-        f32_copy16(dst + r * FT_STRIDE + word * 4, x + (ok ? (size_t)(m0 + r) * K + k : 0), ok);
-      }
+    for (int c = tid; c < rows * WORDS; c += THREADS) {
+      const int word = c % WORDS, r = c / WORDS, in_part = p.at + word * 4, k = p.from + in_part;
+      const bool ok = in_part < len && k < K && r0 + r < limit;
+      f32_copy16(dst + r * FT_STRIDE + word * 4, src + (ok ? (size_t)(r0 + r) * K + k : 0), ok);
     }
-    if (b_side) {
-#pragma unroll
-      for (int c = tid; c < BN * (FT_K / 4); c += THREADS) {
-        const int word = c & 3, r = c >> 2, in_part = base + word * 4, k = part * len + in_part;
-        const bool ok = in_part < len && k < K && n0 + r < N;
-        f32_copy16(dst + (BM + r) * FT_STRIDE + word * 4, w + (ok ? (size_t)(n0 + r) * K + k : 0), ok);
-      }
-    }
+    p.at += FT_K;
+    if (p.at >= len) { p.at = 0; p.from += len; }
   };
+  Place of_x = {0, first_part * len}, of_w = of_x;
+  auto load_x = [&](int stage) { load(of_x, BM, m0, M, x, smem + stage * FT_STAGE); };
+  auto load_w = [&](int stage) { load(of_w, BN, n0, N, w, smem + stage * FT_STAGE + BM * FT_STRIDE); };
 #pragma unroll
-  for (int s = 0; s < FT_STAGES - 1; ++s) load(s, s, false, true);        // weights first (total is at least four steps)
+  for (int s = 0; s < FT_STAGES - 1; ++s) load_w(s);        // weights first (total is at least four steps)
   pdl_wait();
 #pragma unroll
-  for (int s = 0; s < FT_STAGES - 1; ++s) { load(s, s, true, false); f32_commit(); }
+  for (int s = 0; s < FT_STAGES - 1; ++s) { load_x(s); f32_commit(); }
 
   float acc[TM][TN], group[TM][TN];
-  int step = 0;
+  int step = 0, stage = 0;
   for (int g = 0; g < GROUPS; ++g) {
     for (int p = 0; p < 4; ++p) {
 #pragma unroll
@@ -220,10 +219,15 @@ __global__ void __launch_bounds__(FT_THREADS) gemm_f32_tile_kernel(const float* 
       for (int b = 0; b < steps; ++b, ++step) {
         f32_wait<FT_STAGES - 2>();
         __syncthreads();
-        if (step + FT_STAGES - 1 < total) load(step + FT_STAGES - 1, (step + FT_STAGES - 1) % FT_STAGES, true, true);
+        if (step + FT_STAGES - 1 < total) {
+          const int free = stage == 0 ? FT_STAGES - 1 : stage - 1;      // read in the step before this one
+          load_x(free);
+          load_w(free);
+        }
         f32_commit();
-        const float* as = smem + (step % FT_STAGES) * FT_STAGE + ty * FT_STRIDE;
-        const float* bs = smem + (step % FT_STAGES) * FT_STAGE + (BM + tx) * FT_STRIDE;
+        const float* as = smem + stage * FT_STAGE + ty * FT_STRIDE;
+        const float* bs = smem + stage * FT_STAGE + (BM + tx) * FT_STRIDE;
+        stage = stage == FT_STAGES - 1 ? 0 : stage + 1;
 #pragma unroll
         for (int k = 0; k < FT_K; k += 4) {
           float4 a[TM];
@@ -248,14 +252,13 @@ __global__ void __launch_bounds__(FT_THREADS) gemm_f32_tile_kernel(const float* 
 #pragma unroll
         for (int j = 0; j < TN; ++j) group[i][j] = p == 0 ? acc[i][j] : group[i][j] + acc[i][j];
     }
-    // SPLIT 1: the sum of the groups so far; else one group beside the other (a thread's own words: no barrier)
-    float* mine = kept + (SPLIT == 1 ? 0 : g * OUTS * THREADS) + tid;
+    float* mine = kept + tid;        // the sum of the groups so far (a thread's own words: no barrier)
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
         float* o = mine + (i * TN + j) * THREADS;
-        *o = (SPLIT == 1 && g > 0) ? *o + group[i][j] : group[i][j];
+        *o = g > 0 ? *o + group[i][j] : group[i][j];
       }
   }
   f32_wait<0>();
@@ -271,7 +274,7 @@ __global__ void __launch_bounds__(FT_THREADS) gemm_f32_tile_kernel(const float* 
     cluster.sync();
     const float* of_group[4];
 #pragma unroll
-    for (int g = 0; g < 4; ++g) of_group[g] = cluster.map_shared_rank(kept, g / GROUPS) + (g % GROUPS) * OUTS * THREADS + tid;
+    for (int g = 0; g < 4; ++g) of_group[g] = cluster.map_shared_rank(kept, g) + tid;
     constexpr int SHARE = OUTS / SPLIT;
 #pragma unroll 4
     for (int o = (int)blockIdx.z * SHARE; o < ((int)blockIdx.z + 1) * SHARE; ++o)
@@ -283,18 +286,24 @@ __global__ void __launch_bounds__(FT_THREADS) gemm_f32_tile_kernel(const float* 
 template <int SPLIT>
 static int launch_tile(const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
   auto kernel = gemm_f32_tile_kernel<SPLIT>;
-  // the ring, and the sums of the CTA's groups
-  const int smem = (FT_STAGES * FT_STAGE + (SPLIT == 2 ? 2 : 1) * FT_M * FT_N) * (int)sizeof(float);
+  constexpr int own = (FT_STAGES * FT_STAGE + FT_M * FT_N) * (int)sizeof(float);      // the ring, and the CTA's sums
+  constexpr int sm_bytes = 228 * 1024;
   static bool ready[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64 || !ready[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_bytes / 2 + 1024);
     if (e != cudaSuccess) return (int)e;
     if (dev < 64) ready[dev] = true;
   }
   if ((M + FT_M - 1) / FT_M > 65535) return TS_ERR_BAD_ARGUMENT;
   const dim3 grid((N + FT_N - 1) / FT_N, (M + FT_M - 1) / FT_M, SPLIT);
+  // A grid of a few CTAs an SM starts while the kernel before it drains and piles up on the SMs that drain first: 64 rows of
+  // 1,024 x 3,072, 128 CTAs, took 41 us on half of the SMs and take 24 us when no SM has room for two. So a CTA asks for as
+  // much shared memory as lets no SM hold more than its share.
+  const long long per_sm = ((long long)grid.x * grid.y * grid.z + 147) / 148;
+  const int share = per_sm <= 3 ? sm_bytes / ((int)per_sm + 1) + 1024 : 0;
+  const int smem = share > own ? share : own;
   if (SPLIT == 1) return launch(kernel, grid, FT_THREADS, smem, stream, x, w, out, M, N, K);
   return launch_cluster(kernel, grid, FT_THREADS, smem, stream, dim3(1, 1, SPLIT), x, w, out, M, N, K);
 }
@@ -303,17 +312,17 @@ static int launch_tile(const float* x, const float* w, float* out, int M, int N,
 
 using namespace ts;
 
-// `form`: 0 = chosen here; 1, 2 = a few rows, one or two weight rows a thread; 3, 4, 5 = tiles, K over 1, 2, 4 CTAs.
+// `form`: 0 = chosen here; 1, 2 = a few rows, one or two weight rows a thread; 3, 4 = tiles, K over 1, 4 CTAs.
 extern "C" int ts_gemm_f32(const float* x, const float* w, float* out, int M, int N, int K, int form, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
-  if (K <= 0 || form < 0 || form > 5) return TS_ERR_BAD_ARGUMENT;
+  if (K <= 0 || form < 0 || form > 4) return TS_ERR_BAD_ARGUMENT;
   if (K % 4 != 0 || (((uintptr_t)x | (uintptr_t)w) & 15) != 0) return TS_ERR_UNSUPPORTED;
   if (form == 0) {
     const long long tiles = (long long)((M + FT_M - 1) / FT_M) * ((N + FT_N - 1) / FT_N);
-    // (tiles: 150 rows of 1,024 x 2,048, 80 tiles: 64 / 47 / 35 us over 1 / 2 / 4 CTAs; 600 of 4,096 x 1,024, 1,216 tiles:
-    // 164 / 158 / 165 us; 17 rows of the head, 2,374 tiles: 301 / 295 / 309 us)
+    // (K over 4 CTAs / over one: 128 rows of 4,096 x 1,024, 256 tiles, 39 / 42 us; 190 rows, 384 tiles, 53 / 53; 190 of
+    // 6,144 x 1,024, 576 tiles, 79 / 67; 64 of 1,024 x 3,072, 32 tiles, 24 / 73)
     if (M <= 16) form = M > 2 && N >= 2048 ? 2 : 1;
-    else form = tiles <= 400 ? 5 : tiles <= 1300 ? 4 : 3;
+    else form = tiles <= 400 ? 4 : 3;
   }
   if (form <= 2) {
     if ((M + 7) / 8 > 65535) return TS_ERR_BAD_ARGUMENT;
@@ -325,6 +334,5 @@ extern "C" int ts_gemm_f32(const float* x, const float* w, float* out, int M, in
     }
     return M <= 4 ? launch_rows<4, 2>(x, w, out, M, N, K, stream) : launch_rows<8, 2>(x, w, out, M, N, K, stream);
   }
-  if (form == 3) return launch_tile<1>(x, w, out, M, N, K, stream);
-  return form == 4 ? launch_tile<2>(x, w, out, M, N, K, stream) : launch_tile<4>(x, w, out, M, N, K, stream);
+  return form == 3 ? launch_tile<1>(x, w, out, M, N, K, stream) : launch_tile<4>(x, w, out, M, N, K, stream);
 }
