@@ -310,7 +310,9 @@ def test_clamped_feed_forward_products(rows, inter, k) -> None:
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("tokens, experts, top, hidden, ff, shared", [
     (1, 8, 3, 256, 64, True), (5, 5, 2, 48, 24, True), (300, 8, 3, 128, 64, False), (77, 3, 3, 64, 16, True),
-    (513, 64, 6, 128, 96, False), (40, 2, 1, 36, 12, True), (9, 33, 32, 32, 8, False)])
+    (513, 64, 6, 128, 96, False), (40, 2, 1, 36, 12, True), (9, 33, 32, 32, 8, False),
+    # up to 8 and up to 16 tokens: the products of a few rows, with the last block of K and the ring partly filled
+    (8, 4, 2, 1056, 32, False), (9, 4, 2, 1184, 1120, True), (16, 3, 3, 64, 2080, False), (17, 4, 2, 64, 64, True)])
 def test_routed_expert_kernels(dtype, tokens, experts, top, hidden, ff, shared) -> None:
     from tinyserve_b200.kernels import ops
 
@@ -422,6 +424,29 @@ def _router_case(ops, dtype, tokens, experts, top, hidden) -> None:
     assert torch.equal(plan["ids"], want["ids"]) and torch.equal(plan["offsets"], want["offsets"])
     torch.testing.assert_close(plan["weights"], want["weights"], atol=2e-3, rtol=2e-3)
     assert sorted(plan["row_of"].tolist()) == list(range(tokens * top)) and counts.abs().max() == 0
+
+
+def test_products_of_a_few_tokens_take_tiles_of_more_rows_than_expected() -> None:
+    """Routing sends a token whose logits are not numbers to expert 0 with every pick: the tile then has more rows than the
+    step has tokens, and the products of a few rows go over it in several passes."""
+    from tinyserve_b200.kernels import ops
+
+    tokens, experts, top, hidden, ff = 7, 4, 3, 64, 64
+    bf = torch.bfloat16
+    logits = _rand(tokens, experts, seed=1)
+    logits[2:6] = float("nan")
+    plan = ops.moe_route(logits, top, torch.zeros(experts, dtype=torch.int32, device="cuda"), Arena())
+    offsets, token_of = plan["offsets"].long(), plan["token_of"].long()
+    assert int(offsets[1]) > 8
+    x = _rand(tokens, hidden, seed=2, dtype=bf)
+    w1, w2 = _rand(experts, 2 * ff, hidden, seed=3, scale=0.1, dtype=bf), _rand(experts, hidden, ff, seed=4, scale=0.1, dtype=bf)
+    act, y = torch.empty(tokens * top, ff, dtype=bf, device="cuda"), torch.empty(tokens * top, hidden, dtype=bf, device="cuda")
+    ops.moe_gemm(x, w1, act, plan, gated=True, gather=True)
+    ops.moe_gemm(act, w2, y, plan, gated=False, gather=False)
+    expert = torch.bucketize(torch.arange(tokens * top, device="cuda"), offsets[1:], right=True)
+    gu = torch.einsum("rk,rnk->rn", x[token_of].float(), w1[expert].float())
+    torch.testing.assert_close(act.float(), torch.nn.functional.silu(gu[:, :ff]) * gu[:, ff:], atol=1e-3, rtol=2 ** -7)
+    torch.testing.assert_close(y.float(), torch.einsum("rk,rnk->rn", act.float(), w2[expert].float()), atol=1e-3, rtol=2 ** -7)
 
 
 def test_a_token_alone_and_in_a_crowd_takes_the_same_experts_path() -> None:

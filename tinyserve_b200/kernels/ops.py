@@ -108,7 +108,7 @@ _SIGNATURES: dict[str, list[Any]] = {
     "ts_moe_route_fused": [_vp, _vp, _i, _i, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _vp],
     "ts_moe_gather": [_vp, _vp, _vp, _i, _i, _vp, _vp],
     "ts_moe_gemm_tcgen05": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _f, _vp, _vp, _vp, _vp, _i, _vp, _vp],
-    "ts_moe_gemm": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _f, _i, _i, _vp],
+    "ts_moe_gemm": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _f, _i, _i, _i, _vp],
     "ts_moe_combine": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _i, _i, _vp],
     "ts_sample": [_vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
 }
@@ -2134,8 +2134,7 @@ def moe_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, plan: dict[str
         _dev(x, "x"), plan["token_of"].data_ptr() if gather else None, _dev(w, "w"), _dev(out, "out"),
         plan["offsets"].data_ptr(), plan["tile_expert"].data_ptr(), plan["tile_row0"].data_ptr(),
         plan["num_tiles"].data_ptr(), plan["max_tiles"], n, k, int(bool(gated)), _opt(row_weight, "row_weight"), float(limit),
-        _code(x.dtype), int(MOE_TENSOR_CORES),
-        _stream()), "moe_gemm")
+        _code(x.dtype), int(MOE_TENSOR_CORES), picks // plan["top"], _stream()), "moe_gemm")
 
 
 def moe_combine(y: torch.Tensor, plan: dict[str, Any], shared_out: torch.Tensor | None, out: torch.Tensor,
