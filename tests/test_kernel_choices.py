@@ -89,3 +89,18 @@ def test_parts_of_the_sums_of_squares_that_the_stream_product_leaves() -> None:
             p = parts(m, n, 1024)
             assert p in (n // 16, n // 8)
             assert p == n // 16 or p <= 128
+
+
+def test_one_head_or_two_a_cta_in_the_prompt_attention() -> None:
+    """One head where its CTAs all run at once, two where one head's would queue; windows and single tokens count as they run."""
+    from types import SimpleNamespace
+
+    def choice(query_lens, context_lens, heads=16, kv_heads=8, window=0):
+        return ops._prefill_heads_per_cta(SimpleNamespace(query_lens=query_lens, context_lens=context_lens), heads, kv_heads, window)
+
+    assert choice([512], [512]) == 1 and choice([512], [4096]) == 1
+    assert choice([2048], [2048]) == 1 and choice([2048], [9001]) == 2 and choice([8192], [8192]) == 2
+    assert choice([290] * 7, [290] * 7) == 2
+    assert choice([2048, 1, 1], [9001, 500, 70]) == 2 and choice([1], [100]) == 1
+    assert choice([2048], [9001], window=128) == choice([2048], [2176], window=128)
+    assert choice([8192], [8192], heads=24) == 1          # three heads a group: no pairs

@@ -44,7 +44,11 @@
 // 2,048 tokens 41 -> 35 us, 8,192 tokens 640 -> 810 TFLOP/s with one head a CTA. Doing every second
 // exponential as a polynomial on the FMA pipe made the step longer (the softmax warps are short of
 // issue slots, not only of the exponential unit). With two heads a CTA the tensor core works for one
-// head while the other's softmax runs: 920 TFLOP/s at 8,192 tokens. Every operand read from shared
+// head while the other's softmax runs, and the MMA warp serves both in turn, 16 instructions a head and tile: issued from a
+// branch on the lane an instruction took 77 cycles (its operands go to uniform registers one by one) and that warp set the
+// pace; issued by the converged warp, 8,192 tokens 300 -> 266 us (1,035 TFLOP/s), 2,048 tokens at 9,001 positions 179 -> 158
+// us. An MMA warp per head was slower (369 us: the heads fall into step), and so were two score buffers of 64 keys per head
+// (289 us at best: what a step costs whatever its size is paid twice). Every operand read from shared
 // memory and every TMA write goes through the same 128 bytes per cycle, which is why P stays in tensor
 // memory.
 // Every wait is on an mbarrier, is bounded and gives up at once when another role has: the CTA
@@ -157,7 +161,8 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
 
   pdl_trigger();
   unsigned char* smem = (unsigned char*)(((uintptr_t)fa_raw + 1023) & ~(uintptr_t)1023);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // two heads: known to the compiler to be the same in the whole warp, so that the MMA warp's operands are (umma_bf16_by)
+  const int warp = NQ == 1 ? (int)(threadIdx.x >> 5) : __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < FA_KV_STAGES; ++s) {
       mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
@@ -470,22 +475,32 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
   } else {
     // =========================================================== MMA issuer
     bool ok = fa_warp_wait(&q_ready, 0, failed);
+    // One head: a branch on the lane, whose 1,700 cycles a tile the softmax hides (issued by the converged warp instead, prompts
+    // of up to 2,048 tokens took 1 us longer). Two heads: the converged warp.
+    const uint32_t elected = NQ == 1 ? 1u : elect_one();
+    auto by_one = [&](auto&& issue) {
+      if constexpr (NQ == 1) {
+        if (lane == 0) issue();
+      } else {
+        issue();
+      }
+    };
     const uint32_t q_addr = smem_u32(smem + L::OFF_Q);
     const uint32_t k_addr = smem_u32(smem + L::OFF_K), v_addr = smem_u32(smem + L::OFF_V);
     // S_q = Q_q K^T of tile j into the head's buffer j % SPB
     auto issue_s = [&](int j, int q) {
       const int st = j % FA_KV_STAGES, bq = q * SPB + j % SPB;
-      if (lane == 0) {
+      by_one([&] {
 #pragma unroll
         for (int i = 0; i < (PAIR ? 4 : D / 16); ++i) {
           const int ks = PAIR ? 4 * q + i : i;
           const uint64_t ad = sw128_desc(q_addr + (PAIR ? 0 : q) * L::Q_BYTES + (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32);
           const uint64_t bd = sw128_desc(k_addr + st * L::KV_BYTES + (ks >> 2) * (BN * 128) + (ks & 3) * 32);
-          umma_bf16(tmem_base + L::TMEM_SP + (uint32_t)(bq * BN), ad, bd, IDESC_S, i != 0);
+          umma_bf16_by(elected, tmem_base + L::TMEM_SP + (uint32_t)(bq * BN), ad, bd, IDESC_S, i != 0);
         }
-        umma_commit(&s_full[q][j % SPB]);
-        if (q == NQ - 1) umma_commit(&k_empty[st]);       // the K stage is free once the last head's S has read it
-      }
+        umma_commit_by(elected, &s_full[q][j % SPB]);
+        if (q == NQ - 1) umma_commit_by(elected, &k_empty[st]);       // the K stage is free once the last head's S has read it
+      });
       __syncwarp();
     };
     // O_q += P_q V of tile j, P read from the head's buffer in tensor memory
@@ -493,16 +508,16 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
       const int st = j % FA_KV_STAGES, b = j % SPB;
       if (!fa_warp_wait(&p_full[q][b], (j / SPB) & 1, failed)) return false;
       tc_fence_after();
-      if (lane == 0) {
+      by_one([&] {
 #pragma unroll
         for (int ks = 0; ks < BN / 16; ++ks) {
           const uint64_t bd = sw128_desc_mn(v_addr + st * L::KV_BYTES + ks * (16 * 128), BN * 128);
-          umma_bf16_ta(tmem_base + L::TMEM_O + (uint32_t)(q * D),
+          umma_bf16_ta_by(elected, tmem_base + L::TMEM_O + (uint32_t)(q * D),
                        tmem_base + L::TMEM_SP + (uint32_t)((q * SPB + b) * BN + ks * 8), bd, IDESC_PV, (j | ks) != 0);
         }
-        umma_commit(&pv_done[q][b]);
-        if (q == NQ - 1) umma_commit(&v_empty[st]);
-      }
+        umma_commit_by(elected, &pv_done[q][b]);
+        if (q == NQ - 1) umma_commit_by(elected, &v_empty[st]);
+      });
       __syncwarp();
       return true;
     };

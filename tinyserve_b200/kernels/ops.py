@@ -10,6 +10,7 @@ dtype (bfloat16 or float32) and selects the kernel instantiation.
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
 from dataclasses import dataclass
@@ -389,17 +390,49 @@ MIN_KEYS_PER_SPLIT = 64
 MAX_SPLITS = 32
 
 
-def _prefill_heads_per_cta(ctx: Any, num_heads: int, num_kv_heads: int) -> int:
-    """Two query heads of a kv group in a CTA share its key and value tiles, which is worth more
-    than anything once the pairs alone give every SM a CTA (measured on B200, 16 / 8 heads of 128:
-    2,048 tokens 39 us with one head, 46 us with two; 3,072 tokens 79 / 64 us; 8,192 tokens
-    428 / 292 us)."""
+# What a tile of 128 keys costs a CTA of the tcgen05 prompt kernel with one head and with two, and what a CTA costs whatever
+# its tiles (B200 cycles, fitted to the times below).
+PREFILL_TILE_CYCLES = {1: 2560, 2: 4050}
+PREFILL_CTA_CYCLES = 15000
+
+
+def _prefill_cycles(tiles: list[int], heads: int, heads_per_cta: int) -> float:
+    """Estimated cycles of a launch whose query tiles see ``tiles`` (longest first) tiles of keys each, for ``heads`` heads:
+    no less than its longest CTA, than its work spread over the SMs, nor, for every k, than k + 1 times the
+    k * 148-th longest CTA (one SM runs k + 1 that are as long)."""
+    per_tile = heads // heads_per_cta
+    cost = [PREFILL_CTA_CYCLES + t * PREFILL_TILE_CYCLES[heads_per_cta] for t in tiles]
+    bound = max(cost[0], sum(cost) * per_tile / 148)
+    for k in range(1, (len(tiles) * per_tile - 1) // 148 + 1):
+        bound = max(bound, (k + 1) * cost[k * 148 // per_tile])
+    return bound
+
+
+@functools.lru_cache(maxsize=256)
+def _one_head_or_two(query_lens: tuple[int, ...], context_lens: tuple[int, ...], num_heads: int, window: int) -> int:
+    tiles = []
+    for n, total in zip(query_lens, context_lens):
+        if n > 1:
+            for q0 in range(0, n, 128):
+                first = total - n + q0                                  # the tile's first position
+                last = min(first + 128, total)
+                tiles.append((last + 127) // 128 - (max(0, first - window + 1) // 128 if window else 0))
+    tiles.sort(reverse=True)
+    return 1 if not tiles or _prefill_cycles(tiles, num_heads, 1) <= _prefill_cycles(tiles, num_heads, 2) else 2
+
+
+def _prefill_heads_per_cta(ctx: Any, num_heads: int, num_kv_heads: int, window: int = 0) -> int:
+    """Two query heads of a kv group in a CTA share its key and value tiles and keep the tensor core busier, but make half as
+    many CTAs, twice as long: whichever is estimated to end first (by the step's lengths alone, so the layers of a step, and
+    steps alike, share the estimate). Measured on B200, 16 / 8 heads of 128, one head / two: 512 tokens 15 / 17 us, 2,048
+    tokens 40 / 46, 2,048 at 4,096 positions 84 / 80, at 9,001 positions 188 / 158, 3,072 tokens 75 / 64, 8,192 tokens
+    357 / 266, seven prompts of 290 tokens 31 / 25."""
     if (num_heads // num_kv_heads) % 2:
         return 1
     if PREFILL_HEADS_PER_CTA:
         return PREFILL_HEADS_PER_CTA
-    tiles = sum(-(-n // 128) for n in ctx.query_lens if n > 1)
-    return 2 if tiles * (num_heads // 2) > 148 else 1
+    contexts = getattr(ctx, "context_lens", None) or ctx.query_lens      # (a caller of the kernel alone may not know them here)
+    return _one_head_or_two(tuple(ctx.query_lens), tuple(contexts), num_heads, window)
 
 
 def decode_splits(num_decode: int, num_kv_heads: int, group: int, max_context_len: int) -> int:
@@ -518,7 +551,7 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
                 _dev(ctx.context_lens_dev, "context_lens", torch.int32),
                 _dev(ctx.prefill_seqs, "prefill_seqs", torch.int32), num_prefill, ctx.max_query_len,
                 hq, hkv, d, page_size, float(scale), int(window),
-                _prefill_heads_per_cta(ctx, hq, hkv),
+                _prefill_heads_per_cta(ctx, hq, hkv, int(window)),
                 _error_word(q.device).data_ptr(), _opt(sinks, "sinks", torch.float32), keep_first, int(chunk), maps,
                 factor.data_ptr() if maps == 2 else None, float(mult) if maps == 2 else 1.0, float(mix_eps) if maps == 2 else 0.0, _stream()),
                 "prefill_attention_tcgen05")
