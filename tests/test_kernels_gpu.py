@@ -561,6 +561,18 @@ def test_gemm_rows_tcgen05(m, n, k, swiglu, slices) -> None:
     torch.testing.assert_close(out.float(), want.float(), atol=rtol * want.float().abs().mean().item(), rtol=rtol)
 
 
+def test_large_products_of_a_few_rows_off_the_16_byte_grid_stay_with_the_library() -> None:
+    base = rnd(1, 3 * 4096 + 1, dtype=torch.bfloat16, seed=1).flatten()
+    w = rnd(4112, 4096, dtype=torch.bfloat16, seed=2, scale=0.02)
+    x, out, want = base[1:].view(3, 4096), *(torch.empty(3, 4112, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    assert ops.takes_rows_tcgen05(x.clone(), w, out) and not ops.takes_rows_tcgen05(x, w, out)
+    ref.gemm(x, w, want)
+    for rows in (x.clone(), x):
+        out.fill_(float("nan"))
+        ops.gemm(rows, w, out)
+        torch.testing.assert_close(out.float(), want.float(), atol=2e-2, rtol=2e-2)
+
+
 def test_gemm_skinny_refuses_what_it_cannot_take() -> None:
     x, w = rnd(4, 80, dtype=torch.bfloat16), rnd(32, 80, dtype=torch.bfloat16)
     with pytest.raises(ops.KernelError, match="not supported"):

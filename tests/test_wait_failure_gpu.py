@@ -76,6 +76,19 @@ def test_gemm_tcgen05_gives_up_and_recovers(swiglu, pairs) -> None:
     torch.testing.assert_close(out.float(), want.float(), **tol(BF16))
 
 
+@pytest.mark.parametrize("slices", [1, 4])
+def test_gemm_rows_tcgen05_gives_up_and_recovers(slices) -> None:
+    x, w = rnd(9, 1024, dtype=BF16, seed=1), rnd(512, 1024, dtype=BF16, seed=2, scale=0.05)
+    out, want = torch.zeros(9, 512, device="cuda", dtype=BF16), torch.empty(9, 512, device="cuda", dtype=BF16)
+    ref.gemm(x, w, want)
+    with lost_copies():
+        ops.gemm_rows_tcgen05(x, w, out, slices=slices)
+        assert error_code() == 1
+    ops.gemm_rows_tcgen05(x, w, out, slices=slices)
+    ops.check_device_errors()
+    torch.testing.assert_close(out.float(), want.float(), **tol(BF16))
+
+
 @pytest.mark.parametrize("kernel,lens,d,page,code", [
     ("tcgen05", [(300, 300), (700, 130)], 128, 16, 2),        # tcgen05 prefill attention
     ("mma", [(300, 300), (700, 130)], 64, 8, 3),              # mma.sync prefill attention with TMA tiles

@@ -754,7 +754,7 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
         else:       # rows that do not start on a 16-byte boundary
             _check(_fn("ts_gemm_simt")(px, pw, _dev(out, "out"), m, n, k, _F32, _F32, _stream()), "gemm")
         return
-    if takes_rows_tcgen05(m, n * k, k) and out.dtype == x.dtype:
+    if takes_rows_tcgen05(x, w, out):
         gemm_rows_tcgen05(x, w, out)
         return
     if m <= SKINNY_MAX_ROWS and k % 32 == 0 and n % 16 == 0 and (n * k <= SKINNY_MAX_WEIGHTS or out.dtype != x.dtype):
@@ -784,9 +784,12 @@ SKINNY_MAX_WEIGHTS = 1 << 24
 ROWS_TCGEN05_MAX_ROWS = 16
 
 
-def takes_rows_tcgen05(m: int, weights: int, k: int) -> bool:
-    """Whether a bf16 product of ``m`` rows with a matrix of so many ``weights`` goes to :func:`gemm_rows_tcgen05`."""
-    return m <= ROWS_TCGEN05_MAX_ROWS and weights >= SKINNY_MAX_WEIGHTS and k % 8 == 0
+def takes_rows_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether a bf16 product of ``x [M, K]`` with a matrix ``w [N, K]`` (or a merged gate and up matrix) goes to
+    :func:`gemm_rows_tcgen05`: a few rows, a large matrix, rows and pointers on the 16-byte grid of its copies."""
+    return (x.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and x.shape[0] <= ROWS_TCGEN05_MAX_ROWS
+            and w.shape[0] * w.shape[1] >= SKINNY_MAX_WEIGHTS and w.shape[1] % 8 == 0
+            and (x.data_ptr() | w.data_ptr() | out.data_ptr()) % 16 == 0)
 
 
 def rows_tcgen05_slices(tiles: int, k: int) -> int:
@@ -946,7 +949,7 @@ def gemm_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, are
         _check(_fn("ts_gemm_skinny_swiglu")(_dev(x, "x"), _dev(w_gate_up, "w_gate_up"), _dev(out, "out"), m, inter, k,
                                             _stream()), "gemm_swiglu")
         return
-    if x.dtype == torch.bfloat16 and takes_rows_tcgen05(m, 2 * inter * k, k):
+    if takes_rows_tcgen05(x, w_gate_up, out):
         gemm_rows_tcgen05(x, w_gate_up, out, swiglu=True)
         return
     tiles = tcgen05_tiles(m, inter, 128)
