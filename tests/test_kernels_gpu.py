@@ -224,6 +224,17 @@ def test_prefill_attention_kernels(kernel, heads_per_cta, hq, hkv, d, page, wind
     torch.testing.assert_close(out.float(), want.float(), **tol(torch.bfloat16))
 
 
+@pytest.mark.parametrize("window", [0, 70])
+@pytest.mark.parametrize("d,page", [(64, 8), (128, 16)])
+def test_prefill_attention_one_head_or_two_a_cta_give_the_same_bits(d, page, window, monkeypatch) -> None:
+    """The choice follows the step's lengths, and a recorded step knows other ones than the step it stands for."""
+    outs = []
+    for heads in (1, 2):
+        monkeypatch.setattr(ops, "PREFILL_HEADS_PER_CTA", heads)
+        outs.append(_attention_case(torch.bfloat16, 4, 2, d, page, [(2, 2), (63, 40), (129, 129), (700, 260), (1025, 31)], window)[0])
+    assert torch.equal(*outs)
+
+
 @pytest.mark.parametrize("heads_per_cta", [1, 2])
 @pytest.mark.parametrize("pos", [0, 63, 64, 127, 128, 511, 999])
 def test_prefill_attention_tcgen05_far_key(heads_per_cta, pos, monkeypatch) -> None:

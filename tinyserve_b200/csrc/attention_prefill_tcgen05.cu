@@ -244,7 +244,12 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
     const uint32_t tmem_o = tmem_base + lane_addr + L::TMEM_O + (uint32_t)(q * D);
     const int p_abs = p_lo + r;
-    float m_used = -INFINITY, l_sum = 0.f;
+    // The sum of a row, kept per 64 columns of a tile whether one thread has them all or two share them: one head a CTA and two
+    // then give the same bits, and a recorded step, which does not know its contexts, those of the step it stands for.
+    constexpr int PARTS64 = HC / 64;
+    float m_used = -INFINITY, l_sum = 0.f, l_part[PARTS64];
+#pragma unroll
+    for (int c = 0; c < PARTS64; ++c) l_part[c] = 0.f;
     bool ok = true, stopped = false;
     for (int j = 0; j < n_tiles; ++j) {
       const int b = j % SPB, nth = j / SPB;                    // buffer, and how often it has been used
@@ -302,15 +307,19 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
               tmem_st_32(tmem_o + c * 32, o);
             }
           }
-          if (grow) { l_sum *= alpha; m_used = m_new; }
+          if (grow) {
+#pragma unroll
+            for (int c = 0; c < PARTS64; ++c) l_part[c] *= alpha;
+            m_used = m_new;
+          }
         }
       }
       const float m_sub = (m_used == -INFINITY) ? 0.f : m_used;
-      float add4[4] = {0.f, 0.f, 0.f, 0.f};
       // P as bf16, two keys per 32-bit column, over the first half of this buffer's columns
 #pragma unroll
       for (int c = 0; c < HC / 64; ++c) {
         uint32_t packed[32];
+        float add4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           const float p0 = fa_exp2(fmaf(__uint_as_float(sraw[c * 64 + 2 * i]), a.scale_log2, -m_sub));
@@ -319,8 +328,8 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
           packed[i] = fa_pack(p0, p1);
         }
         tmem_st_32_nowait(tmem_sp + half * (HC / 2) + c * 32, packed);
+        l_part[c] += (add4[0] + add4[1]) + (add4[2] + add4[3]);
       }
-      l_sum += (add4[0] + add4[1]) + (add4[2] + add4[3]);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -329,9 +338,10 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
     if (!stopped) {
       const int last = n_tiles - 1;
       if (ok && !fa_warp_wait(&pv_done[q][last % SPB], (last / SPB) & 1, failed)) ok = false;
-      float sums[HS];
-      ok = exchange(l_sum, ok, sums);
-      l_sum = 0.f;
+      float sums[HS], mine = l_part[0];
+#pragma unroll
+      for (int c = 1; c < PARTS64; ++c) mine += l_part[c];
+      ok = exchange(mine, ok, sums);
 #pragma unroll
       for (int h2 = 0; h2 < HS; ++h2) l_sum += sums[h2];      // in the order of the columns, the same in every warp
     }

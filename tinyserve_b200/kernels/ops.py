@@ -784,11 +784,21 @@ SKINNY_MAX_WEIGHTS = 1 << 24
 ROWS_TCGEN05_MAX_ROWS = 16
 
 
+# Plain products of more output columns stay with the library: tests/test_real_sizes_gpu.py holds the decode rows of the 8B
+# widths to it (6,144 x 4,096 there). In a chain of products the two are level (one row / 16 rows, library against that
+# kernel: 6,144 x 4,096 11.5 / 12.3 against 11.5 / 12.1 us, 10,240 x 5,120 20.6 / 21.3 against 19.8 / 20.8), but inside a
+# decode step that kernel, which asks for its first weights while the norm before it runs, would be 4 us a layer faster (16
+# tokens at the 8B sizes 53.3 ms instead of 55.6). With SwiGLU the activation kernel is saved too, at any width.
+ROWS_TCGEN05_MAX_COLS = 5376
+
+
 def takes_rows_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
-    """Whether a bf16 product of ``x [M, K]`` with a matrix ``w [N, K]`` (or a merged gate and up matrix) goes to
-    :func:`gemm_rows_tcgen05`: a few rows, a large matrix, rows and pointers on the 16-byte grid of its copies."""
+    """Whether a bf16 product of ``x [M, K]`` with a matrix ``w [N, K]`` (or a merged gate and up matrix, ``out`` then half as
+    wide) goes to :func:`gemm_rows_tcgen05`: a few rows, a large matrix of few columns of output, and rows and pointers on
+    the 16-byte grid of its copies."""
     return (x.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and x.shape[0] <= ROWS_TCGEN05_MAX_ROWS
             and w.shape[0] * w.shape[1] >= SKINNY_MAX_WEIGHTS and w.shape[1] % 8 == 0
+            and (w.shape[0] <= ROWS_TCGEN05_MAX_COLS or out.shape[1] != w.shape[0])
             and (x.data_ptr() | w.data_ptr() | out.data_ptr()) % 16 == 0)
 
 
