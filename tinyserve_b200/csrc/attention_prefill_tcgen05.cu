@@ -159,7 +159,6 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
   const int head0 = (int)blockIdx.x * NQ;                     // PAIR: the (head, map) pairs 2 head and 2 head + 1
   const int kvh = head0 / (a.num_heads / a.num_kv_heads);
 
-  pdl_trigger();
   unsigned char* smem = (unsigned char*)(((uintptr_t)fa_raw + 1023) & ~(uintptr_t)1023);
   // two heads: known to the compiler to be the same in the whole warp, so that the MMA warp's operands are (umma_bf16_by)
   const int warp = NQ == 1 ? (int)(threadIdx.x >> 5) : __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -178,6 +177,7 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
+  pdl_trigger();   // behind the allocation (tmem_alloc)
   pdl_wait();      // q and the cache rows of this step are written by the kernels before
 
   if (warp < FA_SOFTMAX_WARPS) {

@@ -47,7 +47,6 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_tcgen05_kernel(const __g
   __shared__ uint32_t tmem_base_slot;
   __shared__ int failed;
 
-  pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slices = gridDim.y, slice = blockIdx.y, n0 = blockIdx.x * OUT;
   const int all_kb = (K + GR_BK - 1) / GR_BK;
@@ -64,6 +63,7 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_tcgen05_kernel(const __g
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_slot;
+  pdl_trigger();           // behind the allocation (tmem_alloc)
 
   if (warp == 0) {
     // ---------------- TMA producer (one lane)

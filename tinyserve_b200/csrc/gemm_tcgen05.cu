@@ -209,15 +209,9 @@ __global__ void __launch_bounds__(TG_THREADS) gemm_tcgen05_kernel(const __grid_c
   __shared__ uint32_t tmem_base_slot;
   __shared__ int failed;
 
-  pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   static_assert(!SWIGLU || BN == 256, "the fused activation pairs 128 gate with 128 up columns");
   constexpr int BN_OUT = SWIGLU ? BN / 2 : BN;          // output columns per tile
-  const bool grouped = grp.tile_expert != nullptr;
-  if (grouped) pdl_wait();            // the list of tiles is the work of the kernels before this one
-  const int tiles_m = grouped ? *(const volatile int*)grp.num_tiles : (M + TG_BM - 1) / TG_BM, tiles_n = (N + BN_OUT - 1) / BN_OUT;
-  const int num_tiles = tiles_m * tiles_n;
-  const int num_kb = (K + TG_BK - 1) / TG_BK;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -230,6 +224,12 @@ __global__ void __launch_bounds__(TG_THREADS) gemm_tcgen05_kernel(const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
+  pdl_trigger();                      // behind the allocation (tmem_alloc)
+  const bool grouped = grp.tile_expert != nullptr;
+  if (grouped) pdl_wait();            // the list of tiles is the work of the kernels before this one
+  const int tiles_m = grouped ? *(const volatile int*)grp.num_tiles : (M + TG_BM - 1) / TG_BM, tiles_n = (N + BN_OUT - 1) / BN_OUT;
+  const int num_tiles = tiles_m * tiles_n;
+  const int num_kb = (K + TG_BK - 1) / TG_BK;
 
   if (warp == 0) {
     // ---------------- TMA producer (one lane)
@@ -360,7 +360,6 @@ __global__ void __launch_bounds__(TG_THREADS) gemm_tcgen05_pair_kernel(const __g
   __shared__ uint32_t tmem_base_slot;
   __shared__ int failed;
 
-  pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();
   const bool leader = rank == 0;
@@ -381,6 +380,7 @@ __global__ void __launch_bounds__(TG_THREADS) gemm_tcgen05_pair_kernel(const __g
   cluster_sync_all();      // both CTAs' barriers and tensor memory exist before either uses the other's
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
+  pdl_trigger();           // behind the allocation (tmem_alloc)
   const uint32_t full0 = smem_of_cta(&full_bar[0], 0), acc_empty0 = smem_of_cta(&acc_empty[0], 0);
 
   if (warp == 0) {

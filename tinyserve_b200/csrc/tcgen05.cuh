@@ -29,6 +29,12 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
 }
+// Tensor memory of an SM is shared by the CTAs on it, and an allocation that does not fit blocks, without a bound, until
+// another CTA frees its columns. So a kernel lets the kernels behind it start (pdl_trigger) only once all its threads know
+// that the CTA has its columns: a CTA that holds columns while it waits for an earlier kernel (pdl_wait) then never keeps a
+// CTA of that kernel from its own, because all of those had theirs before it was started. (With the trigger in front, a
+// prompt attention with heads of 64, 512 columns and 112 KB of shared memory, and a product of a few rows behind it, 91 KB,
+// fit one SM and could each have waited for the other.)
 __device__ __forceinline__ void tmem_alloc(uint32_t* result_in_smem, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(result_in_smem)), "r"(cols) : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
