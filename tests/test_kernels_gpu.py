@@ -584,6 +584,18 @@ def test_large_products_of_a_few_rows_off_the_16_byte_grid_stay_with_the_library
         torch.testing.assert_close(out.float(), want.float(), atol=2e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("which", ["x", "w", "out"])
+def test_gemm_rows_tcgen05_refuses_pointers_off_its_grid(which) -> None:
+    def view(rows, cols, off):
+        return torch.zeros(rows * cols + 8, device="cuda", dtype=torch.bfloat16)[off: off + rows * cols].view(rows, cols)
+
+    x, w, out = (view(*shape, 1 if which == name else 0) for name, shape in (("x", (3, 64)), ("w", (128, 64)), ("out", (3, 128))))
+    for swiglu in (False, True):
+        with pytest.raises(ops.KernelError, match="not supported"):
+            ops.gemm_rows_tcgen05(x, w, out if not swiglu else out.view(-1)[: 3 * 64].view(3, 64), swiglu=swiglu)
+    assert not out.any()
+
+
 def test_gemm_skinny_refuses_what_it_cannot_take() -> None:
     x, w = rnd(4, 80, dtype=torch.bfloat16), rnd(32, 80, dtype=torch.bfloat16)
     with pytest.raises(ops.KernelError, match="not supported"):

@@ -231,7 +231,7 @@ extern "C" int ts_gemm_rows_tcgen05(const void* x, const void* w, void* out, int
   if (M <= 0 || N <= 0) return 0;
   if (slices < 1 || slices > GR_MAX_SLICES) return TS_ERR_BAD_ARGUMENT;
   if (M > 64 || K <= 0 || K % 8 != 0 || slices > (K + GR_BK - 1) / GR_BK || error_flag == nullptr) return TS_ERR_UNSUPPORTED;
-  if (((uintptr_t)x | (uintptr_t)w) & 15) return TS_ERR_UNSUPPORTED;
+  if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15) return TS_ERR_UNSUPPORTED;        // copies of 16 bytes, stores of 8
   return swiglu ? dispatch_rows_tc<true>(x, w, (bf16*)out, M, N, K, slices, error_flag, stream)
                 : dispatch_rows_tc<false>(x, w, (bf16*)out, M, N, K, slices, error_flag, stream);
 }
