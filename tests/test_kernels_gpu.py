@@ -683,6 +683,31 @@ def test_sample_nucleus_of_wide_rows(vocab) -> None:
         assert out[5].item() == vocab // 2
 
 
+def test_sample_with_top_p_on_two_streams_at_once() -> None:
+    """The chunks of a row meet in their cluster alone, so launches that run beside each other do not mix their winners
+    (rows with and without top-p, and greedy ones)."""
+    r, vocab = 8, 50000
+    temps = torch.tensor([0.7, 1.0, 0.0, 1.6] * 2, device="cuda")
+    top_p = torch.tensor([0.9, 0.5, 0.9, 1.0] * 2, device="cuda")
+    draws = torch.zeros(r, device="cuda", dtype=torch.int64)
+    sets = [(rnd(r, vocab, seed=s, scale=3.0), torch.arange(r, device="cuda", dtype=torch.int64) + 100 * s) for s in (1, 2)]
+    streams = [torch.cuda.Stream() for _ in sets]
+    want = [torch.empty(r, device="cuda", dtype=torch.int32) for _ in sets]
+    for (logits, seeds), w in zip(sets, want):
+        ops.sample(logits, w, temps, top_p, seeds, draws)
+        torch.cuda.synchronize()
+    assert not torch.equal(*want)
+    got = [[torch.full((r,), -1, device="cuda", dtype=torch.int32) for _ in range(40)] for _ in sets]
+    torch.cuda.synchronize()
+    for i in range(40):
+        for (logits, seeds), stream, outs in zip(sets, streams, got):
+            with torch.cuda.stream(stream):
+                ops.sample(logits, outs[i], temps, top_p, seeds, draws)
+    torch.cuda.synchronize()
+    for w, outs in zip(want, got):
+        assert all(torch.equal(w, o) for o in outs)
+
+
 def test_sample_frequencies_follow_softmax() -> None:
     vocab, n = 8, 4096
     row = torch.tensor([2.0, 1.0, 0.0, -1.0, 0.5, -3.0, 1.5, 0.2], device="cuda")

@@ -11,10 +11,11 @@
 // together by top-p; the race is run on logit / T - log E_i, which orders the same way.
 //
 // A row is cut into chunks, one CTA each; the CTA that arrives last picks the winner among the
-// chunks' winners. A row with top-p needs sums over the whole row, again and again, for the
+// chunks' winners, which meet in one array per device: launches without top-p that may run at the
+// same time (on two streams) would share it. A row with top-p needs sums over the whole row, again and again, for the
 // search of its threshold: its eight chunks are the CTAs of a cluster that keep their weights in
 // registers (20 a thread: 163,840 tokens; a larger vocabulary is read from L2 each time) and add
-// up their sums through distributed shared memory. Bound by the passes over the weights and the
+// up their sums, and pick the winner, through distributed shared memory. Bound by the passes over the weights and the
 // barrier of each: seven thresholds a pass (11 passes instead of 30), and a warp none of whose
 // weights lie between the bounds left keeps its sum from pass to pass. 64 rows of 151,936 tokens: 981 us with one
 // CTA a row and two-way passes, 114 us now.
@@ -332,12 +333,28 @@ __global__ void __launch_bounds__(SM_THREADS) sample_kernel(const float* __restr
     __shared__ NucleusShared sh;
     if (per <= NUCLEUS_HELD * SM_THREADS) threshold = nucleus_threshold<true>(l, begin, end, 1.f / temp, tp, mx, sh);
     else threshold = nucleus_threshold<false>(l, begin, end, 1.f / temp, tp, mx, sh);
-    cg::this_cluster().sync();          // nobody goes on (and leaves) while its sums may still be read
   }
 
-  // ---- this CTA's chunk, then the last CTA picks among the chunks
+  // ---- this CTA's chunk, then one CTA picks among the chunks
   Best best = scan_range(l, begin, end, temp, mx, threshold, k0, k1, d0, d1);
   best = block_best(best, bscratch);
+  if (CLUSTERED) {
+    // the first CTA of the cluster, through distributed shared memory: launches on several streams share nothing
+    __shared__ Best mine;
+    cg::cluster_group cluster = cg::this_cluster();
+    if (threadIdx.x == 0) mine = best;
+    cluster.sync();
+    if (chunk == 0 && threadIdx.x == 0) {
+      Best b[NUCLEUS_CTAS];
+#pragma unroll
+      for (int r = 0; r < NUCLEUS_CTAS; ++r) b[r] = *cluster.map_shared_rank(&mine, r);
+#pragma unroll
+      for (int r = 1; r < NUCLEUS_CTAS; ++r) b[0] = better(b[0], b[r]);
+      out[row] = b[0].i < 0 ? 0 : b[0].i;
+    }
+    cluster.sync();          // nobody leaves while its winner (or its last sums of the search) may still be read
+    return;
+  }
   if (chunks == 1) {
     if (threadIdx.x == 0) out[row] = best.i < 0 ? 0 : best.i;
     return;

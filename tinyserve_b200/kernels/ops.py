@@ -2217,7 +2217,8 @@ def sample(logits: torch.Tensor, out: torch.Tensor, temperature: torch.Tensor | 
     are drawn (``seeds``/``draws`` int64 ``[R]``: the request's seed and how many tokens it
     has drawn so far; ``top_p`` float32 ``[R]`` optional). ``status_out`` (int32, one element):
     receives the device's error word, which kernels with bounded waits set when a wait ran out,
-    so that it reaches the host in the same copy as the tokens."""
+    so that it reaches the host in the same copy as the tokens. Launches without ``top_p`` share scratch
+    memory of the device: one at a time (in the order of a stream); those with it may run beside any other."""
     r, v = logits.shape
     if out.shape != (r,):
         raise KernelError("sample: one output per row")
