@@ -12,13 +12,16 @@
 //
 // A row is cut into chunks, one CTA each; the CTA that arrives last picks the winner among the
 // chunks' winners, which meet in one array per device: launches without top-p that may run at the
-// same time (on two streams) would share it. A row with top-p needs sums over the whole row, again and again, for the
-// search of its threshold: its eight chunks are the CTAs of a cluster that keep their weights in
-// registers (20 a thread: 163,840 tokens; a larger vocabulary is read from L2 each time) and add
-// up their sums, and pick the winner, through distributed shared memory. Bound by the passes over the weights and the
-// barrier of each: seven thresholds a pass (11 passes instead of 30), and a warp none of whose
-// weights lie between the bounds left keeps its sum from pass to pass. 64 rows of 151,936 tokens: 981 us with one
-// CTA a row and two-way passes, 114 us now.
+// same time (on two streams) would share it. A row with top-p needs sums over the whole row, again
+// and again, for the search of its threshold: its chunks are the CTAs of a cluster (one to eight, by
+// the vocabulary) that keep their weights in registers (20 a thread: 163,840 tokens; a larger
+// vocabulary is read from L2 each time) and add up their sums, and pick the winner, through
+// distributed shared memory. Bound by the passes over the weights and the barrier of each: seven
+// thresholds a pass (11 passes instead of 30), and a warp none of whose weights lie between the
+// bounds left leaves its sums where they are. Normal logits, deviation 3, top-p 0.95, one CTA a row
+// with two-way passes / eight CTAs for every vocabulary, closed warps adding up again / now, 1, 64
+// and 256 rows: 151,936 tokens 1,023, 1,044, 2,110 / 48, 233, 834 / 43, 207, 740 us; 32,768 tokens 128,
+// 129, 253 / 41, 196, 699 / 42, 43, 161; 1,000 tokens 19, 19, 36 / 35, 166, 593 / 15, 16, 30.
 #define TS_PDL_CLASS PDL_SAMPLING
 #include <cooperative_groups.h>
 
@@ -163,9 +166,9 @@ __device__ __forceinline__ Best scan_range(const float* __restrict__ l, int begi
   return best;
 }
 
-// The nucleus threshold of one row by the cluster of its NUCLEUS_CTAS chunks: the smallest bit pattern b in
+// The nucleus threshold of one row by the cluster of its CTAS chunks: the smallest bit pattern b in
 // [0, bits(1.0)] with mass{weight > float(b)} < top_p * mass{all}. Tokens of [begin, end) are this CTA's.
-constexpr int NUCLEUS_CTAS = 8, NUCLEUS_HELD = 20, NUCLEUS_WAYS = 8;
+constexpr int NUCLEUS_WAYS = 8, NUCLEUS_HELD = 20, NUCLEUS_HELD_SMALL = 4;
 
 struct NucleusShared {
   float scratch[33];
@@ -174,33 +177,40 @@ struct NucleusShared {
   float whole[2][NUCLEUS_WAYS - 1];     // the cluster's
 };
 
-// `whole` of COUNT values per CTA over the cluster: their sums in the order of the CTAs, or the largest. `turn`
-// alternates from call to call, so that one cluster barrier a call is enough.
-template <int COUNT, bool MAX>
-__device__ __forceinline__ void nucleus_exchange(NucleusShared& sh, int turn) {
-  cg::cluster_group cluster = cg::this_cluster();
-  cluster.sync();                       // everyone's `mine` of this turn is written
-  if (threadIdx.x < COUNT) {
-    float v[NUCLEUS_CTAS];
+// COUNT values per CTA over the cluster: their sums in the order of the CTAs, or the largest. `turn` alternates from
+// call to call, so that one barrier of all CTAs a call is enough.
+template <int CTAS, int COUNT, bool MAX>
+__device__ __forceinline__ const float* nucleus_exchange(NucleusShared& sh, int turn) {
+  if constexpr (CTAS == 1) {
+    __syncthreads();
+    return sh.mine[turn];
+  } else {
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();                       // everyone's `mine` of this turn is written
+    if (threadIdx.x < COUNT) {
+      float v[CTAS];
 #pragma unroll
-    for (int r = 0; r < NUCLEUS_CTAS; ++r) v[r] = *cluster.map_shared_rank(&sh.mine[turn][threadIdx.x], r);
-    float t = v[0];
+      for (int r = 0; r < CTAS; ++r) v[r] = *cluster.map_shared_rank(&sh.mine[turn][threadIdx.x], r);
+      float t = v[0];
 #pragma unroll
-    for (int r = 1; r < NUCLEUS_CTAS; ++r) t = MAX ? fmaxf(t, v[r]) : t + v[r];
-    sh.whole[turn][threadIdx.x] = t;
+      for (int r = 1; r < CTAS; ++r) t = MAX ? fmaxf(t, v[r]) : t + v[r];
+      sh.whole[turn][threadIdx.x] = t;
+    }
+    __syncthreads();
+    return sh.whole[turn];
   }
-  __syncthreads();
 }
 
-template <bool HELD>
+// HELD: weights a thread keeps in registers, 0: they are read and raised again in every pass.
+template <int CTAS, int HELD>
 __device__ __forceinline__ float nucleus_threshold(const float* __restrict__ l, int begin, int end, float inv_t, float top_p,
                                                    float& row_max, NucleusShared& sh) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  float e[NUCLEUS_HELD];
+  float e[HELD ? HELD : 1];
   float mx = -INFINITY;
   if (HELD) {
 #pragma unroll
-    for (int j = 0; j < NUCLEUS_HELD; ++j) {
+    for (int j = 0; j < HELD; ++j) {
       const int i = begin + tid + j * SM_THREADS;
       e[j] = i < end ? l[i] : -INFINITY;
       mx = fmaxf(mx, scaled(e[j], inv_t));
@@ -210,14 +220,13 @@ __device__ __forceinline__ float nucleus_threshold(const float* __restrict__ l, 
   }
   mx = block_max(mx, sh.scratch);
   if (tid == 0) sh.mine[0][0] = mx;
-  nucleus_exchange<1, true>(sh, 0);
-  mx = sh.whole[0][0];
+  mx = nucleus_exchange<CTAS, 1, true>(sh, 0)[0];
   row_max = mx;
 
   float z = 0.f;
   if (HELD) {
 #pragma unroll
-    for (int j = 0; j < NUCLEUS_HELD; ++j) {
+    for (int j = 0; j < HELD; ++j) {
       e[j] = begin + tid + j * SM_THREADS < end ? weight_of(e[j], inv_t, mx) : 0.f;     // 0 is above no threshold
       z += e[j];
     }
@@ -226,26 +235,22 @@ __device__ __forceinline__ float nucleus_threshold(const float* __restrict__ l, 
   }
   z = block_sum(z, sh.scratch);
   if (tid == 0) sh.mine[1][0] = z;
-  nucleus_exchange<1, false>(sh, 1);
-  const float target = top_p * sh.whole[1][0];
+  const float target = top_p * nucleus_exchange<CTAS, 1, false>(sh, 1)[0];
 
   uint32_t lo = 0u, hi = 0x3f800000u;
   int turn = 0;
   bool open = true;                     // whether a weight of this warp may lie between the bounds
-  float settled = 0.f;                  // if not: this thread's sum, the same for every threshold left
   while (lo < hi) {
-    float t[NUCLEUS_WAYS - 1], mass[NUCLEUS_WAYS - 1];
+    if (open) {        // else the warp's sums, the same for every threshold left, are where it has put them
+      float t[NUCLEUS_WAYS - 1], mass[NUCLEUS_WAYS - 1];
 #pragma unroll
-    for (int q = 0; q < NUCLEUS_WAYS - 1; ++q) {
-      t[q] = __uint_as_float(lo + (uint32_t)(((unsigned long long)(hi - lo) * (q + 1)) / NUCLEUS_WAYS));
-      mass[q] = settled;
-    }
-    if (open) {
-#pragma unroll
-      for (int q = 0; q < NUCLEUS_WAYS - 1; ++q) mass[q] = 0.f;
+      for (int q = 0; q < NUCLEUS_WAYS - 1; ++q) {
+        t[q] = __uint_as_float(lo + (uint32_t)(((unsigned long long)(hi - lo) * (q + 1)) / NUCLEUS_WAYS));
+        mass[q] = 0.f;
+      }
       if (HELD) {
 #pragma unroll
-        for (int j = 0; j < NUCLEUS_HELD; ++j)
+        for (int j = 0; j < HELD; ++j)
 #pragma unroll
           for (int q = 0; q < NUCLEUS_WAYS - 1; ++q)
             if (e[j] > t[q]) mass[q] += e[j];
@@ -257,18 +262,18 @@ __device__ __forceinline__ float nucleus_threshold(const float* __restrict__ l, 
             if (v > t[q]) mass[q] += v;
         }
       }
-    }
 #pragma unroll
-    for (int q = 0; q < NUCLEUS_WAYS - 1; ++q) {
-      const float v = warp_sum(mass[q]);
-      if (lane == 0) sh.by_warp[q][warp] = v;
+      for (int q = 0; q < NUCLEUS_WAYS - 1; ++q) {
+        const float v = warp_sum(mass[q]);
+        if (lane == 0) sh.by_warp[q][warp] = v;
+      }
     }
     __syncthreads();
     if (warp < NUCLEUS_WAYS - 1) {
       const float v = warp_sum(sh.by_warp[warp][lane]);
       if (lane == 0) sh.mine[turn][warp] = v;
     }
-    nucleus_exchange<NUCLEUS_WAYS - 1, false>(sh, turn);
+    const float* whole = nucleus_exchange<CTAS, NUCLEUS_WAYS - 1, false>(sh, turn);
     // sums of the same terms in the same order grow as the threshold falls: the first one below the target ends the search
     uint32_t below = lo, next = hi;
     bool found = false;
@@ -276,7 +281,7 @@ __device__ __forceinline__ float nucleus_threshold(const float* __restrict__ l, 
     for (int q = 0; q < NUCLEUS_WAYS - 1; ++q) {
       const uint32_t mid = lo + (uint32_t)(((unsigned long long)(hi - lo) * (q + 1)) / NUCLEUS_WAYS);
       if (!found) {
-        if (sh.whole[turn][q] < target) { next = mid; found = true; }
+        if (whole[q] < target) { next = mid; found = true; }
         else below = mid + 1u;
       }
     }
@@ -289,19 +294,22 @@ __device__ __forceinline__ float nucleus_threshold(const float* __restrict__ l, 
       bool between = false;
       float above = 0.f;
 #pragma unroll
-      for (int j = 0; j < NUCLEUS_HELD; ++j) {
+      for (int j = 0; j < HELD; ++j) {
         between = between || (e[j] > low && e[j] <= high);
         if (e[j] > high) above += e[j];
       }
       open = __any_sync(0xffffffffu, between);
-      settled = above;
+      if (!open) {
+        above = warp_sum(above);
+        if (lane < NUCLEUS_WAYS - 1) sh.by_warp[lane][warp] = above;
+      }
     }
   }
   return __uint_as_float(lo);
 }
 
-// CLUSTERED: some rows have a top-p; the chunks of a row are the NUCLEUS_CTAS CTAs of a cluster.
-template <bool CLUSTERED>
+// CTAS > 0: some rows have a top-p; the chunks of a row are the CTAS CTAs of a cluster.
+template <int CTAS, int HELD>
 __global__ void __launch_bounds__(SM_THREADS) sample_kernel(const float* __restrict__ logits, int vocab,
                                                             const float* __restrict__ temperature,
                                                             const float* __restrict__ top_p,
@@ -329,27 +337,26 @@ __global__ void __launch_bounds__(SM_THREADS) sample_kernel(const float* __restr
   per = (per + 3) & ~3;
   const int begin = chunk * per, end = min(vocab, begin + per);     // empty behind the last token
   float mx = 0.f, threshold = 0.f;
-  if (CLUSTERED && tp < 1.f) {
+  if constexpr (CTAS > 0) if (tp < 1.f) {
     __shared__ NucleusShared sh;
-    if (per <= NUCLEUS_HELD * SM_THREADS) threshold = nucleus_threshold<true>(l, begin, end, 1.f / temp, tp, mx, sh);
-    else threshold = nucleus_threshold<false>(l, begin, end, 1.f / temp, tp, mx, sh);
+    threshold = nucleus_threshold<CTAS, HELD>(l, begin, end, 1.f / temp, tp, mx, sh);
   }
 
   // ---- this CTA's chunk, then one CTA picks among the chunks
   Best best = scan_range(l, begin, end, temp, mx, threshold, k0, k1, d0, d1);
   best = block_best(best, bscratch);
-  if (CLUSTERED) {
+  if constexpr (CTAS > 1) {
     // the first CTA of the cluster, through distributed shared memory: launches on several streams share nothing
     __shared__ Best mine;
     cg::cluster_group cluster = cg::this_cluster();
     if (threadIdx.x == 0) mine = best;
     cluster.sync();
     if (chunk == 0 && threadIdx.x == 0) {
-      Best b[NUCLEUS_CTAS];
+      Best b[CTAS];
 #pragma unroll
-      for (int r = 0; r < NUCLEUS_CTAS; ++r) b[r] = *cluster.map_shared_rank(&mine, r);
+      for (int r = 0; r < CTAS; ++r) b[r] = *cluster.map_shared_rank(&mine, r);
 #pragma unroll
-      for (int r = 1; r < NUCLEUS_CTAS; ++r) b[0] = better(b[0], b[r]);
+      for (int r = 1; r < CTAS; ++r) b[0] = better(b[0], b[r]);
       out[row] = b[0].i < 0 ? 0 : b[0].i;
     }
     cluster.sync();          // nobody leaves while its winner (or its last sums of the search) may still be read
@@ -393,9 +400,25 @@ extern "C" int ts_sample(const float* logits, int num_rows, int vocab, const flo
   if (num_rows <= 0) return 0;
   if (vocab <= 0 || num_rows > SM_MAX_ROWS) return TS_ERR_BAD_ARGUMENT;
   if (temperature != nullptr && (seeds == nullptr || draws == nullptr)) return TS_ERR_BAD_ARGUMENT;
-  if (temperature != nullptr && top_p != nullptr)
-    return launch_cluster(sample_kernel<true>, dim3(num_rows, NUCLEUS_CTAS), SM_THREADS, 0, stream, dim3(1, NUCLEUS_CTAS), logits, vocab,
-                          temperature, top_p, seeds, draws, out, NUCLEUS_CTAS, status_in, status_out);
+  if (temperature != nullptr && top_p != nullptr) {
+    // As few CTAs a row as hold its weights in registers: one CTA fits an SM, so eight let 18 rows run at once, and what a
+    // pass costs besides its tokens (the cluster's barrier and exchange) is paid by each. The number of rows has no say: a
+    // row's sums are the same in any batch.
+    constexpr int one = NUCLEUS_HELD * SM_THREADS;
+#define TS_NUCLEUS(CTAS_, HELD_)                                                                                                    \
+    return launch_cluster(sample_kernel<CTAS_, HELD_>, dim3(num_rows, CTAS_), SM_THREADS, 0, stream, dim3(1, CTAS_), logits, vocab, \
+                          temperature, top_p, seeds, draws, out, CTAS_, status_in, status_out)
+    if (vocab <= one) {
+      auto kernel = vocab <= NUCLEUS_HELD_SMALL * SM_THREADS ? sample_kernel<1, NUCLEUS_HELD_SMALL> : sample_kernel<1, NUCLEUS_HELD>;
+      return launch(kernel, dim3(num_rows), SM_THREADS, 0, stream, logits, vocab, temperature, top_p, seeds, draws, out, 1, status_in,
+                    status_out);
+    }
+    if (vocab <= 2 * one) TS_NUCLEUS(2, NUCLEUS_HELD);
+    if (vocab <= 4 * one) TS_NUCLEUS(4, NUCLEUS_HELD);
+    if (vocab <= 8 * one) TS_NUCLEUS(8, NUCLEUS_HELD);
+    TS_NUCLEUS(8, 0);
+#undef TS_NUCLEUS
+  }
   // as many CTAs as run at once (two of 1024 threads per SM), never a partly filled second
   // round, each with at least a few thousand tokens
   int chunks = (148 * 2) / num_rows;
@@ -403,6 +426,6 @@ extern "C" int ts_sample(const float* logits, int num_rows, int vocab, const flo
   if (chunks > most) chunks = most;
   if (chunks > SM_MAX_CHUNKS) chunks = SM_MAX_CHUNKS;
   if (chunks < 1) chunks = 1;
-  return launch(sample_kernel<false>, dim3(num_rows, chunks), SM_THREADS, 0, stream, logits, vocab, temperature, top_p,
+  return launch(sample_kernel<0, 0>, dim3(num_rows, chunks), SM_THREADS, 0, stream, logits, vocab, temperature, top_p,
                 seeds, draws, out, chunks, status_in, status_out);
 }
