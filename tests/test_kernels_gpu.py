@@ -656,12 +656,12 @@ def test_sample_temperature_and_top_p_match_reference(vocab) -> None:
         assert out.tolist() == want.tolist()
 
 
-@pytest.mark.parametrize("vocab", [3, 31, 32768, 151936, 163841])
+@pytest.mark.parametrize("vocab", [3, 31, 20480, 20481, 32768, 40961, 81920, 81921, 151936, 163840, 163841])
 def test_sample_nucleus_of_wide_rows(vocab) -> None:
-    """The eight chunks of a row (some empty at the smallest vocabularies; weights held in registers up to 163,840
-    tokens, read again beyond) find the same nucleus as a sort does: with the temperature low and the noise removed
-    by comparing eligibility, every drawn token's more likely tokens hold less than top_p, and the most likely token
-    is always eligible. A row of -inf but one token, and greedy rows beside it."""
+    """The chunks of a row (one to eight by the vocabulary, some empty; weights held in registers up to 163,840 tokens,
+    read again beyond) find the nucleus that a sort finds: a drawn token's more likely tokens hold less than top_p, and of
+    all tokens of which that is true the drawn one won the race, so the nucleus is neither too large nor too small. A row
+    of -inf but one token, and greedy rows beside it."""
     r = 12
     logits = rnd(r, vocab, seed=6, scale=3.0)
     logits[5, :] = float("-inf")
@@ -671,6 +671,9 @@ def test_sample_nucleus_of_wide_rows(vocab) -> None:
     seeds = torch.arange(r, device="cuda", dtype=torch.int64) + 77
     z = logits.double() / torch.where(temps > 0, temps, torch.ones_like(temps)).double()[:, None]
     p = torch.softmax(z, -1)
+    ranked, order = p.sort(-1, descending=True)
+    first = torch.searchsorted(-ranked, -ranked)            # equal probabilities share the mass above the first of them
+    above = torch.zeros_like(p).scatter_(1, order, (ranked.cumsum(-1) - ranked).gather(1, first))
     for draw in range(6):
         out = torch.empty(r, device="cuda", dtype=torch.int32)
         ops.sample(logits, out, temps, top_p, seeds, torch.full((r,), draw, device="cuda", dtype=torch.int64))
@@ -680,6 +683,10 @@ def test_sample_nucleus_of_wide_rows(vocab) -> None:
                 assert tok == int(logits[b].argmax())
             else:           # 32-bit sums of up to 163,841 weights: 1e-5 of slack
                 assert float(p[b][p[b] > p[b][tok]].sum()) < float(top_p[b]) + 1e-5
+                inside = (above[b] < float(top_p[b]) - 1e-5) | (above[b] == 0)
+                score = z[b] - torch.log(ref.exponential_noise(vocab, int(seeds[b]), draw).to("cuda").double())
+                # scores are made of 32-bit values of up to 40: 1e-4 of slack
+                assert float(score[tok]) > float(score[inside].max()) - 1e-4
         assert out[5].item() == vocab // 2
 
 
