@@ -104,3 +104,17 @@ def test_one_head_or_two_a_cta_in_the_prompt_attention() -> None:
     assert choice([2048, 1, 1], [9001, 500, 70]) == 2 and choice([1], [100]) == 1
     assert choice([2048], [9001], window=128) == choice([2048], [2176], window=128)
     assert choice([8192], [8192], heads=24) == 1          # three heads a group: no pairs
+
+
+def test_expert_products_of_a_few_tokens_by_their_ctas_per_k() -> None:
+    """On either side of the line, shapes measured on both; never beyond the 16 rows that the form holds."""
+    take = ops.moe_takes_few_rows
+    for tokens, experts, top, n, k, gated in [(4, 16, 3, 768, 1024, True), (4, 16, 3, 1024, 768, False), (2, 8, 2, 14336, 4096, True),
+                                              (8, 8, 2, 4096, 14336, False), (4, 128, 8, 1536, 4096, True), (1, 16, 3, 768, 256, True),
+                                              (8, 128, 8, 2048, 768, False), (16, 4, 2, 512, 512, False)]:
+        assert take(tokens, experts, top, n, k, gated)
+    for tokens, experts, top, n, k, gated in [(8, 8, 2, 14336, 4096, True), (16, 128, 8, 1536, 4096, True), (8, 16, 3, 768, 256, True),
+                                              (16, 128, 8, 2048, 768, False), (8, 64, 8, 1024, 384, False), (16, 64, 6, 1408, 2048, True),
+                                              (17, 4, 2, 64, 4096, True), (17, 4, 2, 64, 4096, False)]:
+        assert not take(tokens, experts, top, n, k, gated)
+    assert take(1, 2, 2, 64, 64, True) and not take(1, 2, 2, 1 << 20, 64, True)

@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(TG_THREADS) moe_gemm_mma_kernel(
 }
 
 // The form for steps of up to 16 tokens, where an expert has one row or a few and the products are the stream of the picked
-// experts' weights. A CTA takes 16 weight rows (GATED: 8 gate and the 8 matching up rows) of one tile; its 8 warps share K,
+// experts' weights (which of those steps take it: moe_takes_few_rows in kernels/ops.py). A CTA takes 16 weight rows (GATED: 8 gate and the 8 matching up rows) of one tile; its 8 warps share K,
 // each asking for four blocks of 32 k at a time straight from global memory into the mma operands (x is the A operand: rows
 // g and, XR = 2, g + 8, fetched through the token list), and add up in shared memory in the order of the warps. Tiles of 64
 // rows staged through shared memory, which these steps took before, multiplied some sixty rows of zeros with every weight

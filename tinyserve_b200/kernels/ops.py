@@ -2143,6 +2143,26 @@ def moe_route(logits: torch.Tensor, top: int, counts: torch.Tensor, arena: Any, 
     return plan
 
 
+def moe_takes_few_rows(tokens: int, experts: int, top: int, n: int, k: int, gated: bool) -> bool:
+    """Whether the experts' bf16 products of a step of up to 16 tokens stream the weights into the mma operands (one CTA per
+    8 or 16 weight rows of an expert) instead of taking tiles of 64 rows. A CTA of the former has its start, its list of rows
+    and its reduction to pay for with K, so the line is a number of CTAs per K, of the experts that even routing would pick.
+    Measured on B200 at 30 shapes of 4 to 256 experts, K and N of 64 to 14,336, weights from memory, streamed / tiles of 64:
+    gate and up, 16 experts, top 3, 1,024 x 768, 4 tokens 15 / 20 us; 8, 2, 4,096 x 14,336, 2 and 8 tokens 283 / 297 and
+    488 / 472; 128, 8, 4,096 x 1,536, 4 and 16 tokens 226 / 245 and 656 / 580; 16, 3, 256 x 768, 1 and 8 tokens 6 / 8 and
+    13 / 10; the product back, 8, 2, 14,336 x 4,096, 8 tokens 265 / 365; 128, 8, 768 x 2,048, 8 and 16 tokens 58 / 61 and
+    115 / 96; 64, 8, 384 x 1,024, 8 tokens 25 / 19. By this line nothing measured is more than 6 % slower than the faster of
+    its two sides where that is the tiles of 64."""
+    if tokens > 16:
+        return False
+    ctas = experts * (1.0 - (1.0 - min(1.0, top / experts)) ** tokens) * n / (8 if gated else 16)
+    if gated:
+        return ctas <= (2.0 if tokens <= 8 else 1.25) * k
+    if tokens <= 8:
+        return k >= 768 or ctas <= 1.75 * k
+    return ctas <= (2.0 if k >= 1024 else 0.5) * k
+
+
 def moe_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, plan: dict[str, Any], gated: bool, gather: bool,
              arena: Any = None, limit: float = 0.0) -> None:
     """The experts' products over the sorted order of ``plan``: for every sorted row r of expert e,
@@ -2176,11 +2196,13 @@ def moe_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, plan: dict[str
             plan["tile_row0"].data_ptr(), plan["num_tiles"].data_ptr(), plan["max_tiles"],
             _error_word(x.device).data_ptr(), _stream()), "moe_gemm_tcgen05")
         return
+    tokens = picks // plan["top"]
     _check(_fn("ts_moe_gemm")(
         _dev(x, "x"), plan["token_of"].data_ptr() if gather else None, _dev(w, "w"), _dev(out, "out"),
         plan["offsets"].data_ptr(), plan["tile_expert"].data_ptr(), plan["tile_row0"].data_ptr(),
         plan["num_tiles"].data_ptr(), plan["max_tiles"], n, k, int(bool(gated)), _opt(row_weight, "row_weight"), float(limit),
-        _code(x.dtype), int(MOE_TENSOR_CORES), picks // plan["top"], _stream()), "moe_gemm")
+        _code(x.dtype), int(MOE_TENSOR_CORES), tokens if moe_takes_few_rows(tokens, e, plan["top"], n, k, gated) else 17,
+        _stream()), "moe_gemm")
 
 
 def moe_combine(y: torch.Tensor, plan: dict[str, Any], shared_out: torch.Tensor | None, out: torch.Tensor,
