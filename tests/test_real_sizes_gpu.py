@@ -85,14 +85,15 @@ def real_8b(tmp_path_factory):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_8b_layer_widths_under_every_cut(real_8b, dtype, monkeypatch) -> None:
     """At these widths another set of kernels runs than at the 0.6B ones: the decode rows' products
-    leave the skinny kernel for the library (the matrices are larger than it is tuned for), the
+    leave the skinny kernel (the matrices are larger than it is tuned for) for the tcgen05 kernel of a
+    few rows or the library, whichever is measured to be faster, the
     norms run as kernels of their own (the stream is wider than the fusion takes), products of a
     hundred-odd rows go to the library too (their tiles would not fill the machine), and four
     query heads share a kv head. The test also checks that those are the kernels that ran."""
     from tinyserve_b200.kernels import ops
     from tinyserve_b200.model import DecoderModel
 
-    seen = {"mm": 0, "tcgen05": 0, "norm": 0, "normed": 0, "skinny": 0, "fused_attention": 0}
+    seen = {"mm": 0, "rows": 0, "tcgen05": 0, "norm": 0, "normed": 0, "skinny": 0, "fused_attention": 0}
 
     def counted(name, fn):
         def wrapper(*a, **k):
@@ -102,7 +103,7 @@ def test_8b_layer_widths_under_every_cut(real_8b, dtype, monkeypatch) -> None:
 
     monkeypatch.setattr(ops.torch, "mm", counted("mm", torch.mm))
     for name, attr in (("tcgen05", "gemm_tcgen05"), ("norm", "add_rms_norm"), ("normed", "gemm_normed"),
-                       ("skinny", "gemm_skinny"), ("fused_attention", "decode_attention_fused")):
+                       ("skinny", "gemm_skinny"), ("rows", "gemm_rows_tcgen05"), ("fused_attention", "decode_attention_fused")):
         monkeypatch.setattr(ops, attr, counted(name, getattr(ops, attr)))
     folder, reqs, want = real_8b
     model = DecoderModel.from_folder(folder, dtype, "cuda")
@@ -116,10 +117,12 @@ def test_8b_layer_widths_under_every_cut(real_8b, dtype, monkeypatch) -> None:
     assert seen["norm"] > 0 and seen["normed"] == 0
     if dtype == torch.bfloat16:
         # (the only tcgen05 product here is the output head over a whole prompt's 150 rows: 1,188 tiles)
-        assert seen["mm"] > 100 and seen["tcgen05"] <= 2 and seen["fused_attention"] > 0
+        # four products a layer and step; the few rows' output, gate/up and down products are the rows kernel's in any case
+        assert seen["mm"] > 0 and seen["rows"] > 100 and seen["mm"] + seen["rows"] > 300
+        assert seen["tcgen05"] <= 2 and seen["fused_attention"] > 0
         assert seen["skinny"] > 0          # the output head of a few rows still streams through the skinny kernel
     else:
-        assert seen["mm"] == 0 and seen["tcgen05"] == 0
+        assert seen["mm"] == 0 and seen["rows"] == 0 and seen["tcgen05"] == 0
 
 
 def test_8b_layer_widths_long_prompt_on_the_tcgen05_products(real_8b, monkeypatch) -> None:
