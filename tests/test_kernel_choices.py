@@ -4,6 +4,7 @@ attention cuts a request."""
 from __future__ import annotations
 
 import pytest
+import torch
 
 from tinyserve_b200.kernels import ops
 
@@ -118,3 +119,18 @@ def test_expert_products_of_a_few_tokens_by_their_ctas_per_k() -> None:
                                               (17, 4, 2, 64, 4096, True), (17, 4, 2, 64, 4096, False)]:
         assert not take(tokens, experts, top, n, k, gated)
     assert take(1, 2, 2, 64, 64, True) and not take(1, 2, 2, 1 << 20, 64, True)
+
+
+def test_few_rows_of_large_matrices_by_the_shape_of_the_matrix() -> None:
+    """The tcgen05 kernel of a few rows takes the matrices that it was measured to stream faster than the library, whatever
+    kind of product they come from; single products on either side of each line."""
+    def take(m, n, k, swiglu=False, dtype=torch.bfloat16):
+        def like(*shape):
+            return torch.empty(1, dtype=dtype).expand(shape)          # (sizes and types decide: no memory behind it)
+        return ops.takes_rows_tcgen05(like(m, k), like(2 * n if swiglu else n, k), like(m, n), swiglu)
+
+    assert take(1, 4096, 4096) and take(16, 6144, 4096) and take(5, 10240, 5120) and take(1, 2048, 8192)
+    assert not take(17, 6144, 4096) and not take(1, 10248, 5120) and not take(1, 2040, 16384) and not take(1, 8192, 2560)
+    assert not take(1, 4096, 4088) and not take(1, 4096, 4100) and not take(1, 4096, 4096, dtype=torch.float32)
+    assert take(1, 12288, 4096, True) and take(16, 1024, 8192, True) and take(1, 16384, 512, True)
+    assert not take(1, 512, 16384, True) and not take(1, 32768, 256, True) and not take(17, 12288, 4096, True)

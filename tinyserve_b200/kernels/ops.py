@@ -784,22 +784,33 @@ SKINNY_MAX_WEIGHTS = 1 << 24
 ROWS_TCGEN05_MAX_ROWS = 16
 
 
-# Plain products of more output columns stay with the library: tests/test_real_sizes_gpu.py holds the decode rows of the 8B
-# widths to it (6,144 x 4,096 there). In a chain of products the two are level (one row / 16 rows, library against that
-# kernel: 6,144 x 4,096 11.5 / 12.3 against 11.5 / 12.1 us, 10,240 x 5,120 20.6 / 21.3 against 19.8 / 20.8), but inside a
-# decode step that kernel, which asks for its first weights while the norm before it runs, would be 4 us a layer faster (16
-# tokens at the 8B sizes 53.3 ms instead of 55.6). With SwiGLU the activation kernel is saved too, at any width.
-ROWS_TCGEN05_MAX_COLS = 5376
+# Where the matrix gives the kernel enough CTAs (a tile of 128 rows of w, K over up to eight of them) with enough to stream
+# each, and not more tiles than it balances better than the library. Measured on B200, library / that kernel, one row and
+# 16: behind a norm, 768 x 25,600 16 / 24 and 15 / 25 us, 1,536 x 16,384 19 / 20 and 18 / 20, 2,048 x 12,288 26 / 17 and 17 /
+# 16, 4,096 x 8,192 20 / 15 and 15 / 16, 5,120 x 8,192 18 / 18 and 20 / 18, 9,728 x 2,560 11 / 12 and 13 / 13, 65,536 x 1,024
+# 24 / 26 and 24 / 28; the qkv product of a recorded decode step of 8 layers, time a layer, 8,192 x 6,144 130 / 128 and 137 /
+# 133, 10,240 x 5,120 113 / 112 and 119 / 116, 12,288 x 4,096 80 / 81 and 85 / 86, 15,360 x 5,120 112 / 112 and 117 / 120;
+# 6,144 x 4,096, 36 layers, 85 / 86 and 91 / 91, 16 tokens of one request through the engine 55.8 / 53.6 ms.
+ROWS_TCGEN05_COLS = (2048, 10240)
+ROWS_TCGEN05_MIN_K = 3072
+# With SwiGLU the activation kernel is saved too: 1,024 x 8,192 21 / 11 and 14 / 11 us, 512 x 16,384 16 / 17 and 16 / 19,
+# 16,384 x 512 9.3 / 7.9 and 9.3 / 8.8, 32,768 x 256 9.7 / 10.4 and 9.9 / 12.3, 28,672 x 8,192 150 / 143 and 162 / 146.
+ROWS_TCGEN05_SWIGLU_MIN_COLS = 1024
+ROWS_TCGEN05_SWIGLU_MIN_K = 512
 
 
-def takes_rows_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
-    """Whether a bf16 product of ``x [M, K]`` with a matrix ``w [N, K]`` (or a merged gate and up matrix, ``out`` then half as
-    wide) goes to :func:`gemm_rows_tcgen05`: a few rows, a large matrix of few columns of output, and rows and pointers on
-    the 16-byte grid of its copies."""
-    return (x.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and x.shape[0] <= ROWS_TCGEN05_MAX_ROWS
-            and w.shape[0] * w.shape[1] >= SKINNY_MAX_WEIGHTS and w.shape[1] % 8 == 0
-            and (w.shape[0] <= ROWS_TCGEN05_MAX_COLS or out.shape[1] != w.shape[0])
-            and (x.data_ptr() | w.data_ptr() | out.data_ptr()) % 16 == 0)
+def takes_rows_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, swiglu: bool = False) -> bool:
+    """Whether a bf16 product of ``x [M, K]`` with ``w [N, K]`` (``swiglu``: a merged gate and up matrix, twice as many rows as
+    ``out`` has columns) goes to :func:`gemm_rows_tcgen05`: a few rows, a large matrix of a shape that suits it, rows and
+    pointers on the 16-byte grid of its copies."""
+    if not (x.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and x.shape[0] <= ROWS_TCGEN05_MAX_ROWS):
+        return False
+    n, k = w.shape
+    if swiglu:
+        suits = n >= 2 * ROWS_TCGEN05_SWIGLU_MIN_COLS and k >= ROWS_TCGEN05_SWIGLU_MIN_K
+    else:
+        suits = ROWS_TCGEN05_COLS[0] <= n <= ROWS_TCGEN05_COLS[1] and k >= ROWS_TCGEN05_MIN_K
+    return suits and n * k >= SKINNY_MAX_WEIGHTS and k % 8 == 0 and (x.data_ptr() | w.data_ptr() | out.data_ptr()) % 16 == 0
 
 
 def rows_tcgen05_slices(tiles: int, k: int) -> int:
@@ -959,7 +970,7 @@ def gemm_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, are
         _check(_fn("ts_gemm_skinny_swiglu")(_dev(x, "x"), _dev(w_gate_up, "w_gate_up"), _dev(out, "out"), m, inter, k,
                                             _stream()), "gemm_swiglu")
         return
-    if takes_rows_tcgen05(x, w_gate_up, out):
+    if takes_rows_tcgen05(x, w_gate_up, out, swiglu=True):
         gemm_rows_tcgen05(x, w_gate_up, out, swiglu=True)
         return
     tiles = tcgen05_tiles(m, inter, 128)
