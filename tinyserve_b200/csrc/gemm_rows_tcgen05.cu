@@ -1,10 +1,11 @@
-// out[M, N] = x[M, K] * w[N, K]^T for up to 64 rows and a large matrix, bf16, on the 5th-generation tensor cores with the
-// operands' places changed: 128 rows of w are the A operand, the rows of x (16, 32 or 64 of them, zeros beyond M) the B
-// operand, so that a tile of the accumulator is 128 columns of the output and no work is done for rows that are not there
-// beyond the next 16. Optionally the SwiGLU product of a merged matrix (64 gate and the 64 matching up rows make a tile).
+// out[M, N] = x[M, K] * w[N, K]^T for a few rows and a large matrix, bf16, on the 5th-generation tensor cores with the
+// operands' places changed: 128 rows of w are the A operand, 16 rows of x (zeros beyond M) the B operand, so that a tile of
+// the accumulator is 128 columns of the output and no work is done for rows that are not there beyond the next 16 (more than
+// 16 rows are several tiles, each of which reads w again; the library is faster there). Optionally the SwiGLU product of a
+// merged matrix (64 gate and the 64 matching up rows make a tile).
 //
 // Bound by the stream of the weights. A CTA takes one tile of w and a slice of K; TMA copies of 128 rows x 64 k (16 KB,
-// 128-byte swizzle) go through a ring of 4 or 5 stages, the first ones asked for before the wait for the kernels before
+// 128-byte swizzle) go through a ring of 5 stages, the first ones asked for before the wait for the kernels before
 // this one; one thread issues the MMAs. No register holds a weight, so what is in flight does not depend on occupancy, and
 // two CTAs fit an SM. The slices of a tile are a thread-block cluster: each CTA leaves its sums in shared memory (where
 // the ring was) and the cluster adds them up in the order of the slices through distributed shared memory, so there is no
@@ -18,25 +19,18 @@
 namespace ts {
 namespace cg = cooperative_groups;
 
-constexpr int GR_BN = 128, GR_BK = 64, GR_THREADS = 128, GR_MAX_SLICES = 8;
-constexpr uint32_t GR_W_BYTES = GR_BN * GR_BK * 2;
+constexpr int GR_BN = 128, GR_BK = 64, GR_XN = 16, GR_THREADS = 128, GR_MAX_SLICES = 8, GR_STAGES = 5;
+constexpr uint32_t GR_W_BYTES = GR_BN * GR_BK * 2, GR_STAGE = GR_W_BYTES + GR_XN * GR_BK * 2;
+constexpr uint32_t GR_TMEM_COLS = 32;       // the least there is; 16 are used
+constexpr size_t GR_SMEM = GR_STAGES * (size_t)GR_STAGE + 1024;
+static_assert(GR_BN * GR_XN * 4 <= GR_STAGES * (int)GR_STAGE, "the sums take the place of the ring");
 
-template <int XN>
-struct RowsTile {
-  static constexpr uint32_t X_BYTES = XN * GR_BK * 2, STAGE = GR_W_BYTES + X_BYTES;
-  static constexpr int STAGES = XN == 64 ? 4 : 5;
-  static constexpr uint32_t TMEM_COLS = XN < 32 ? 32 : XN;
-  static constexpr size_t SMEM = STAGES * (size_t)STAGE + 1024;
-  static_assert(GR_BN * XN * 4 <= STAGES * (int)STAGE, "the sums take the place of the ring");
-};
-
-template <int XN, bool SWIGLU>
+template <bool SWIGLU>
 __global__ void __launch_bounds__(GR_THREADS) gemm_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x,
                                                                        const __grid_constant__ CUtensorMap map_w,
-                                                                       bf16* __restrict__ out, int M, int N, int K,
+                                                                       bf16* __restrict__ out, int all_rows, int N, int K,
                                                                        int* __restrict__ error_flag) {
-  using Tile = RowsTile<XN>;
-  constexpr int STAGES = Tile::STAGES, OUT = SWIGLU ? GR_BN / 2 : GR_BN;
+  constexpr int STAGES = GR_STAGES, XN = GR_XN, OUT = SWIGLU ? GR_BN / 2 : GR_BN;
   // instruction descriptor: D = f32, A = B = bf16, both K-major, N = XN, M = 128
   constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(XN >> 3) << 17) | ((uint32_t)(GR_BN >> 4) << 24);
   extern __shared__ unsigned char smem_raw[];
@@ -49,6 +43,8 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_tcgen05_kernel(const __g
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slices = gridDim.y, slice = blockIdx.y, n0 = blockIdx.x * OUT;
+  const int m0 = blockIdx.z * XN, M = min(XN, all_rows - m0);       // this tile's rows
+  out += (size_t)m0 * N;
   const int all_kb = (K + GR_BK - 1) / GR_BK;
   const int kb0 = (int)((long long)all_kb * slice / slices), num_kb = (int)((long long)all_kb * (slice + 1) / slices) - kb0;
 
@@ -58,7 +54,7 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_tcgen05_kernel(const __g
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc(&tmem_base_slot, Tile::TMEM_COLS);
+  if (warp == 1) tmem_alloc(&tmem_base_slot, GR_TMEM_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -70,8 +66,8 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_tcgen05_kernel(const __g
     if (lane == 0 && !wait_test_unarmed()) {
       auto load_w = [&](int i) {
         const int s = i % STAGES;
-        unsigned char* a = ring + (size_t)s * Tile::STAGE;
-        mbar_expect_tx(&full_bar[s], Tile::STAGE);
+        unsigned char* a = ring + (size_t)s * GR_STAGE;
+        mbar_expect_tx(&full_bar[s], GR_STAGE);
         tma_load_2d(a, &map_w, &full_bar[s], (kb0 + i) * GR_BK, n0);
         if constexpr (SWIGLU) tma_load_2d(a + GR_W_BYTES / 2, &map_w, &full_bar[s], (kb0 + i) * GR_BK, N + n0);      // boxes of 64 rows
       };
@@ -85,7 +81,7 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_tcgen05_kernel(const __g
           if (!mbar_wait(&empty_bar[s], ((i / STAGES) & 1) ^ 1)) { *(volatile int*)&failed = 1; break; }
           load_w(i);
         }
-        tma_load_2d(ring + (size_t)s * Tile::STAGE + GR_W_BYTES, &map_x, &full_bar[s], (kb0 + i) * GR_BK, 0);
+        tma_load_2d(ring + (size_t)s * GR_STAGE + GR_W_BYTES, &map_x, &full_bar[s], (kb0 + i) * GR_BK, m0);
       }
       // after a failure: copies in flight may still land in this CTA's shared memory
       if (*(volatile int*)&failed)
@@ -101,7 +97,7 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_tcgen05_kernel(const __g
         ok = mbar_wait(&full_bar[s], (i / STAGES) & 1);
         if (!ok) { *(volatile int*)&failed = 1; break; }
         tc_fence_after();
-        const uint32_t a_addr = smem_u32(ring + (size_t)s * Tile::STAGE);
+        const uint32_t a_addr = smem_u32(ring + (size_t)s * GR_STAGE);
         const uint64_t adesc = sw128_desc(a_addr), bdesc = sw128_desc(a_addr + GR_W_BYTES);
 #pragma unroll
         for (int k = 0; k < GR_BK / 16; ++k) umma_bf16(tmem, adesc + 2 * k, bdesc + 2 * k, IDESC, (i | k) != 0);
@@ -120,26 +116,23 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_tcgen05_kernel(const __g
   tc_fence_after();
   __syncthreads();         // the ring is free: all its copies have arrived and all MMAs have read them
   float* sums = reinterpret_cast<float*>(ring);        // [row of x][row of the tile]
-#pragma unroll
-  for (int c = 0; c < XN; c += 32) {
-    if (c >= M) break;
+  {
     uint32_t v[32];
-    tmem_ld_32(tmem + ((uint32_t)(warp * 32) << 16) + c, v);
+    tmem_ld_32(tmem + ((uint32_t)(warp * 32) << 16), v);
 #pragma unroll
-    for (int j = 0; j < (XN < 32 ? XN : 32); ++j) {
-      const int m = c + j;
+    for (int m = 0; m < XN; ++m) {
       if (m < M) {
         if (!SWIGLU && slices == 1) {
-          if (n0 + (int)threadIdx.x < N) out[(size_t)m * N + n0 + threadIdx.x] = from_float<bf16>(__uint_as_float(v[j]));
+          if (n0 + (int)threadIdx.x < N) out[(size_t)m * N + n0 + threadIdx.x] = from_float<bf16>(__uint_as_float(v[m]));
         } else {
-          sums[m * GR_BN + threadIdx.x] = __uint_as_float(v[j]);
+          sums[m * GR_BN + threadIdx.x] = __uint_as_float(v[m]);
         }
       }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem, Tile::TMEM_COLS);
+  if (warp == 1) tmem_dealloc(tmem, GR_TMEM_COLS);
   if (!SWIGLU && slices == 1) return;
   cg::cluster_group cluster = cg::this_cluster();
   if (slices > 1) cluster.sync();
@@ -197,27 +190,19 @@ static bool rows_map(CUtensorMap* map, const void* base, int rows, int K, int bo
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, promotion, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int XN, bool SWIGLU>
+template <bool SWIGLU>
 static int launch_rows_tc(const void* x, const void* w, bf16* out, int M, int N, int K, int slices, int* error_flag, cudaStream_t stream) {
-  using Tile = RowsTile<XN>;
   constexpr int OUT = SWIGLU ? GR_BN / 2 : GR_BN;
   CUtensorMap mx, mw;
-  if (!rows_map(&mx, x, M, K, XN, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) ||
+  if (!rows_map(&mx, x, M, K, GR_XN, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) ||
       !rows_map(&mw, w, SWIGLU ? 2 * N : N, K, OUT, CU_TENSOR_MAP_L2_PROMOTION_L2_256B))
     return TS_ERR_UNSUPPORTED;
-  auto kern = gemm_rows_tcgen05_kernel<XN, SWIGLU>;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile::SMEM);
+  auto kern = gemm_rows_tcgen05_kernel<SWIGLU>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GR_SMEM);
   if (e != cudaSuccess) return (int)e;
-  const dim3 grid((N + OUT - 1) / OUT, slices);
-  if (slices == 1) return launch(kern, grid, GR_THREADS, Tile::SMEM, stream, mx, mw, out, M, N, K, error_flag);
-  return launch_cluster(kern, grid, GR_THREADS, Tile::SMEM, stream, dim3(1, slices), mx, mw, out, M, N, K, error_flag);
-}
-
-template <bool SWIGLU>
-static int dispatch_rows_tc(const void* x, const void* w, bf16* out, int M, int N, int K, int slices, int* error_flag, cudaStream_t stream) {
-  if (M <= 16) return launch_rows_tc<16, SWIGLU>(x, w, out, M, N, K, slices, error_flag, stream);
-  if (M <= 32) return launch_rows_tc<32, SWIGLU>(x, w, out, M, N, K, slices, error_flag, stream);
-  return launch_rows_tc<64, SWIGLU>(x, w, out, M, N, K, slices, error_flag, stream);
+  const dim3 grid((N + OUT - 1) / OUT, slices, (M + GR_XN - 1) / GR_XN);
+  if (slices == 1) return launch(kern, grid, GR_THREADS, GR_SMEM, stream, mx, mw, out, M, N, K, error_flag);
+  return launch_cluster(kern, grid, GR_THREADS, GR_SMEM, stream, dim3(1, slices), mx, mw, out, M, N, K, error_flag);
 }
 
 }  // namespace ts
@@ -232,6 +217,6 @@ extern "C" int ts_gemm_rows_tcgen05(const void* x, const void* w, void* out, int
   if (slices < 1 || slices > GR_MAX_SLICES) return TS_ERR_BAD_ARGUMENT;
   if (M > 64 || K <= 0 || K % 8 != 0 || slices > (K + GR_BK - 1) / GR_BK || error_flag == nullptr) return TS_ERR_UNSUPPORTED;
   if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15) return TS_ERR_UNSUPPORTED;        // copies of 16 bytes, stores of 8
-  return swiglu ? dispatch_rows_tc<true>(x, w, (bf16*)out, M, N, K, slices, error_flag, stream)
-                : dispatch_rows_tc<false>(x, w, (bf16*)out, M, N, K, slices, error_flag, stream);
+  return swiglu ? launch_rows_tc<true>(x, w, (bf16*)out, M, N, K, slices, error_flag, stream)
+                : launch_rows_tc<false>(x, w, (bf16*)out, M, N, K, slices, error_flag, stream);
 }

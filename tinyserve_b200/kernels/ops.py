@@ -780,7 +780,7 @@ SKINNY_MAX_ROWS = 16
 # 46 / 37.5 / 36.3 us; 16 rows 13.3 / 9.6 / 9.4, 38 / 22 / 20, 145 / 46 / 44, 54 / 38.0 / 37.4 us. At the 0.6B shapes
 # (4,096 x 1,024) the skinny kernel is ahead, 3.3 / 5.4 / 4.5 us.
 SKINNY_MAX_WEIGHTS = 1 << 24
-# Up to this many rows: at 64 rows the library is level or ahead (4,096 x 12,288 22 / 23 us, 4,096 x 4,096 10 / 12 us).
+# Up to this many rows, one tile of x; at 17, two tiles, the library takes 22 us where that kernel takes 35 (4,096 x 12,288).
 ROWS_TCGEN05_MAX_ROWS = 16
 
 
@@ -822,7 +822,8 @@ def rows_tcgen05_slices(tiles: int, k: int) -> int:
 
 def gemm_rows_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, swiglu: bool = False, slices: int = 0) -> None:
     """bf16 ``out[M, N] = x[M, K] @ w[N, K]^T`` (``swiglu``: ``silu(x Wgate^T) * (x Wup^T)``, ``w`` = ``2 N`` rows) for
-    ``M <= 64`` and ``K % 8 == 0``: weight tiles as the A operand of tcgen05.mma (``csrc/gemm_rows_tcgen05.cu``).
+    ``M <= 64`` (16 rows at a time) and ``K % 8 == 0``: weight tiles as the A operand of tcgen05.mma
+    (``csrc/gemm_rows_tcgen05.cu``).
     ``slices``: CTAs that share K (0: chosen by the size)."""
     m, k = x.shape
     n = out.shape[1]
