@@ -229,6 +229,39 @@ def test_replayed_prompt_portions_match_eager_and_plain(real) -> None:
                  plain_rows(pcfg, w16, toks, places), torch.bfloat16)
 
 
+def test_a_recorded_portion_has_a_form_for_each_context(real) -> None:
+    """2,048 tokens without context take one head a CTA, behind 2,048 others two: both are recorded, each portion replays
+    its own, and both give the bits of the step launched kernel by kernel."""
+    from tinyserve_b200.engine.step import StepEntry
+    from tinyserve_b200.kernels import ops
+    from tinyserve_b200.model import DecoderModel
+
+    model = DecoderModel.from_folder(real[0], torch.bfloat16, "cuda")
+    fleet = Fleet(model, buckets=[1], max_context=4096, pages=300, prefill_graphs=(2048,))
+    runner, cache = fleet.runner, fleet.cache
+    graph = runner.prefill_graphs[2048]
+    assert graph.form_of(2048) == (1,) and graph.form_of(4096) == (2,) and set(graph.graphs) == {(1,), (2,)}
+    toks = random_prompt(4096, VOCAB, 78)
+    rows = {}
+    for mode in ("own", "swapped", "eager"):
+        recordings = graph.graphs
+        if mode == "swapped":
+            graph.graphs = {(1,): recordings[2,], (2,): recordings[1,]}
+        elif mode == "eager":
+            runner.prefill_graphs = {}
+        req = cache.new_request()
+        rows[mode] = []
+        for a in (0, 2048):
+            cache.append(req, 2048)
+            rows[mode].append(runner.step([StepEntry(req, toks[a: a + 2048])]).clone())
+        cache.free(req)
+        graph.graphs = recordings
+    ops.check_device_errors()
+    assert runner.num_graph_steps == 4
+    for mode in ("own", "swapped"):
+        assert all(torch.equal(x, y) for x, y in zip(rows[mode], rows["eager"]))
+
+
 @pytest.mark.parametrize("ahead", [True, False])
 def test_engine_with_recorded_steps_launched_ahead(real, ahead) -> None:
     """Through ``Engine``: eight requests of different lengths, recorded decode steps (launched ahead

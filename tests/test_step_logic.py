@@ -60,3 +60,31 @@ def test_every_cut_gives_the_plain_logits(name: str, tmp_path: Path) -> None:
             assert len(got[rid]) == len(toks)
             for pos, row in got[rid].items():
                 torch.testing.assert_close(row, want[rid][pos], atol=2e-5, rtol=2e-5)
+
+
+def test_a_recorded_portion_replays_the_form_of_its_own_context() -> None:
+    """The recording of a prompt portion serves every context up to a limit: it is chosen by the request's own length, not
+    by the limit; a choice that was not recorded takes the recording that shares most of it."""
+    from tinyserve_b200.engine.step import PrefillGraph
+
+    class Recording:
+        def __init__(self, name: str) -> None:
+            self.name = name
+
+        def replay(self) -> None:
+            replayed.append(self.name)
+
+    replayed: list[str] = []
+    g = object.__new__(PrefillGraph)
+    g.tokens, g.layouts = 2048, {(16, 8, 0): 2, (16, 16, 0): 1}
+    assert g.form_of(2048) == (1, 1) and g.form_of(9001) == (2, 1)
+    g.graphs = {(1, 1): Recording("one"), (2, 1): Recording("two")}
+    for total in (2048, 9001, 2100, 8192):
+        g.replay(total)
+    assert replayed == ["one", "two", "one", "two"]
+    g.layouts = {(16, 8, 0): 2, (32, 8, 0): 2, (16, 16, 0): 1}
+    g.graphs = {(1, 1, 1): Recording("a"), (2, 2, 1): Recording("b")}
+    assert g.form_of(2048) == (1, 2, 1)
+    g.replay(9001)
+    g.replay(2048)
+    assert replayed[4] == "b" and replayed[5] in "ab"

@@ -179,7 +179,14 @@ class PrefillGraph:
     a long prompt, as chunked prefill cuts them) on top of any context up to ``max_context``.
     A step of a few thousand tokens launches some 250 kernels whose host-side cost is as long
     as their run time at small model sizes; replayed from a recording it costs one launch. The
-    logits of the portion's last token are always computed (a mid-prompt portion ignores them)."""
+    logits of the portion's last token are always computed (a mid-prompt portion ignores them).
+
+    The prompt attention has two forms, one head a CTA or two, with the same results; which is faster
+    depends on the context (2,048 tokens of 16 / 8 heads: one head without context, 36 against 45 us a
+    layer; two at 9,001 positions, 183 against 160). So the step is recorded once for every choice that
+    some context up to ``max_context`` makes, and a step replays the one that its own context makes."""
+
+    MOST_FORMS = 4        # recordings; layouts whose choices change at many contexts share the nearest
 
     def __init__(self, runner: "ModelRunner", tokens: int, max_context: int) -> None:
         self.tokens = t = tokens
@@ -215,44 +222,63 @@ class PrefillGraph:
             buf[st] = g.pad_page
         self.dev.copy_(self.host)
         self._arange = np.arange(t, dtype=np.int64)
-        self.graph: torch.cuda.CUDAGraph | None = None
+        self.layouts: dict[tuple[int, int, int], int] = {}                    # of the model's prompt attention
+        self.graphs: dict[tuple[int, ...], torch.cuda.CUDAGraph] = {}         # heads a CTA of each layout -> recording
         self.logits: torch.Tensor | None = None
 
-    def context(self, runner: "ModelRunner") -> StepContext:
+    def form_of(self, total: int) -> tuple[int, ...]:
+        """Heads a CTA of each layout when the request holds ``total`` tokens after the step."""
+        return tuple(ops.prefill_heads_per_cta((self.tokens,), (total,), *layout) for layout in self.layouts)
+
+    def context(self, runner: "ModelRunner", total: int) -> StepContext:
+        """``total``: the tokens of the request that the kernels' forms are chosen for."""
         t, dev, w = self.tokens, self.dev, self.width
         cache = runner.cache
         kv = {g.index: KVGroupContext(g.page_size, dev[st].view(1, w), dev[ss])
               for g, ss, st in zip(cache.groups, self.s_slots, self.s_tables)}
         cap = w * cache.page_size
         return StepContext(
-            num_tokens=t, num_seqs=1, query_lens=[t], context_lens=[cap],
+            num_tokens=t, num_seqs=1, query_lens=[t], context_lens=[total],
             tokens=dev[self.s_tokens], positions=dev[self.s_pos], cu_query_lens=dev[self.s_cu],
             context_lens_dev=dev[self.s_ctx], decode_seqs=dev[self.s_dec], prefill_seqs=dev[self.s_pre],
             num_decode=0, num_prefill=1, max_query_len=t, max_context_len=cap, kv=kv,
             state_slots=dev[self.s_state] if cache.has_state else None, state_slots_host=[0],
-            arena=self.arena, dtype=runner.model.dtype, recorded=True)
+            arena=self.arena, dtype=runner.model.dtype, recorded=True, prompt_heads=self.layouts)
 
     def record(self, runner: "ModelRunner") -> None:
         model, caches = runner.model, runner.cache.entries
 
-        def run() -> torch.Tensor:
+        def run(total: int) -> torch.Tensor:
             self.arena.begin_step()
             with ops.stream_scope():
-                return model.forward(self.context(runner), caches, self.dev[self.s_rows], 1)
+                return model.forward(self.context(runner, total), caches, self.dev[self.s_rows], 1)
 
-        run()
-        run()
-        reserved = self.arena.reserved_bytes
-        torch.cuda.synchronize()
-        graph = torch.cuda.CUDAGraph()
-        before = ops.launch_count
-        with torch.cuda.graph(graph):
-            logits = run()
-        self.num_kernels = ops.launch_count - before
-        ops.launch_count = before          # recorded, not run
-        if self.arena.reserved_bytes != reserved:
-            raise RuntimeError("scratch memory moved while a prefill graph was being recorded")
-        self.graph, self.logits = graph, logits
+        run(self.tokens)
+        cap = self.width * runner.cache.page_size
+        forms: dict[tuple[int, ...], int] = {}                    # a choice -> a context that makes it
+        for total in [*range(self.tokens, cap, 128), cap]:
+            forms.setdefault(self.form_of(total), total)
+        for form, total in list(forms.items())[: self.MOST_FORMS]:
+            run(total)
+            reserved = self.arena.reserved_bytes
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            before = ops.launch_count
+            with torch.cuda.graph(graph):
+                logits = run(total)
+            self.num_kernels = ops.launch_count - before
+            ops.launch_count = before          # recorded, not run
+            if self.arena.reserved_bytes != reserved or (self.logits is not None and self.logits.data_ptr() != logits.data_ptr()):
+                raise RuntimeError("scratch memory moved while a prefill graph was being recorded")
+            self.graphs[form], self.logits = graph, logits
+
+    def replay(self, total: int) -> None:
+        """Launch the recording for a request that holds ``total`` tokens, the step's included."""
+        form = self.form_of(total)
+        graph = self.graphs.get(form)
+        if graph is None:
+            graph = self.graphs[max(self.graphs, key=lambda f: sum(a == b for a, b in zip(f, form)))]
+        graph.replay()
 
     def fill(self, runner: "ModelRunner", entry: StepEntry) -> None:
         self.copied.synchronize()          # the last copy must have left the host buffer
@@ -492,7 +518,7 @@ class ModelRunner:
         pgraph = self._prefill_graph_for(entries, want)
         if pgraph is not None:
             pgraph.fill(self, entries[0])
-            pgraph.graph.replay()
+            pgraph.replay(entries[0].cache.num_tokens)
             ops.launch_count += pgraph.num_kernels
             self.num_steps += 1
             self.num_graph_steps += 1

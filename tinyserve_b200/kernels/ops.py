@@ -421,18 +421,30 @@ def _one_head_or_two(query_lens: tuple[int, ...], context_lens: tuple[int, ...],
     return 1 if not tiles or _prefill_cycles(tiles, num_heads, 1) <= _prefill_cycles(tiles, num_heads, 2) else 2
 
 
-def _prefill_heads_per_cta(ctx: Any, num_heads: int, num_kv_heads: int, window: int = 0) -> int:
+def prefill_heads_per_cta(query_lens: Sequence[int], context_lens: Sequence[int], num_heads: int, num_kv_heads: int,
+                          window: int = 0) -> int:
     """Two query heads of a kv group in a CTA share its key and value tiles and keep the tensor core busier, but make half as
     many CTAs, twice as long: whichever is estimated to end first (by the step's lengths alone, so the layers of a step, and
-    steps alike, share the estimate). Measured on B200, 16 / 8 heads of 128, one head / two: 512 tokens 15 / 17 us, 2,048
-    tokens 40 / 46, 2,048 at 4,096 positions 84 / 80, at 9,001 positions 188 / 158, 3,072 tokens 75 / 64, 8,192 tokens
-    357 / 266, seven prompts of 290 tokens 31 / 25."""
+    steps alike, share the estimate). Measured on B200, 16 / 8 heads of 128, one head / two: 512 tokens 13 / 18 us, 2,048
+    tokens 36 / 45, 2,048 at 4,096 positions 79 / 78, at 9,001 positions 183 / 160, 3,072 tokens 70 / 61, 8,192 tokens
+    350 / 273, seven prompts of 290 tokens 31 / 25. The same constants serve every layout the kernel takes: over 280 steps
+    with 16, 32 and 64 heads of 128 and 4 to 32 of 64, groups of 2, 4 and 8, windows or none, the choice took as long as
+    the faster form to within the noise for heads of 128 and 0.3 % longer on average (17 % at worst) for heads of 64."""
     if (num_heads // num_kv_heads) % 2:
         return 1
     if PREFILL_HEADS_PER_CTA:
         return PREFILL_HEADS_PER_CTA
+    return _one_head_or_two(tuple(query_lens), tuple(context_lens), num_heads, window)
+
+
+def _prefill_heads_per_cta(ctx: Any, num_heads: int, num_kv_heads: int, window: int = 0) -> int:
+    """:func:`prefill_heads_per_cta` of a step, noted in its ``prompt_heads`` if that is asked for."""
     contexts = getattr(ctx, "context_lens", None) or ctx.query_lens      # (a caller of the kernel alone may not know them here)
-    return _one_head_or_two(tuple(ctx.query_lens), tuple(contexts), num_heads, window)
+    heads = prefill_heads_per_cta(ctx.query_lens, contexts, num_heads, num_kv_heads, window)
+    notes = getattr(ctx, "prompt_heads", None)
+    if notes is not None:
+        notes[num_heads, num_kv_heads, window] = heads
+    return heads
 
 
 def decode_splits(num_decode: int, num_kv_heads: int, group: int, max_context_len: int) -> int:
@@ -551,7 +563,7 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
                 _dev(ctx.context_lens_dev, "context_lens", torch.int32),
                 _dev(ctx.prefill_seqs, "prefill_seqs", torch.int32), num_prefill, ctx.max_query_len,
                 hq, hkv, d, page_size, float(scale), int(window),
-                _prefill_heads_per_cta(ctx, hq, hkv, int(window)),
+                1 if chunk or maps == 2 else _prefill_heads_per_cta(ctx, hq, hkv, int(window)),       # (those have one form)
                 _error_word(q.device).data_ptr(), _opt(sinks, "sinks", torch.float32), keep_first, int(chunk), maps,
                 factor.data_ptr() if maps == 2 else None, float(mult) if maps == 2 else 1.0, float(mix_eps) if maps == 2 else 0.0, _stream()),
                 "prefill_attention_tcgen05")
