@@ -159,6 +159,7 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
   const int head0 = (int)blockIdx.x * NQ;                     // PAIR: the (head, map) pairs 2 head and 2 head + 1
   const int kvh = head0 / (a.num_heads / a.num_kv_heads);
 
+  pdl_trigger();
   unsigned char* smem = (unsigned char*)(((uintptr_t)fa_raw + 1023) & ~(uintptr_t)1023);
   // two heads: known to the compiler to be the same in the whole warp, so that the MMA warp's operands are (umma_bf16_by)
   const int warp = NQ == 1 ? (int)(threadIdx.x >> 5) : __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -172,12 +173,8 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
     failed_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == FA_SOFTMAX_WARPS + 2 * PW) tmem_alloc(&tmem_base_slot, L::TMEM_COLS);
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = tmem_base_slot;
-  pdl_trigger();   // behind the allocation (tmem_alloc)
+  uint32_t tmem_base = 0;
   pdl_wait();      // q and the cache rows of this step are written by the kernels before
 
   if (warp < FA_SOFTMAX_WARPS) {
@@ -213,6 +210,8 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
       __syncwarp();
       if (lane == 0) mbar_arrive(&q_ready);
     }
+    tmem_meet<5, (FA_SOFTMAX_WARPS + 1) * 32>();
+    tmem_base = tmem_base_slot;
     // The HS warps of a row quarter meet twice per exchange (named barrier 1 + its index, 32 HS threads):
     // after writing and after reading. Each also says whether its waits have held, so that they stop
     // together: a warp that left alone would leave its partner at the barrier.
@@ -484,6 +483,9 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
     }
   } else {
     // =========================================================== MMA issuer
+    tmem_alloc(&tmem_base_slot, L::TMEM_COLS);
+    tmem_meet<5, (FA_SOFTMAX_WARPS + 1) * 32>();
+    tmem_base = tmem_base_slot;
     bool ok = fa_warp_wait(&q_ready, 0, failed);
     // One head: a branch on the lane, whose 1,700 cycles a tile the softmax hides (issued by the converged warp instead, prompts
     // of up to 2,048 tokens took 1 us longer). Two heads: the converged warp.
@@ -627,7 +629,7 @@ static int launch_fa(const AttnArgs& a, long long cache_rows, int max_query_len,
   const CUtensorMap* mk = fa_cache_map(a.k_cache, cache_rows, L::D, BR);
   const CUtensorMap* mv = fa_cache_map(a.v_cache, cache_rows, L::D, BR);
   if (mk == nullptr || mv == nullptr) return TS_ERR_UNSUPPORTED;
-  const size_t smem = (size_t)L::TOTAL + 1024;
+  const size_t smem = L::TOTAL + 1024 > TMEM_ALONE_SMEM ? L::TOTAL + 1024 : TMEM_ALONE_SMEM;
   auto kern = prefill_attn_tc_kernel<D64, BR, NQ, PAIR, CHUNKED>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;

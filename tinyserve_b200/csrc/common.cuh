@@ -138,11 +138,10 @@ static inline int launch_status() {
 // ---- programmatic dependent launch
 // Kernels of one step form a chain on one stream. When this switch is on they are launched so
 // that the next kernel's CTAs may be scheduled while the previous kernel is still draining:
-// every kernel calls pdl_trigger() at its start (one that allocates tensor memory: behind the
-// allocation, see tmem_alloc) and pdl_wait() before it reads anything an
-// earlier kernel wrote or writes anything at all. pdl_wait() returns once every earlier kernel
-// of the chain has finished and its writes are visible, so ordering is what it was; only the
-// launch latency and the part of a kernel that needs no input (index arithmetic, prefetch of
+// every kernel calls pdl_trigger() at its start and pdl_wait() before it reads anything an
+// earlier kernel wrote, writes anything at all or allocates tensor memory (tmem_alloc).
+// pdl_wait() returns once every earlier kernel of the chain has finished and its writes are
+// visible, so ordering is what it was; only the launch latency and the part of a kernel that needs no input (index arithmetic, prefetch of
 // weights) overlap the predecessor. Off, the two calls do nothing.
 // The switch is a mask of kernel classes, so that the overlap can be limited to the kernels that
 // gain from it.

@@ -23,6 +23,7 @@ constexpr int GR_BN = 128, GR_BK = 64, GR_XN = 16, GR_THREADS = 128, GR_MAX_SLIC
 constexpr uint32_t GR_W_BYTES = GR_BN * GR_BK * 2, GR_STAGE = GR_W_BYTES + GR_XN * GR_BK * 2;
 constexpr uint32_t GR_TMEM_COLS = 32;       // the least there is; 16 are used
 constexpr size_t GR_SMEM = GR_STAGES * (size_t)GR_STAGE + 1024;
+static_assert(GR_SMEM >= TMEM_WAITING_SMEM, "beside no other kernel's CTA with tensor memory");
 static_assert(GR_BN * GR_XN * 4 <= GR_STAGES * (int)GR_STAGE, "the sums take the place of the ring");
 
 template <bool SWIGLU>
@@ -41,6 +42,7 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_tcgen05_kernel(const __g
   __shared__ uint32_t tmem_base_slot;
   __shared__ int failed;
 
+  pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slices = gridDim.y, slice = blockIdx.y, n0 = blockIdx.x * OUT;
   const int m0 = blockIdx.z * XN, M = min(XN, all_rows - m0);       // this tile's rows
@@ -54,12 +56,11 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_tcgen05_kernel(const __g
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc(&tmem_base_slot, GR_TMEM_COLS);
+  if (warp == 1) tmem_alloc(&tmem_base_slot, GR_TMEM_COLS);      // in front of the wait: see TMEM_WAITING_SMEM
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_slot;
-  pdl_trigger();           // behind the allocation (tmem_alloc)
 
   if (warp == 0) {
     // ---------------- TMA producer (one lane)

@@ -209,9 +209,15 @@ __global__ void __launch_bounds__(TG_THREADS) gemm_tcgen05_kernel(const __grid_c
   __shared__ uint32_t tmem_base_slot;
   __shared__ int failed;
 
+  pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   static_assert(!SWIGLU || BN == 256, "the fused activation pairs 128 gate with 128 up columns");
   constexpr int BN_OUT = SWIGLU ? BN / 2 : BN;          // output columns per tile
+  const bool grouped = grp.tile_expert != nullptr;
+  if (grouped) pdl_wait();            // the list of tiles is the work of the kernels before this one
+  const int tiles_m = grouped ? *(const volatile int*)grp.num_tiles : (M + TG_BM - 1) / TG_BM, tiles_n = (N + BN_OUT - 1) / BN_OUT;
+  const int num_tiles = tiles_m * tiles_n;
+  const int num_kb = (K + TG_BK - 1) / TG_BK;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -219,17 +225,8 @@ __global__ void __launch_bounds__(TG_THREADS) gemm_tcgen05_kernel(const __grid_c
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc(&tmem_base_slot, TMEM_COLS);
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = tmem_base_slot;
-  pdl_trigger();                      // behind the allocation (tmem_alloc)
-  const bool grouped = grp.tile_expert != nullptr;
-  if (grouped) pdl_wait();            // the list of tiles is the work of the kernels before this one
-  const int tiles_m = grouped ? *(const volatile int*)grp.num_tiles : (M + TG_BM - 1) / TG_BM, tiles_n = (N + BN_OUT - 1) / BN_OUT;
-  const int num_tiles = tiles_m * tiles_n;
-  const int num_kb = (K + TG_BK - 1) / TG_BK;
+  uint32_t tmem_base = 0;
 
   if (warp == 0) {
     // ---------------- TMA producer (one lane)
@@ -276,6 +273,10 @@ __global__ void __launch_bounds__(TG_THREADS) gemm_tcgen05_kernel(const __grid_c
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (one lane)
+    pdl_wait();
+    tmem_alloc(&tmem_base_slot, TMEM_COLS);
+    tmem_meet<1, TG_THREADS - 32>();
+    tmem_base = tmem_base_slot;
     if (lane == 0) {
       int it = 0, t = 0;
       for (int tile = blockIdx.x; tile < num_tiles && !failed; tile += gridDim.x, ++t) {
@@ -304,6 +305,8 @@ __global__ void __launch_bounds__(TG_THREADS) gemm_tcgen05_kernel(const __grid_c
   } else {
     // ---------------- epilogue: warps 2..5; warp w may touch TMEM lanes 32 (w % 4) .. + 31
     pdl_wait();      // out may be written only once the kernel before this one is done
+    tmem_meet<1, TG_THREADS - 32>();
+    tmem_base = tmem_base_slot;
     const int quad = warp & 3;
     int t = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++t) {
@@ -357,9 +360,11 @@ __global__ void __launch_bounds__(TG_THREADS) gemm_tcgen05_pair_kernel(const __g
   __shared__ __align__(8) uint64_t empty_bar[STAGES];     // in each CTA: the MMAs have read this stage
   __shared__ __align__(8) uint64_t acc_full[2];           // in each CTA: the accumulator is complete
   __shared__ __align__(8) uint64_t acc_empty[2];          // used in the even CTA: 2 x 4 epilogue warps are done with it
+  __shared__ __align__(8) uint64_t peer_ready;            // used in the even CTA: the odd one has its tensor memory
   __shared__ uint32_t tmem_base_slot;
   __shared__ int failed;
 
+  pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();
   const bool leader = rank == 0;
@@ -371,16 +376,13 @@ __global__ void __launch_bounds__(TG_THREADS) gemm_tcgen05_pair_kernel(const __g
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
+    mbar_init(&peer_ready, 1);
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc_pair(&tmem_base_slot, TMEM_COLS);
-  tc_fence_before();
   __syncthreads();
-  cluster_sync_all();      // both CTAs' barriers and tensor memory exist before either uses the other's
-  tc_fence_after();
-  const uint32_t tmem_base = tmem_base_slot;
-  pdl_trigger();           // behind the allocation (tmem_alloc)
+  cluster_sync_all();      // both CTAs' barriers exist before either uses the other's
+  uint32_t tmem_base = 0;
   const uint32_t full0 = smem_of_cta(&full_bar[0], 0), acc_empty0 = smem_of_cta(&acc_empty[0], 0);
 
   if (warp == 0) {
@@ -421,8 +423,14 @@ __global__ void __launch_bounds__(TG_THREADS) gemm_tcgen05_pair_kernel(const __g
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (one lane of the even CTA)
+    pdl_wait();
+    tmem_alloc_pair(&tmem_base_slot, TMEM_COLS);
+    tmem_meet<1, TG_THREADS - 32>();
+    tmem_base = tmem_base_slot;
+    if (lane == 0 && !leader) mbar_arrive_cluster(smem_of_cta(&peer_ready, 0));
     if (lane == 0 && leader) {
       int it = 0, t = 0;
+      if (!mbar_wait(&peer_ready, 0)) failed = 1;
       for (int tile = pair; tile < num_tiles && !failed; tile += num_pairs, ++t) {
         const int b = t & 1;
         if (!mbar_wait(&acc_empty[b], ((t >> 1) & 1) ^ 1)) { failed = 1; break; }
@@ -445,6 +453,8 @@ __global__ void __launch_bounds__(TG_THREADS) gemm_tcgen05_pair_kernel(const __g
   } else {
     // ---------------- epilogue: warps 2..5 of each CTA drain their own CTA's tensor memory
     pdl_wait();
+    tmem_meet<1, TG_THREADS - 32>();
+    tmem_base = tmem_base_slot;
     const int quad = warp & 3;
     int t = 0;
     for (int tile = pair; tile < num_tiles; tile += num_pairs, ++t) {
@@ -503,7 +513,8 @@ template <int BN, int STAGES, typename TOut, int SWIGLU = false>
 static int launch_tc(const CUtensorMap& mx, const CUtensorMap& mw, TOut* out, int M, int N, int K, int* error_flag,
                      cudaStream_t stream, float act_limit = 0.f, const GemmGroup& grp = GemmGroup(), int max_row_tiles = 0,
                      const bf16* act_bias = nullptr) {
-  const size_t smem = (size_t)STAGES * (TG_BM + BN) * TG_BK * 2 + 1024;
+  constexpr size_t smem = (size_t)STAGES * (TG_BM + BN) * TG_BK * 2 + 1024;
+  static_assert(smem >= TMEM_ALONE_SMEM, "no CTA that waits with tensor memory of its own fits beside one");
   auto kern = gemm_tcgen05_kernel<BN, STAGES, TOut, SWIGLU>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
@@ -517,7 +528,8 @@ static int launch_tc(const CUtensorMap& mx, const CUtensorMap& mw, TOut* out, in
 template <int STAGES, typename TOut, int SWIGLU>
 static int launch_tc_pair(const CUtensorMap& mx, const CUtensorMap& mw, TOut* out, int M, int N, int K, int* error_flag,
                           cudaStream_t stream, float act_limit = 0.f, const bf16* act_bias = nullptr) {
-  const size_t smem = (size_t)STAGES * (TG_BM + 128) * TG_BK * 2 + 1024;
+  constexpr size_t smem = (size_t)STAGES * (TG_BM + 128) * TG_BK * 2 + 1024;
+  static_assert(smem >= TMEM_ALONE_SMEM, "no CTA that waits with tensor memory of its own fits beside one");
   auto kern = gemm_tcgen05_pair_kernel<STAGES, TOut, SWIGLU>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;

@@ -30,14 +30,27 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
       ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
 }
 // Tensor memory of an SM is shared by the CTAs on it, and an allocation that does not fit blocks, without a bound, until
-// another CTA frees its columns. So a kernel lets the kernels behind it start (pdl_trigger) only once all its threads know
-// that the CTA has its columns: a CTA that holds columns while it waits for an earlier kernel (pdl_wait) then never keeps a
-// CTA of that kernel from its own, because all of those had theirs before it was started. (With the trigger in front, a
-// prompt attention with heads of 64, 512 columns and 112 KB of shared memory, and a product of a few rows behind it, 91 KB,
-// fit one SM and could each have waited for the other.)
+// another CTA frees its columns. A CTA that is started early (pdl_trigger) and holds columns while it waits for the kernels
+// before it (pdl_wait) could keep a CTA of one of these from its own, each waiting for the other. Two rules exclude that:
+//  * A kernel allocates behind its wait; the MMA warp does it while the first tiles of x, q or the keys, which it needs too,
+//    are on their way. The warps that use the columns meet it at a named barrier (tmem_meet), after which they may read the
+//    address. (2,048 prompt tokens behind 7,000, 28 layers: 6.75 ms; allocated in front of the wait, with the trigger behind
+//    the allocation, 6.89.)
+//  * The product of a few rows, whose MMAs follow the wait at once (1.3 us more a launch otherwise), allocates in front of it.
+//    It takes TMEM_WAITING_SMEM of shared memory at least and the other kernels that allocate TMEM_ALONE_SMEM at least, so
+//    it is never on an SM with one of their CTAs; as many as fit of its own kind find their 32 columns.
+constexpr size_t TMEM_WAITING_SMEM = 91 * 1024, TMEM_ALONE_SMEM = 138 * 1024;
+static_assert(TMEM_WAITING_SMEM + TMEM_ALONE_SMEM > 228 * 1024, "the shared memory of an SM");
 __device__ __forceinline__ void tmem_alloc(uint32_t* result_in_smem, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(result_in_smem)), "r"(cols) : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+template <int BARRIER, int THREADS>
+__device__ __forceinline__ void tmem_meet() {
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  asm volatile("bar.sync %0, %1;" ::"n"(BARRIER), "n"(THREADS) : "memory");
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
