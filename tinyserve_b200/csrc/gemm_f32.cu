@@ -16,12 +16,14 @@
 // row, 64 x 64 tiles of all K before / now: 4,096 x 1,024 70 / 11 us, 1,024 x 3,072 205 / 8 us, the head 92 us (6.8 TB/s).
 //
 // More rows: bound by the multiply-adds and, below some hundred rows, by the latency of the chains. Register tiles of
-// 4 x 4 outputs a thread, 32 x 64 a CTA, operands in shared memory as [row][32 k] read in 16-byte words (rows a thread owns lie a stride apart, so that eight neighbouring threads read
-// eight different groups of banks), three cp.async stages. Where the tiles are too few for the machine, the four
-// groups of K go to the four CTAs of a cluster, which leave their sums in shared memory; each then adds up its
-// share of the tile through distributed shared memory. Measured, one kernel of 64 x 64 tiles for all sizes (which these
-// replace) / now: 45 rows of 4,096 x 1,024 76 / 20 us, 64 rows of 1,024 x 3,072 221 / 24 us, 190 rows of 6,144 x 1,024 115 /
-// 67 us; many rows reach 38 TFLOP/s. Steps of 16 k, with a division per copy, took 25, 40 and 80 us. Tiles of 64 x 64 and
+// 4 x 4 outputs a thread, 32 x 64 a CTA, operands in shared memory as [row][32 k] read in 16-byte words (rows a thread
+// owns lie a stride apart, so that eight neighbouring threads read eight different groups of banks), three cp.async
+// stages. Where the tiles are too few for the machine, the four groups of K go to the four CTAs of a cluster, which leave
+// their sums in shared memory; each then adds up its share of the tile through distributed shared memory. Where parts are
+// no whole steps of 32 k, a step runs over their ends (a part of its own steps multiplied mostly zeros: 1,000 rows of
+// 10,000 x 100 298 us, of 512 x 64 24 us). Measured, one kernel of 64 x 64 tiles for all sizes (which these replace) /
+// now: 45 rows of 4,096 x 1,024 76 / 20 us, 64 rows of 1,024 x 3,072 221 / 24 us, 190 rows of 6,144 x 1,024 115 / 67 us,
+// 1,000 rows of 10,000 x 100 86 / 80 us, of 512 x 64 6.7 / 6.8; many rows reach 38 TFLOP/s. Tiles of 64 x 64 and
 // 128 x 128 (8 outputs a thread and side) were no faster at any of 1 to 600 rows: they leave too few warps on an SM.
 #define TS_PDL_CLASS PDL_OTHER
 #include <cooperative_groups.h>
@@ -52,7 +54,8 @@ struct F32Rows {
   static constexpr int STAGE = FP_PARTS * ROWS * FR_STRIDE + MT * FP_PARTS * FR_SLAB;     // floats
 };
 
-template <int MT, int R>
+// SHORT: a part is shorter than a slab.
+template <int MT, int R, bool SHORT>
 __global__ void __launch_bounds__(FR_THREADS) gemm_f32_rows_kernel(const float* x, const float* __restrict__ w, float* out,
                                                                   int M, int N, int K) {
   using Rows = F32Rows<MT, R>;
@@ -114,8 +117,7 @@ __global__ void __launch_bounds__(FR_THREADS) gemm_f32_rows_kernel(const float* 
     const float* stage = smem + (s % FR_STAGES) * Rows::STAGE;
     const float* ws = stage + (part * ROWS + row) * FR_STRIDE;
     const float* xs = stage + FP_PARTS * ROWS * FR_STRIDE + part * FR_SLAB;
-#pragma unroll
-    for (int i = 0; i < FR_SLAB; i += 4) {
+    auto quad = [&](int i) {
       float4 b[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) b[r] = *reinterpret_cast<const float4*>(ws + r * 8 * FR_STRIDE + i);
@@ -130,6 +132,12 @@ __global__ void __launch_bounds__(FR_THREADS) gemm_f32_rows_kernel(const float* 
           acc[r][m] = fmaf(a.w, b[r].w, acc[r][m]);
         }
       }
+    };
+    if constexpr (SHORT) {
+      for (int i = 0; i < len; i += 4) quad(i);
+    } else {
+#pragma unroll
+      for (int i = 0; i < FR_SLAB; i += 4) quad(i);
     }
   }
 #pragma unroll
@@ -148,128 +156,160 @@ __global__ void __launch_bounds__(FR_THREADS) gemm_f32_rows_kernel(const float* 
   }
 }
 
-template <int MT, int R>
-static int launch_rows(const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
+template <int MT, int R, bool SHORT>
+static int launch_rows_form(const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
   using Rows = F32Rows<MT, R>;
   const int most = FR_STAGES * Rows::STAGE * (int)sizeof(float);
   static bool ready[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64 || !ready[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<MT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<MT, R, SHORT>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (e != cudaSuccess) return (int)e;
     if (dev < 64) ready[dev] = true;
   }
   // fewer slabs than stages: room for those alone, so that more CTAs fit an SM
   const int slabs = (f32_part_length(K) + FR_SLAB - 1) / FR_SLAB, smem = slabs < FR_STAGES ? most / FR_STAGES * slabs : most;
   const dim3 grid((N + Rows::ROWS - 1) / Rows::ROWS, (M + MT - 1) / MT);
-  return launch(gemm_f32_rows_kernel<MT, R>, grid, FR_THREADS, smem, stream, x, w, out, M, N, K);
+  return launch(gemm_f32_rows_kernel<MT, R, SHORT>, grid, FR_THREADS, smem, stream, x, w, out, M, N, K);
+}
+
+template <int MT, int R>
+static int launch_rows(const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
+  return f32_part_length(K) < FR_SLAB ? launch_rows_form<MT, R, true>(x, w, out, M, N, K, stream)
+                                      : launch_rows_form<MT, R, false>(x, w, out, M, N, K, stream);
 }
 
 // -------------------------------------------------------------------------------------------------- more rows
 constexpr int FT_M = 32, FT_N = 64, FT_OWN = 4, FT_K = 32, FT_STRIDE = FT_K + 4, FT_STAGES = 3;
 constexpr int FT_THREADS = (FT_M / FT_OWN) * (FT_N / FT_OWN), FT_STAGE = (FT_M + FT_N) * FT_STRIDE;     // floats
 
-template <int SPLIT>
-__global__ void __launch_bounds__(FT_THREADS) gemm_f32_tile_kernel(const float* x, const float* __restrict__ w, float* out,
+// WHOLE: parts are whole steps of 32 k; else a step may hold the ends of several.
+template <int SPLIT, bool WHOLE>
+__global__ void __launch_bounds__(FT_THREADS, 4) gemm_f32_tile_kernel(const float* x, const float* __restrict__ w, float* out,
                                                                    int M, int N, int K) {
   static_assert(SPLIT == 1 || SPLIT == 4, "all groups of K in one CTA, or one in each");
   constexpr int BM = FT_M, BN = FT_N, TM = FT_OWN, TN = FT_OWN;
   constexpr int THREADS = FT_THREADS, GROUPS = 4 / SPLIT, OUTS = TM * TN;
   extern __shared__ float smem[];
-  float* kept = smem + FT_STAGES * FT_STAGE;           // [output of a thread][thread]
+  float* kept = smem + FT_STAGES * FT_STAGE;           // SPLIT 4: [output of a thread][thread]
   pdl_trigger();
   const int tid = threadIdx.x;
   const int tx = tid % (BN / TN), ty = tid / (BN / TN);
   const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
-  const int len = f32_part_length(K), steps = (len + FT_K - 1) / FT_K;    // steps of a part
-  const int first_part = blockIdx.z * GROUPS * 4, total = GROUPS * 4 * steps;
+  const int len = f32_part_length(K), range = GROUPS * 4 * len;           // k of a part, and of this CTA
+  const int k_first = blockIdx.z * range, mine = max(0, min(range, K - k_first)), total = (mine + FT_K - 1) / FT_K;
 
-  // Step by step in order: `at` is the place of the next step inside its part, `from` the part's first k. Either side (x or
-  // w) keeps its own, because the first steps of w are asked for before x may be read.
+  // Steps of 32 k, whatever parts they hold; either side (x or w) keeps its place, because the first steps of w are asked
+  // for before x may be read. Zeros beyond the CTA's range and the matrix; parts beyond the matrix would add nothing
+  // and are left out.
   constexpr int WORDS = FT_K / 4;
-  struct Place { int at, from; };
-  auto load = [&](Place& p, int rows, int r0, int limit, const float* src, float* dst) {
+  auto load = [&](int& at, int rows, int r0, int limit, const float* src, float* dst) {
 #pragma unroll
     for (int c = tid; c < rows * WORDS; c += THREADS) {
-      const int word = c % WORDS, r = c / WORDS, in_part = p.at + word * 4, k = p.from + in_part;
-      const bool ok = in_part < len && k < K && r0 + r < limit;
+      const int word = c % WORDS, r = c / WORDS, k = k_first + at + word * 4;
+      const bool ok = at + word * 4 < mine && r0 + r < limit;
       f32_copy16(dst + r * FT_STRIDE + word * 4, src + (ok ? (size_t)(r0 + r) * K + k : 0), ok);
     }
-    p.at += FT_K;
-    if (p.at >= len) { p.at = 0; p.from += len; }
+    at += FT_K;
   };
-  Place of_x = {0, first_part * len}, of_w = of_x;
+  int of_x = 0, of_w = 0;
   auto load_x = [&](int stage) { load(of_x, BM, m0, M, x, smem + stage * FT_STAGE); };
   auto load_w = [&](int stage) { load(of_w, BN, n0, N, w, smem + stage * FT_STAGE + BM * FT_STRIDE); };
 #pragma unroll
-  for (int s = 0; s < FT_STAGES - 1; ++s) load_w(s);        // weights first (total is at least four steps)
+  for (int s = 0; s < FT_STAGES - 1; ++s) load_w(s);        // weights first
   pdl_wait();
 #pragma unroll
   for (int s = 0; s < FT_STAGES - 1; ++s) { load_x(s); f32_commit(); }
 
-  float acc[TM][TN], group[TM][TN];
-  int step = 0, stage = 0;
-  for (int g = 0; g < GROUPS; ++g) {
-    for (int p = 0; p < 4; ++p) {
+  float acc[TM][TN], group[TM][TN], sum[TM][TN];        // of a part, of a group, of the groups so far
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-      for (int b = 0; b < steps; ++b, ++step) {
-        f32_wait<FT_STAGES - 2>();
-        __syncthreads();
-        if (step + FT_STAGES - 1 < total) {
-          const int free = stage == 0 ? FT_STAGES - 1 : stage - 1;      // read in the step before this one
-          load_x(free);
-          load_w(free);
-        }
-        f32_commit();
-        const float* as = smem + stage * FT_STAGE + ty * FT_STRIDE;
-        const float* bs = smem + stage * FT_STAGE + (BM + tx) * FT_STRIDE;
-        stage = stage == FT_STAGES - 1 ? 0 : stage + 1;
-#pragma unroll
-        for (int k = 0; k < FT_K; k += 4) {
-          float4 a[TM];
-#pragma unroll
-          for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(as + i * (BM / TM) * FT_STRIDE + k);
-#pragma unroll
-          for (int j = 0; j < TN; ++j) {
-            const float4 v = *reinterpret_cast<const float4*>(bs + j * (BN / TN) * FT_STRIDE + k);
-#pragma unroll
-            for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].x, v.x, acc[i][j]);
-#pragma unroll
-            for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].y, v.y, acc[i][j]);
-#pragma unroll
-            for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].z, v.z, acc[i][j]);
-#pragma unroll
-            for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].w, v.w, acc[i][j]);
-          }
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) group[i][j] = p == 0 ? acc[i][j] : group[i][j] + acc[i][j];
-    }
-    float* mine = kept + tid;        // the sum of the groups so far (a thread's own words: no barrier)
+    for (int j = 0; j < TN; ++j) acc[i][j] = group[i][j] = sum[i][j] = 0.f;
+  auto end_part = [&]() {
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
+      for (int j = 0; j < TN; ++j) { group[i][j] += acc[i][j]; acc[i][j] = 0.f; }
+  };
+  auto end_group = [&]() {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) { sum[i][j] += group[i][j]; group[i][j] = 0.f; }
+  };
+  int stage = 0, part = 0, left = len / 4, ahead = (mine + 3) / 4;       // of the part and of all, in steps of four
+  for (int step = 0; step < total; ++step) {
+    f32_wait<FT_STAGES - 2>();
+    __syncthreads();
+    if (step + FT_STAGES - 1 < total) {
+      const int free = stage == 0 ? FT_STAGES - 1 : stage - 1;      // read in the step before this one
+      load_x(free);
+      load_w(free);
+    }
+    f32_commit();
+    const float* as = smem + stage * FT_STAGE + ty * FT_STRIDE;
+    const float* bs = smem + stage * FT_STAGE + (BM + tx) * FT_STRIDE;
+    stage = stage == FT_STAGES - 1 ? 0 : stage + 1;
+    auto four = [&](int k) {
+      float4 a[TM];
+#pragma unroll
+      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(as + i * (BM / TM) * FT_STRIDE + k);
+#pragma unroll
       for (int j = 0; j < TN; ++j) {
-        float* o = mine + (i * TN + j) * THREADS;
-        *o = g > 0 ? *o + group[i][j] : group[i][j];
+        const float4 v = *reinterpret_cast<const float4*>(bs + j * (BN / TN) * FT_STRIDE + k);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].x, v.x, acc[i][j]);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].y, v.y, acc[i][j]);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].z, v.z, acc[i][j]);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].w, v.w, acc[i][j]);
       }
+    };
+    auto forward = [&](int fours_done) {
+      left -= fours_done;
+      if (left == 0) {
+        left = len / 4;
+        end_part();
+        if ((++part & 3) == 0) end_group();
+      }
+    };
+    if constexpr (WHOLE) {
+#pragma unroll
+      for (int q = 0; q < WORDS; ++q) four(4 * q);
+      forward(WORDS);
+    } else {
+      const int fours = ahead < WORDS ? ahead : WORDS;
+      ahead -= fours;
+      for (int done = 0; done < fours;) {
+        const int run = left < fours - done ? left : fours - done;
+        if (run == WORDS) {
+#pragma unroll
+          for (int q = 0; q < WORDS; ++q) four(4 * q);
+        } else {
+          for (int q = 0; q < run; ++q) four(4 * (done + q));
+        }
+        done += run;
+        forward(run);
+      }
+    }
   }
+  end_part();         // (of a part that the matrix ends in; else they add zeros)
+  end_group();
   f32_wait<0>();
   auto store = [&](int o, float v) {
     const int r = m0 + ty + (o / TN) * (BM / TM), c = n0 + tx + (o % TN) * (BN / TN);
     if (r < M && c < N) out[(size_t)r * N + c] = v;
   };
   if (SPLIT == 1) {
-#pragma unroll 4
-    for (int o = 0; o < OUTS; ++o) store(o, kept[o * THREADS + tid]);
+#pragma unroll
+    for (int o = 0; o < OUTS; ++o) store(o, sum[o / TN][o % TN]);
   } else {
+#pragma unroll
+    for (int o = 0; o < OUTS; ++o) kept[o * THREADS + tid] = sum[o / TN][o % TN];
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
     const float* of_group[4];
@@ -283,10 +323,10 @@ __global__ void __launch_bounds__(FT_THREADS) gemm_f32_tile_kernel(const float* 
   }
 }
 
-template <int SPLIT>
-static int launch_tile(const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
-  auto kernel = gemm_f32_tile_kernel<SPLIT>;
-  constexpr int own = (FT_STAGES * FT_STAGE + FT_M * FT_N) * (int)sizeof(float);      // the ring, and the CTA's sums
+template <int SPLIT, bool WHOLE>
+static int launch_tile_form(const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
+  auto kernel = gemm_f32_tile_kernel<SPLIT, WHOLE>;
+  constexpr int own = (FT_STAGES * FT_STAGE + (SPLIT == 1 ? 0 : FT_M * FT_N)) * (int)sizeof(float);      // the ring, and the CTA's sums
   constexpr int sm_bytes = 228 * 1024;
   static bool ready[64] = {};
   int dev = 0;
@@ -308,6 +348,12 @@ static int launch_tile(const float* x, const float* w, float* out, int M, int N,
   return launch_cluster(kernel, grid, FT_THREADS, smem, stream, dim3(1, 1, SPLIT), x, w, out, M, N, K);
 }
 
+template <int SPLIT>
+static int launch_tile(const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
+  return f32_part_length(K) % FT_K == 0 ? launch_tile_form<SPLIT, true>(x, w, out, M, N, K, stream)
+                                        : launch_tile_form<SPLIT, false>(x, w, out, M, N, K, stream);
+}
+
 }  // namespace ts
 
 using namespace ts;
@@ -320,9 +366,11 @@ extern "C" int ts_gemm_f32(const float* x, const float* w, float* out, int M, in
   if (form == 0) {
     const long long tiles = (long long)((M + FT_M - 1) / FT_M) * ((N + FT_N - 1) / FT_N);
     // (K over 4 CTAs / over one: 128 rows of 4,096 x 1,024, 256 tiles, 39 / 42 us; 190 rows, 384 tiles, 53 / 53; 190 of
-    // 6,144 x 1,024, 576 tiles, 79 / 67; 64 of 1,024 x 3,072, 32 tiles, 24 / 73)
+    // 6,144 x 1,024, 576 tiles, 79 / 67; 64 of 1,024 x 3,072, 32 tiles, 24 / 73. The cluster's meeting weighs more the
+    // shorter K: 300 rows of 1,024 x 128, 160 tiles, 9.3 / 8.9; of 2,048 x 256, 320 tiles, 20 / 18; 40 of 4,096 x 64, 128
+    // tiles, 6.7 / 5.4; 128 of 2,048 x 256, 128 tiles, 9.4 / 10.6)
     if (M <= 16) form = M > 2 && N >= 2048 ? 2 : 1;
-    else form = tiles <= 400 ? 4 : 3;
+    else form = tiles <= 400 && tiles <= 100 + K / 2 ? 4 : 3;
   }
   if (form <= 2) {
     if ((M + 7) / 8 > 65535) return TS_ERR_BAD_ARGUMENT;
