@@ -428,6 +428,14 @@ def test_gemm_f32_forms_agree_bit_for_bit(m, n, k) -> None:
     assert torch.equal(row[0], out[m - 1])
 
 
+@pytest.mark.parametrize("m", [ops.F32_MAX_ROWS, ops.F32_MAX_ROWS + 1])
+def test_gemm_f32_of_millions_of_rows(m) -> None:
+    x, w = rnd(m, 4, seed=1), rnd(3, 4, seed=2)
+    out = torch.full((m, 3), float("nan"), device="cuda")
+    ops.gemm(x, w, out)
+    torch.testing.assert_close(out, (x.double() @ w.double().T).float(), atol=1e-5, rtol=1e-5)
+
+
 def test_gemm_f32_rows_off_the_16_byte_grid_take_the_general_kernel() -> None:
     x, w = rnd(7, 33, seed=1), rnd(20, 33, seed=2)
     out = torch.empty(7, 20, device="cuda")

@@ -761,9 +761,9 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
         return
     if x.dtype == torch.float32:
         px, pw = _dev(x, "x"), _dev(w, "w")
-        if k % 4 == 0 and (px | pw) % 16 == 0:
+        if k % 4 == 0 and (px | pw) % 16 == 0 and m <= F32_MAX_ROWS:
             _check(_fn("ts_gemm_f32")(px, pw, _dev(out, "out"), m, n, k, 0, _stream()), "gemm")
-        else:       # rows that do not start on a 16-byte boundary
+        else:       # rows that do not start on a 16-byte boundary, or more than a grid of the tiles holds
             _check(_fn("ts_gemm_simt")(px, pw, _dev(out, "out"), m, n, k, _F32, _F32, _stream()), "gemm")
         return
     if takes_rows_tcgen05(x, w, out):
@@ -784,6 +784,8 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
         torch.mm(x, w.t(), out_dtype=torch.float32, out=out)
 
 
+# The 32-bit product's tiles hold 32 rows, a grid 65,535 of them (the general kernel twice as many).
+F32_MAX_ROWS = 65535 * 32
 # Up to this many rows a bf16 product streams the weights through the skinny kernel ...
 SKINNY_MAX_ROWS = 16
 # ... if the matrix is smaller than this (or the output head's): larger ones go to the tcgen05 kernel that streams the
