@@ -207,6 +207,17 @@ def test_attention_mixed_batch(dtype, hq, hkv, d, page) -> None:
     torch.testing.assert_close(out.float(), want.float(), **tol(dtype))
 
 
+@pytest.mark.parametrize("dtype,hq,hkv,d", [(torch.float32, 8, 8, 64), (torch.float32, 16, 8, 128), (torch.float32, 24, 8, 64),
+                                            (torch.float32, 64, 8, 128), (torch.float32, 16, 8, 256), (torch.bfloat16, 16, 8, 256),
+                                            (torch.bfloat16, 64, 8, 192)])
+def test_single_tokens_of_many_requests_on_cuda_cores(dtype, hq, hkv, d) -> None:
+    """As many CTAs as fill the machine have four warps instead of eight; contexts shorter and longer than a batch of keys."""
+    lens = [(1 + (7 * i) % 41, 1) for i in range(70)]
+    out, want = _attention_case(dtype, hq, hkv, d, 16, lens, 0)
+    assert not out.isnan().any()
+    torch.testing.assert_close(out.float(), want.float(), **tol(dtype))
+
+
 @pytest.mark.parametrize("kernel,heads_per_cta", [("tcgen05", 1), ("tcgen05", 2), ("mma", 0)])
 @pytest.mark.parametrize("hq,hkv,d,page", [(16, 8, 128, 16), (4, 2, 64, 8), (8, 2, 128, 32), (6, 1, 64, 48),
                                            (5, 5, 128, 8)])

@@ -29,7 +29,8 @@ constexpr float NEG_INF = -INFINITY;
 // cost six shared-memory instructions for eight multiply-adds), float tiles come by cp.async into the second buffer
 // while the first one is worked on, and a step with few CTAs is cut into tiles of 16 queries instead of 32. Whatever the
 // cut, a row's scores are one chain over the head's elements, its sums go over the keys in order and are rescaled every
-// 32 keys, so its result does not depend on the batch. B200, float, 16 / 8 heads of 128: see launch_prefill_dj.
+// 32 keys, so its result does not depend on the batch. B200, float, 16 / 8 heads of 128, staged and multiplied element by
+// element / now: 45 tokens 24 / 15 us, 300 tokens 119 / 80, 64 tokens at 2,000 positions 615 / 358, 2,000 tokens 1,290 / 1,098.
 constexpr int PF_TK = 32;       // keys per tile
 constexpr int PF_THREADS = 128;
 
@@ -280,8 +281,10 @@ __global__ void __launch_bounds__(PF_THREADS) prefill_attn_kernel(AttnArgs a, in
 }
 
 // ================================================================ decode (split-K)
-constexpr int DC_WARPS = 8;
-constexpr int DC_THREADS = DC_WARPS * 32;
+// A CTA has eight warps, or four when there are this many CTAs, three an SM, to fill the machine (float, 12 / 3 heads of 64,
+// 64 requests of 200 positions, 576 CTAs: 26 us with eight, 18 with four; 16 / 8 of 128, 16 of 1,000, 640 CTAs, 54 / 40; one
+// of 500, 56 CTAs, 9.3 / 10.3).
+constexpr int DC_MANY_CTAS = 444;
 constexpr int DC_MAX_COUNTERS = 1 << 16;
 
 // One arrival counter per (request, CTA row of the grid): the CTA that arrives last merges the
@@ -293,12 +296,13 @@ static __device__ unsigned int g_decode_counters[DC_MAX_COUNTERS];
 // LPK = lanes that share a key; CPL = 16-byte chunks of a key per lane; U = keys per lane group whose loads are in flight.
 // Bound by its chain of latencies: block table, keys, the sums over the lanes of a key, the exponentials. Few lanes a key
 // make few exchanges (three steps for four keys at once with LPK = 8, five for one with 32), and the number of lanes is
-// known to the compiler so that the exchanges of all keys and heads overlap.
-template <typename T, int GT, int CPL, int LPK, int U>
-__global__ void __launch_bounds__(DC_THREADS) decode_attn_kernel(AttnArgs a, int passes) {
+// known to the compiler so that the exchanges of all keys and heads overlap. Float, 16 / 8 heads of 128, 32 lanes a key and
+// four warps / now: one request of 500 positions 21 / 9 us, 16 of 1,000 111 / 40; 32 / 8 heads, 64 of 200 95 / 54.
+template <typename T, int GT, int CPL, int LPK, int U, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) decode_attn_kernel(AttnArgs a, int passes) {
   constexpr int VEC = Vec<T>::N;
   constexpr int EPL = VEC * CPL;                 // elements of a key per lane
-  extern __shared__ float smem[];                // [DC_WARPS][GT][D + 2]
+  extern __shared__ float smem[];                // [WARPS][GT][D + 2]
   __shared__ int is_last;
   pdl_trigger();
   const int D = a.head_dim;
@@ -358,7 +362,7 @@ __global__ void __launch_bounds__(DC_THREADS) decode_attn_kernel(AttnArgs a, int
     for (int e = 0; e < EPL; ++e) acc[g][e] = 0.f;
   }
 
-  const int stride = DC_WARPS * KPW * U;
+  const int stride = WARPS * KPW * U;
   for (int base = k_begin + (warp * U) * KPW; base < k_end; base += stride) {
     // ---- all loads of this batch first: U keys and U values per lane group, kept packed
     Vec<T> kraw[U][CPL], vraw[U][CPL];
@@ -473,14 +477,14 @@ __global__ void __launch_bounds__(DC_THREADS) decode_attn_kernel(AttnArgs a, int
     }
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < ng * D; idx += DC_THREADS) {
+  for (int idx = threadIdx.x; idx < ng * D; idx += WARPS * 32) {
     const int g = idx / D, d = idx - g * D;
     float mm = NEG_INF;
 #pragma unroll
-    for (int w = 0; w < DC_WARPS; ++w) mm = fmaxf(mm, smem[((size_t)w * GT + g) * WS + D]);
+    for (int w = 0; w < WARPS; ++w) mm = fmaxf(mm, smem[((size_t)w * GT + g) * WS + D]);
     float num = 0.f, den = 0.f;
 #pragma unroll
-    for (int w = 0; w < DC_WARPS; ++w) {
+    for (int w = 0; w < WARPS; ++w) {
       const float* ws = smem + ((size_t)w * GT + g) * WS;
       const float c = (ws[D] == NEG_INF) ? 0.f : exp2f(ws[D] - mm);
       num += ws[d] * c;
@@ -533,22 +537,29 @@ static int launch_prefill(const AttnArgs& a, int max_query_len, cudaStream_t str
   return launch_prefill_qj<T, 4>(a, max_query_len, stream);
 }
 
-template <typename T, int GT, int CPL, int LPK>
-static int launch_decode_gc(const AttnArgs& a, cudaStream_t stream) {
+template <typename T, int GT, int CPL, int LPK, int WARPS>
+static int launch_decode_warps(const AttnArgs& a, int passes, cudaStream_t stream) {
   constexpr int U = CPL >= 8 ? 1 : CPL >= 4 ? 2 : (CPL == 1 && GT <= 4) ? 8 : 4;
-  const int G = a.num_heads / a.num_kv_heads;
-  const int passes = (G + GT - 1) / GT;
-  if ((long long)a.num_seqs * a.num_kv_heads * passes > DC_MAX_COUNTERS && a.num_splits > 1) return TS_ERR_UNSUPPORTED;
   // the warps' sums; the merge of the ranges keeps its (max, sum) pairs in the same memory
-  const size_t sums = (size_t)DC_WARPS * GT * (a.head_dim + 2), pairs = (size_t)GT * a.num_splits * 2;
+  const size_t sums = (size_t)WARPS * GT * (a.head_dim + 2), pairs = (size_t)GT * a.num_splits * 2;
   const size_t smem = sizeof(float) * (sums > pairs ? sums : pairs);
-  auto kern = decode_attn_kernel<T, GT, CPL, LPK, U>;
+  auto kern = decode_attn_kernel<T, GT, CPL, LPK, U, WARPS>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
   dim3 grid(a.num_seqs, a.num_kv_heads * passes, a.num_splits);
-  return launch(kern, grid, DC_THREADS, smem, stream, a, passes);
+  return launch(kern, grid, WARPS * 32, smem, stream, a, passes);
+}
+
+template <typename T, int GT, int CPL, int LPK>
+static int launch_decode_gc(const AttnArgs& a, cudaStream_t stream) {
+  const int G = a.num_heads / a.num_kv_heads;
+  const int passes = (G + GT - 1) / GT;
+  const long long rows = (long long)a.num_seqs * a.num_kv_heads * passes;
+  if (rows > DC_MAX_COUNTERS && a.num_splits > 1) return TS_ERR_UNSUPPORTED;
+  return rows * a.num_splits >= DC_MANY_CTAS ? launch_decode_warps<T, GT, CPL, LPK, 4>(a, passes, stream)
+                                             : launch_decode_warps<T, GT, CPL, LPK, 8>(a, passes, stream);
 }
 
 template <typename T>
@@ -557,24 +568,35 @@ static int launch_decode(const AttnArgs& a, cudaStream_t stream) {
   const int chunks = a.head_dim / VEC;
   const int G = a.num_heads / a.num_kv_heads;
   if (chunks > 64) return TS_ERR_UNSUPPORTED;
+  // Lanes a key and 16-byte chunks a lane: few lanes make few exchanges, but each holds its elements of every head's query
+  // and sum, and too many of them leave no registers for keys in flight and no room for CTAs (float, 4 / 2 heads of 256, 16
+  // requests of 1,000 positions: 8 lanes 43 us, 16 lanes 25; 32 / 8 of 128, 64 of 200: 32 lanes 113, 16 lanes 82; bf16, 16 / 2
+  // of 256, 16 of 1,000, eight heads a CTA: 16 lanes 119, 32 lanes 81).
   if (G <= 2) {
-    // up to eight lanes a key: the heads' queries and sums still fit the registers
-#define TS_DECODE_CASE(GT_)                                                   \
-    if (chunks <= 4) return launch_decode_gc<T, GT_, 1, 4>(a, stream);        \
-    if (chunks <= 8) return launch_decode_gc<T, GT_, 1, 8>(a, stream);        \
-    if (chunks <= 16) return launch_decode_gc<T, GT_, 2, 8>(a, stream);       \
-    if (chunks <= 32) return launch_decode_gc<T, GT_, 4, 8>(a, stream);       \
-    if constexpr (VEC == 4) return launch_decode_gc<T, GT_, 8, 8>(a, stream)
+#define TS_DECODE_CASE(GT_)                                                                \
+    if (chunks <= 4) return launch_decode_gc<T, GT_, 1, 4>(a, stream);                     \
+    if (chunks <= 8) return launch_decode_gc<T, GT_, 1, 8>(a, stream);                     \
+    if (chunks <= 16) return launch_decode_gc<T, GT_, 2, 8>(a, stream);                    \
+    if constexpr (VEC == 4) {                                                              \
+      if (chunks <= 32) return launch_decode_gc<T, GT_, 4, 8>(a, stream);                  \
+      return launch_decode_gc<T, GT_, 4, 16>(a, stream);                                   \
+    } else {                                                                               \
+      if (chunks <= 32) return launch_decode_gc<T, GT_, 2, 16>(a, stream);                 \
+    }
     if (G == 1) { TS_DECODE_CASE(1); return TS_ERR_UNSUPPORTED; }
     TS_DECODE_CASE(2);
     return TS_ERR_UNSUPPORTED;
 #undef TS_DECODE_CASE
   }
 #define TS_DECODE_CASE(GT_)                                                   \
-  if (chunks <= 4) return launch_decode_gc<T, GT_, 1, 4>(a, stream);          \
-  if (chunks <= 8) return launch_decode_gc<T, GT_, 1, 8>(a, stream);          \
-  if (chunks <= 16) return launch_decode_gc<T, GT_, 1, 16>(a, stream);        \
-  if (chunks <= 32) return launch_decode_gc<T, GT_, 1, 32>(a, stream);        \
+  if (chunks <= 4) return launch_decode_gc<T, GT_, 1, 4>(a, stream);                           \
+  if (chunks <= 8) return launch_decode_gc<T, GT_, 1, 8>(a, stream);                           \
+  if (chunks <= 16) return launch_decode_gc<T, GT_, GT_ == 4 ? 2 : 1, GT_ == 4 ? 8 : 16>(a, stream);   \
+  if constexpr (VEC == 4 || GT_ == 4) {                                                        \
+    if (chunks <= 32) return launch_decode_gc<T, GT_, 2, 16>(a, stream);                       \
+  } else {                                                                                     \
+    if (chunks <= 32) return launch_decode_gc<T, GT_, 1, 32>(a, stream);                       \
+  }                                                                                            \
   if constexpr (VEC == 4) return launch_decode_gc<T, GT_, 2, 32>(a, stream)
   if (G <= 4) { TS_DECODE_CASE(4); return TS_ERR_UNSUPPORTED; }
   TS_DECODE_CASE(8);
