@@ -46,8 +46,8 @@
 // issue slots, not only of the exponential unit). With two heads a CTA the tensor core works for one
 // head while the other's softmax runs, and the MMA warp serves both in turn, 16 instructions a head and tile: issued from a
 // branch on the lane an instruction took 77 cycles (its operands go to uniform registers one by one) and that warp set the
-// pace; issued by the converged warp, 8,192 tokens 300 -> 266 us (1,035 TFLOP/s), 2,048 tokens at 9,001 positions 179 -> 158
-// us. An MMA warp per head was slower (369 us: the heads fall into step), and so were two score buffers of 64 keys per head
+// pace; issued by the converged warp, 8,192 tokens 300 -> 273 us (1,010 TFLOP/s), 2,048 tokens at 9,001 positions 179 -> 160
+// us (with the sums of a row kept per 64 columns, which take 3 % of that). An MMA warp per head was slower (369 us: the heads fall into step), and so were two score buffers of 64 keys per head
 // (289 us at best: what a step costs whatever its size is paid twice). Every operand read from shared
 // memory and every TMA write goes through the same 128 bytes per cycle, which is why P stays in tensor
 // memory.
