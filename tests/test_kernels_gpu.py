@@ -63,6 +63,25 @@ def test_add_rms_norm(dtype, hidden, with_delta) -> None:
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("hidden", [4, 132, 2048, 2052, 4100, 8192, 12288, 16384, 16388])
+@pytest.mark.parametrize("t", [1, 40])
+def test_add_rms_norm_of_a_cta_a_row(dtype, hidden, t) -> None:
+    """Rows in the registers of one CTA: one, two or four times four elements a thread, a last warp that is not full; from
+    16,388 columns on the kernel of two passes over memory. Sums of squares in 32 bits in any order: within (hidden + 2)
+    roundings of one another, half of that in the norm, then the two roundings of a bf16 result (2^-8 each)."""
+    resid, delta = rnd(t, hidden, seed=1, scale=3.0), rnd(t, hidden, dtype=dtype, seed=2)
+    w = (1 + rnd(hidden, seed=3, scale=0.1)).to(dtype)
+    for d in (delta, None):
+        r1, out = resid.clone(), torch.full((t, hidden), float("nan"), device="cuda", dtype=dtype)
+        ops.add_rms_norm(r1, d, w, 1e-5, out)
+        x = resid if d is None else resid + d.float()
+        assert torch.equal(r1, x)
+        want = x.double() * torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True) + 1e-5) * w.double()
+        step = 2.0 ** -24 * (hidden / 2 + 4) if dtype == torch.float32 else 2.0 ** -7 + 2.0 ** -15 + 2.0 ** -24 * hidden
+        assert bool(((out.double() - want).abs() <= step * want.abs() + 1e-30).all())
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("hidden", [256, 512, 1024, 2048])
 @pytest.mark.parametrize("t", [256, 1027])
 def test_add_rms_norm_of_many_rows(dtype, hidden, t) -> None:

@@ -71,64 +71,97 @@ __global__ void add_rms_norm_kernel(float* __restrict__ resid, const T* __restri
   }
 }
 
-// The same with 16-byte accesses on the 32-bit stream and 8-byte (bf16) or 16-byte (float)
-// accesses on the rest: 4 elements per thread and step. Needs hidden % 4 == 0 and the row cache.
-template <typename T>
-__global__ void add_rms_norm_vec_kernel(float* __restrict__ resid, const T* __restrict__ delta,
-                                        const T* __restrict__ weight, T* __restrict__ out,
-                                        const int* __restrict__ rows, int hidden, float eps) {
-  extern __shared__ float xs[];
-  __shared__ float scratch[33];
+// Four neighbouring elements as they lie in memory: half the registers of their 32-bit values where T is bf16.
+template <typename T> struct Packed;
+template <> struct Packed<float> {
+  float4 raw;
+  __device__ __forceinline__ void load(const float* p) { raw = *reinterpret_cast<const float4*>(p); }
+  __device__ __forceinline__ void zero() { raw = make_float4(0.f, 0.f, 0.f, 0.f); }
+  __device__ __forceinline__ void values(float* f) const { f[0] = raw.x; f[1] = raw.y; f[2] = raw.z; f[3] = raw.w; }
+};
+template <> struct Packed<bf16> {
+  uint2 raw;
+  __device__ __forceinline__ void load(const bf16* p) { raw = *reinterpret_cast<const uint2*>(p); }
+  __device__ __forceinline__ void zero() { raw = make_uint2(0u, 0u); }
+  __device__ __forceinline__ void values(float* f) const {
+    f[0] = __uint_as_float(raw.x << 16); f[1] = __uint_as_float(raw.x & 0xffff0000u);
+    f[2] = __uint_as_float(raw.y << 16); f[3] = __uint_as_float(raw.y & 0xffff0000u);
+  }
+};
+
+// The same with 16-byte accesses on the 32-bit stream and 8-byte (bf16) or 16-byte (float) accesses on the rest: a CTA
+// takes a row, a thread NV times 4 of its elements, which stay in registers between the two passes. Bound by latency (one
+// to 64 rows between two products): so the weights, which no kernel before this one writes, are asked for in front of the
+// wait, all loads of the row are in flight at once, and the sum of squares meets at one barrier. Registers are held to what
+// lets four CTAs of 512 threads share an SM, where many rows are bound by throughput. Needs hidden % 4 == 0. One after the
+// other with the weights in L2, row kept in shared memory, two barriers, weights asked for last / now: bf16, 4,096 columns, 1
+// row 2.4 / 2.1 us, 16 rows 2.6 / 2.1, 190 rows 4.3 / 3.2, 512 rows 4.4 / 4.0; 8,192 columns, 16 rows 3.6 / 2.8; 12,288
+// columns (before: element by element) 11.8 / 3.3; 32 bits, 4,096 columns, 16 rows 2.6 / 2.2.
+template <typename T, int NV>
+__global__ void __launch_bounds__(NV == 4 ? 1024 : 512, NV == 4 ? 1 : NV == 2 && sizeof(T) == 4 ? 3 : 4)
+    add_rms_norm_vec_kernel(float* __restrict__ resid, const T* __restrict__ delta, const T* __restrict__ weight,
+                            T* __restrict__ out, const int* __restrict__ rows, int hidden, float eps) {
+  __shared__ float parts[32];
   pdl_trigger();
+  Packed<T> w[NV], add[NV];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int i = (threadIdx.x + j * blockDim.x) * 4;
+    w[j].zero();
+    if (i < hidden) w[j].load(weight + i);
+  }
   pdl_wait();
   const int r = blockIdx.x;
   const int row = rows ? rows[r] : r;
   float* x = resid + (size_t)row * hidden;
   const T* d = delta ? delta + (size_t)row * hidden : nullptr;
   const bool write_back = (rows == nullptr) && (d != nullptr);
-  float ss = 0.f;
-  for (int i = threadIdx.x * 4; i < hidden; i += blockDim.x * 4) {
-    float4 v = *reinterpret_cast<const float4*>(x + i);
-    if (d) {
-      if constexpr (sizeof(T) == 2) {
-        const uint2 raw = *reinterpret_cast<const uint2*>(d + i);
-        v.x += __uint_as_float(raw.x << 16); v.y += __uint_as_float(raw.x & 0xffff0000u);
-        v.z += __uint_as_float(raw.y << 16); v.w += __uint_as_float(raw.y & 0xffff0000u);
-      } else {
-        const float4 dv = *reinterpret_cast<const float4*>(d + i);
-        v.x += dv.x; v.y += dv.y; v.z += dv.z; v.w += dv.w;
-      }
+  float v[NV][4];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int i = (threadIdx.x + j * blockDim.x) * 4;
+    add[j].zero();
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[j][e] = 0.f;
+    if (i < hidden) {
+      Quad<float>::load(x + i, v[j]);
+      if (d) add[j].load(d + i);
     }
-    if (write_back) *reinterpret_cast<float4*>(x + i) = v;
-    *reinterpret_cast<float4*>(xs + i) = v;
-    ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
   }
-  ss = block_sum(ss, scratch);
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    if (d) {
+      float more[4];
+      add[j].values(more);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[j][e] += more[e];
+    }
+    ss += v[j][0] * v[j][0] + v[j][1] * v[j][1] + v[j][2] * v[j][2] + v[j][3] * v[j][3];
+  }
+  const int lane = threadIdx.x & 31;
+  ss = warp_sum(ss);
+  if (lane == 0) parts[threadIdx.x >> 5] = ss;
+  if (write_back) {
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int i = (threadIdx.x + j * blockDim.x) * 4;
+      if (i < hidden) Quad<float>::store(x + i, v[j]);
+    }
+  }
+  __syncthreads();
+  ss = warp_sum(lane < (int)(blockDim.x >> 5) ? parts[lane] : 0.f);
   const float rstd = rsqrtf(ss / (float)hidden + eps);
   T* o = out + (size_t)r * hidden;
-  for (int i = threadIdx.x * 4; i < hidden; i += blockDim.x * 4) {
-    const float4 v = *reinterpret_cast<const float4*>(xs + i);
-    const float f[4] = {v.x, v.y, v.z, v.w};
-    float w[4], res[4];
-    if constexpr (sizeof(T) == 2) {
-      const uint2 raw = *reinterpret_cast<const uint2*>(weight + i);
-      w[0] = __uint_as_float(raw.x << 16); w[1] = __uint_as_float(raw.x & 0xffff0000u);
-      w[2] = __uint_as_float(raw.y << 16); w[3] = __uint_as_float(raw.y & 0xffff0000u);
-    } else {
-      const float4 wv = *reinterpret_cast<const float4*>(weight + i);
-      w[0] = wv.x; w[1] = wv.y; w[2] = wv.z; w[3] = wv.w;
-    }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) res[e] = round_to<T>(f[e] * rstd) * w[e];
-    if constexpr (sizeof(T) == 2) {
-      __nv_bfloat162 a = __floats2bfloat162_rn(res[0], res[1]), b = __floats2bfloat162_rn(res[2], res[3]);
-      uint2 pk;
-      pk.x = *reinterpret_cast<uint32_t*>(&a);
-      pk.y = *reinterpret_cast<uint32_t*>(&b);
-      *reinterpret_cast<uint2*>(o + i) = pk;
-    } else {
-      *reinterpret_cast<float4*>(o + i) = make_float4(res[0], res[1], res[2], res[3]);
-    }
+  for (int j = 0; j < NV; ++j) {
+    const int i = (threadIdx.x + j * blockDim.x) * 4;
+    if (i >= hidden) continue;
+    float res[4], gain[4];
+    w[j].values(gain);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) res[e] = round_to<T>(v[j][e] * rstd) * gain[e];
+    Quad<T>::store(o + i, res);
   }
 }
 
@@ -329,6 +362,20 @@ static int launch_add_rms_norm_warp(float* resid, const T* delta, const T* weigh
 }
 constexpr int NORM_WARP_ROWS = 256;      // from this many rows on a warp takes a row
 
+constexpr int NORM_MOST_QUADS = 4 * 1024;
+template <typename T>
+static int launch_add_rms_norm_vec(float* resid, const T* delta, const T* weight, T* out, const int* rows, int num_rows,
+                                   int hidden, float eps, cudaStream_t stream) {
+  const int quads = hidden / 4;
+  const int per = quads <= 512 ? 1 : quads <= 1024 ? 2 : 4;       // of a thread
+  const int threads = ((quads + per - 1) / per + 31) / 32 * 32;
+  if (per == 1)
+    return launch(add_rms_norm_vec_kernel<T, 1>, num_rows, threads, 0, stream, resid, delta, weight, out, rows, hidden, eps);
+  if (per == 2)
+    return launch(add_rms_norm_vec_kernel<T, 2>, num_rows, threads, 0, stream, resid, delta, weight, out, rows, hidden, eps);
+  return launch(add_rms_norm_vec_kernel<T, 4>, num_rows, threads, 0, stream, resid, delta, weight, out, rows, hidden, eps);
+}
+
 extern "C" int ts_add_rms_norm(float* resid, const void* delta, const void* weight, void* out,
                                const int* rows, int num_rows, int hidden, float eps, int dtype,
                                cudaStream_t stream) {
@@ -346,14 +393,13 @@ extern "C" int ts_add_rms_norm(float* resid, const void* delta, const void* weig
                                             hidden, eps, stream);
     return TS_ERR_BAD_ARGUMENT;
   }
-  if (cache_row && hidden % 4 == 0 && aligned) {
-    const int vthreads = hidden >= 4096 ? 512 : (hidden >= 1024 ? 256 : 128);
+  if (hidden % 4 == 0 && hidden <= NORM_MOST_QUADS * 4 && aligned) {
     if (dtype == TS_DTYPE_F32)
-      return launch(add_rms_norm_vec_kernel<float>, num_rows, vthreads, smem, stream, resid, (const float*)delta,
-                    (const float*)weight, (float*)out, rows, hidden, eps);
+      return launch_add_rms_norm_vec<float>(resid, (const float*)delta, (const float*)weight, (float*)out, rows, num_rows,
+                                            hidden, eps, stream);
     if (dtype == TS_DTYPE_BF16)
-      return launch(add_rms_norm_vec_kernel<bf16>, num_rows, vthreads, smem, stream, resid, (const bf16*)delta,
-                    (const bf16*)weight, (bf16*)out, rows, hidden, eps);
+      return launch_add_rms_norm_vec<bf16>(resid, (const bf16*)delta, (const bf16*)weight, (bf16*)out, rows, num_rows, hidden,
+                                           eps, stream);
     return TS_ERR_BAD_ARGUMENT;
   }
   if (dtype == TS_DTYPE_F32)
