@@ -324,6 +324,17 @@ def test_decode_attention_cluster_merge_gives_the_same_bits(hq, hkv, d, page, sp
     torch.testing.assert_close(out.float(), want.float(), **tol(torch.bfloat16))
 
 
+@pytest.mark.parametrize("hq,hkv,d,page", [(16, 8, 128, 16), (8, 4, 64, 8)])
+@pytest.mark.parametrize("batch", [2, 16, 18, 19, 37, 38, 50])
+def test_decode_attention_with_an_sm_for_every_cta_or_several_ctas_an_sm(hq, hkv, d, page, batch) -> None:
+    """Up to 148 CTAs (requests x kv heads x key ranges) keep four tiles a warp in flight, more of them two."""
+    lens = [(1 + (i * 53) % 700, 1) for i in range(batch - 1)] + [(1500, 1)]
+    out, want = _attention_case(torch.bfloat16, hq, hkv, d, page, lens, 0, seed=3, spike=(batch - 1, 1100))
+    ops.check_device_errors()
+    assert not out.isnan().any()
+    torch.testing.assert_close(out.float(), want.float(), **tol(torch.bfloat16))
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("new", [1, 5])
 @pytest.mark.parametrize("pos", [0, 15, 16, 511, 700])

@@ -27,10 +27,14 @@
 
 namespace ts {
 
-#ifndef DM_STAGES_N
-#define DM_STAGES_N 2
-#endif
-constexpr int DM_WARPS = 4, DM_THREADS = DM_WARPS * 32, DM_TK = 16, DM_STAGES = DM_STAGES_N;
+constexpr int DM_WARPS = 4, DM_THREADS = DM_WARPS * 32, DM_TK = 16;
+constexpr int DM_STAGES = 2;
+// Up to this many CTAs (half the SMs: clusters of eight, one CTA an SM, then still find room) have eight warps: with an SM
+// to itself a CTA is bound by its warps' chains of products and exponentials, some 1,900 cycles a tile. One request of 16 / 8
+// heads of 128, four warps / eight: 1,000 keys 6.0 / 5.8 us, 4,000 11.4 / 9.5, 9,000 21.2 / 15.7, 20,000 40.9 / 29.7. (Four
+// tiles in flight a warp instead of two: 20.7 us at 9,000 keys, and clusters that found no room, 12 us instead of 6.5 for
+// two requests of 1,000. More ranges that merge through memory: 19.1 us with 16, and 10.2 instead of 6.0 at 1,000 keys.)
+constexpr int DM_FEW_CTAS = 74;
 constexpr int DM_MAX_COUNTERS = 1 << 16;
 
 static __device__ unsigned int g_dt_arrivals[DM_MAX_COUNTERS];
@@ -248,22 +252,32 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attn_tma_kernel(const __gri
   const int* table = a.block_tables + (size_t)seq * a.table_width;
 
   // One lane fetches a tile: the 16 positions from k0 lie in one page (BR = 16) or in two pages
-  // of 8. Row of the cache matrix = (page * kv_heads + kvh) * page_size + offset in the page.
-  auto load_tile = [&](int tile, int stage) {
+  // of 8. Row of the cache matrix = (page * kv_heads + kvh) * page_size + offset in the page. The pages are looked up apart
+  // from the copies and earlier: the look-up is a trip to L2 of its own.
+  constexpr int BOXES = DM_TK / BR;
+  auto box_pos = [&](int tile, int part) {
+    const int k0 = lo_al + tile * DM_TK, kpos = k0 + part * BR;
+    return kpos >= ctx ? k0 : kpos;      // a part wholly past the end: fetch any valid rows, they are masked
+  };
+  auto look_up = [&](int tile, int (&page)[BOXES]) {
+    if (lane != 0) return;
+#pragma unroll
+    for (int part = 0; part < BOXES; ++part) {
+      const int kpos = box_pos(tile, part);
+      page[part] = table[a.page_shift >= 0 ? kpos >> a.page_shift : kpos / a.page_size];
+    }
+  };
+  auto load_tile = [&](int tile, int stage, const int (&page)[BOXES]) {
     if (lane != 0 || wait_test_unarmed()) return;
-    const int k0 = lo_al + tile * DM_TK;
     unsigned char* kd = my + (size_t)stage * 2 * TILE_BYTES;
     unsigned char* vd = kd + TILE_BYTES;
     uint64_t* bar = &bars[warp][stage];
     dm_bar_arrive_tx(bar, 2u * TILE_BYTES);
 #pragma unroll
-    for (int part = 0; part < DM_TK / BR; ++part) {
-      int kpos = k0 + part * BR;
-      if (kpos >= ctx) kpos = k0;      // a part wholly past the end: fetch any valid rows, they are masked
-      int page, off;
-      if (a.page_shift >= 0) { page = table[kpos >> a.page_shift]; off = kpos & (a.page_size - 1); }
-      else { const int idx = kpos / a.page_size; page = table[idx]; off = kpos - idx * a.page_size; }
-      const int y = (page * a.num_kv_heads + kvh) * a.page_size + off;
+    for (int part = 0; part < BOXES; ++part) {
+      const int kpos = box_pos(tile, part);
+      const int off = a.page_shift >= 0 ? kpos & (a.page_size - 1) : kpos % a.page_size;
+      const int y = (page[part] * a.num_kv_heads + kvh) * a.page_size + off;
 #pragma unroll
       for (int h = 0; h < D64; ++h) {
         dm_tensor_copy(kd + h * 2048 + part * BR * 128, &map_k, h * 64, y, bar);
@@ -282,9 +296,14 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attn_tma_kernel(const __gri
 
   // this warp's tiles: tile_begin + warp, + WARPS, ...
   const int first = tile_begin + warp;
+  int pages[DM_STAGES][BOXES];
+#pragma unroll
+  for (int s = 0; s < DM_STAGES; ++s)
+    if (first + s * WARPS < tile_end) look_up(first + s * WARPS, pages[s]);
+#pragma unroll
   for (int s = 0; s < DM_STAGES; ++s) {
     const int tile = first + s * WARPS;
-    if (tile < tile_end && (FUSED || tile < ntiles_all - 1)) load_tile(tile, s);
+    if (tile < tile_end && (FUSED || tile < ntiles_all - 1)) load_tile(tile, s, pages[s]);
   }
   // (fused form) constants of the model and host-made inputs of the step, before the wait too
   const bool owns_last = tile_begin < tile_end && tile_end == ntiles_all;   // this range ends at the newest key
@@ -299,9 +318,10 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attn_tma_kernel(const __gri
   }
   pdl_wait();
   if constexpr (!FUSED) {
+#pragma unroll
     for (int s = 0; s < DM_STAGES; ++s) {
       const int tile = first + s * WARPS;
-      if (tile < tile_end && tile == ntiles_all - 1) load_tile(tile, s);
+      if (tile < tile_end && tile == ntiles_all - 1) load_tile(tile, s, pages[s]);
     }
   }
 
@@ -367,6 +387,9 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attn_tma_kernel(const __gri
   for (int tile = first; tile < tile_end; tile += WARPS, ++n) {
     const int stage = n % DM_STAGES;
     const uint32_t parity = (n / DM_STAGES) & 1;
+    const int nxt = tile + DM_STAGES * WARPS;      // takes this tile's place
+    int next_page[BOXES];
+    if (nxt < tile_end) look_up(nxt, next_page);
     if (!dm_bar_wait(&bars[warp][stage], parity)) { failed = true; break; }
     unsigned char* kt = my + (size_t)stage * 2 * TILE_BYTES;
     unsigned char* vt = kt + TILE_BYTES;
@@ -467,8 +490,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attn_tma_kernel(const __gri
     // order this warp's accesses to the stage (reads, and the zeroing above) before the copy
     // engine's next write into it
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    const int nxt = tile + DM_STAGES * WARPS;
-    if (nxt < tile_end) load_tile(nxt, stage);
+    if (nxt < tile_end) load_tile(nxt, stage, next_page);
   }
   if (failed && lane == 0) atomicExch(error_flag, WAIT_FAILED_DECODE_TMA);
 
@@ -661,9 +683,12 @@ static int launch_dt(const AttnArgs& a, long long cache_rows, int* error_flag, c
   if (D64 == 2 && a.num_splits == 1 && ctas > 3 * 148 && ctas <= 4 * 148)
     return launch_dt_w<D64, BR, FUSED, 3, false>(a, cache_rows, error_flag, stream, f);
   // 2 to 8 key ranges (the portable cluster size) merge inside a cluster
-  if (g_decode_cluster_merge && a.num_splits >= 2 && a.num_splits <= 8)
-    return launch_dt_w<D64, BR, FUSED, 4, true>(a, cache_rows, error_flag, stream, f);
-  return launch_dt_w<D64, BR, FUSED, 4, false>(a, cache_rows, error_flag, stream, f);
+  const bool cluster = g_decode_cluster_merge && a.num_splits >= 2 && a.num_splits <= 8;
+  if (ctas <= DM_FEW_CTAS)
+    return cluster ? launch_dt_w<D64, BR, FUSED, 8, true>(a, cache_rows, error_flag, stream, f)
+                   : launch_dt_w<D64, BR, FUSED, 8, false>(a, cache_rows, error_flag, stream, f);
+  return cluster ? launch_dt_w<D64, BR, FUSED, 4, true>(a, cache_rows, error_flag, stream, f)
+                 : launch_dt_w<D64, BR, FUSED, 4, false>(a, cache_rows, error_flag, stream, f);
 }
 
 }  // namespace ts
