@@ -469,6 +469,18 @@ def test_gemm_f32_forms_agree_bit_for_bit(m, n, k) -> None:
     assert torch.equal(row[0], out[m - 1])
 
 
+@pytest.mark.parametrize("m,n,k", [(33, 64, 1024), (40, 132, 68), (130, 1000, 132), (5, 24, 64)])
+def test_gemm_f32_stores_to_an_output_off_the_16_byte_grid(m, n, k) -> None:
+    x, w = rnd(m, k, seed=1), rnd(n, k, seed=2)
+    want = torch.empty(m, n, device="cuda")
+    ops.gemm(x, w, want)
+    for form in range(5):
+        buf = torch.full((m * n + 2,), float("nan"), device="cuda")
+        ops._check(ops._fn("ts_gemm_f32")(x.data_ptr(), w.data_ptr(), buf[1:].data_ptr(), m, n, k, form, ops._stream()), "gemm")
+        assert torch.equal(buf[1:-1].view(m, n), want), form
+        assert bool(buf[0].isnan()) and bool(buf[-1].isnan())
+
+
 @pytest.mark.parametrize("m", [ops.F32_MAX_ROWS, ops.F32_MAX_ROWS + 1])
 def test_gemm_f32_of_millions_of_rows(m) -> None:
     x, w = rnd(m, 4, seed=1), rnd(3, 4, seed=2)

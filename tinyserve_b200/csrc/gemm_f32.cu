@@ -15,18 +15,24 @@
 // word of w (8 rows of the 151,936 x 1,024 head: 207 us with one, 165 us with two). Measured back to back on B200, one
 // row, 64 x 64 tiles of all K before / now: 4,096 x 1,024 70 / 11 us, 1,024 x 3,072 205 / 8 us, the head 92 us (6.8 TB/s).
 //
-// More rows: bound by the multiply-adds and, below some hundred rows, by the latency of the chains. Register tiles of
-// 4 x 4 outputs a thread, 32 x 64 a CTA, operands in shared memory as [row][32 k] read in 16-byte words (rows a thread
-// owns lie a stride apart, so that eight neighbouring threads read eight different groups of banks), three cp.async
-// stages. Where the tiles are too few for the machine, the four groups of K go to the four CTAs of a cluster, which leave
-// their sums in shared memory; each then adds up its share of the tile through distributed shared memory. Where parts are
-// no whole steps of 32 k, a step runs over their ends (a part of its own steps multiplied mostly zeros: 1,000 rows of
-// 10,000 x 100 298 us, of 512 x 64 24 us). Measured, one kernel of 64 x 64 tiles for all sizes (which these replace) /
-// now: 45 rows of 4,096 x 1,024 76 / 20 us, 64 rows of 1,024 x 3,072 221 / 24 us, 190 rows of 6,144 x 1,024 115 / 67 us,
-// 1,000 rows of 10,000 x 100 86 / 80 us, of 512 x 64 6.7 / 6.8; many rows reach 38 TFLOP/s. Tiles of 64 x 64 and
-// 128 x 128 (8 outputs a thread and side) were no faster at any of 1 to 600 rows: they leave too few warps on an SM.
+// More rows: bound by the multiply-adds and, below some hundred rows, by the latency of the chains. A warp owns a tile of
+// 32 x 64 outputs, 8 x 8 a thread (a thread reads 16 words of shared memory for 64 multiply-adds; the 4 x 4 tiles that this
+// replaces read 32 for as many), and one stretch of K, so a CTA's four warps share a tile of outputs and nothing else: each
+// copies its own rows of x and w, in steps of 16 k and three cp.async stages, and none waits for another before the sums
+// meet in shared memory. Where the tiles are too few for the machine, a CTA takes one of the four groups, a warp one of its
+// parts, and the groups' CTAs are a cluster that adds up through distributed shared memory; else a warp takes a group and
+// keeps its parts' sums in shared memory. Parts shorter than a step (K up to 192) go to a kernel of thread tiles of 4 x 4
+// whose steps hold several parts (600 rows of 10,000 x 100 50 us, in steps of their own 73). Measured, 4 x 4 tiles for all / now: 64 rows of
+// 1,024 x 2,048 15.1 / 12.3 us, of 1,024 x 3,072 21.1 / 16.7, 128 rows of 4,096 x 1,024 39.9 / 32.7, of 1,024 x 3,072 32.8 / 24.6,
+// 190 rows of 6,144 x 1,024 70.8 / 64.5, 600 rows 216 / 203 (37 TFLOP/s: two or three warps a scheduler, which issue 72 % of
+// the time, 78 % of it multiply-adds; two at a time, fma.rn.f32x2, come to no more than 45 TFLOP/s in registers alone, one
+// at a time to 66). K over 4 CTAs / over one: 64 rows of 4,096 x 1,024, 128 tiles, 21 / 21 us, of 6,144 x 1,024, 192 tiles, 31 / 32;
+// 128 rows, 256 and 384 tiles, 41 / 33 and 58 / 52; 600 rows of 1,024 x 2,048, 304 tiles, 76 / 93; 64 and 128 rows of 2,048 x
+// 256, 64 and 128 tiles, 5.9 / 7.6 and 12.3 / 7.8: the cluster's meeting weighs more the shorter K.
 #define TS_PDL_CLASS PDL_OTHER
 #include <cooperative_groups.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -181,46 +187,218 @@ static int launch_rows(const float* x, const float* w, float* out, int M, int N,
 }
 
 // -------------------------------------------------------------------------------------------------- more rows
-constexpr int FT_M = 32, FT_N = 64, FT_OWN = 4, FT_K = 32, FT_STRIDE = FT_K + 4, FT_STAGES = 3;
-constexpr int FT_THREADS = (FT_M / FT_OWN) * (FT_N / FT_OWN), FT_STAGE = (FT_M + FT_N) * FT_STRIDE;     // floats
+constexpr int FT_M = 32, FT_N = 64, FT_OWN = 8, FT_K = 16, FT_TEAMS = 4, FT_STAGES = 3;
+constexpr int FT_THREADS = FT_TEAMS * 32, FT_STAGE = (FT_M + FT_N) * FT_K;       // floats of a warp's stage
+constexpr int FT_SUM_STRIDE = FT_N + 8, FT_SUMS = FT_M * FT_SUM_STRIDE;          // of a warp's sums: no two lanes in one bank
+static_assert(FT_SUMS <= FT_STAGES * FT_STAGE, "with K over a cluster the sums take the place of the ring");
 
-// WHOLE: parts are whole steps of 32 k; else a step may hold the ends of several.
-template <int SPLIT, bool WHOLE>
-__global__ void __launch_bounds__(FT_THREADS, 4) gemm_f32_tile_kernel(const float* x, const float* __restrict__ w, float* out,
-                                                                   int M, int N, int K) {
+// A warp's tile in one stage: rows of 16 k in four words of 16 bytes, whose places within a row are swapped by the row, so
+// that eight neighbouring rows read at the same word lie in different banks.
+__device__ __forceinline__ int f32_word_at(int row, int word) { return row * FT_K + ((word ^ ((row >> 1) & 3)) << 2); }
+
+// SPLIT 1: warp = one of the four groups of K. SPLIT 4: the CTA has one group, warp = one of its parts.
+// CTAS: CTAs of an SM, what the registers of a thread are held to.
+template <int SPLIT, int CTAS>
+__global__ void __launch_bounds__(FT_THREADS, CTAS) gemm_f32_tile_kernel(const float* x, const float* __restrict__ w,
+                                                                                     float* out, int M, int N, int K) {
   static_assert(SPLIT == 1 || SPLIT == 4, "all groups of K in one CTA, or one in each");
-  constexpr int BM = FT_M, BN = FT_N, TM = FT_OWN, TN = FT_OWN;
-  constexpr int THREADS = FT_THREADS, GROUPS = 4 / SPLIT, OUTS = TM * TN;
+  constexpr int PARTS = SPLIT == 1 ? 4 : 1, OWN = FT_OWN;       // parts a warp goes through
   extern __shared__ float smem[];
-  float* kept = smem + FT_STAGES * FT_STAGE;           // SPLIT 4: [output of a thread][thread]
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, team = threadIdx.x >> 5;
+  const int tx = lane & 7, ty = lane >> 3;
+  const int n0 = blockIdx.x * FT_N, m0 = blockIdx.y * FT_M;
+  const int len = f32_part_length(K), first_part = SPLIT == 1 ? 4 * team : 4 * blockIdx.z + team;
+  float* ring = smem + team * (FT_STAGES * FT_STAGE);
+  float* sums = SPLIT == 1 ? smem + FT_TEAMS * (FT_STAGES * FT_STAGE) : smem;       // [team][row][column]
+
+  // ---- copies: four lanes a row. A step holds 16 k of one part (fewer at its end); x and w keep their own places in the
+  // sequence of steps, because the first steps of w are asked for before x may be read.
+  const int row = lane >> 2, word = lane & 3;
+  const float* x_row = x + (size_t)(m0 + row) * K + word * 4;
+  const float* w_row = w + (size_t)(n0 + row) * K + word * 4;
+  struct Place { int part, at, stage; };       // the next step: of which part, from which of its k, into which stage
+  auto k_end = [&](int part) { return max(0, min(len, K - (first_part + part) * len)); };
+  auto skip_empty = [&](Place& p) { while (p.part < PARTS && p.at >= k_end(p.part)) { ++p.part; p.at = 0; } };
+  auto copy = [&](Place& p, auto rows, const float* src, int limit, int offset) {
+    if (p.part < PARTS) {
+      const int k = (first_part + p.part) * len + p.at;
+      const bool ok = p.at + word * 4 < k_end(p.part);
+      float* dst = ring + p.stage * FT_STAGE + offset;
+#pragma unroll
+      for (int i = 0; i < decltype(rows)::value / 8; ++i) {
+        const bool in = ok && row + 8 * i < limit;
+        f32_copy16(dst + f32_word_at(row + 8 * i, word), in ? src + (size_t)(8 * i) * K + k : w, in);
+      }
+      p.at += FT_K;
+      p.stage = p.stage == FT_STAGES - 1 ? 0 : p.stage + 1;
+      skip_empty(p);
+    }
+  };
+  Place of_x = {0, 0, 0}, of_w = {0, 0, 0}, now = {0, 0, 0};
+  skip_empty(of_x);
+  of_w = now = of_x;
+  auto load_x = [&]() { copy(of_x, std::integral_constant<int, FT_M>(), x_row, M - m0, 0); };
+  auto load_w = [&]() { copy(of_w, std::integral_constant<int, FT_N>(), w_row, N - n0, FT_M * FT_K); };
+#pragma unroll
+  for (int s = 0; s < FT_STAGES - 1; ++s) load_w();        // weights first
+  pdl_wait();
+#pragma unroll
+  for (int s = 0; s < FT_STAGES - 1; ++s) { load_x(); f32_commit(); }
+
+  float acc[OWN][OWN];
+#pragma unroll
+  for (int i = 0; i < OWN; ++i)
+#pragma unroll
+    for (int j = 0; j < OWN; ++j) acc[i][j] = 0.f;
+  float* my_sums = sums + team * FT_SUMS + ty * FT_SUM_STRIDE + tx;
+  for (int part = 0; part < PARTS; ++part) {
+    const int end = k_end(part);
+    for (int at = 0; at < end; at += FT_K) {
+      f32_wait<FT_STAGES - 2>();
+      __syncwarp();        // the step's words have arrived for every lane, and the step before it has been read by every lane
+      const float* as = ring + now.stage * FT_STAGE + ty * FT_K;
+      const float* bs = ring + now.stage * FT_STAGE + FT_M * FT_K + tx * FT_K;
+      now.stage = now.stage == FT_STAGES - 1 ? 0 : now.stage + 1;
+      load_x();
+      load_w();
+      f32_commit();
+      auto four = [&](int q) {
+        float4 a[OWN];
+#pragma unroll
+        for (int i = 0; i < OWN; ++i)       // rows ty + 4 i
+          a[i] = *reinterpret_cast<const float4*>(as + 4 * i * FT_K + ((q ^ (((ty >> 1) + 2 * i) & 3)) << 2));
+#pragma unroll
+        for (int j = 0; j < OWN; ++j) {     // rows tx + 8 j
+          const float4 b = *reinterpret_cast<const float4*>(bs + 8 * j * FT_K + ((q ^ ((tx >> 1) & 3)) << 2));
+#pragma unroll
+          for (int i = 0; i < OWN; ++i) acc[i][j] = fmaf(a[i].x, b.x, acc[i][j]);
+#pragma unroll
+          for (int i = 0; i < OWN; ++i) acc[i][j] = fmaf(a[i].y, b.y, acc[i][j]);
+#pragma unroll
+          for (int i = 0; i < OWN; ++i) acc[i][j] = fmaf(a[i].z, b.z, acc[i][j]);
+#pragma unroll
+          for (int i = 0; i < OWN; ++i) acc[i][j] = fmaf(a[i].w, b.w, acc[i][j]);
+        }
+      };
+      if (end - at >= FT_K) {
+#pragma unroll
+        for (int q = 0; q < FT_K / 4; ++q) four(q);
+      } else {
+        for (int q = 0; q < (end - at) / 4; ++q) four(q);
+      }
+    }
+    if (SPLIT == 1) {      // the part's sums join the group's, which wait in shared memory (nobody else touches these)
+#pragma unroll
+      for (int i = 0; i < OWN; ++i)
+#pragma unroll
+        for (int j = 0; j < OWN; ++j) {
+          float* s = my_sums + 4 * i * FT_SUM_STRIDE + 8 * j;
+          *s = part == 0 ? acc[i][j] : *s + acc[i][j];
+          acc[i][j] = 0.f;
+        }
+    }
+  }
+  f32_wait<0>();
+  if (SPLIT == 4) {
+    __syncthreads();       // every warp has read its ring to the end
+#pragma unroll
+    for (int i = 0; i < OWN; ++i)
+#pragma unroll
+      for (int j = 0; j < OWN; ++j) my_sums[4 * i * FT_SUM_STRIDE + 8 * j] = acc[i][j];
+  }
+  __syncthreads();
+  // ---- the four sums of an output (of groups, or of the group's parts) added left to right, four neighbouring columns a
+  // thread
+  auto add_up = [&](const float* const (&of)[4], int o) {
+    float4 s = *reinterpret_cast<const float4*>(of[0] + o);
+#pragma unroll
+    for (int q = 1; q < 4; ++q) {
+      const float4 v = *reinterpret_cast<const float4*>(of[q] + o);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    return s;
+  };
+  const bool by_fours = N % 4 == 0 && ((uintptr_t)out & 15) == 0;
+  auto store = [&](int r, int c, float4 s) {
+    if (m0 + r >= M) return;
+    float* o = out + (size_t)(m0 + r) * N + n0 + c;
+    if (by_fours && n0 + c < N) {
+      *reinterpret_cast<float4*>(o) = s;
+    } else {
+      const float v[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (n0 + c + e < N) o[e] = v[e];
+    }
+  };
+  constexpr int QUADS = FT_N / 4;
+  const float* of_team[4] = {sums, sums + FT_SUMS, sums + 2 * FT_SUMS, sums + 3 * FT_SUMS};
+  if (SPLIT == 1) {
+    for (int q = threadIdx.x; q < FT_M * QUADS; q += FT_THREADS) {
+      const int r = q / QUADS, c = q % QUADS * 4;
+      store(r, c, add_up(of_team, r * FT_SUM_STRIDE + c));
+    }
+  } else {
+    for (int q = threadIdx.x; q < FT_M * QUADS; q += FT_THREADS) {      // in place of the first part's
+      const int o = q / QUADS * FT_SUM_STRIDE + q % QUADS * 4;
+      *reinterpret_cast<float4*>(sums + o) = add_up(of_team, o);
+    }
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    const float* of_group[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) of_group[g] = cluster.map_shared_rank(sums, g);
+    constexpr int SHARE = FT_M / SPLIT;        // rows
+    for (int q = threadIdx.x; q < SHARE * QUADS; q += FT_THREADS) {
+      const int r = (int)blockIdx.z * SHARE + q / QUADS, c = q % QUADS * 4;
+      store(r, c, add_up(of_group, r * FT_SUM_STRIDE + c));
+    }
+    cluster.sync();        // nobody leaves while its sums are still read
+  }
+}
+
+// ----------------------------------------------------------------------------------- more rows, parts of 4 to 12 k
+constexpr int FS_OWN = 4, FS_K = 32, FS_STRIDE = FS_K + 4, FS_STAGES = 3;
+constexpr int FS_THREADS = (FT_M / FS_OWN) * (FT_N / FS_OWN), FS_STAGE = (FT_M + FT_N) * FS_STRIDE;     // floats
+
+// Thread tiles of 4 x 4 whose CTA goes through K in steps of 32 k that hold several parts each.
+template <int SPLIT>
+__global__ void __launch_bounds__(FS_THREADS, 4) gemm_f32_short_kernel(const float* x, const float* __restrict__ w, float* out, int M,
+                                                                    int N, int K) {
+  static_assert(SPLIT == 1 || SPLIT == 4, "all groups of K in one CTA, or one in each");
+  constexpr int BM = FT_M, BN = FT_N, TM = FS_OWN, TN = FS_OWN;
+  constexpr int THREADS = FS_THREADS, GROUPS = 4 / SPLIT, OUTS = TM * TN;
+  extern __shared__ float smem[];
+  float* kept = smem + FS_STAGES * FS_STAGE;           // SPLIT 4: [output of a thread][thread]
   pdl_trigger();
   const int tid = threadIdx.x;
   const int tx = tid % (BN / TN), ty = tid / (BN / TN);
   const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
   const int len = f32_part_length(K), range = GROUPS * 4 * len;           // k of a part, and of this CTA
-  const int k_first = blockIdx.z * range, mine = max(0, min(range, K - k_first)), total = (mine + FT_K - 1) / FT_K;
+  const int k_first = blockIdx.z * range, mine = max(0, min(range, K - k_first)), total = (mine + FS_K - 1) / FS_K;
 
   // Steps of 32 k, whatever parts they hold; either side (x or w) keeps its place, because the first steps of w are asked
   // for before x may be read. Zeros beyond the CTA's range and the matrix; parts beyond the matrix would add nothing
   // and are left out.
-  constexpr int WORDS = FT_K / 4;
+  constexpr int WORDS = FS_K / 4;
   auto load = [&](int& at, int rows, int r0, int limit, const float* src, float* dst) {
 #pragma unroll
     for (int c = tid; c < rows * WORDS; c += THREADS) {
       const int word = c % WORDS, r = c / WORDS, k = k_first + at + word * 4;
       const bool ok = at + word * 4 < mine && r0 + r < limit;
-      f32_copy16(dst + r * FT_STRIDE + word * 4, src + (ok ? (size_t)(r0 + r) * K + k : 0), ok);
+      f32_copy16(dst + r * FS_STRIDE + word * 4, src + (ok ? (size_t)(r0 + r) * K + k : 0), ok);
     }
-    at += FT_K;
+    at += FS_K;
   };
   int of_x = 0, of_w = 0;
-  auto load_x = [&](int stage) { load(of_x, BM, m0, M, x, smem + stage * FT_STAGE); };
-  auto load_w = [&](int stage) { load(of_w, BN, n0, N, w, smem + stage * FT_STAGE + BM * FT_STRIDE); };
+  auto load_x = [&](int stage) { load(of_x, BM, m0, M, x, smem + stage * FS_STAGE); };
+  auto load_w = [&](int stage) { load(of_w, BN, n0, N, w, smem + stage * FS_STAGE + BM * FS_STRIDE); };
 #pragma unroll
-  for (int s = 0; s < FT_STAGES - 1; ++s) load_w(s);        // weights first
+  for (int s = 0; s < FS_STAGES - 1; ++s) load_w(s);        // weights first
   pdl_wait();
 #pragma unroll
-  for (int s = 0; s < FT_STAGES - 1; ++s) { load_x(s); f32_commit(); }
+  for (int s = 0; s < FS_STAGES - 1; ++s) { load_x(s); f32_commit(); }
 
   float acc[TM][TN], group[TM][TN], sum[TM][TN];        // of a part, of a group, of the groups so far
 #pragma unroll
@@ -241,24 +419,24 @@ __global__ void __launch_bounds__(FT_THREADS, 4) gemm_f32_tile_kernel(const floa
   };
   int stage = 0, part = 0, left = len / 4, ahead = (mine + 3) / 4;       // of the part and of all, in steps of four
   for (int step = 0; step < total; ++step) {
-    f32_wait<FT_STAGES - 2>();
+    f32_wait<FS_STAGES - 2>();
     __syncthreads();
-    if (step + FT_STAGES - 1 < total) {
-      const int free = stage == 0 ? FT_STAGES - 1 : stage - 1;      // read in the step before this one
+    if (step + FS_STAGES - 1 < total) {
+      const int free = stage == 0 ? FS_STAGES - 1 : stage - 1;      // read in the step before this one
       load_x(free);
       load_w(free);
     }
     f32_commit();
-    const float* as = smem + stage * FT_STAGE + ty * FT_STRIDE;
-    const float* bs = smem + stage * FT_STAGE + (BM + tx) * FT_STRIDE;
-    stage = stage == FT_STAGES - 1 ? 0 : stage + 1;
+    const float* as = smem + stage * FS_STAGE + ty * FS_STRIDE;
+    const float* bs = smem + stage * FS_STAGE + (BM + tx) * FS_STRIDE;
+    stage = stage == FS_STAGES - 1 ? 0 : stage + 1;
     auto four = [&](int k) {
       float4 a[TM];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(as + i * (BM / TM) * FT_STRIDE + k);
+      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(as + i * (BM / TM) * FS_STRIDE + k);
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
-        const float4 v = *reinterpret_cast<const float4*>(bs + j * (BN / TN) * FT_STRIDE + k);
+        const float4 v = *reinterpret_cast<const float4*>(bs + j * (BN / TN) * FS_STRIDE + k);
 #pragma unroll
         for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].x, v.x, acc[i][j]);
 #pragma unroll
@@ -277,24 +455,13 @@ __global__ void __launch_bounds__(FT_THREADS, 4) gemm_f32_tile_kernel(const floa
         if ((++part & 3) == 0) end_group();
       }
     };
-    if constexpr (WHOLE) {
-#pragma unroll
-      for (int q = 0; q < WORDS; ++q) four(4 * q);
-      forward(WORDS);
-    } else {
-      const int fours = ahead < WORDS ? ahead : WORDS;
-      ahead -= fours;
-      for (int done = 0; done < fours;) {
-        const int run = left < fours - done ? left : fours - done;
-        if (run == WORDS) {
-#pragma unroll
-          for (int q = 0; q < WORDS; ++q) four(4 * q);
-        } else {
-          for (int q = 0; q < run; ++q) four(4 * (done + q));
-        }
-        done += run;
-        forward(run);
-      }
+    const int fours = ahead < WORDS ? ahead : WORDS;
+    ahead -= fours;
+    for (int done = 0; done < fours;) {
+      const int run = left < fours - done ? left : fours - done;
+      for (int q = 0; q < run; ++q) four(4 * (done + q));
+      done += run;
+      forward(run);
     }
   }
   end_part();         // (of a part that the matrix ends in; else they add zeros)
@@ -323,35 +490,41 @@ __global__ void __launch_bounds__(FT_THREADS, 4) gemm_f32_tile_kernel(const floa
   }
 }
 
-template <int SPLIT, bool WHOLE>
-static int launch_tile_form(const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
-  auto kernel = gemm_f32_tile_kernel<SPLIT, WHOLE>;
-  constexpr int own = (FT_STAGES * FT_STAGE + (SPLIT == 1 ? 0 : FT_M * FT_N)) * (int)sizeof(float);      // the ring, and the CTA's sums
-  constexpr int sm_bytes = 228 * 1024;
-  static bool ready[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 64 || !ready[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_bytes / 2 + 1024);
-    if (e != cudaSuccess) return (int)e;
-    if (dev < 64) ready[dev] = true;
-  }
-  if ((M + FT_M - 1) / FT_M > 65535) return TS_ERR_BAD_ARGUMENT;
-  const dim3 grid((N + FT_N - 1) / FT_N, (M + FT_M - 1) / FT_M, SPLIT);
-  // A grid of a few CTAs an SM starts while the kernel before it drains and piles up on the SMs that drain first: 64 rows of
-  // 1,024 x 3,072, 128 CTAs, took 41 us on half of the SMs and take 24 us when no SM has room for two. So a CTA asks for as
-  // much shared memory as lets no SM hold more than its share.
+// A grid of a few CTAs an SM starts while the kernel before it drains and piles up on the SMs that drain first: 64 rows of
+// 1,024 x 3,072, 128 CTAs, took 41 us on half of the SMs and take 24 us when no SM has room for two. So a CTA asks for as
+// much shared memory as lets no SM hold more than its share.
+constexpr int F32_SM_BYTES = 228 * 1024;
+template <typename Kernel>
+static int launch_spread(Kernel kernel, dim3 grid, int threads, int own, int cluster, const float* x, const float* w, float* out, int M,
+                         int N, int K, cudaStream_t stream) {
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F32_SM_BYTES / 2 + 1024);
+  if (e != cudaSuccess) return (int)e;
   const long long per_sm = ((long long)grid.x * grid.y * grid.z + 147) / 148;
-  const int share = per_sm <= 3 ? sm_bytes / ((int)per_sm + 1) + 1024 : 0;
+  const int share = per_sm <= 3 ? F32_SM_BYTES / ((int)per_sm + 1) + 1024 : 0;
   const int smem = share > own ? share : own;
-  if (SPLIT == 1) return launch(kernel, grid, FT_THREADS, smem, stream, x, w, out, M, N, K);
-  return launch_cluster(kernel, grid, FT_THREADS, smem, stream, dim3(1, 1, SPLIT), x, w, out, M, N, K);
+  if (cluster == 1) return launch(kernel, grid, threads, smem, stream, x, w, out, M, N, K);
+  return launch_cluster(kernel, grid, threads, smem, stream, dim3(1, 1, cluster), x, w, out, M, N, K);
 }
+
+// How many CTAs one SM runs of a grid of `ctas`, `per` of them at a time.
+static long long f32_rounds(long long ctas, int per) { return (ctas + 148 * per - 1) / (148 * per) * per; }
 
 template <int SPLIT>
 static int launch_tile(const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
-  return f32_part_length(K) % FT_K == 0 ? launch_tile_form<SPLIT, true>(x, w, out, M, N, K, stream)
-                                        : launch_tile_form<SPLIT, false>(x, w, out, M, N, K, stream);
+  if ((M + FT_M - 1) / FT_M > 65535) return TS_ERR_BAD_ARGUMENT;
+  const dim3 grid((N + FT_N - 1) / FT_N, (M + FT_M - 1) / FT_M, SPLIT);
+  if (f32_part_length(K) < FT_K) {
+    constexpr int own = (FS_STAGES * FS_STAGE + (SPLIT == 1 ? 0 : FT_M * FT_N)) * (int)sizeof(float);      // the ring, and the CTA's sums
+    return launch_spread(gemm_f32_short_kernel<SPLIT>, grid, FS_THREADS, own, SPLIT, x, w, out, M, N, K, stream);
+  }
+  constexpr int own = FT_TEAMS * (FT_STAGES * FT_STAGE + (SPLIT == 1 ? FT_SUMS : 0)) * (int)sizeof(float);
+  // Two CTAs an SM have registers to look further ahead, three hide more by taking turns; what counts more is the CTAs that an
+  // SM is given in the end (see f32_rounds). K over four CTAs, 1,024 columns and K = 2,048, two / three: 128 rows (256
+  // CTAs) 17.6 / 20.0 us, 190 rows (384) 33.7 / 27.1, 600 rows (1,216) 80.7 / 76.4; 64 rows of 4,096 x 1,024 (512) 21.3 / 26.4.
+  const long long ctas = (long long)grid.x * grid.y * grid.z;
+  if (SPLIT == 4 && f32_rounds(ctas, 3) <= f32_rounds(ctas, 2))
+    return launch_spread(gemm_f32_tile_kernel<SPLIT, SPLIT == 4 ? 3 : 2>, grid, FT_THREADS, own, SPLIT, x, w, out, M, N, K, stream);
+  return launch_spread(gemm_f32_tile_kernel<SPLIT, 2>, grid, FT_THREADS, own, SPLIT, x, w, out, M, N, K, stream);
 }
 
 }  // namespace ts
@@ -365,12 +538,13 @@ extern "C" int ts_gemm_f32(const float* x, const float* w, float* out, int M, in
   if (K % 4 != 0 || (((uintptr_t)x | (uintptr_t)w) & 15) != 0) return TS_ERR_UNSUPPORTED;
   if (form == 0) {
     const long long tiles = (long long)((M + FT_M - 1) / FT_M) * ((N + FT_N - 1) / FT_N);
-    // (K over 4 CTAs / over one: 128 rows of 4,096 x 1,024, 256 tiles, 39 / 42 us; 190 rows, 384 tiles, 53 / 53; 190 of
-    // 6,144 x 1,024, 576 tiles, 79 / 67; 64 of 1,024 x 3,072, 32 tiles, 24 / 73. The cluster's meeting weighs more the
-    // shorter K: 300 rows of 1,024 x 128, 160 tiles, 9.3 / 8.9; of 2,048 x 256, 320 tiles, 20 / 18; 40 of 4,096 x 64, 128
-    // tiles, 6.7 / 5.4; 128 of 2,048 x 256, 128 tiles, 9.4 / 10.6)
+    // K over four CTAs where an SM is then given less than a quarter as many CTAs' worth, the cluster's meeting counted as 384 k;
+    // many tiles, or a few hundred of a short K, fill the machine as they are (640 tiles of K = 1,024 81 / 88 us with one / four)
+    const long long four = f32_rounds(4 * tiles, 2) < f32_rounds(4 * tiles, 3) ? f32_rounds(4 * tiles, 2) : f32_rounds(4 * tiles, 3);
+    const bool split = f32_part_length(K) < FT_K ? tiles <= 400 && tiles <= 100 + K / 2
+                                                 : tiles <= (K < 512 ? 100 : 320) && four + 384.0 / K < 4.0 * f32_rounds(tiles, 1);
     if (M <= 16) form = M > 2 && N >= 2048 ? 2 : 1;
-    else form = tiles <= 400 && tiles <= 100 + K / 2 ? 4 : 3;
+    else form = split ? 4 : 3;
   }
   if (form <= 2) {
     if ((M + 7) / 8 > 65535) return TS_ERR_BAD_ARGUMENT;
