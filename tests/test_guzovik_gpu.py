@@ -73,6 +73,38 @@ def test_norms_around_a_sub_layer_kernel(dtype, rows, hidden) -> None:
         torch.testing.assert_close(got3.float(), want3.float(), **_tol(dtype))
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("rows, hidden", [(1, 4), (3, 2048), (7, 2052), (2, 4096), (2, 4100), (511, 256), (512, 256)])
+def test_norms_around_a_sub_layer_in_registers_and_in_shared_memory(dtype, rows, hidden) -> None:
+    """Rows on the 16-byte grid (few of them: a CTA a row, in registers) against the same values a single element off it, which
+    go the general way, with every optional operand: sums of squares in another order, 2^-21 of them at most, which may move
+    a result to its neighbour."""
+    from tinyserve_b200.kernels import ops
+
+    def off(t):
+        base = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")
+        base[1:] = t.flatten()
+        return base[1:].view(t.shape)
+
+    x, added = _rand(rows, hidden, seed=1, scale=2.0), _rand(rows, hidden, seed=6)
+    y, second = (_rand(rows, hidden, seed=s, scale=3.0, dtype=dtype) for s in (2, 7))
+    post, scale, w, bias, vec = (_rand(hidden, seed=s, scale=0.3, dtype=dtype) for s in (3, 4, 5, 8, 9))
+    pick = torch.tensor([rows - 1, 0], dtype=torch.int32, device="cuda")
+    close = {"atol": 1e-6, "rtol": 2.0 ** -20 if dtype == torch.float32 else 2.0 ** -7}
+    for delta, of_post, of_scale, extra in [
+            (y, post, scale, {}), (y, None, scale, {"delta_bias": bias}), (None, None, None, {"add_rows": added}),
+            (y, None, None, {"second": second, "second_scale": 0.5, "add_vec": vec}), (y, post, None, {"rows": pick})]:
+        res = []
+        for place in (lambda t: t.clone(), off):
+            on = lambda t: None if t is None else place(t)
+            stream, out = place(x), torch.empty(2 if "rows" in extra else rows, hidden, dtype=dtype, device="cuda")
+            more = {k: place(v) if isinstance(v, torch.Tensor) and k != "rows" else v for k, v in extra.items()}
+            ops.post_norm_add_rms_norm(stream, on(delta), on(of_post), on(of_scale), 1e-5, True, place(w), True, 1e-6, out, **more)
+            res.append((stream, out))
+        torch.testing.assert_close(res[0][0], res[1][0], atol=1e-5, rtol=1e-5)
+        torch.testing.assert_close(res[0][1].float(), res[1][1].float(), **close)
+
+
 def _tables(lens: list[int], page: int, seed: int):
     """Block tables over shuffled pages (two spare pages stay NaN), as a device tensor and lists."""
     need = [-(-n // page) for n in lens]
@@ -145,6 +177,32 @@ def test_latent_attention_kernels(dtype, heads, nope, rank, rot, rotary, page, w
     got, want, *_ = _latent_case(dtype, heads, nope, rank, rot, rotary, page, lens, news, window)
     assert not got.isnan().any()
     torch.testing.assert_close(got, want, **_tol(dtype))
+
+
+@pytest.mark.parametrize("tokens, heads, rank, rot, rotary", [(1, 1, 8, 8, 8), (4, 16, 512, 64, 64), (150, 5, 64, 16, 8), (700, 17, 24, 8, 0),
+                                                              (3, 2, 2048, 8, 8), (2, 2, 2056, 8, 8)])
+def test_latent_prepare_in_wide_pieces_and_by_elements(tokens, heads, rank, rot, rotary) -> None:
+    """Rows on the 16-byte grid against the same a single element off it, which go the general way: the queries bit for bit,
+    the latent to a neighbour (its sum of squares runs in another order)."""
+    from tinyserve_b200.kernels import ops
+
+    nope, d = 24, rank + rot
+    q_in, folded = _rand(tokens, heads * (nope + rot), seed=1, dtype=torch.bfloat16), _rand(heads, tokens, rank, seed=2, dtype=torch.bfloat16)
+    ckr, w = _rand(tokens, d + 8, seed=3, dtype=torch.bfloat16)[:, :d], _rand(rank, seed=4, dtype=torch.bfloat16)
+    angle = _rand(tokens, rotary // 2, seed=5) if rotary else None
+    cos, sin = (None, None) if angle is None else (angle.cos(), angle.sin())
+    slots = torch.randperm(tokens + 3, generator=torch.Generator().manual_seed(6))[:tokens].int().cuda()
+    for with_keys in (True, False):
+        res = []
+        for first in (0, 1):
+            q = torch.full((tokens * heads * d + 1,), float("nan"), dtype=torch.bfloat16, device="cuda")
+            cache = torch.full((tokens + 3, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+            out = q[first: first + tokens * heads * d].view(tokens, heads, d)
+            ops.latent_prepare(q_in, folded, ckr if with_keys else None, w if with_keys else None, 1e-5, cos, sin, rotary, True,
+                               slots if with_keys else None, cache if with_keys else None, heads, nope, rank, rot, out)
+            res.append((out.clone(), cache))
+        assert torch.equal(*[r[0] for r in res])
+        torch.testing.assert_close(res[0][1].float(), res[1][1].float(), equal_nan=True, atol=0, rtol=2.0 ** -7)
 
 
 @pytest.mark.parametrize("lens, news, window", [([1500, 700, 64, 3000], [1, 1, 1, 1], 0), ([1500, 130], [1, 1], 1024),
