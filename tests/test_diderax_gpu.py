@@ -173,6 +173,21 @@ def test_latent_attention_with_sinks_kernels(dtype, heads, rank, rot, page) -> N
         assert (none - got).abs().max() > 1e-2, "the sink changes nothing"
 
 
+@pytest.mark.parametrize("splits", [1, 2, 5, 8])
+@pytest.mark.parametrize("heads, rank, rot", [(1, 16, 0), (16, 512, 64), (17, 128, 16), (5, 512, 192), (33, 272, 32)])
+def test_latent_attention_of_single_tokens_over_any_number_of_ranges(heads, rank, rot, splits, monkeypatch) -> None:
+    """Keys around the 16 of a warp and the 64 or 128 of a round, fewer of them than ranges, heads around the 16 of a CTA, rows
+    so long that half the warps take keys, with and without sinks. In bfloat16 as everywhere: the probabilities are rounded to
+    it, so a sum of values of at most about 5 is off by 5 x 2^-9 and rounded once more."""
+    from tinyserve_b200.kernels import ops
+
+    monkeypatch.setattr(ops, "latent_splits", lambda *args: splits)
+    lens = [1, 15, 16, 17, 64, 65, 127, 128, 129, 256, 257, 1000]
+    for sinks in (None, _rand(heads, seed=9, scale=2.0)):
+        got, want, *_ = _sink_case(torch.bfloat16, heads, rank, rot, 16, lens, [1] * len(lens), sinks)
+        torch.testing.assert_close(got, want, **_tol(torch.bfloat16))
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("new", [1, 2, 70])
 @pytest.mark.parametrize("rank, rot, page", [(16, 8, 16), (64, 32, 16), (24, 2, 4)])

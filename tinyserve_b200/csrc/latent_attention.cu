@@ -14,9 +14,12 @@
 //    A warp owns a row at a time: each lane scores one key of the tile, then each lane owns
 //    output columns. Rows of other requests or beyond a request's positions are never loaded.
 #define TS_PDL_CLASS PDL_ATTENTION
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace ts {
+namespace cg = cooperative_groups;
 
 // ------------------------------------------------------------------------ prepare
 struct LatentPrepArgs {
@@ -88,6 +91,71 @@ __global__ void latent_prepare_kernel(LatentPrepArgs a) {
         from_float<T>(rotated(qi + (size_t)h * (a.nope + a.rot) + a.nope, i, c, s, rdim, a.interleaved));
   }
 }
+
+// The same where rows and pieces of 8 elements lie on the 16-byte grid (bf16): the folded queries travel as 16-byte pieces,
+// and a token's heads go to `gridDim.y` CTAs, of which the first also norms the latent. Bound by latency: with a CTA a
+// token, element by element and two divisions each, four tokens of 16 heads of 512 + 64 elements took 10.9 us, with this 2.7;
+// 2,048 tokens 44.5 and 15.5.
+__global__ void latent_prepare_vec_kernel(LatentPrepArgs a) {
+  __shared__ float parts[32];
+  pdl_trigger();
+  const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int D = a.rank + a.rot;
+  const bf16* w = (const bf16*)a.norm_weight;
+  const bool owner = a.slots && blockIdx.y == 0;       // of the token's latent
+  Vec<bf16> gain[2];                                   // constants of the model: in front of the wait
+  const int pieces = a.rank >> 3;
+  if (owner)
+    for (int j = 0; j < 2; ++j)
+      if ((int)threadIdx.x + j * (int)blockDim.x < pieces) gain[j].load(w + 8 * (threadIdx.x + j * blockDim.x));
+  pdl_wait();
+  const float* c = a.cos_t ? a.cos_t + (size_t)t * (a.rotary_dim >> 1) : nullptr;
+  const float* s = a.sin_t ? a.sin_t + (size_t)t * (a.rotary_dim >> 1) : nullptr;
+  const int rdim = c ? a.rotary_dim : 0;
+  // ---- the queries: a warp takes a head
+  const int share = (a.heads + gridDim.y - 1) / gridDim.y;
+  const int h_end = min(a.heads, ((int)blockIdx.y + 1) * share);
+  for (int h = blockIdx.y * share + warp; h < h_end; h += warps) {
+    bf16* qo = (bf16*)a.q_out + ((size_t)t * a.heads + h) * D;
+    const bf16* qf = (const bf16*)a.q_folded + ((size_t)h * a.num_tokens + t) * a.rank;
+    for (int i = lane; i < pieces; i += 32) *reinterpret_cast<uint4*>(qo + 8 * i) = *reinterpret_cast<const uint4*>(qf + 8 * i);
+    const bf16* qi = (const bf16*)a.q_in + (size_t)t * a.q_stride + (size_t)h * (a.nope + a.rot) + a.nope;
+    for (int i = 2 * lane; i < a.rot; i += 64)
+      *reinterpret_cast<__nv_bfloat162*>(qo + a.rank + i) = __floats2bfloat162_rn(
+          rotated(qi, i, c, s, rdim, a.interleaved), rotated(qi, i + 1, c, s, rdim, a.interleaved));
+  }
+  if (!owner) return;
+  // ---- the latent and the shared key part
+  const bf16* row = (const bf16*)a.ckr + (size_t)t * a.ckr_stride;
+  bf16* dst = (bf16*)a.cache + (size_t)a.slots[t] * D;
+  float v[2][8], ss = 0.f;
+  for (int j = 0; j < 2; ++j) {
+    const int i = threadIdx.x + j * blockDim.x;
+    if (i >= pieces) continue;
+    Vec<bf16> raw;
+    raw.load(row + 8 * i);
+    raw.unpack(v[j]);
+    for (int e = 0; e < 8; ++e) ss = fmaf(v[j][e], v[j][e], ss);
+  }
+  for (int i = threadIdx.x; i < a.rot; i += blockDim.x)
+    dst[a.rank + i] = from_float<bf16>(rotated(row + a.rank, i, c, s, rdim, a.interleaved));
+  ss = warp_sum(ss);
+  if (lane == 0) parts[warp] = ss;
+  __syncthreads();
+  ss = warp_sum(lane < warps ? parts[lane] : 0.f);
+  const float rstd = rsqrtf(ss / (float)a.rank + a.eps);
+  for (int j = 0; j < 2; ++j) {
+    const int i = threadIdx.x + j * blockDim.x;
+    if (i >= pieces) continue;
+    float g[8];
+    gain[j].unpack(g);
+    for (int e = 0; e < 8; ++e) g[e] = v[j][e] * rstd * g[e];
+    Vec<bf16> o;
+    o.pack(g);
+    o.store(dst + 8 * i);
+  }
+}
+constexpr int LATENT_PREP_THREADS = 128;
 
 // ---------------------------------------------------------------------- attention
 struct LatentAttnArgs {
@@ -260,8 +328,6 @@ static int launch_latent(const LatentAttnArgs& a, int max_query_len, cudaStream_
 // P V to its columns, V being the first R elements of the very same rows in shared memory (read
 // transposed by ldmatrix). Both warps of a row group form the same S; that costs a third of the
 // multiply-adds again and saves exchanging P through shared memory.
-// With `splits` > 1 (steps of single tokens) a CTA takes one range of the keys and leaves an
-// unnormalised partial result; latent_merge_kernel adds the ranges up.
 constexpr int LM_THREADS = 256, LM_ROWS = 64, LM_TK = 32;
 
 __device__ __forceinline__ void lm_cp_async16(void* smem, const void* gmem, bool valid) {
@@ -290,15 +356,9 @@ __device__ __forceinline__ uint32_t lm_pack(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-struct LatentSplit {
-  int splits;
-  float* part_acc;   // [T, H, splits, R]
-  float* part_ml;    // [T, H, splits, 2]
-};
-
 // NB: blocks of 8 output columns a warp owns at most (its half of R is 8 NB columns or fewer).
 template <int NB>
-__global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(LatentAttnArgs a, LatentSplit sp, int ld) {
+__global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(LatentAttnArgs a, int ld) {
   extern __shared__ __align__(16) unsigned char lm_raw[];
   bf16* Qs = (bf16*)lm_raw;                        // [LM_ROWS][ld]
   bf16* Ks = Qs + (size_t)LM_ROWS * ld;            // [2][LM_TK][ld]
@@ -311,8 +371,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(Lat
   const int t0 = blockIdx.x * a.tokens_per_cta;
   if (t0 >= n) return;
   const int nt = min(a.tokens_per_cta, n - t0);
-  const int chunk = blockIdx.z / sp.splits, split = blockIdx.z - chunk * sp.splits;
-  const int h0 = chunk * a.heads_per_cta;
+  const int h0 = blockIdx.z * a.heads_per_cta;
   const int nh = min(a.heads_per_cta, a.heads - h0);
   const int nrows = nt * nh;
   const int ctx = a.ctx_lens[seq];
@@ -325,13 +384,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(Lat
   const int chunks = D >> 3;                       // 16-byte pieces of a row
 
   const int qpos_first = first_pos + t0, qpos_last = first_pos + t0 + nt - 1;
-  int k_lo = a.window > 0 ? max(0, qpos_first - a.window + 1) : 0;
-  int k_hi = qpos_last + 1;
-  if (sp.splits > 1) {
-    const int per = (((k_hi - k_lo) + sp.splits - 1) / sp.splits + LM_TK - 1) / LM_TK * LM_TK;
-    k_lo = k_lo + split * per;
-    k_hi = min(k_hi, k_lo + per);
-  }
+  const int k_lo = a.window > 0 ? max(0, qpos_first - a.window + 1) : 0, k_hi = qpos_last + 1;
   const int k_begin = (k_lo / LM_TK) * LM_TK;
   const int tiles = k_hi > k_begin ? (k_hi - k_begin + LM_TK - 1) / LM_TK : 0;
 
@@ -501,75 +554,300 @@ __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(Lat
     const int tt = r / nh, hh = r - tt * nh;
     const size_t orow = (size_t)(row0 + t0 + tt) * a.heads + h0 + hh;
     const float l = half ? l_b : l_a, m = half ? m_b : m_a;
-    if (sp.splits == 1) {
-      float den = l, keep = 1.f;
-      if (a.sinks) {
-        const float sk = a.sinks[h0 + hh] * 1.4426950408889634f;
-        const float m_new = fmaxf(m, sk);
-        keep = exp2f(m - m_new);                      // m = -inf gives 0
-        den = den * keep + exp2f(sk - m_new);
-      }
-      const float inv = den > 0.f ? keep / den : 0.f;
-      bf16* out = (bf16*)a.out + orow * R;
+    float den = l, keep = 1.f;
+    if (a.sinks) {
+      const float sk = a.sinks[h0 + hh] * 1.4426950408889634f;
+      const float m_new = fmaxf(m, sk);
+      keep = exp2f(m - m_new);                        // m = -inf gives 0
+      den = den * keep + exp2f(sk - m_new);
+    }
+    const float inv = den > 0.f ? keep / den : 0.f;
+    bf16* out = (bf16*)a.out + orow * R;
 #pragma unroll
-      for (int j = 0; j < NB; ++j) {
-        const int col = col_base + j * 8 + (lane & 3) * 2;
-        if (col < R) *reinterpret_cast<__nv_bfloat162*>(out + col) = __floats2bfloat162_rn(o[j][half * 2] * inv, o[j][half * 2 + 1] * inv);
-      }
-    } else {
-      float* acc = sp.part_acc + (orow * sp.splits + split) * R;
-#pragma unroll
-      for (int j = 0; j < NB; ++j) {
-        const int col = col_base + j * 8 + (lane & 3) * 2;
-        if (col < R) *reinterpret_cast<float2*>(acc + col) = make_float2(o[j][half * 2], o[j][half * 2 + 1]);
-      }
-      if (ch == 0 && (lane & 3) == 0) {
-        sp.part_ml[(orow * sp.splits + split) * 2] = m;
-        sp.part_ml[(orow * sp.splits + split) * 2 + 1] = l;
-      }
+    for (int j = 0; j < NB; ++j) {
+      const int col = col_base + j * 8 + (lane & 3) * 2;
+      if (col < R) *reinterpret_cast<__nv_bfloat162*>(out + col) = __floats2bfloat162_rn(o[j][half * 2] * inv, o[j][half * 2 + 1] * inv);
     }
   }
 }
 
-// out[row, :] = sum_s 2^(m_s - M) acc_s / sum_s 2^(m_s - M) l_s over the key ranges of a row.
-// With sinks, head (row % heads) adds 2^(sink log2(e) - M) to the denominator.
-__global__ void latent_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, bf16* __restrict__ out,
-                                    int splits, int R, const float* __restrict__ sinks, int heads) {
+// ------------------------------------------- attention of single tokens, tensor cores
+// A step in which every request brings one token: the 16 heads of a CTA are the 16 rows of an mma tile. Bound by the latency
+// of the chain from the cached rows to the result, so that chain is kept short: a CTA of eight warps takes `key_warps` x 16
+// keys of its range at a time. A warp fetches 16 of them (those of earlier steps in front of the wait for the
+// kernels before this one) and scores them for all heads; the warps agree on the maxima and leave their probabilities in
+// shared memory, and each then sums all keys of the round for an eighth of the output columns. The key ranges
+// of a request are the CTAs of a cluster, which add up their results through distributed shared memory.
+// (A kernel of 64-row tiles, three quarters of them empty, which walked over 32 keys at a time and left its ranges to a second
+// kernel, as this replaces / this, four requests of 16 heads of 512 + 64 elements: 60 keys 13.2 / 9.2 us, 500 24.3 / 10.4, 1,024
+// 27.4 / 9.5, 4,000 55 / 29.6.)
+constexpr int LD_WARPS = 8, LD_THREADS = LD_WARPS * 32, LD_HEADS = 16, LD_MAX_KEYS = LD_WARPS * 16, LD_MAX_SPLITS = 8, LD_P_STRIDE = LD_MAX_KEYS + 8;
+
+__host__ __device__ __forceinline__ size_t latent_single_smem(int ld, int key_warps) {
+  return sizeof(bf16) * ((size_t)(LD_HEADS + 16 * key_warps) * ld + LD_HEADS * LD_P_STRIDE);
+}
+
+// NB: blocks of 8 output columns of a warp, an even number.
+template <int NB>
+__global__ void __launch_bounds__(LD_THREADS, 1) latent_single_kernel(LatentAttnArgs a, int ld, int key_warps, int splits) {
+  extern __shared__ __align__(16) unsigned char lm_raw[];
+  bf16* Qs = (bf16*)lm_raw;                              // [LD_HEADS][ld]
+  bf16* Ks = Qs + (size_t)LD_HEADS * ld;                 // [16 key_warps][ld]; at the end the CTA's sums, [LD_HEADS][R] floats
+  bf16* Ps = Ks + (size_t)16 * key_warps * ld;           // [LD_HEADS][LD_P_STRIDE]
+  __shared__ float warp_max_s[LD_WARPS][LD_HEADS], warp_sum_s[LD_WARPS][LD_HEADS];
+  __shared__ float range_m[LD_HEADS], range_l[LD_HEADS], share_s[LD_MAX_SPLITS][LD_HEADS];
   pdl_trigger();
+  const int R = a.rank, D = a.rank + a.rot;
+  const int seq = blockIdx.y;
+  const int row = a.cu_q[seq];
+  if (a.cu_q[seq + 1] == row) return;                    // (the whole cluster)
+  const int chunk = blockIdx.z / splits, split = blockIdx.z - chunk * splits;
+  const int h0 = chunk * LD_HEADS, nh = min(LD_HEADS, a.heads - h0);
+  const int ctx = a.ctx_lens[seq];
+  const int* table = a.block_tables + (size_t)seq * a.table_width;
+  const bf16* cache = (const bf16*)a.cache;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int pieces = D >> 3;                             // 16-byte pieces of a row
+  const int keys_round = 16 * key_warps;
+  const int first = a.window > 0 ? max(0, ctx - a.window) : 0;
+  const int per = ((ctx - first + splits - 1) / splits + 15) / 16 * 16;
+  const int k_lo = first + split * per, k_hi = min(ctx, k_lo + per);
+
+  // This warp's 16 keys of the round that starts at k0: those below `end` only, then (`rest`) the others.
+  auto load_keys = [&](int k0, int end, bool rest) {
+    if (warp >= key_warps) return;
+    const int kpos = k0 + 16 * warp + (lane & 15);
+    int crow = 0;
+    if (kpos < k_hi) {
+      const int pg = kpos / a.page_size;
+      crow = table[pg] * a.page_size + (kpos - pg * a.page_size);
+    }
+    for (int r = 0; r < 16; ++r) {
+      const int pos = k0 + 16 * warp + r;
+      const int cr = __shfl_sync(0xffffffffu, crow, r);
+      if ((pos < end) == rest) continue;                 // warp-uniform
+      const bool ok = pos < k_hi;
+      const bf16* src = cache + (size_t)cr * D;
+      bf16* dst = Ks + (size_t)(16 * warp + r) * ld;
+      for (int i = lane; i < pieces; i += 32) lm_cp_async16(dst + 8 * i, src + 8 * i, ok);
+    }
+  };
+  const int before = min(k_hi, ctx - 1);                 // the newest row is written by the kernels before this one
+  if (k_lo < k_hi) load_keys(k_lo, before, false);
   pdl_wait();
-  const size_t row = blockIdx.x;
-  const float* ml = part_ml + row * splits * 2;
-  float mm = -INFINITY;
-  for (int s = 0; s < splits; ++s) mm = fmaxf(mm, ml[2 * s]);
-  float den = 0.f;
-  if (sinks) {
-    const float sk = sinks[row % heads] * 1.4426950408889634f;
-    mm = fmaxf(mm, sk);
-    den = exp2f(sk - mm);
+  for (int r = warp; r < LD_HEADS; r += LD_WARPS) {
+    const bf16* src = (const bf16*)a.q + ((size_t)row * a.heads + h0 + (r < nh ? r : 0)) * D;
+    for (int i = lane; i < pieces; i += 32) lm_cp_async16(Qs + (size_t)r * ld + 8 * i, src + 8 * i, r < nh);
   }
-  for (int s = 0; s < splits; ++s) den += ml[2 * s] == -INFINITY ? 0.f : ml[2 * s + 1] * exp2f(ml[2 * s] - mm);
-  const float inv = den > 0.f ? 1.f / den : 0.f;
-  for (int c = threadIdx.x; c < R; c += blockDim.x) {
-    float num = 0.f;
-    for (int s = 0; s < splits; ++s)
-      if (ml[2 * s] != -INFINITY) num += part_acc[(row * splits + s) * R + c] * exp2f(ml[2 * s] - mm);
-    out[row * R + c] = from_float<bf16>(num * inv);
+  if (k_lo < k_hi) load_keys(k_lo, before, true);
+  lm_commit();
+
+  const uint32_t q_base = (uint32_t)__cvta_generic_to_shared(Qs), k_base = (uint32_t)__cvta_generic_to_shared(Ks),
+                 p_base = (uint32_t)__cvta_generic_to_shared(Ps);
+  const int g = lane >> 2, t = lane & 3;                 // this thread's rows g and g + 8
+  const int col_base = warp * NB * 8;
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};      // of the rows; l: this warp's keys alone
+  float o[NB][4];
+#pragma unroll
+  for (int j = 0; j < NB; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
+  for (int k0 = k_lo; k0 < k_hi; k0 += keys_round) {
+    if (k0 > k_lo) {
+      __syncthreads();                                   // the round before has been read
+      load_keys(k0, k_hi, false);
+      load_keys(k0, k_hi, true);
+      lm_commit();
+    }
+    lm_wait<0>();
+    __syncthreads();
+    float s[2][4], mx[2] = {-INFINITY, -INFINITY};
+    if (warp < key_warps) {
+      // ---- S = Q K^T of 16 heads x 16 keys: two chains for each of two blocks of 8 keys
+      float c[2][2][4] = {};
+      const uint32_t qrow = q_base + 2u * (uint32_t)((lane & 15) * ld + (lane >> 4) * 8);
+      const uint32_t krow = k_base + 2u * (uint32_t)((16 * warp + (lane & 7) + ((lane >> 4) << 3)) * ld + ((lane >> 3) & 1) * 8);
+      for (int kk = 0; kk < D; kk += 32) {
+        uint32_t qa[2][4], kb[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          if (kk + 16 * i < D) {
+            lm_ldmatrix(qa[i], qrow + 2u * (kk + 16 * i));
+            lm_ldmatrix(kb[i], krow + 2u * (kk + 16 * i));
+          }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          if (kk + 16 * i < D) {
+            lm_mma(c[i][0], qa[i], kb[i][0], kb[i][1]);
+            lm_mma(c[i][1], qa[i], kb[i][2], kb[i][3]);
+          }
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int kpos = k0 + 16 * warp + j * 8 + 2 * t + (e & 1);
+          s[j][e] = kpos < k_hi ? (c[0][j][e] + c[1][j][e]) * a.scale_log2 : -INFINITY;
+          mx[e >> 1] = fmaxf(mx[e >> 1], s[j][e]);
+        }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
+        mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
+        if (t == 0) warp_max_s[warp][g + 8 * h] = mx[h];
+      }
+    }
+    __syncthreads();
+    float corr[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float m_new = m[h];
+      for (int w = 0; w < key_warps; ++w) m_new = fmaxf(m_new, warp_max_s[w][g + 8 * h]);
+      corr[h] = m_new == -INFINITY ? 1.f : exp2f(m[h] - m_new);      // m = -inf gives 0
+      m[h] = m_new;
+      l[h] *= corr[h];
+    }
+    if (warp < key_warps) {
+      float sum[2] = {0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          s[j][e] = s[j][e] == -INFINITY ? 0.f : exp2f(s[j][e] - m[e >> 1]);
+          sum[e >> 1] += s[j][e];
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          *reinterpret_cast<uint32_t*>(Ps + (g + 8 * h) * LD_P_STRIDE + 16 * warp + 8 * j + 2 * t) = lm_pack(s[j][2 * h], s[j][2 * h + 1]);
+      }
+      l[0] += sum[0];
+      l[1] += sum[1];
+    }
+    __syncthreads();
+    // ---- O = O corr + P V over this warp's columns, V being the first R elements of the keys
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      o[j][0] *= corr[0]; o[j][1] *= corr[0];
+      o[j][2] *= corr[1]; o[j][3] *= corr[1];
+    }
+    const int steps = (min(keys_round, k_hi - k0) + 15) / 16;
+    const uint32_t prow = p_base + 2u * (uint32_t)((lane & 15) * LD_P_STRIDE + (lane >> 4) * 8);
+    const uint32_t vrow = k_base + 2u * (uint32_t)(((lane & 7) + ((lane >> 3) & 1) * 8) * ld + (lane >> 4) * 8);
+    for (int ks = 0; ks < steps; ++ks) {
+      uint32_t pf[4];
+      lm_ldmatrix(pf, prow + 2u * 16 * ks);
+#pragma unroll
+      for (int j = 0; j < NB; j += 2) {
+        const int col = col_base + 8 * j;
+        if (col < R) {                                   // warp-uniform; R % 16 == 0
+          uint32_t vf[4];
+          lm_ldmatrix_t(vf, vrow + 2u * (uint32_t)(ks * 16 * ld + col));
+          lm_mma(o[j], pf, vf[0], vf[1]);
+          lm_mma(o[j + 1], pf, vf[2], vf[3]);
+        }
+      }
+    }
   }
+  // ---- the range's maximum, weight and sums, where the keys were
+  lm_wait<0>();
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
+    l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
+    if (t == 0) warp_sum_s[warp][g + 8 * h] = l[h];
+    if (warp == 0 && t == 0) range_m[g + 8 * h] = m[h];
+  }
+  __syncthreads();
+  float* sums = reinterpret_cast<float*>(Ks);            // [LD_HEADS][R]
+#pragma unroll
+  for (int j = 0; j < NB; ++j) {
+    const int col = col_base + 8 * j + 2 * t;
+    if (col < R) {
+      *reinterpret_cast<float2*>(sums + (size_t)g * R + col) = make_float2(o[j][0], o[j][1]);
+      *reinterpret_cast<float2*>(sums + (size_t)(g + 8) * R + col) = make_float2(o[j][2], o[j][3]);
+    }
+  }
+  if (tid < LD_HEADS) {
+    float sum = 0.f;
+    for (int w = 0; w < key_warps; ++w) sum += warp_sum_s[w][tid];
+    range_l[tid] = sum;
+  }
+  cg::cluster_group cluster = cg::this_cluster();
+  if (splits > 1) cluster.sync(); else __syncthreads();
+  // ---- every range's share of a head's result: 2^(m_range - M) / sum over the ranges (and the sink)
+  if (tid < LD_HEADS && tid < nh) {
+    float top = -INFINITY, mr[LD_MAX_SPLITS], lr[LD_MAX_SPLITS];
+#pragma unroll
+    for (int q = 0; q < LD_MAX_SPLITS; ++q) {
+      mr[q] = q < splits ? (splits > 1 ? cluster.map_shared_rank(range_m, q) : range_m)[tid] : -INFINITY;
+      lr[q] = q < splits ? (splits > 1 ? cluster.map_shared_rank(range_l, q) : range_l)[tid] : 0.f;
+      top = fmaxf(top, mr[q]);
+    }
+    float den = 0.f;
+    if (a.sinks) {
+      const float sk = a.sinks[h0 + tid] * 1.4426950408889634f;
+      top = fmaxf(top, sk);
+      den = exp2f(sk - top);
+    }
+#pragma unroll
+    for (int q = 0; q < LD_MAX_SPLITS; ++q) {
+      mr[q] = mr[q] == -INFINITY ? 0.f : exp2f(mr[q] - top);
+      den += lr[q] * mr[q];
+    }
+    const float inv = den > 0.f ? 1.f / den : 0.f;
+#pragma unroll
+    for (int q = 0; q < LD_MAX_SPLITS; ++q)
+      if (q < splits) share_s[q][tid] = mr[q] * inv;
+  }
+  __syncthreads();
+  const float* of_range[LD_MAX_SPLITS];
+#pragma unroll
+  for (int q = 0; q < LD_MAX_SPLITS; ++q) of_range[q] = splits > 1 && q < splits ? cluster.map_shared_rank(sums, q) : sums;
+  const int quads = R / 4;
+  for (int idx = split * LD_THREADS + tid; idx < nh * quads; idx += splits * LD_THREADS) {
+    const int h = idx / quads, at = idx * 4;             // [LD_HEADS][R] without gaps
+    float4 v[LD_MAX_SPLITS];
+#pragma unroll
+    for (int q = 0; q < LD_MAX_SPLITS; ++q)
+      if (q < splits) v[q] = *reinterpret_cast<const float4*>(of_range[q] + at);
+    float r[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int q = 0; q < LD_MAX_SPLITS; ++q)
+      if (q < splits) {
+        const float by = share_s[q][h];
+        r[0] = fmaf(v[q].x, by, r[0]); r[1] = fmaf(v[q].y, by, r[1]);
+        r[2] = fmaf(v[q].z, by, r[2]); r[3] = fmaf(v[q].w, by, r[3]);
+      }
+    Quad<bf16>::store((bf16*)a.out + ((size_t)row * a.heads + h0) * R + at, r);
+  }
+  if (splits > 1) cluster.sync();                        // nobody leaves while its sums are still read
 }
 
 template <int NB>
-static int launch_latent_mma(const LatentAttnArgs& a, const LatentSplit& sp, int max_query_len, cudaStream_t stream) {
-  const int D = a.rank + a.rot;
-  int ld = D + 8;
-  if (((ld >> 3) & 1) == 0) ld += 8;                 // rows 16 (odd) bytes apart: ldmatrix reads without bank conflicts
+static int launch_latent_single(const LatentAttnArgs& a, int ld, int splits, cudaStream_t stream) {
+  const int key_warps = latent_single_smem(ld, LD_WARPS) <= 200 * 1024 ? LD_WARPS : LD_WARPS / 2;
+  const size_t smem = latent_single_smem(ld, key_warps);
+  auto kern = latent_single_kernel<NB>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  const dim3 grid(1, a.num_seqs, (a.heads + LD_HEADS - 1) / LD_HEADS * splits);
+  if (splits == 1) return launch(kern, grid, LD_THREADS, smem, stream, a, ld, key_warps, splits);
+  return launch_cluster(kern, grid, LD_THREADS, smem, stream, dim3(1, 1, splits), a, ld, key_warps, splits);
+}
+
+// Elements from one row to the next in shared memory: an odd number of 16 bytes, so that ldmatrix reads without bank conflicts.
+static int latent_row_length(int D) { return ((D + 8) >> 3) & 1 ? D + 8 : D + 16; }
+
+template <int NB>
+static int launch_latent_mma(const LatentAttnArgs& a, int max_query_len, cudaStream_t stream) {
+  const int ld = latent_row_length(a.rank + a.rot);
   const size_t smem = sizeof(bf16) * (size_t)(LM_ROWS + 2 * LM_TK) * ld;
   if (smem > 220 * 1024) return TS_ERR_UNSUPPORTED;
   auto kern = latent_attention_mma_kernel<NB>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  const int chunks = (a.heads + a.heads_per_cta - 1) / a.heads_per_cta;
-  dim3 grid((max_query_len + a.tokens_per_cta - 1) / a.tokens_per_cta, a.num_seqs, chunks * sp.splits);
-  return launch(kern, grid, LM_THREADS, smem, stream, a, sp, ld);
+  dim3 grid((max_query_len + a.tokens_per_cta - 1) / a.tokens_per_cta, a.num_seqs, (a.heads + a.heads_per_cta - 1) / a.heads_per_cta);
+  return launch(kern, grid, LM_THREADS, smem, stream, a, ld);
 }
 
 }  // namespace ts
@@ -591,6 +869,15 @@ extern "C" int ts_latent_prepare(const void* q_in, long long q_stride, const voi
   a.norm_weight = norm_weight; a.eps = eps; a.cos_t = rotary_dim ? cos_t : nullptr; a.sin_t = rotary_dim ? sin_t : nullptr;
   a.rotary_dim = rotary_dim; a.interleaved = interleaved; a.slots = slots; a.cache = cache; a.q_out = q_out;
   a.num_tokens = num_tokens; a.heads = heads; a.nope = nope; a.rank = rank; a.rot = rot;
+  const bool grid16 = ((uintptr_t)q_folded | (uintptr_t)(slots ? ckr : nullptr) | (uintptr_t)(slots ? norm_weight : nullptr) |
+                       (uintptr_t)(slots ? cache : nullptr) | (uintptr_t)q_out) % 16 == 0;
+  if (dtype == TS_DTYPE_BF16 && grid16 && rank % 8 == 0 && rot % 8 == 0 && ckr_stride % 8 == 0 && rank <= 16 * LATENT_PREP_THREADS) {
+    // a CTA takes a token's heads where the tokens fill the machine, else a share of them, at least a head a warp
+    const int most = (heads + LATENT_PREP_THREADS / 32 - 1) / (LATENT_PREP_THREADS / 32);
+    int cut = 4 * 148 / num_tokens;
+    cut = cut < 1 ? 1 : cut > most ? most : cut;
+    return launch(latent_prepare_vec_kernel, dim3(num_tokens, cut), LATENT_PREP_THREADS, 0, stream, a);
+  }
   if (dtype == TS_DTYPE_F32) return launch(latent_prepare_kernel<float>, num_tokens, 256, 0, stream, a);
   if (dtype == TS_DTYPE_BF16) return launch(latent_prepare_kernel<bf16>, num_tokens, 256, 0, stream, a);
   return TS_ERR_BAD_ARGUMENT;
@@ -599,21 +886,17 @@ extern "C" int ts_latent_prepare(const void* q_in, long long q_stride, const voi
 // Largest latent size the kernel takes (32 output columns per lane and step, 16 steps).
 extern "C" int ts_latent_attention_max_rank() { return 512; }
 
-// Whether the tensor-core form takes these sizes (bf16 only).
+// Whether the tensor-core forms take these sizes (bf16 only).
 extern "C" int ts_latent_attention_mma_takes(int rank, int rot) {
   const int D = rank + rot;
-  int ld = D + 8;
-  if (((ld >> 3) & 1) == 0) ld += 8;
-  return rank % 16 == 0 && D % 16 == 0 && rank <= 512 && sizeof(bf16) * (size_t)(LM_ROWS + 2 * LM_TK) * ld <= 220 * 1024;
+  return rank % 16 == 0 && D % 16 == 0 && rank <= 512 && sizeof(bf16) * (size_t)(LM_ROWS + 2 * LM_TK) * latent_row_length(D) <= 220 * 1024;
 }
 
-// `splits` > 1 (steps of single tokens, tensor-core form only): key ranges per request, with scratch
-// part_acc [T, heads, splits, rank] and part_ml [T, heads, splits, 2] floats.
+// `splits`: key ranges per request, 1 to 8 (more than one: steps of single tokens, tensor-core form only).
 extern "C" int ts_latent_attention(const void* q, void* out, const void* cache, const int* block_tables, int table_width,
                                    const int* cu_q, const int* ctx_lens, int num_seqs, int max_query_len, int heads,
                                    int rank, int rot, int page_size, float scale, int window, int dtype, int use_mma,
-                                   int splits, float* part_acc, float* part_ml, int num_tokens, const float* sinks,
-                                   cudaStream_t stream) {
+                                   int splits, const float* sinks, cudaStream_t stream) {
   if (num_seqs <= 0 || max_query_len <= 0) return 0;
   if (heads <= 0 || rank <= 0 || rank > 512 || rot < 0 || page_size <= 0 || window < 0) return TS_ERR_BAD_ARGUMENT;
   LatentAttnArgs a;
@@ -623,20 +906,21 @@ extern "C" int ts_latent_attention(const void* q, void* out, const void* cache, 
   a.sinks = sinks;
   if (dtype == TS_DTYPE_BF16 && use_mma && ts_latent_attention_mma_takes(rank, rot) &&
       (((uintptr_t)q | (uintptr_t)cache | (uintptr_t)out) & 15) == 0) {
-    if (splits < 1 || (splits > 1 && (max_query_len != 1 || !part_acc || !part_ml))) return TS_ERR_BAD_ARGUMENT;
+    if (splits < 1 || splits > LD_MAX_SPLITS || (splits > 1 && max_query_len != 1)) return TS_ERR_BAD_ARGUMENT;
+    if (max_query_len == 1) {
+      const int ld = latent_row_length(rank + rot);
+      const int nb = (rank + 127) / 128 * 2;        // blocks of 8 columns per warp, an even number
+      if (nb <= 2) return launch_latent_single<2>(a, ld, splits, stream);
+      if (nb <= 4) return launch_latent_single<4>(a, ld, splits, stream);
+      return launch_latent_single<8>(a, ld, splits, stream);
+    }
     // 64 rows a CTA where the step has them: up to 64 heads of as many tokens as fit
     a.heads_per_cta = heads < LM_ROWS ? heads : LM_ROWS;
-    a.tokens_per_cta = max_query_len == 1 ? 1 : (LM_ROWS / a.heads_per_cta);
-    LatentSplit sp;
-    sp.splits = splits; sp.part_acc = part_acc; sp.part_ml = part_ml;
+    a.tokens_per_cta = LM_ROWS / a.heads_per_cta;
     const int nb = (rank / 2 + 15) / 16 * 2;        // blocks of 8 columns per half, an even number
-    int st;
-    if (nb <= 8) st = launch_latent_mma<8>(a, sp, max_query_len, stream);
-    else if (nb <= 16) st = launch_latent_mma<16>(a, sp, max_query_len, stream);
-    else st = launch_latent_mma<32>(a, sp, max_query_len, stream);
-    if (st != 0 || splits == 1) return st;
-    return launch(latent_merge_kernel, num_tokens * heads, 128, 0, stream, (const float*)part_acc, (const float*)part_ml,
-                  (bf16*)out, splits, rank, sinks, heads);
+    if (nb <= 8) return launch_latent_mma<8>(a, max_query_len, stream);
+    if (nb <= 16) return launch_latent_mma<16>(a, max_query_len, stream);
+    return launch_latent_mma<32>(a, max_query_len, stream);
   }
   // 32 rows a CTA where the step has them: 8 heads of 4 tokens (a single token: 8 heads)
   a.heads_per_cta = heads < 8 ? heads : 8;

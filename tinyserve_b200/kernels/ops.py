@@ -102,7 +102,7 @@ _SIGNATURES: dict[str, list[Any]] = {
     "ts_gemm_skinny_gated": [_vp, _vp, _vp, _i, _i, _i, _i, _f, _vp],
     "ts_latent_prepare": [_vp, _c.c_longlong, _vp, _vp, _c.c_longlong, _vp, _f, _vp, _vp, _i, _i, _vp, _vp, _vp, _i, _i, _i,
                           _i, _i, _i, _vp],
-    "ts_latent_attention": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _i, _i, _vp, _vp, _i, _vp, _vp],
+    "ts_latent_attention": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _i, _i, _vp, _vp],
     "ts_latent_attention_mma_takes": [_i, _i],
     "ts_moe_route": [_vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _i,
                      _vp],
@@ -1925,15 +1925,15 @@ def talking_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
 # ------------------------------------------------------------- latent attention
 LATENT_MAX_RANK = 512
 LATENT_TENSOR_CORES = True        # bf16 at sizes the mma.sync form takes; False: CUDA cores always
-LATENT_MAX_SPLITS = 16
-LATENT_MIN_KEYS_PER_SPLIT = 64
+LATENT_MAX_SPLITS = 8              # the CTAs of a cluster
+LATENT_KEYS_PER_SPLIT = 128        # what a CTA takes at a time
 
 
 def latent_splits(num_seqs: int, heads: int, keys: int) -> int:
-    """Key ranges per request for a step of single tokens: enough CTAs (one per request, 64 heads and
-    range) to give every SM one, no range shorter than 64 keys. Depends only on the step's shape."""
-    ctas = max(1, num_seqs * -(-heads // 64))
-    return max(1, min(SM_COUNT // ctas, keys // LATENT_MIN_KEYS_PER_SPLIT, LATENT_MAX_SPLITS))
+    """Key ranges per request for a step of single tokens: as many CTAs (one per request, 16 heads and range) as the SMs hold
+    one each, no range shorter than what a CTA takes at a time. Depends only on the step's shape."""
+    ctas = max(1, num_seqs * -(-heads // 16))
+    return max(1, min(SM_COUNT // ctas, -(-keys // LATENT_KEYS_PER_SPLIT), LATENT_MAX_SPLITS))
 
 
 def latent_prepare(q_in: torch.Tensor, q_folded: torch.Tensor, ckr: torch.Tensor | None, norm_weight: torch.Tensor | None,
@@ -1987,20 +1987,15 @@ def latent_attention(q: torch.Tensor, cache: torch.Tensor, page_size: int, block
         raise KernelError("latent_attention: sinks must be float32, one per head")
     _check_indices("latent_attention", block_tables, ctx, page_size, cache.shape[0] // page_size)
     mma = bool(LATENT_TENSOR_CORES and dt == torch.bfloat16 and _fn("ts_latent_attention_mma_takes")(rank, d - rank))
-    splits, part_acc, part_ml = 1, None, None
+    splits = 1
     if mma and ctx.max_query_len == 1:
-        keys = min(ctx.max_context_len, window) if window else ctx.max_context_len
-        splits = latent_splits(ctx.num_seqs, heads, keys)
-        if splits > 1:
-            part_acc = ctx.arena.take((t, heads, splits, rank), torch.float32)
-            part_ml = ctx.arena.take((t, heads, splits, 2), torch.float32)
+        splits = latent_splits(ctx.num_seqs, heads, min(ctx.max_context_len, window) if window else ctx.max_context_len)
     _check(_fn("ts_latent_attention")(
         _dev(q, "q"), _dev(out, "out"), _dev(cache, "cache"), _dev(block_tables, "block_tables", torch.int32),
         block_tables.shape[1], _dev(ctx.cu_query_lens, "cu_query_lens", torch.int32),
         _dev(ctx.context_lens_dev, "context_lens", torch.int32), ctx.num_seqs, ctx.max_query_len, heads, rank, d - rank,
-        page_size, float(scale), int(window), _code(dt), int(mma), splits, _opt(part_acc, "part_acc"),
-        _opt(part_ml, "part_ml"), t, _opt(sinks, "sinks", torch.float32), _stream()), "latent_attention",
-        kernels=2 if splits > 1 else 1)
+        page_size, float(scale), int(window), _code(dt), int(mma), splits, _opt(sinks, "sinks", torch.float32), _stream()),
+        "latent_attention")
 
 
 def bmm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
