@@ -203,3 +203,26 @@ def test_steps_launched_ahead_change_nothing(setup, name) -> None:
             assert e.requests[ids[0]].output == want[0]
             assert e.requests[ids[1]].output == want[1][: want[1].index(want[1][3]) + 1]
     assert outs[0] == outs[1]
+
+
+def test_prompts_of_every_kind_become_the_same_request(setup) -> None:
+    """Lists, tuples, ranges, arrays, tensors and iterators of numbers give the same ids, as ints; a portion is a slice of
+    them, across the border to the drawn tokens too; ids outside the vocabulary, however large, are refused."""
+    import numpy as np
+
+    model, page, _, _ = setup["A"]
+    ids = [3, 5, 7, 9]
+    kinds = [ids, tuple(ids), range(3, 11, 2), np.array(ids), np.array(ids, dtype=np.uint16), torch.tensor(ids), iter(ids), [3.0, 5, np.int64(7), 9.9]]
+    for prompt in kinds:
+        e = engine(model, page, 40)
+        r = e.requests[e.add_request(prompt, 4)]
+        assert r.prompt == ids and all(type(t) is int for t in r.prompt)
+        r.output.extend([11, 12])
+        for start in range(6):
+            for end in range(start + 1, 7):
+                assert list(r.token_slice(start, end)) == (ids + [11, 12])[start:end]
+    for bad in ([-1], [model.vocab_size], [1, 1 << 31], [1, 1 << 63], [1 << 80], np.array([1 << 40])):
+        with pytest.raises(ValueError, match="token id outside"):
+            engine(model, page, 40).add_request(bad, 4)
+    with pytest.raises(ValueError):
+        engine(model, page, 40).add_request([], 4)

@@ -19,6 +19,7 @@ import time
 from dataclasses import dataclass, field
 from typing import Callable, Sequence
 
+import numpy as np
 import torch
 
 from ..cache.manager import CacheManager
@@ -28,6 +29,17 @@ from ..sampling.sampler import SampleTicket, Sampler, TokenLogprobs, derive_seed
 from .request import Request, Status
 from .scheduler import Scheduler
 from .step import ModelRunner, StepEntry
+
+
+def _as_ids(prompt: Sequence[int]) -> tuple[list[int], "np.ndarray | None"]:
+    """A prompt as a list of ints and, where its elements are numbers of 64 bits, as an array too."""
+    if not hasattr(prompt, "__len__"):
+        prompt = list(prompt)
+    try:
+        ids = np.fromiter(prompt, dtype=np.int64, count=len(prompt))
+    except (TypeError, ValueError, OverflowError):
+        return [int(t) for t in prompt], None
+    return ids.tolist(), ids
 
 
 @dataclass
@@ -132,13 +144,13 @@ class Engine:
     # ------------------------------------------------------------------ requests
     def add_request(self, prompt: Sequence[int], max_new_tokens: int,
                     eos_ids: frozenset[int] = frozenset(), sampling: SamplingParams | None = None) -> int:
-        prompt = [int(t) for t in prompt]
         vocab = self.model.vocab_size
-        if any(t < 0 or t >= vocab for t in prompt):
+        prompt, ids = _as_ids(prompt)
+        if any(t < 0 or t >= vocab for t in ((ids.min(), ids.max()) if ids is not None and len(ids) else prompt)):
             raise ValueError(f"prompt has a token id outside 0..{vocab - 1}")
         rid = self._next_id
         params = sampling or SamplingParams()
-        req = Request(rid, prompt, max_new_tokens, frozenset(eos_ids), params)
+        req = Request(rid, prompt, max_new_tokens, frozenset(eos_ids), params, prompt_ids=None if ids is None else ids.astype(np.int32))
         self.scheduler.add(req)
         self._next_id += 1
         self.requests[rid] = req
@@ -197,8 +209,8 @@ class Engine:
         self._mark(marks)
         sampled = reqs if ahead is not None else [r for r in reqs if not r.in_prefill()]
         if self.logits_log is not None and sampled:
-            rows = logits[: len(sampled)].clone()      # a step launched ahead reuses the buffer before this one is read
-            self.logits_log.extend((r.request_id, r.cache.num_tokens - 1, rows[j]) for j, r in enumerate(sampled))
+            rows = logits[: len(sampled)].clone().unbind()     # a step launched ahead reuses the buffer before this one is read
+            self.logits_log.extend((r.request_id, r.cache.num_tokens - 1, row) for r, row in zip(sampled, rows))
         ticket = None
         if sampled:
             drawn = 1 if ahead is not None else 0        # the token under way counts as drawn

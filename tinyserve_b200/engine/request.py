@@ -17,6 +17,8 @@ from __future__ import annotations
 from dataclasses import dataclass, field
 from enum import Enum
 
+import numpy as np
+
 from ..cache.manager import RequestCache
 from ..sampling.params import SamplingParams
 
@@ -39,6 +41,8 @@ class Request:
     cache: RequestCache | None = None
     num_scheduled: int = 0        # tokens given to the last scheduled step
     num_preemptions: int = 0
+    # the prompt as int32, if its maker has it: a portion is then a slice of it
+    prompt_ids: "np.ndarray | None" = field(default=None, compare=False, repr=False)
 
     def __post_init__(self) -> None:
         if len(self.prompt) == 0:
@@ -50,11 +54,11 @@ class Request:
     def tokens(self) -> list[int]:
         return [*self.prompt, *self.output]
 
-    def token_slice(self, start: int, end: int) -> list[int]:
+    def token_slice(self, start: int, end: int) -> "list[int] | np.ndarray":
         """``tokens[start:end]`` without building the whole list (a decode step needs one token)."""
         n = len(self.prompt)
         if end <= n:
-            return self.prompt[start:end]
+            return (self.prompt if self.prompt_ids is None else self.prompt_ids)[start:end]
         if start >= n:
             return self.output[start - n: end - n]
         return self.prompt[start:] + self.output[: end - n]

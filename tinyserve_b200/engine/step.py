@@ -378,20 +378,23 @@ class ModelRunner:
         self._staging(off)
         buf = self._host_np
 
-        # ---- fill
-        tok = buf[s_tokens]
-        pos = buf[s_pos]
-        cu = buf[s_cu]
+        # ---- fill: whole columns at a time, a loop only over what differs in length from request to request
+        tok, pos, cu = buf[s_tokens], buf[s_pos], buf[s_cu]
+        lens = np.array(query_lens, dtype=np.int32)
         cu[0] = 0
+        np.cumsum(lens, out=cu[1:])
+        of = np.repeat(np.arange(b, dtype=np.int32), lens)             # the request of each token
+        first = np.array(totals, dtype=np.int32) - lens                # the position of a request's first token
+        np.subtract(np.arange(t, dtype=np.int32), (cu[:-1] - first)[of], out=pos)
         at = 0
-        dec: list[int] = []
-        pre: list[int] = []
-        for i, (e, n, total) in enumerate(zip(entries, query_lens, totals)):
-            tok[at: at + n] = e.tokens
-            pos[at: at + n] = np.arange(total - n, total, dtype=np.int32)
+        for e, n in zip(entries, query_lens):
+            if n == 1:
+                tok[at] = e.tokens[0]
+            else:
+                tok[at: at + n] = e.tokens
             at += n
-            cu[i + 1] = at
-            (dec if n == 1 else pre).append(i)
+        dec = [i for i, n in enumerate(query_lens) if n == 1]
+        pre = [i for i, n in enumerate(query_lens) if n != 1]
         buf[s_ctx] = totals
         buf[s_dec][: len(dec)] = dec
         buf[s_pre][: len(pre)] = pre
@@ -399,16 +402,12 @@ class ModelRunner:
         buf[s_state] = [e.cache.state_slot for e in entries]
         for g, ss, st, w in zip(groups, s_slots, s_tables, widths):
             ps = g.page_size
-            slots = buf[ss]
             table = buf[st].reshape(b, w)
             table[:] = 0
-            at = 0
-            for i, (e, n, total) in enumerate(zip(entries, query_lens, totals)):
+            for i, e in enumerate(entries):
                 pages = e.cache.tables[g.index].pages_array()
                 table[i, : pages.shape[0]] = pages
-                p = pos[at: at + n]
-                slots[at: at + n] = pages[p // ps] * ps + p % ps
-                at += n
+            buf[ss] = table[of, pos // ps] * ps + pos % ps
 
         dev = self._dev
         dev[:off].copy_(self._host[:off], non_blocking=True)
