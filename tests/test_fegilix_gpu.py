@@ -178,6 +178,65 @@ def test_mlstm_scan_kernel(dtype, heads, d, dv) -> None:
     assert got[2].abs().max() == 0 and got[4].abs().max() == 0
 
 
+def _mlstm_in_64_bits(x, offs, gates, gb, cap, q_scale, state, step, heads, d, dv):
+    """The recurrence token by token; ``state`` (a copy, 64-bit) advances too. Returns the outputs ``[T, heads, dv]``."""
+    x, z = x.double().cpu(), gates.double().cpu() + gb.double().cpu()
+    li, lf = cap * torch.tanh(z[:, :heads] / cap), torch.nn.functional.logsigmoid(cap * torch.tanh(z[:, heads:] / cap))
+    q, k, v = (x[:, o: o + heads * w].view(-1, heads, w) for o, w in zip(offs, (d, d, dv)))
+    out, cu = torch.empty(len(x), heads, dv, dtype=torch.float64), step.cu_query_lens.tolist()
+    copies = -(-dv // 32)
+    for b, slot in enumerate(step.state_slots.tolist()):
+        st = state[slot].view(heads, -1)
+        S, n, m = st[:, : d * dv].reshape(heads, d, dv).clone(), st[:, d * dv: d * dv + d].clone(), st[:, d * dv + d].clone()
+        for t in range(cu[b], cu[b + 1]):
+            top = torch.maximum(lf[t] + m, li[t])
+            keep, take, m = torch.exp(lf[t] + m - top), torch.exp(li[t] - top), top
+            S = keep[:, None, None] * S + take[:, None, None] * k[t][:, :, None] * v[t][:, None, :]
+            n = keep[:, None] * n + take[:, None] * k[t]
+            qt = q[t] * q_scale
+            out[t] = torch.einsum("hkv,hk->hv", S, qt) / (torch.maximum((n * qt).sum(-1).abs(), torch.exp(-m)) + 1e-6)[:, None]
+        st[:, : d * dv] = S.reshape(heads, -1)
+        for c in range(copies):
+            at = d * dv + c * (d + 1)
+            st[:, at: at + d], st[:, at + d] = n, m
+    return out
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads, d, dv, lens", [(2, 128, 128, [200, 64, 1, 129]), (3, 64, 96, [128, 65]), (1, 48, 50, [300]),
+                                                (2, 70, 33, [63, 191, 0, 128]), (1, 1, 1, [130])])
+def test_mlstm_scan_over_chunks(dtype, heads, d, dv, lens, monkeypatch) -> None:
+    """Portions as products over chunks of 64 tokens and token by token, from a fresh state and from the one that leaves,
+    then single tokens from its state, both against 64 bits: the chunks as close as the other form, row by row in the
+    middle (a tenth and two roundings of slack for sums in another order) and at worst within eight times (either's worst row
+    is one whose denominator is a small difference)."""
+    from tinyserve_b200.kernels import ops
+
+    slots, size, gb = list(range(len(lens))), ops.mlstm_state_size(heads, d, dv), _rand(2 * heads, seed=1)
+    offs = (8, 8 + heads * d, 8 + 2 * heads * d)
+    errors = {}
+    for chunks in (True, False):
+        monkeypatch.setattr(ops, "MLSTM_CHUNKS", chunks)
+        state = torch.zeros(len(lens) + 1, size, device="cuda")
+        exact = state.double().cpu()
+        for i, news in enumerate((lens, lens[::-1], [1] * len(lens))):
+            t, step = sum(news), FakeStep(news, slots, "cuda")
+            x = _rand(t, 8 + 2 * heads * d + heads * dv, seed=20 + i, dtype=dtype)
+            gates = _rand(t, 2 * heads, seed=30 + i, scale=4.0)
+            out = torch.full((t, heads, dv), float("nan"), device="cuda")
+            ops.mlstm_scan(x, *offs, gates, gb, 5.0, d ** -0.5, state, step, heads, d, dv, out)
+            want = _mlstm_in_64_bits(x, offs, gates, gb, 5.0, d ** -0.5, exact, step, heads, d, dv)
+            for what, got, ref in (("out", out, want), ("state", state, exact)):
+                width = dv if what == "out" else size
+                diff, rows = (got.double().cpu() - ref).view(-1, width).norm(dim=-1), ref.reshape(-1, width).norm(dim=-1)
+                off = (diff / rows)[rows > 0]
+                errors.setdefault((i, what), []).append((float(off.median()), float(off.max())))
+        assert state[-1].abs().max() == 0
+    for key, (over_chunks, token_by_token) in errors.items():
+        assert over_chunks[0] <= 1.1 * token_by_token[0] + 2.0 ** -23, (key, over_chunks, token_by_token)
+        assert over_chunks[1] <= 8 * token_by_token[1] + 2.0 ** -22, (key, over_chunks, token_by_token)
+
+
 def _attention_case(dtype, heads, groups, d, dv, page, lens, news, rot, sink_shift=0.0, far=None):
     """Requests with ``lens`` tokens of which the last ``news`` are this step's; the earlier ones are
     already in the cache (written by a first call). Returns kernel and reference outputs of the step."""

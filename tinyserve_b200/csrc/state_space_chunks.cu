@@ -15,20 +15,13 @@
 // holds 4 x 4 or 8 x 4 sums and spends a 16-byte read of shared memory on eight or eleven multiply-adds, where the
 // token-by-token form spends one on four. The running sums are kept in 64-bit: the difference of two of them is what decays a weight, and
 // in 32-bit it would lose the digits that a long or fast decaying chunk has accumulated. Every exponent is at most zero.
-//
-// Chunks are numbered over the whole step, request b's from cu_q[b] / 64 + b on (gaps of at most one), so scratch and
-// grid follow the step's tokens, however unequal the requests are; a request of one token costs one chunk of one row.
 #define TS_PDL_CLASS PDL_OTHER
 #include <cuda_pipeline_primitives.h>
 
 #include "common.cuh"
+#include "scan_chunks.cuh"
 
 namespace ts {
-
-constexpr int SC_Q = 64;              // tokens of a chunk
-constexpr int SC_V = 64;              // value columns of a CTA
-constexpr int SC_LD = SC_Q + 4;       // row of a tile whose fast index is the token (16-byte aligned, spread over the banks)
-constexpr int SC_MAX_STATE = 128;
 
 struct ScanChunkArgs {
   const float* c; int c_stride;       // [T, G * N] rows c_stride apart
@@ -46,19 +39,6 @@ struct ScanChunkArgs {
 };
 
 __device__ __forceinline__ float sc_softplus(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
-
-// The request and the tokens of chunk g of the step; false for a number that belongs to no chunk.
-__device__ __forceinline__ bool find_chunk(const ScanChunkArgs& a, int g, int& t0, int& nt) {
-  int lo = 0, hi = a.num_seqs - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (a.cu_q[mid] / SC_Q + mid <= g) lo = mid; else hi = mid - 1;
-  }
-  const int start = a.cu_q[lo], end = a.cu_q[lo + 1];
-  t0 = start + (g - (start / SC_Q + lo)) * SC_Q;
-  nt = min(SC_Q, end - t0);
-  return nt > 0;
-}
 
 // By one warp: dt and the running sums of the chunk's tokens for head h (two tokens a lane); tokens past the end have dt 0.
 __device__ __forceinline__ void chunk_steps(const ScanChunkArgs& a, int h, int t0, int nt, int lane, float* dt_s, double* cum_s) {
@@ -83,63 +63,6 @@ __device__ __forceinline__ void chunk_steps(const ScanChunkArgs& a, int h, int t
   cum_s[2 * lane + 1] = run;
 }
 
-// acc[4 A][4] += A^T B over k rows: A's rows hold the 4 A-wide operand (row `lda` floats, this thread's part from `ar`), B's
-// the 4-wide one. Both 16-byte aligned.
-template <int A>
-__device__ __forceinline__ void tile_product(float (&acc)[4 * A][4], const float* ar, int lda, const float* br, int ldb, int k) {
-#pragma unroll 4
-  for (int i = 0; i < k; ++i) {
-    const float4 b = *reinterpret_cast<const float4*>(br + i * ldb);
-#pragma unroll
-    for (int q = 0; q < A; ++q) {
-      const float4 a = *reinterpret_cast<const float4*>(ar + i * lda + 4 * q);
-      const float av[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        acc[4 * q + r][0] = fmaf(av[r], b.x, acc[4 * q + r][0]);
-        acc[4 * q + r][1] = fmaf(av[r], b.y, acc[4 * q + r][1]);
-        acc[4 * q + r][2] = fmaf(av[r], b.z, acc[4 * q + r][2]);
-        acc[4 * q + r][3] = fmaf(av[r], b.w, acc[4 * q + r][3]);
-      }
-    }
-  }
-}
-
-// Loads in flight per thread before the first is stored to shared memory: one after the other each would wait for memory.
-constexpr int SC_LOADS = 8;
-
-// [nt rows of `width`] -> tile [SC_Q][ld], zero past the edges; four columns an access where the source allows it.
-__device__ __forceinline__ void load_rows(const float* src, int stride, int rows, int width, bool vec, float* dst, int ld, int cols,
-                                          int total_rows, int tid, int threads) {
-  const int quads = cols / 4, total = total_rows * quads;
-  for (int base = tid; base < total; base += threads * SC_LOADS) {
-    float4 v[SC_LOADS];
-#pragma unroll
-    for (int u = 0; u < SC_LOADS; ++u) {
-      const int idx = base + u * threads, r = idx / quads, c = (idx - r * quads) * 4;
-      v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (idx < total && r < rows) {
-        const float* p = src + (size_t)r * stride + c;
-        if (vec && c + 4 <= width) {
-          v[u] = *reinterpret_cast<const float4*>(p);
-        } else {
-          if (c < width) v[u].x = p[0];
-          if (c + 1 < width) v[u].y = p[1];
-          if (c + 2 < width) v[u].z = p[2];
-          if (c + 3 < width) v[u].w = p[3];
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < SC_LOADS; ++u) {
-      const int idx = base + u * threads, r = idx / quads, c = (idx - r * quads) * 4;
-      if (idx < total) *reinterpret_cast<float4*>(dst + r * ld + c) = v[u];
-    }
-  }
-}
-
-__device__ __forceinline__ bool rows_aligned(const float* p, int stride) { return (((uintptr_t)p) & 15) == 0 && (stride & 3) == 0; }
-
 // What a chunk leaves: [N x dv] per head. A CTA is (chunk, head, 64 value columns); NP = the state size rounded up to 64.
 template <int NP>
 __global__ void __launch_bounds__(2 * NP) chunk_leave_kernel(ScanChunkArgs a) {
@@ -153,7 +76,7 @@ __global__ void __launch_bounds__(2 * NP) chunk_leave_kernel(ScanChunkArgs a) {
   pdl_wait();
   int t0, nt;
   const int g = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * SC_V;
-  if (!find_chunk(a, g, t0, nt)) return;
+  if (!find_chunk(a.cu_q, a.num_seqs, g, t0, nt)) return;
   const int tid = threadIdx.x, lane = tid & 31;
   const int grp = h / a.per_group, N = a.N;
   if (tid < 32) chunk_steps(a, h, t0, nt, lane, dt_s, cum_s);
@@ -238,41 +161,6 @@ __global__ void chunk_combine_kernel(ScanChunkArgs a) {
   for (int e = 0; e < VEC; ++e) slot[e] = s[e];
 }
 
-// The token rows of C or B, transposed: tile [n][SC_LD] with the token as fast index, zero past the chunk's end and past N.
-__device__ __forceinline__ void load_transposed(const float* src, int stride, int nt, int N, int NP, float* dst, int warp, int warps, int lane) {
-  const bool vec = rows_aligned(src, stride);
-  const int t_local = lane & 7, n4 = (lane >> 3) * 4;      // a warp takes 8 tokens x 16 columns
-  const int tiles = (SC_Q / 8) * (NP / 16);
-  for (int base = warp; base < tiles; base += warps * SC_LOADS) {
-    float v[SC_LOADS][4];
-#pragma unroll
-    for (int u = 0; u < SC_LOADS; ++u) {
-      const int tile = base + u * warps, t = (tile & 7) * 8 + t_local, n = (tile >> 3) * 16 + n4;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) v[u][e] = 0.f;
-      if (tile < tiles && t < nt) {
-        const float* p = src + (size_t)t * stride + n;
-        if (vec && n + 4 <= N) {
-          const float4 q = *reinterpret_cast<const float4*>(p);
-          v[u][0] = q.x; v[u][1] = q.y; v[u][2] = q.z; v[u][3] = q.w;
-        } else {
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            if (n + e < N) v[u][e] = p[e];
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < SC_LOADS; ++u) {
-      const int tile = base + u * warps, t = (tile & 7) * 8 + t_local, n = (tile >> 3) * 16 + n4;
-      if (tile < tiles) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) dst[(n + e) * SC_LD + t] = v[u][e];
-      }
-    }
-  }
-}
-
 // The read-outs of a chunk. A CTA is (chunk, some heads of one group, 64 value columns).
 constexpr int SC_READ_THREADS = 256;  // (64 / 4) x (64 / 4) tiles of 4 x 4: two CTAs of eight warps an SM
 template <int NP>
@@ -288,7 +176,7 @@ __global__ void __launch_bounds__(SC_READ_THREADS, 2) chunk_read_kernel(ScanChun
   pdl_wait();
   int t0, nt;
   const int g = blockIdx.x, v0 = blockIdx.z * SC_V, N = a.N;
-  if (!find_chunk(a, g, t0, nt)) return;
+  if (!find_chunk(a.cu_q, a.num_seqs, g, t0, nt)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int h0 = blockIdx.y * a.heads_per_cta, grp = h0 / a.per_group;
   load_transposed(a.c + (size_t)t0 * a.c_stride + grp * N, a.c_stride, nt, N, NP, c_s, warp, SC_READ_THREADS / 32, lane);

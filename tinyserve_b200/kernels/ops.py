@@ -60,6 +60,7 @@ _SIGNATURES: dict[str, list[Any]] = {
     "ts_head_norm_gate": [_vp, _i, _vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _f, _i, _i, _i, _i, _vp],
     "ts_post_norm_add_rms_norm": [_vp, _vp, _vp, _vp, _f, _i, _f, _vp, _i, _f, _vp, _vp, _i, _i, _vp, _vp, _f, _vp, _vp, _i, _vp],
     "ts_mlstm_scan": [_vp, _i, _i, _i, _i, _vp, _vp, _f, _f, _vp, _i, _vp, _vp, _i, _i, _i, _i, _vp, _i, _vp],
+    "ts_mlstm_chunks": [_vp, _i, _i, _i, _i, _vp, _vp, _f, _f, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp],
     "ts_delta_scan": [_vp, _i, _i, _i, _i, _vp, _i, _i, _vp, _vp, _vp, _i, _f, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp],
     "ts_causal_conv_silu": [_vp, _i, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _vp, _i, _i, _vp],
     "ts_qkv_prepare": [_vp, _i, _vp, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp, _f, _vp, _vp, _i, _vp, _vp, _vp, _i, _i, _i, _i,
@@ -1442,6 +1443,17 @@ def mlstm_state_size(heads: int, d: int, dv: int) -> int:
     return heads * (d * dv + -(-dv // 32) * (d + 1))
 
 
+# Long portions as products over chunks; False: token by token always. Measured on B200, 8 heads of 128 x 128, token by token / over
+# chunks: 129 tokens 54.7 / 54.8 us, 256 102 / 57, 650 252 / 63, 2,048 780 / 114; portions of 100, 370 and 650 265 / 89, eight of 800
+# 392 / 325. The kernel's tiles hold keys of up to 128; its scratch is a chunk's sums per head, and a step that would need more
+# than this of it goes token by token.
+MLSTM_CHUNKS = True
+MLSTM_CHUNK = 64                  # tokens of a chunk, as the kernel is built
+MLSTM_CHUNKS_MIN_TOKENS = 128
+MLSTM_CHUNKS_MAX_KEY_DIM = 128
+MLSTM_CHUNKS_SCRATCH_BYTES = 1 << 30
+
+
 def mlstm_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: torch.Tensor, gate_bias: torch.Tensor,
                cap: float, q_scale: float, state: torch.Tensor, ctx: Any, heads: int, d: int, dv: int,
                out: torch.Tensor) -> None:
@@ -1456,11 +1468,20 @@ def mlstm_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: tor
     if d > SCAN_MAX_KEY_DIM:
         raise KernelError("mlstm_scan: key size")
     state_ptr, state_stride = _state_rows(state, mlstm_state_size(heads, d, dv), "mlstm_scan")
+    common = (_dev(qkv, "qkv"), qkv.shape[1], q_off, k_off, v_off, _dev(gates, "gates", torch.float32),
+              _dev(gate_bias, "gate_bias", torch.float32), float(cap), float(q_scale), state_ptr, state_stride,
+              _dev(ctx.cu_query_lens, "cu_query_lens", torch.int32), _dev(ctx.state_slots, "state_slots", torch.int32), ctx.num_seqs)
+    chunks = t // MLSTM_CHUNK + ctx.num_seqs
+    if (MLSTM_CHUNKS and ctx.max_query_len >= MLSTM_CHUNKS_MIN_TOKENS and d <= MLSTM_CHUNKS_MAX_KEY_DIM
+            and 4 * chunks * heads * d * dv <= MLSTM_CHUNKS_SCRATCH_BYTES):
+        # long portions: 32-bit products over chunks of 64 tokens (``csrc/mlstm_chunks.cu``)
+        left, left_n = ctx.arena.take((chunks, heads, d, dv), torch.float32), ctx.arena.take((chunks, heads, d), torch.float32)
+        ends, starts = ctx.arena.take((chunks, heads, 2), torch.float64), ctx.arena.take((chunks, heads), torch.float32)
+        _check(_fn("ts_mlstm_chunks")(*common, t, heads, d, dv, left.data_ptr(), left_n.data_ptr(), ends.data_ptr(), starts.data_ptr(),
+                                      _dev(out, "out", torch.float32), _code(qkv.dtype), _stream()), "mlstm_scan", kernels=3)
+        return
     _check(_fn("ts_mlstm_scan")(
-        _dev(qkv, "qkv"), qkv.shape[1], q_off, k_off, v_off, _dev(gates, "gates", torch.float32),
-        _dev(gate_bias, "gate_bias", torch.float32), float(cap), float(q_scale), state_ptr, state_stride,
-        _dev(ctx.cu_query_lens, "cu_query_lens", torch.int32), _dev(ctx.state_slots, "state_slots", torch.int32),
-        ctx.num_seqs, heads, d, dv, _dev(out, "out", torch.float32), _code(qkv.dtype), _stream()), "mlstm_scan")
+        *common, heads, d, dv, _dev(out, "out", torch.float32), _code(qkv.dtype), _stream()), "mlstm_scan")
 
 
 def delta_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, a: torch.Tensor, dt_bias: torch.Tensor,
