@@ -237,6 +237,23 @@ def test_mlstm_scan_over_chunks(dtype, heads, d, dv, lens, monkeypatch) -> None:
         assert over_chunks[1] <= 8 * token_by_token[1] + 2.0 ** -22, (key, over_chunks, token_by_token)
 
 
+def test_mlstm_scan_into_an_output_off_the_16_byte_grid() -> None:
+    """A long portion whose read-outs go to a place that the chunks' wide stores do not take."""
+    from tinyserve_b200.kernels import ops
+
+    heads, d, dv, t = 2, 32, 32, 140
+    x, gates, gb = _rand(t, 2 * heads * d + heads * dv, seed=1), _rand(t, 2 * heads, seed=2), _rand(2 * heads, seed=3)
+    outs = []
+    for first in (0, 1):
+        state = torch.zeros(2, ops.mlstm_state_size(heads, d, dv), device="cuda")
+        buf = torch.full((t * heads * dv + 2,), float("nan"), device="cuda")
+        out = buf[first: first + t * heads * dv].view(t, heads, dv)
+        ops.mlstm_scan(x, 0, heads * d, 2 * heads * d, gates, gb, 5.0, d ** -0.5, state, FakeStep([t], [0], "cuda"), heads, d, dv, out)
+        assert int(buf.isnan().sum()) == 2
+        outs.append(out.clone())
+    torch.testing.assert_close(*outs, atol=1e-4, rtol=1e-4)
+
+
 def _attention_case(dtype, heads, groups, d, dv, page, lens, news, rot, sink_shift=0.0, far=None):
     """Requests with ``lens`` tokens of which the last ``news`` are this step's; the earlier ones are
     already in the cache (written by a first call). Returns kernel and reference outputs of the step."""

@@ -1473,7 +1473,7 @@ def mlstm_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: tor
               _dev(ctx.cu_query_lens, "cu_query_lens", torch.int32), _dev(ctx.state_slots, "state_slots", torch.int32), ctx.num_seqs)
     chunks = t // MLSTM_CHUNK + ctx.num_seqs
     if (MLSTM_CHUNKS and ctx.max_query_len >= MLSTM_CHUNKS_MIN_TOKENS and d <= MLSTM_CHUNKS_MAX_KEY_DIM
-            and 4 * chunks * heads * d * dv <= MLSTM_CHUNKS_SCRATCH_BYTES):
+            and 4 * chunks * heads * d * dv <= MLSTM_CHUNKS_SCRATCH_BYTES and out.data_ptr() % 16 == 0):
         # long portions: 32-bit products over chunks of 64 tokens (``csrc/mlstm_chunks.cu``)
         left, left_n = ctx.arena.take((chunks, heads, d, dv), torch.float32), ctx.arena.take((chunks, heads, d), torch.float32)
         ends, starts = ctx.arena.take((chunks, heads, 2), torch.float64), ctx.arena.take((chunks, heads), torch.float32)
