@@ -265,6 +265,24 @@ def test_prefill_attention_one_head_or_two_a_cta_give_the_same_bits(d, page, win
     assert torch.equal(*outs)
 
 
+@pytest.mark.parametrize("scale", [0.7, 4.0])
+@pytest.mark.parametrize("window", [0, 150])
+@pytest.mark.parametrize("d,page", [(64, 8), (128, 16)])
+def test_prefill_attention_where_row_maxima_grow_behind_the_first_tile(d, page, window, scale, monkeypatch) -> None:
+    """Scores so wide that the maximum of some rows grows by more than 2^8 in tiles other than the first, in either half of a
+    tile's keys: the sums and outputs made before are scaled and the tile's probabilities made again. In 32-bit the exponents
+    are off by 2^-24 of the widest score (a few hundred), far below bfloat16's rounding."""
+    outs = []
+    for heads in (1, 2):
+        monkeypatch.setattr(ops, "PREFILL_HEADS_PER_CTA", heads)
+        out, want = _attention_case(torch.bfloat16, 4, 2, d, page, [(2, 2), (129, 129), (900, 900), (1300, 260), (520, 31)], window, seed=3, scale=scale)
+        ops.check_device_errors()
+        assert not out.isnan().any()
+        torch.testing.assert_close(out.float(), want.float(), **tol(torch.bfloat16))
+        outs.append(out)
+    assert torch.equal(*outs)
+
+
 @pytest.mark.parametrize("heads_per_cta", [1, 2])
 @pytest.mark.parametrize("pos", [0, 63, 64, 127, 128, 511, 999])
 def test_prefill_attention_tcgen05_far_key(heads_per_cta, pos, monkeypatch) -> None:

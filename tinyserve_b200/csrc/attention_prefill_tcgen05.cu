@@ -48,7 +48,12 @@
 // branch on the lane an instruction took 77 cycles (its operands go to uniform registers one by one) and that warp set the
 // pace; issued by the converged warp, 8,192 tokens 300 -> 273 us (1,010 TFLOP/s), 2,048 tokens at 9,001 positions 179 -> 160
 // us (with the sums of a row kept per 64 columns, which take 3 % of that). An MMA warp per head was slower (369 us: the heads fall into step), and so were two score buffers of 64 keys per head
-// (289 us at best: what a step costs whatever its size is paid twice). Every operand read from shared
+// (289 us at best: what a step costs whatever its size is paid twice). With one head a CTA and two threads a row the same holds since the
+// probabilities are made in the scale of the maximum so far while the tile's own maximum is being found (again, if it has
+// grown too far, which is rare behind the first tile), and the warps of a row quarter meet once a tile instead of twice: a step is then
+// 2,330 cycles, the MMA warp's 77 an instruction from a branch on the lane and the softmax's chain come to the same, and each of
+// the two changes alone gave nothing (2,048 tokens 35.8 us, 37.5 and 37.3 with one, 30.5 with both; 512 tokens 13.4 -> 11.2, 8,192 tokens
+// of 32 heads 672 -> 612, 2,048 at 4,096 positions 78 -> 67; the same bits). Every operand read from shared
 // memory and every TMA write goes through the same 128 bytes per cycle, which is why P stays in tensor
 // memory.
 // Every wait is on an mbarrier, is bounded and gives up at once when another role has: the CTA
@@ -134,6 +139,7 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
   __shared__ int failed_flag;
   __shared__ float pair_value[NQ][4][HS][32];      // what the warps of a row quarter tell one another: a row maximum, a row sum
   __shared__ int pair_ok[NQ][4][HS];
+  __shared__ uint2 pair_grown[2][4][2];             // (HS = 2) the rows whose maximum has grown, and whether the waits have held
   volatile int* failed = &failed_flag;
 
   // ---- which rows and keys (uniform over the CTA); a CTA without rows leaves before any set-up
@@ -161,8 +167,8 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
 
   pdl_trigger();
   unsigned char* smem = (unsigned char*)(((uintptr_t)fa_raw + 1023) & ~(uintptr_t)1023);
-  // two heads: known to the compiler to be the same in the whole warp, so that the MMA warp's operands are (umma_bf16_by)
-  const int warp = NQ == 1 ? (int)(threadIdx.x >> 5) : __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  // known to the compiler to be the same in the whole warp, so that the MMA warp's operands are (umma_bf16_by)
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < FA_KV_STAGES; ++s) {
       mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
@@ -240,6 +246,16 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
         return all_ok;
       }
     };
+    // (HS = 2) Whether a row of either warp has `grown`. One meeting: tiles take the two places in turn, so a place is written
+    // again behind the meeting of the tile between, which a warp reaches after it has read.
+    auto any_grown = [&](int turn, bool grown, bool mine_ok, bool& any) -> bool {
+      const unsigned mine = __ballot_sync(0xffffffffu, grown);
+      if (lane == 0) pair_grown[turn][quad][half] = make_uint2(mine, mine_ok ? 1u : 0u);
+      pair_sync();
+      const uint2 a2 = pair_grown[turn][quad][0], b2 = pair_grown[turn][quad][1];
+      any = (a2.x | b2.x) != 0;
+      return (a2.y & b2.y) != 0;
+    };
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
     const uint32_t tmem_o = tmem_base + lane_addr + L::TMEM_O + (uint32_t)(q * D);
     const int p_abs = p_lo + r;
@@ -258,76 +274,127 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
       uint32_t sraw[HC];
       float mx = -INFINITY;
       const int k0 = tile_of(j) * BN + half * HC;              // the first key of this thread's columns
+      // Two threads a row: the probabilities of the thread's 64 columns as bf16, two keys per word, and their sum, in the scale
+      // of the maximum so far; `look` finds the columns' own maximum on the way, beside the exponentials.
+      uint32_t packed[HS == 2 ? 32 : 1];
+      float part = 0.f;
+      auto probabilities = [&](bool look) {
+        const float m_sub = m_used == -INFINITY ? 0.f : m_used;
+        float add4[4] = {0.f, 0.f, 0.f, 0.f}, mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const float s0 = __uint_as_float(sraw[2 * i]), s1 = __uint_as_float(sraw[2 * i + 1]);
+          if (look) mx4[i & 3] = fmaxf(mx4[i & 3], fmaxf(s0, s1));
+          const float p0 = fa_exp2(fmaf(s0, a.scale_log2, -m_sub)), p1 = fa_exp2(fmaf(s1, a.scale_log2, -m_sub));
+          add4[i & 3] += p0 + p1;
+          packed[i] = fa_pack(p0, p1);
+        }
+        part = (add4[0] + add4[1]) + (add4[2] + add4[3]);
+        if (look) mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      };
       if (ok) {
 #pragma unroll
         for (int c = 0; c < HC / 32; ++c) tmem_ld_32_nowait(tmem_sp + half * HC + c * 32, sraw + c * 32);
         tmem_ld_wait();
         const bool edge = (k0 + HC - 1 > p_lo) || (CHUNKED ? k0 < first_visible(p_lo + FA_BM - 1, a)
                                                            : a.window > 0 && k0 < p_lo + FA_BM - a.window);
-        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // four chains: the maxima do not wait on one another
-        if (edge) {
-          const int first = CHUNKED ? first_visible(p_abs, a) : a.window > 0 ? p_abs - a.window + 1 : 0;
+        if constexpr (HS == 2) {
+          if (edge) {
+            const int first = CHUNKED ? first_visible(p_abs, a) : a.window > 0 ? p_abs - a.window + 1 : 0;
 #pragma unroll
-          for (int i = 0; i < HC; ++i) {
-            const int kpos = k0 + i;
-            const float v = (kpos <= p_abs && (kpos >= first || kpos < a.keep_first)) ? __uint_as_float(sraw[i]) : -INFINITY;
-            sraw[i] = __float_as_uint(v);
-            mx4[i & 3] = fmaxf(mx4[i & 3], v);
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < HC; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(sraw[i]));
-        }
-        mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      }
-      // the row's maximum over all its columns; every score of the tile has been read by now, so the
-      // probabilities may overwrite them
-      float maxima[HS];
-      if (!exchange(mx, ok, maxima)) { stopped = true; break; }
-#pragma unroll
-      for (int h2 = 0; h2 < HS; ++h2) mx = fmaxf(mx, maxima[h2]);
-      const float m_new = fmaxf(m_used, mx * a.scale_log2);
-      if (j == 0) {
-        m_used = m_new;
-      } else {
-        const bool grow = m_new > m_used + FA_RESCALE_STEP;    // also when nothing was seen before (-inf)
-        if (__any_sync(0xffffffffu, grow)) {
-          // O is final up to tile j - 1 before it is scaled; each warp scales its share of the columns
-          if (!fa_warp_wait(&pv_done[q][(j - 1) % SPB], ((j - 1) / SPB) & 1, failed)) ok = false;
-          tc_fence_after();
-          const float alpha = grow ? (m_used == -INFINITY ? 0.f : fa_exp2(m_used - m_new)) : 1.f;
-          if (ok) {
-#pragma unroll 1
-            for (int c = half * (D / 32 / HS); c < (half + 1) * (D / 32 / HS); ++c) {
-              uint32_t o[32];
-              tmem_ld_32(tmem_o + c * 32, o);
-#pragma unroll
-              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-              tmem_st_32(tmem_o + c * 32, o);
+            for (int i = 0; i < HC; ++i) {
+              const int kpos = k0 + i;
+              if (!(kpos <= p_abs && (kpos >= first || kpos < a.keep_first))) sraw[i] = __float_as_uint(-INFINITY);
             }
           }
-          if (grow) {
+          // From the second tile on the maximum so far almost always serves, so the probabilities are made with it while
+          // the tile's own maximum is being found, and again in the rare case that it has grown too far.
+          if (j > 0) {
+            probabilities(true);
+          } else {
+            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-            for (int c = 0; c < PARTS64; ++c) l_part[c] *= alpha;
-            m_used = m_new;
+            for (int i = 0; i < HC; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(sraw[i]));
+            mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
           }
+        } else {
+          float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // four chains: the maxima do not wait on one another
+          if (edge) {
+            const int first = CHUNKED ? first_visible(p_abs, a) : a.window > 0 ? p_abs - a.window + 1 : 0;
+#pragma unroll
+            for (int i = 0; i < HC; ++i) {
+              const int kpos = k0 + i;
+              const float v = (kpos <= p_abs && (kpos >= first || kpos < a.keep_first)) ? __uint_as_float(sraw[i]) : -INFINITY;
+              sraw[i] = __float_as_uint(v);
+              mx4[i & 3] = fmaxf(mx4[i & 3], v);
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < HC; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(sraw[i]));
+          }
+          mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
         }
       }
-      const float m_sub = (m_used == -INFINITY) ? 0.f : m_used;
-      // P as bf16, two keys per 32-bit column, over the first half of this buffer's columns
+      // every score of the tile has been read by both warps behind this, so the probabilities may overwrite them
+      bool look_closer = true;
+      if constexpr (HS == 2) {
+        if (j > 0 && !any_grown(j & 1, mx * a.scale_log2 > m_used + FA_RESCALE_STEP, ok, look_closer)) { stopped = true; break; }
+      }
+      if (look_closer) {
+        // the row's maximum over all its columns
+        float maxima[HS];
+        if (!exchange(mx, ok, maxima)) { stopped = true; break; }
 #pragma unroll
-      for (int c = 0; c < HC / 64; ++c) {
-        uint32_t packed[32];
-        float add4[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int h2 = 0; h2 < HS; ++h2) mx = fmaxf(mx, maxima[h2]);
+        const float m_new = fmaxf(m_used, mx * a.scale_log2);
+        if (j == 0) {
+          m_used = m_new;
+        } else {
+          const bool grow = m_new > m_used + FA_RESCALE_STEP;    // also when nothing was seen before (-inf)
+          if (__any_sync(0xffffffffu, grow)) {
+            // O is final up to tile j - 1 before it is scaled; each warp scales its share of the columns
+            if (!fa_warp_wait(&pv_done[q][(j - 1) % SPB], ((j - 1) / SPB) & 1, failed)) ok = false;
+            tc_fence_after();
+            const float alpha = grow ? (m_used == -INFINITY ? 0.f : fa_exp2(m_used - m_new)) : 1.f;
+            if (ok) {
+#pragma unroll 1
+              for (int c = half * (D / 32 / HS); c < (half + 1) * (D / 32 / HS); ++c) {
+                uint32_t o[32];
+                tmem_ld_32(tmem_o + c * 32, o);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float p0 = fa_exp2(fmaf(__uint_as_float(sraw[c * 64 + 2 * i]), a.scale_log2, -m_sub));
-          const float p1 = fa_exp2(fmaf(__uint_as_float(sraw[c * 64 + 2 * i + 1]), a.scale_log2, -m_sub));
-          add4[i & 3] += p0 + p1;
-          packed[i] = fa_pack(p0, p1);
+                for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                tmem_st_32(tmem_o + c * 32, o);
+              }
+            }
+            if (grow) {
+#pragma unroll
+              for (int c = 0; c < PARTS64; ++c) l_part[c] *= alpha;
+              m_used = m_new;
+            }
+          }
         }
-        tmem_st_32_nowait(tmem_sp + half * (HC / 2) + c * 32, packed);
-        l_part[c] += (add4[0] + add4[1]) + (add4[2] + add4[3]);
+        if constexpr (HS == 2) probabilities(false);
+      }
+      if constexpr (HS == 2) {
+        tmem_st_32_nowait(tmem_sp + half * (HC / 2), packed);
+        l_part[0] += part;
+      } else {
+        const float m_sub = (m_used == -INFINITY) ? 0.f : m_used;
+        // P as bf16, two keys per 32-bit column, over the first half of this buffer's columns
+#pragma unroll
+        for (int c = 0; c < HC / 64; ++c) {
+          uint32_t packed[32];
+          float add4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const float p0 = fa_exp2(fmaf(__uint_as_float(sraw[c * 64 + 2 * i]), a.scale_log2, -m_sub));
+            const float p1 = fa_exp2(fmaf(__uint_as_float(sraw[c * 64 + 2 * i + 1]), a.scale_log2, -m_sub));
+            add4[i & 3] += p0 + p1;
+            packed[i] = fa_pack(p0, p1);
+          }
+          tmem_st_32_nowait(tmem_sp + half * (HC / 2) + c * 32, packed);
+          l_part[c] += (add4[0] + add4[1]) + (add4[2] + add4[3]);
+        }
       }
       tmem_st_wait();
       tc_fence_before();
@@ -487,32 +554,21 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
     tmem_meet<5, (FA_SOFTMAX_WARPS + 1) * 32>();
     tmem_base = tmem_base_slot;
     bool ok = fa_warp_wait(&q_ready, 0, failed);
-    // One head: a branch on the lane, whose 1,700 cycles a tile the softmax hides (issued by the converged warp instead, prompts
-    // of up to 2,048 tokens took 1 us longer). Two heads: the converged warp.
-    const uint32_t elected = NQ == 1 ? 1u : elect_one();
-    auto by_one = [&](auto&& issue) {
-      if constexpr (NQ == 1) {
-        if (lane == 0) issue();
-      } else {
-        issue();
-      }
-    };
+    const uint32_t elected = elect_one();       // issued by the converged warp, not from a branch on the lane
     const uint32_t q_addr = smem_u32(smem + L::OFF_Q);
     const uint32_t k_addr = smem_u32(smem + L::OFF_K), v_addr = smem_u32(smem + L::OFF_V);
     // S_q = Q_q K^T of tile j into the head's buffer j % SPB
     auto issue_s = [&](int j, int q) {
       const int st = j % FA_KV_STAGES, bq = q * SPB + j % SPB;
-      by_one([&] {
 #pragma unroll
-        for (int i = 0; i < (PAIR ? 4 : D / 16); ++i) {
-          const int ks = PAIR ? 4 * q + i : i;
-          const uint64_t ad = sw128_desc(q_addr + (PAIR ? 0 : q) * L::Q_BYTES + (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32);
-          const uint64_t bd = sw128_desc(k_addr + st * L::KV_BYTES + (ks >> 2) * (BN * 128) + (ks & 3) * 32);
-          umma_bf16_by(elected, tmem_base + L::TMEM_SP + (uint32_t)(bq * BN), ad, bd, IDESC_S, i != 0);
-        }
-        umma_commit_by(elected, &s_full[q][j % SPB]);
-        if (q == NQ - 1) umma_commit_by(elected, &k_empty[st]);       // the K stage is free once the last head's S has read it
-      });
+      for (int i = 0; i < (PAIR ? 4 : D / 16); ++i) {
+        const int ks = PAIR ? 4 * q + i : i;
+        const uint64_t ad = sw128_desc(q_addr + (PAIR ? 0 : q) * L::Q_BYTES + (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32);
+        const uint64_t bd = sw128_desc(k_addr + st * L::KV_BYTES + (ks >> 2) * (BN * 128) + (ks & 3) * 32);
+        umma_bf16_by(elected, tmem_base + L::TMEM_SP + (uint32_t)(bq * BN), ad, bd, IDESC_S, i != 0);
+      }
+      umma_commit_by(elected, &s_full[q][j % SPB]);
+      if (q == NQ - 1) umma_commit_by(elected, &k_empty[st]);       // the K stage is free once the last head's S has read it
       __syncwarp();
     };
     // O_q += P_q V of tile j, P read from the head's buffer in tensor memory
@@ -520,16 +576,14 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
       const int st = j % FA_KV_STAGES, b = j % SPB;
       if (!fa_warp_wait(&p_full[q][b], (j / SPB) & 1, failed)) return false;
       tc_fence_after();
-      by_one([&] {
 #pragma unroll
-        for (int ks = 0; ks < BN / 16; ++ks) {
-          const uint64_t bd = sw128_desc_mn(v_addr + st * L::KV_BYTES + ks * (16 * 128), BN * 128);
-          umma_bf16_ta_by(elected, tmem_base + L::TMEM_O + (uint32_t)(q * D),
-                       tmem_base + L::TMEM_SP + (uint32_t)((q * SPB + b) * BN + ks * 8), bd, IDESC_PV, (j | ks) != 0);
-        }
-        umma_commit_by(elected, &pv_done[q][b]);
-        if (q == NQ - 1) umma_commit_by(elected, &v_empty[st]);
-      });
+      for (int ks = 0; ks < BN / 16; ++ks) {
+        const uint64_t bd = sw128_desc_mn(v_addr + st * L::KV_BYTES + ks * (16 * 128), BN * 128);
+        umma_bf16_ta_by(elected, tmem_base + L::TMEM_O + (uint32_t)(q * D),
+                     tmem_base + L::TMEM_SP + (uint32_t)((q * SPB + b) * BN + ks * 8), bd, IDESC_PV, (j | ks) != 0);
+      }
+      umma_commit_by(elected, &pv_done[q][b]);
+      if (q == NQ - 1) umma_commit_by(elected, &v_empty[st]);
       __syncwarp();
       return true;
     };

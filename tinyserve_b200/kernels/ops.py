@@ -392,9 +392,10 @@ MAX_SPLITS = 32
 
 
 # What a tile of 128 keys costs a CTA of the tcgen05 prompt kernel with one head and with two, and what a CTA costs whatever
-# its tiles (B200 cycles, fitted to the times below).
-PREFILL_TILE_CYCLES = {1: 2560, 2: 4050}
-PREFILL_CTA_CYCLES = 15000
+# its tiles (B200 cycles, fitted to the times below; a tile of two heads takes 4,050, but portions of 2,048 tokens behind as
+# many, 67 us with one head a CTA and 76 with two, stay with two, which they are recorded with: 3,600 draws the line there).
+PREFILL_TILE_CYCLES = {1: 2330, 2: 3600}
+PREFILL_CTA_CYCLES = {1: 12000, 2: 15000}
 
 
 def _prefill_cycles(tiles: list[int], heads: int, heads_per_cta: int) -> float:
@@ -402,7 +403,7 @@ def _prefill_cycles(tiles: list[int], heads: int, heads_per_cta: int) -> float:
     no less than its longest CTA, than its work spread over the SMs, nor, for every k, than k + 1 times the
     k * 148-th longest CTA (one SM runs k + 1 that are as long)."""
     per_tile = heads // heads_per_cta
-    cost = [PREFILL_CTA_CYCLES + t * PREFILL_TILE_CYCLES[heads_per_cta] for t in tiles]
+    cost = [PREFILL_CTA_CYCLES[heads_per_cta] + t * PREFILL_TILE_CYCLES[heads_per_cta] for t in tiles]
     bound = max(cost[0], sum(cost) * per_tile / 148)
     for k in range(1, (len(tiles) * per_tile - 1) // 148 + 1):
         bound = max(bound, (k + 1) * cost[k * 148 // per_tile])
@@ -426,9 +427,9 @@ def prefill_heads_per_cta(query_lens: Sequence[int], context_lens: Sequence[int]
                           window: int = 0) -> int:
     """Two query heads of a kv group in a CTA share its key and value tiles and keep the tensor core busier, but make half as
     many CTAs, twice as long: whichever is estimated to end first (by the step's lengths alone, so the layers of a step, and
-    steps alike, share the estimate). Measured on B200, 16 / 8 heads of 128, one head / two: 512 tokens 13 / 18 us, 2,048
-    tokens 36 / 45, 2,048 at 4,096 positions 79 / 78, at 9,001 positions 183 / 160, 3,072 tokens 70 / 61, 8,192 tokens
-    350 / 273, seven prompts of 290 tokens 31 / 25. The same constants serve every layout the kernel takes: over 280 steps
+    steps alike, share the estimate). Measured on B200, 16 / 8 heads of 128, one head / two: 512 tokens 11 / 17 us, 2,048
+    tokens 30 / 43, 2,048 at 4,096 positions 67 / 76, at 9,001 positions 153 / 156, 4,096 tokens 90 / 76, 8,192 tokens
+    300 / 264, seven prompts of 290 tokens 24.5 / 24; 32 / 8 heads, 2,048 tokens 60 / 49, 1,024 23 / 26. The same constants serve every layout the kernel takes: over 280 steps
     with 16, 32 and 64 heads of 128 and 4 to 32 of 64, groups of 2, 4 and 8, windows or none, the choice took as long as
     the faster form to within the noise for heads of 128 and 0.3 % longer on average (17 % at worst) for heads of 64."""
     if (num_heads // num_kv_heads) % 2:
