@@ -16,6 +16,7 @@
 #define TS_PDL_CLASS PDL_ATTENTION
 #include "attention.cuh"
 #include "bounded_wait.cuh"
+#include "launch_list.cuh"
 
 namespace ts {
 
@@ -348,6 +349,7 @@ extern "C" int ts_decode_attention_mma(
   }
   return TS_ERR_UNSUPPORTED;
 }
+TS_LIST_ENTRY(ts_decode_attention_mma);
 
 // How many CTAs of the tensor-core decode kernel fit the machine at once (for the split choice).
 extern "C" int ts_decode_attention_mma_slots(int head_dim) {

@@ -24,6 +24,7 @@
 #include "attention.cuh"
 #include "bounded_wait.cuh"
 #include "cache_map.cuh"
+#include "launch_list.cuh"
 
 namespace ts {
 
@@ -734,6 +735,7 @@ extern "C" int ts_decode_attention_tma(
   }
   return page_size == 8 ? launch_dt<2, 8>(a, rows, error_flag, stream) : launch_dt<2, 16>(a, rows, error_flag, stream);
 }
+TS_LIST_ENTRY(ts_decode_attention_tma);
 
 // The same attention for a step of decode tokens only, fed with the raw output of the qkv product:
 // the kernel normalises (per-head RMSNorm; a null weight skips it) and rotates (rotate-half over
@@ -776,6 +778,7 @@ extern "C" int ts_decode_attention_tma_fused(
   return page_size == 8 ? launch_dt<2, 8, true>(a, rows, error_flag, stream, f)
                         : launch_dt<2, 16, true>(a, rows, error_flag, stream, f);
 }
+TS_LIST_ENTRY(ts_decode_attention_tma_fused);
 
 // How many CTAs of this kernel fit the machine at once (for the split choice).
 extern "C" int ts_decode_attention_tma_slots(int head_dim) {

@@ -14,6 +14,7 @@
 #include <cuda_pipeline_primitives.h>
 
 #include "attention.cuh"
+#include "launch_list.cuh"
 
 namespace ts {
 
@@ -316,3 +317,4 @@ extern "C" int ts_prefill_attention_mma(
   }
   return TS_ERR_UNSUPPORTED;
 }
+TS_LIST_ENTRY(ts_prefill_attention_mma);

@@ -68,6 +68,7 @@
 
 #include "attention.cuh"
 #include "tcgen05.cuh"
+#include "launch_list.cuh"
 
 namespace ts {
 
@@ -758,3 +759,4 @@ extern "C" int ts_prefill_attention_tcgen05(
   TS_FA(2, 16);
 #undef TS_FA
 }
+TS_LIST_ENTRY(ts_prefill_attention_tcgen05);

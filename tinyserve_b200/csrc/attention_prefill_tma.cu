@@ -20,6 +20,7 @@
 
 #include "attention.cuh"
 #include "bounded_wait.cuh"
+#include "launch_list.cuh"
 
 namespace ts {
 
@@ -403,3 +404,4 @@ extern "C" int ts_prefill_attention_tma(
   return page_size == 8 ? launch_pt<2, 8>(a, rows, max_query_len, error_flag, stream)
                         : launch_pt<2, 16>(a, rows, max_query_len, error_flag, stream);
 }
+TS_LIST_ENTRY(ts_prefill_attention_tma);

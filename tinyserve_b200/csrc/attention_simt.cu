@@ -1,6 +1,7 @@
 // Entry point of the CUDA-core paged attention kernels (see attention_simt.cuh).
 #define TS_PDL_CLASS PDL_ATTENTION
 #include "attention_simt.cuh"
+#include "launch_list.cuh"
 
 using namespace ts;
 
@@ -56,3 +57,4 @@ extern "C" int ts_paged_attention_simt(
   }
   return st;
 }
+TS_LIST_ENTRY(ts_paged_attention_simt);

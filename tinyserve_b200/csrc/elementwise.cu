@@ -6,6 +6,7 @@
 // The residual stream itself is kept in 32-bit, so the residual sum is a 32-bit sum.
 #define TS_PDL_CLASS PDL_ELEMENTWISE
 #include "common.cuh"
+#include "launch_list.cuh"
 
 namespace ts {
 
@@ -410,6 +411,7 @@ extern "C" int ts_add_rms_norm(float* resid, const void* delta, const void* weig
                   (const bf16*)weight, (bf16*)out, rows, hidden, eps, cache_row);
   return TS_ERR_BAD_ARGUMENT;
 }
+TS_LIST_ENTRY(ts_add_rms_norm);
 
 extern "C" int ts_rope_tables(const int* positions, const double* inv_freq, float* cos_out, float* sin_out,
                               int num_tokens, int half, double mult, cudaStream_t stream) {
@@ -442,3 +444,4 @@ extern "C" int ts_silu_mul(const void* gate_up, void* out, int num_tokens, int i
     return launch(silu_mul_kernel<bf16>, (int)blocks, 256, 0, stream, (const bf16*)gate_up, (bf16*)out, inter, total);
   return TS_ERR_BAD_ARGUMENT;
 }
+TS_LIST_ENTRY(ts_silu_mul);

@@ -35,6 +35,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "launch_list.cuh"
 
 namespace ts {
 namespace cg = cooperative_groups;
@@ -558,3 +559,4 @@ extern "C" int ts_gemm_f32(const float* x, const float* w, float* out, int M, in
   }
   return form == 3 ? launch_tile<1>(x, w, out, M, N, K, stream) : launch_tile<4>(x, w, out, M, N, K, stream);
 }
+TS_LIST_ENTRY(ts_gemm_f32);

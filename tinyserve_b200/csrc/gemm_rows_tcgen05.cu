@@ -15,6 +15,7 @@
 
 #include "cache_map.cuh"
 #include "tcgen05.cuh"
+#include "launch_list.cuh"
 
 namespace ts {
 namespace cg = cooperative_groups;
@@ -221,3 +222,4 @@ extern "C" int ts_gemm_rows_tcgen05(const void* x, const void* w, void* out, int
   return swiglu ? launch_rows_tc<true>(x, w, (bf16*)out, M, N, K, slices, error_flag, stream)
                 : launch_rows_tc<false>(x, w, (bf16*)out, M, N, K, slices, error_flag, stream);
 }
+TS_LIST_ENTRY(ts_gemm_rows_tcgen05);

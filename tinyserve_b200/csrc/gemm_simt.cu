@@ -7,6 +7,7 @@
 // not depend on which other rows share the batch.
 #define TS_PDL_CLASS PDL_OTHER
 #include "common.cuh"
+#include "launch_list.cuh"
 
 namespace ts {
 
@@ -89,3 +90,4 @@ extern "C" int ts_gemm_simt(const void* x, const void* w, void* out, int M, int 
     return launch(gemm_simt_kernel<bf16, float>, grid, GTHREADS, 0, stream, (const bf16*)x, (const bf16*)w, (float*)out, M, N, K);
   return TS_ERR_BAD_ARGUMENT;
 }
+TS_LIST_ENTRY(ts_gemm_simt);

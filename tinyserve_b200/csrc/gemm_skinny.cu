@@ -37,6 +37,7 @@
 // caller takes another kernel).
 #define TS_PDL_CLASS PDL_SKINNY
 #include "common.cuh"
+#include "launch_list.cuh"
 
 namespace ts {
 
@@ -842,6 +843,7 @@ extern "C" int ts_gemm_skinny(const void* x, const void* w, void* out, int M, in
     return dispatch_skinny<float>((const bf16*)x, (const bf16*)w, (float*)out, M, N, K, stream);
   return TS_ERR_BAD_ARGUMENT;
 }
+TS_LIST_ENTRY(ts_gemm_skinny);
 
 // gelu(x w^T) (the exact form) in bf16, M <= 16: the activation on the 32-bit sums.
 extern "C" int ts_gemm_skinny_gelu(const void* x, const void* w, void* out, int M, int N, int K, cudaStream_t stream) {
@@ -869,6 +871,7 @@ extern "C" int ts_gemm_skinny_swiglu(const void* x, const void* w, void* out, in
   if (M <= 16) return dispatch_swiglu_nt<2>(xp, wp, op, M, inter, K, stream);
   return dispatch_swiglu_nt<4>(xp, wp, op, M, inter, K, stream);
 }
+TS_LIST_ENTRY(ts_gemm_skinny_swiglu);
 
 // The same with a choice of activation: 0 = silu (as above), 1 = the tanh form of GELU, 2 = the clamped form
 // with its `limit`.
@@ -949,6 +952,7 @@ extern "C" int ts_gemm_skinny_normed(const void* resid16, const float* sumsq, in
   }
   return TS_ERR_BAD_ARGUMENT;
 }
+TS_LIST_ENTRY(ts_gemm_skinny_normed);
 
 // resid[M, N] += bf16(x * w^T) in place, resid16 = bf16(resid), and sumsq_out[m * (N / 16) + n / 16]
 // = sum over the 16 columns from n of the new resid[m, .]^2 (RESID above). M <= 16; sumsq_out
@@ -974,3 +978,4 @@ extern "C" int ts_gemm_skinny_to_stream(const void* x, const void* w, float* res
     return launch_skinny<bf16, 1, 1, false, 4, false, true>((const bf16*)x, (const bf16*)w, (bf16*)nullptr, M, N, K, stream, nrm);
   return launch_skinny<bf16, 2, 1, false, 4, false, true>((const bf16*)x, (const bf16*)w, (bf16*)nullptr, M, N, K, stream, nrm);
 }
+TS_LIST_ENTRY(ts_gemm_skinny_to_stream);

@@ -28,6 +28,7 @@
 #include <type_traits>
 
 #include "tcgen05.cuh"
+#include "launch_list.cuh"
 
 namespace ts {
 
@@ -568,6 +569,7 @@ extern "C" int ts_gemm_tcgen05(const void* x, const void* w, void* out, int M, i
   TS_TC(256, 4);
 #undef TS_TC
 }
+TS_LIST_ENTRY(ts_gemm_tcgen05);
 
 // gelu(x w^T) (the exact form) in bf16: the activation in the epilogue, on the 32-bit sums. tile_n: 256, or 512 for pairs of CTAs.
 extern "C" int ts_gemm_tcgen05_gelu(const void* x, const void* w, void* out, int M, int N, int K, int tile_n, int* error_flag,
@@ -594,6 +596,7 @@ extern "C" int ts_gemm_tcgen05_swiglu(const void* x, const void* w, void* out, i
   if (pair) return launch_tc_pair<6, bf16, GATED_SILU>(mx, mw, (bf16*)out, M, inter, K, error_flag, stream);
   return launch_tc<256, 4, bf16, GATED_SILU>(mx, mw, (bf16*)out, M, inter, K, error_flag, stream);
 }
+TS_LIST_ENTRY(ts_gemm_tcgen05_swiglu);
 
 // silu(x gate^T + b_gate) * (x up^T + b_up) in 32-bit, rounded once; bias [2 inter] bf16 (gate, then up).
 extern "C" int ts_gemm_tcgen05_biased_swiglu(const void* x, const void* w, const void* bias, void* out, int M, int inter,

@@ -9,6 +9,7 @@
 // Cache layout: [page, kv_head, offset_in_page, head_dim]; slot = page * page_size + offset.
 #define TS_PDL_CLASS PDL_ELEMENTWISE
 #include "common.cuh"
+#include "launch_list.cuh"
 
 namespace ts {
 
@@ -361,3 +362,4 @@ extern "C" int ts_qk_norm_rope_write(const void* qkv, void* q_out, const void* q
         num_kv_heads, head_dim, write_kv);
   return TS_ERR_BAD_ARGUMENT;
 }
+TS_LIST_ENTRY(ts_qk_norm_rope_write);

@@ -37,12 +37,14 @@ class _Region:
         self.used = 0          # offset in ``buf`` of the next take
         self.demand = 0        # bytes taken since the last reset, wherever they came from
         self.high_water = 0    # the largest demand of any step so far
+        self.moves = 0         # how often ``buf`` has been made anew
 
     def reset(self) -> None:
         if self.high_water > self.buf.numel():
             # The last step outgrew the buffer and was served piecemeal; make one buffer that
             # holds a whole step, so that from now on nothing moves.
             self.buf = torch.empty(self.high_water // _ALIGN * _ALIGN + _ALIGN, dtype=torch.uint8, device=self.device)
+            self.moves += 1
             self._typed = {}
             self._views = {}
         elif len(self._views) > _MOST_VIEWS:
@@ -71,6 +73,7 @@ class _Region:
             # Grow: views handed out earlier keep the old buffer alive until they die.
             grow = max(nbytes, 2 * self.buf.numel(), 1 << 16)
             self.buf = torch.empty((grow + _ALIGN - 1) // _ALIGN * _ALIGN, dtype=torch.uint8, device=self.device)
+            self.moves += 1
             self._typed = {}
             self._views = {}
             start, end = 0, nbytes
@@ -114,6 +117,11 @@ class Arena:
 
     def take_step(self, shape: tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
         return self._step.take(tuple(shape), dtype)
+
+    @property
+    def moves(self) -> int:
+        """Grows whenever a region's buffer is made anew (what was handed out before then lies elsewhere)."""
+        return self._step.moves + sum(f.moves for f in self._frames)
 
     @property
     def reserved_bytes(self) -> int:

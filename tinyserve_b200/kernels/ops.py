@@ -13,6 +13,7 @@ import ctypes
 import functools
 import math
 import os
+import threading
 from dataclasses import dataclass
 from typing import Any, Callable, Sequence
 
@@ -113,8 +114,32 @@ _SIGNATURES: dict[str, list[Any]] = {
     "ts_moe_gemm": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _f, _i, _i, _i, _vp],
     "ts_moe_combine": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _i, _i, _vp],
     "ts_sample": [_vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
+    "ts_library_gemm": [_vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp],
 }
 _fns: dict[str, Any] = {}
+# Functions of the library that only answer a question.
+_QUESTIONS = frozenset({"ts_gemm_skinny_to_stream_parts", "ts_decode_attention_tma_slots", "ts_decode_attention_mma_slots",
+                        "ts_talking_attention_mma_takes", "ts_latent_attention_mma_takes"})
+
+
+# Whether steps that are not recorded launch layers that differ only in their tensors from lists (``kernels.launch_list``);
+# off, every launch goes through the functions below.
+LAUNCH_LISTS = True
+
+
+class _Notes(threading.local):
+    """While ``calls`` is a list, the calls that this thread makes of the library are also written down there, as (name,
+    arguments), for ``kernels.launch_list``."""
+
+    calls: "list[tuple[str, tuple[Any, ...]]] | None" = None
+
+
+notes = _Notes()
+
+
+def _noted(name: str, f: Any, *args: Any) -> int:
+    notes.calls.append((name, args))
+    return f(*args)
 
 # Kernel classes launched with programmatic dependent launch in decode steps. Up to 16 rows: all
 # classes (the L2 prefetch kernel then starts beside the product before it, and nothing small is
@@ -159,6 +184,8 @@ def _fn(name: str) -> Any:
         f.argtypes = _SIGNATURES[name]
         f.restype = _i
         _fns[name] = f
+    if notes.calls is not None and name not in _QUESTIONS:
+        return functools.partial(_noted, name, f)
     return f
 
 
@@ -779,11 +806,20 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
         if tiles:
             gemm_tcgen05(x, w, out, TCGEN05_PAIR_TILE if tiles == "pairs" else 256)
             return
-    _dev(x, "x"), _dev(w, "w"), _dev(out, "out")
+    px, pw, po = _dev(x, "x"), _dev(w, "w"), _dev(out, "out")
+    if notes.calls is not None:
+        notes.calls.append(("ts_library_gemm", (px, pw, po, m, n, k, _code(out.dtype), _library_gemm_function(),
+                                                torch.cuda.current_blas_handle())))
     if out.dtype == torch.bfloat16:
         torch.mm(x, w.t(), out=out)                       # vendor library matrix product
     else:
         torch.mm(x, w.t(), out_dtype=torch.float32, out=out)
+
+
+@functools.lru_cache(maxsize=None)
+def _library_gemm_function() -> int:
+    """Where the vendor library that torch has loaded keeps the function that ``torch.mm`` calls."""
+    return ctypes.cast(ctypes.CDLL("libcublas.so.12").cublasGemmEx, _vp).value
 
 
 # The 32-bit product's tiles hold 32 rows, a grid 65,535 of them (the general kernel twice as many).
@@ -869,7 +905,8 @@ def _error_word(device: torch.device) -> torch.Tensor:
     """A device int32 that kernels with bounded waits set when a wait ran out."""
     w = _error_words.get(device)
     if w is None:
-        w = _error_words[device] = torch.zeros(1, dtype=torch.int32, device=device)
+        with torch.inference_mode(False):      # a step's first launch may be the one that makes it; others clear it later
+            w = _error_words[device] = torch.zeros(1, dtype=torch.int32, device=device)
     return w
 
 

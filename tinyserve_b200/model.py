@@ -10,6 +10,7 @@ wanted rows, apply the final norm to those rows only and multiply by the output 
 
 from __future__ import annotations
 
+from array import array
 from dataclasses import dataclass
 from pathlib import Path
 from typing import Any, Mapping
@@ -17,13 +18,19 @@ from typing import Any, Mapping
 import torch
 
 from . import parts as _parts  # noqa: F401  (registers the built-in parts)
+from .kernels import launch_list, ops
 from .config.base import LayerSpec, ModelConfig, ModelSpec
 from .parts.base import (
     BLOCKS, EMBEDDINGS, HEADS, NORMS, PART_FAMILIES, POSITION_ENCODINGS, STREAM_INPUTS,
-    Block, CacheNeed, PagedNeed, PositionEncoding, ResidualStream, StepContext, StreamInput, TensorSpec,
+    Block, CacheNeed, KVCacheEntry, PagedNeed, PositionEncoding, ResidualStream, StepContext, StreamInput, TensorSpec,
 )
 from .weights.loader import load_tensors, merge_specs
 from .weights.random_init import random_bound_tensors
+
+# Above this estimate of a layer's products (what the product of its tensors' bytes and the step's tokens comes to at the rates
+# of many rows, in a microsecond) its launches are not made from a list.
+LISTED_LAYER_US = 40.0
+BYTE_TOKENS_PER_US = {torch.bfloat16: 1.4e9, torch.float32: 7.4e7}
 
 
 @dataclass
@@ -73,6 +80,14 @@ class ModelParts:
                 self._user_index[(n, role)] = tuple(range(first, first + len(several))) if isinstance(need, tuple) else first
                 self._needs += several if call.reads_cache_of is None else (None,) * len(several)
         self._check_order()
+        self._rows_of_alike = self._find_alike()
+        # of a row, once the parts hold their tensors: where those of each call lie, call by call, and the bytes of each
+        self._tensor_places: dict[int, tuple[list[int], list[int]]] = {}
+        self._cache_indices = []      # of a call: the cache entries that its mixers keep
+        for n, call in enumerate(spec.order):
+            of = [self._user_index[(n, role)] for role in self.layers[call.layer].block.mixers()]
+            self._cache_indices.append([i for index in of for i in (index if isinstance(index, tuple) else (index,))
+                                        if self._needs[i] is not None])
 
     def _encoding(self, spec: Any) -> PositionEncoding:
         cand = POSITION_ENCODINGS.build(spec.kind, **spec.args)
@@ -115,6 +130,83 @@ class ModelParts:
                     raise ValueError(
                         f"order[{n}] reads the cache of call {src}, whose layout differs: {need} vs {other}")
 
+    # ---- layers whose launches are the same but for their tensors
+    MIN_ALIKE = 6      # one layer as it comes, two that are written down, and enough that follow them
+
+    def _find_alike(self) -> dict[int, int]:
+        """Rows of calls of the order that differ in nothing but their tensors: first call -> the one after the last."""
+        def like_next(n: int) -> bool:
+            a, b = self.spec.order[n], self.spec.order[n + 1]
+            if a.layer == b.layer or self.stream_inputs[n] is not None or self.stream_inputs[n + 1] is not None:
+                return False
+            if a.reads_cache_of is not None or b.reads_cache_of is not None:
+                return False
+            one, two = self.layers[a.layer], self.layers[b.layer]
+            return {**vars(one.spec), "prefix": None} == {**vars(two.spec), "prefix": None}
+
+        rows, n, calls = {}, 0, len(self.spec.order)
+        while n < calls:
+            end = n + 1
+            block = self.layers[self.spec.order[n].layer].block
+            if block.same_launches and all(p.same_launches for p in block.parts.values()):
+                while end < calls and like_next(end - 1):
+                    end += 1
+            if end - n >= self.MIN_ALIKE:
+                rows[n] = end
+            n = end
+        return rows
+
+    def _place_tensors(self) -> None:
+        """For each such row, where the tensors of its layers lie (the attributes of their parts, which change by ``bind``
+        alone). A row whose layers' tensors differ in their forms, or in how they lie to one another (a view of another
+        tensor in one layer and none in the next) is given up."""
+        self._tensor_places = {}
+        for n, end in self._rows_of_alike.items():
+            places, form, sizes = [], None, []
+            for call in range(n, end):
+                block = self.layers[self.spec.order[call].layer].block
+                named = [(role, name, t) for role, part in block.parts.items() for name, t in vars(part).items()
+                         if isinstance(t, torch.Tensor)]
+                storages = [t.untyped_storage().data_ptr() for _, _, t in named]
+                at = [t.data_ptr() for _, _, t in named]
+                first = [storages.index(s) for s in storages]          # the first tensor of the same memory
+                mine = [(role, name, t.shape, t.dtype, t.stride(), first[i], at[i] - at[first[i]])
+                        for i, (role, name, t) in enumerate(named)]
+                if form is None:
+                    form, sizes = mine, [t.numel() * t.element_size() for _, _, t in named]
+                if mine != form:
+                    break
+                places += at
+            else:
+                self._tensor_places[n] = places, sizes
+
+    def weight_bytes(self, row: int) -> int:
+        """The bytes of the tensors of one layer of such a row."""
+        return sum(self._tensor_places[row][1])
+
+    def alike_from(self, n: int) -> int:
+        """If a row of calls starts at ``n`` whose launches are the same but for their tensors, the call after its last
+        one; else 0."""
+        return self._rows_of_alike[n] if n in self._tensor_places else 0
+
+    def places_of_alike(self, row: int, calls: range, caches: list[Any]) -> "tuple[array[int], list[int]] | None":
+        """Where the tensors of these calls of the row that starts at ``row`` lie, weights and caches, call by call, and the
+        bytes of each of a call's; ``None`` if the caches are not alike."""
+        weights, sizes = self._tensor_places[row]
+        like = [caches[i] for i in self._cache_indices[calls[0]]]
+        if any(type(e) is not KVCacheEntry for e in like):
+            return None
+        form = [(e.group, e.page_size, e.k.shape, e.v.shape) for e in like]
+        count, places = len(sizes), []
+        for n in calls:
+            places += weights[(n - row) * count: (n - row + 1) * count]
+            for i, (group, page_size, k_shape, v_shape) in zip(self._cache_indices[n], form):
+                e = caches[i]
+                if type(e) is not KVCacheEntry or e.group != group or e.page_size != page_size or e.k.shape != k_shape or e.v.shape != v_shape:
+                    return None
+                places += (e.k.data_ptr(), e.v.data_ptr())
+        return array("Q", places), sizes + [t.numel() * t.element_size() for e in like for t in (e.k, e.v)]
+
     # ---- weights
     def _each_part(self):
         yield "", self.embedding
@@ -142,6 +234,7 @@ class ModelParts:
     def bind(self, tensors: Mapping[str, torch.Tensor]) -> None:
         for prefix, part in self._each_part():
             part.bind(prefix, tensors)
+        self._place_tensors()
 
     # ---- cache
     def cache_needs(self) -> list[CacheNeed | None]:
@@ -230,6 +323,51 @@ class DecoderModel:
             ctx.position_tables[key] = encoding.prepare(ctx)
         return ctx.position_tables[key]
 
+    def _lists_launches(self, n: int, ctx: StepContext) -> int:
+        """If the calls of this step from ``n`` on may be launched from a list, the call after them; else 0: not while the step is
+        being recorded (a recording runs what else it has beside the step), nor where each call is checked on the host, nor
+        where the products alone keep the device busy for longer than ``LISTED_LAYER_US`` a layer: the host is then ahead of
+        it without a list, and what a list takes to make is time that the device waits."""
+        if not ops.LAUNCH_LISTS or ctx.recorded or self.device.type != "cuda" or ops.CHECK_INDICES:
+            return 0
+        end = self.parts.alike_from(n)
+        if end and self.parts.weight_bytes(n) * ctx.num_tokens > LISTED_LAYER_US * BYTE_TOKENS_PER_US[self.dtype]:
+            return 0
+        return end
+
+    def _run_call(self, n: int, stream: ResidualStream, ctx: StepContext, caches: list[Any]) -> None:
+        parts, call = self.parts, self.spec.order[n]
+        layer = parts.layers[call.layer]
+        if parts.stream_inputs[n] is not None:
+            parts.stream_inputs[n].forward(stream, ctx)
+        if layer.positions:
+            tables = {role: self._position_data(p, ctx) for role, p in layer.positions.items()}
+        else:
+            tables = None if layer.position is None else self._position_data(layer.position, ctx)
+        ctx.upcoming_caches = parts.caches_of_call(n + 1, caches) if n + 1 < len(self.spec.order) else {}
+        layer.block.forward(stream, ctx, parts.caches_of_call(n, caches), call.reads_cache_of is None, tables)
+
+    def _run_alike(self, n: int, end: int, stream: ResidualStream, ctx: StepContext, caches: list[Any]) -> None:
+        """Calls ``n`` to ``end``, which differ in nothing but their tensors: the first as it comes (it may find another
+        stream than the rest), the next two written down, one in each half of the arena, and what follows
+        launched from those two lists, as long as the arena stayed where it was."""
+        self._run_call(n, stream, ctx, caches)
+        moves = ctx.arena.moves
+        noted, left = [], []
+        for m in (n + 1, n + 2):
+            with launch_list.Noting() as calls:
+                self._run_call(m, stream, ctx, caches)
+            noted.append(calls)
+            left.append(stream.state())
+        at = self.parts.places_of_alike(n, range(n + 1, end), caches) if ctx.arena.moves == moves else None
+        if at is not None and launch_list.run(noted, *at):
+            if (end - n - 3) % 2:           # the last layer worked where the first of the two did
+                ctx.arena.next_frame()
+                stream.set_state(left[0])
+            return
+        for m in range(n + 3, end):
+            self._run_call(m, stream, ctx, caches)
+
     def forward(self, ctx: StepContext, caches: list[Any], want_rows: torch.Tensor | None,
                 num_want: int) -> torch.Tensor | None:
         """Run this step's tokens; return float32 logits ``[num_want, vocab]`` at ``want_rows``
@@ -238,16 +376,14 @@ class DecoderModel:
         stream = ResidualStream(parts.embedding.forward(ctx))
         if parts.keeps_origin:
             stream.origin = parts.embedding.forward(ctx)      # a second copy that no layer adds to
-        for n, call in enumerate(self.spec.order):
-            layer = parts.layers[call.layer]
-            if parts.stream_inputs[n] is not None:
-                parts.stream_inputs[n].forward(stream, ctx)
-            if layer.positions:
-                tables = {role: self._position_data(p, ctx) for role, p in layer.positions.items()}
+        n, calls = 0, len(self.spec.order)
+        while n < calls:
+            end = self._lists_launches(n, ctx)
+            if end:
+                self._run_alike(n, end, stream, ctx, caches)
             else:
-                tables = None if layer.position is None else self._position_data(layer.position, ctx)
-            ctx.upcoming_caches = parts.caches_of_call(n + 1, caches) if n + 1 < len(self.spec.order) else {}
-            layer.block.forward(stream, ctx, parts.caches_of_call(n, caches), call.reads_cache_of is None, tables)
+                self._run_call(n, stream, ctx, caches)
+            n = max(n + 1, end)
         ctx.arena.step_region()
         for join in ctx.at_step_end:
             join()

@@ -23,6 +23,7 @@ from .base import (EVERY_STEP, KVCacheEntry, KVNeed, LatentNeed, LazyNormed, Mix
 
 class GQAAttention(Mixer):
     recordable = EVERY_STEP
+    same_launches = True
 
     def __init__(self, prefix: str, hidden_size: int, num_heads: int, num_kv_heads: int,
                  head_dim: int, scale: float, qk_norm: bool = False, qk_norm_eps: float = 1e-6,

@@ -319,6 +319,13 @@ class ResidualStream:
         self._sumsq_buf: torch.Tensor | None = None
         self._resid16_buf: torch.Tensor | None = None
 
+    def state(self) -> tuple[Any, ...]:
+        return tuple(getattr(self, name) for name in self.__slots__)
+
+    def set_state(self, state: tuple[Any, ...]) -> None:
+        for name, value in zip(self.__slots__, state):
+            setattr(self, name, value)
+
     def fusion_buffers(self, ctx: "StepContext") -> tuple[torch.Tensor, torch.Tensor]:
         """Scratch for the stream's copy in the model dtype and for the parts of the rows' sums
         of squares (up to 16 rows x a part per 8 columns: two floats per column)."""
@@ -402,6 +409,12 @@ class Part:
     # allows nothing; the built-in parts allow both (``EVERY_STEP``). A mixer with state of its own
     # can allow "decode" by indexing its state with ``ctx.state_slots`` on the device.
     recordable: frozenset = frozenset()
+
+    # True if, in a step that is not being recorded, two parts of this class with equal arguments launch the same kernels
+    # with the same arguments but for their own tensors (attributes of the part), their cache entries and the place of
+    # what they take from the arena, and do nothing else: then the launches of one layer can stand for those of
+    # the next ones (``kernels.launch_list``).
+    same_launches: bool = False
 
     def tensor_specs(self, prefix: str) -> list[TensorSpec]:
         return []
@@ -518,6 +531,7 @@ class Block:
 
     roles: Mapping[str, str] = {}
     optional_roles: frozenset = frozenset()
+    same_launches: bool = False        # as for Part: the block does nothing but run its parts on the stream
 
     def __init__(self, parts: Mapping[str, Part]) -> None:
         self.parts = dict(parts)

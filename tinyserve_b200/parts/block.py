@@ -23,6 +23,7 @@ class PreNormBlock(Block):
     roles = {"mixer_norm": "norm", "mixer": "mixer", "second_mixer": "mixer", "feed_forward_norm": "norm",
              "feed_forward": "feed_forward"}
     optional_roles = frozenset({"second_mixer", "feed_forward_norm", "feed_forward"})
+    same_launches = True
 
     def __init__(self, parts: Mapping[str, Part], mixer_scale: float = 1.0, second_mixer_scale: float = 1.0) -> None:
         super().__init__(parts)

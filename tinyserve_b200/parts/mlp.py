@@ -19,6 +19,7 @@ from .base import (EVERY_STEP, FeedForward, LazyNormed, ResidualStream, StepCont
 
 class SwiGLU(FeedForward):
     recordable = EVERY_STEP
+    same_launches = True
 
     def __init__(self, prefix: str, hidden_size: int, intermediate_size: int) -> None:
         self.prefix = prefix

@@ -26,6 +26,7 @@ from .base import EVERY_STEP, LazyNormed, Norm, ResidualStream, StepContext, Ten
 
 class RMSNorm(Norm):
     recordable = EVERY_STEP
+    same_launches = True
 
     def __init__(self, name: str, size: int, eps: float, unit_offset: bool = False, round_once: bool = False) -> None:
         self.name, self.size, self.eps = name, int(size), float(eps)
