@@ -769,6 +769,53 @@ def test_sample_nucleus_of_wide_rows(vocab) -> None:
         assert out[5].item() == vocab // 2
 
 
+@pytest.mark.parametrize("vocab", [31, 1000, 1024, 1025, 5000, 40000, 163840, 163841])
+def test_sample_nucleus_of_ties_and_of_few_or_many_weights_between_the_bounds(vocab) -> None:
+    """Rows whose threshold falls on equal weights (two or a thousand of them, or all tokens), on the likeliest token, or a long
+    way down; the numbers of weights that are left to sort lie on both sides of a CTA's threads. A drawn token's more likely
+    tokens hold less than top_p, and of all tokens of which that is true the drawn one won the race of the row drawn without
+    top_p; sums within 1e-5 of top_p may fall to either side. Infinities and NaN draw something."""
+    g = torch.Generator(device="cuda").manual_seed(vocab)
+    flat = torch.zeros(vocab, device="cuda")
+    two = flat.clone()
+    two[: vocab // 2] = 1.0
+    steps = (torch.arange(vocab, device="cuda") % max(1, vocab // 700)).float() * 0.01
+    narrow, wide = torch.randn(vocab, device="cuda", generator=g) * 1e-3, torch.randn(vocab, device="cuda", generator=g) * 4
+    peak = flat.clone()
+    peak[vocab // 3] = 30.0
+    cases = [(flat, 0.5), (two, 0.3), (two, 0.9), (steps, 0.37), (narrow, 0.5), (narrow, 0.99), (wide, 0.05), (wide, 0.95), (wide, 0.999995), (peak, 0.9)]
+    r = 2 * len(cases)
+    logits = torch.stack([c[0] for c in cases for _ in range(2)])
+    top_p = torch.tensor([c[1] for c in cases for _ in range(2)], device="cuda")
+    temps, seeds = torch.ones(r, device="cuda"), torch.arange(r, device="cuda")
+    p = torch.softmax(logits.double(), -1)
+    order = p.sort(-1, descending=True)
+    before = order.values.cumsum(-1) - order.values
+    first = torch.searchsorted(-order.values, -p, right=False)       # of the equal ones the first
+    above = before.gather(1, first)
+    out = torch.empty(r, dtype=torch.int32, device="cuda")
+    for draw in range(3):
+        draws = torch.full((r,), draw, device="cuda", dtype=torch.int64)
+        ops.sample(logits, out, temps, top_p, seeds, draws)
+        alone = torch.empty(1, dtype=torch.int32, device="cuda")
+        for b in range(r):
+            tok = int(out[b])
+            assert float(above[b, tok]) < float(top_p[b]) + 1e-5
+            ops.sample(logits[b: b + 1].contiguous(), alone, temps[b: b + 1], top_p[b: b + 1], seeds[b: b + 1].contiguous(), draws[b: b + 1])
+            assert int(alone) == tok, "the rows beside it have a say"
+            sure = logits[b].clone()
+            sure[above[b] >= float(top_p[b]) - 1e-5] = float("-inf")     # (without top_p: the race of the tokens that are surely in it)
+            sure[int(p[b].argmax())] = logits[b, int(p[b].argmax())]
+            ops.sample(sure[None].contiguous(), alone, temps[b: b + 1], torch.ones(1, device="cuda"), seeds[b: b + 1].contiguous(), draws[b: b + 1])
+            unsure = (above[b] - float(top_p[b])).abs() <= 1e-5
+            assert int(alone) == tok or bool(unsure[tok])
+    odd = torch.randn(4, vocab, device="cuda", generator=g)
+    odd[0, 3], odd[1, 5], odd[2], odd[3, 1:] = float("inf"), float("nan"), float("-inf"), float("-inf")
+    out = torch.full((4,), -1, dtype=torch.int32, device="cuda")
+    ops.sample(odd, out, torch.ones(4, device="cuda"), torch.full((4,), 0.9, device="cuda"), torch.arange(4, device="cuda"), torch.zeros(4, dtype=torch.int64, device="cuda"))
+    assert bool(((out >= 0) & (out < vocab)).all()) and int(out[3]) == 0
+
+
 def test_sample_with_top_p_on_two_streams_at_once() -> None:
     """The chunks of a row meet in their cluster alone, so launches that run beside each other do not mix their winners
     (rows with and without top-p, and greedy ones)."""

@@ -16,12 +16,13 @@
 // and again, for the search of its threshold: its chunks are the CTAs of a cluster (one to eight, by
 // the vocabulary) that keep their weights in registers (20 a thread: 163,840 tokens; a larger
 // vocabulary is read from L2 each time) and add up their sums, and pick the winner, through
-// distributed shared memory. Bound by the passes over the weights and the barrier of each: seven
-// thresholds a pass (11 passes instead of 30), and a warp none of whose weights lie between the
-// bounds left leaves its sums where they are. Normal logits, deviation 3, top-p 0.95, one CTA a row
-// with two-way passes / eight CTAs for every vocabulary, closed warps adding up again / now, 1, 64
-// and 256 rows: 151,936 tokens 1,023, 1,044, 2,110 / 48, 233, 834 / 43, 207, 740 us; 32,768 tokens 128,
-// 129, 253 / 41, 196, 699 / 42, 43, 161; 1,000 tokens 19, 19, 36 / 35, 166, 593 / 15, 16, 30.
+// distributed shared memory. Bound by the passes over the weights and the barrier of each: seven thresholds a pass, a warp none
+// of whose weights lie between the bounds left leaves its sums where they are, the search starts from a bound that the mean
+// weight gives, and as soon as no more than 1,024 weights are left between the bounds, every CTA sorts these and sums them up
+// itself. Normal logits, top-p 0.95 at deviation 3 and 0.99 at 8, passes to the end (11 of them) / now: 151,936 tokens, 1 row
+// 46.8, 30.5 / 39.2, 22.7 us, 64 rows 226, 158 / 192, 105, 256 rows 823, 572 / 698, 392; 32,768 tokens, 1 row 43.3, 31.1 / 31.8, 17.7, 256
+// rows 172, 129 / 130, 81; 1,000 tokens, 1 row 15.5, 13.9 / 11.6, 8.9. (One CTA a row and two-way passes took 1,023 us for a row of
+// 151,936.) Beyond 163,840 tokens nothing is sorted: 200,000 tokens 72.5 / 72.7.
 #define TS_PDL_CLASS PDL_SAMPLING
 #include <cooperative_groups.h>
 
@@ -169,13 +170,75 @@ __device__ __forceinline__ Best scan_range(const float* __restrict__ l, int begi
 // The nucleus threshold of one row by the cluster of its CTAS chunks: the smallest bit pattern b in
 // [0, bits(1.0)] with mass{weight > float(b)} < top_p * mass{all}. Tokens of [begin, end) are this CTA's.
 constexpr int NUCLEUS_WAYS = 8, NUCLEUS_HELD = 20, NUCLEUS_HELD_SMALL = 4;
+constexpr int NUCLEUS_LIST = SM_THREADS;      // weights that are sorted at the end, one a thread
 
 struct NucleusShared {
   float scratch[33];
   float by_warp[NUCLEUS_WAYS - 1][32];
-  float mine[2][NUCLEUS_WAYS - 1];      // this CTA's sums, read by the whole cluster; alternating
-  float whole[2][NUCLEUS_WAYS - 1];     // the cluster's
+  float mine[2][NUCLEUS_WAYS];          // this CTA's sums (the last: how many weights lie between the bounds), read by the whole
+                                        // cluster; alternating
+  float whole[2][NUCLEUS_WAYS];         // the cluster's
+  int listed[2];                        // this CTA's weights between the bounds, alternating ...
+  float list[NUCLEUS_LIST];             // ... and the weights, in any order, if there are no more than these
+  float sorted[NUCLEUS_LIST];
+  float found;
 };
+
+// Where the sum of the weights in descending order, on top of `base`, first reaches `target`: the weight there, or `none`. The
+// cluster's lists (of turn `turn`) hold `n` <= NUCLEUS_LIST of them, which every CTA sorts for itself: equal weights are
+// alike, so neither the order within a list nor anything else of the launch shows in the result.
+template <int CTAS>
+__device__ __forceinline__ float nucleus_from_lists(NucleusShared& sh, int turn, int n, float base, float target, float none) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float v = 0.f;
+  if constexpr (CTAS == 1) {
+    if (tid < n) v = sh.list[tid];
+  } else {
+    cg::cluster_group cluster = cg::this_cluster();
+    int count[CTAS], at = tid;
+#pragma unroll
+    for (int r = 0; r < CTAS; ++r) count[r] = *cluster.map_shared_rank(&sh.listed[turn], r);
+#pragma unroll
+    for (int r = 0; r < CTAS; ++r) {
+      if (at >= 0 && at < count[r]) v = *cluster.map_shared_rank(&sh.list[at], r);
+      at -= count[r];
+    }
+  }
+  int size = 32;
+  while (size < n) size <<= 1;
+  for (int k = 2; k <= size; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {      // bitonic, descending
+      float other;
+      if (j >= 32) {
+        __syncthreads();
+        sh.sorted[tid] = v;
+        __syncthreads();
+        other = sh.sorted[tid ^ j];
+      } else {
+        other = __shfl_xor_sync(0xffffffffu, v, j);
+      }
+      v = (((tid & j) == 0) == ((tid & k) == 0)) ? fmaxf(v, other) : fminf(v, other);
+    }
+  float sum = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float below = __shfl_up_sync(0xffffffffu, sum, o);
+    if (lane >= o) sum += below;
+  }
+  if (lane == 31) sh.scratch[warp] = sum;
+  if (tid == 0) sh.found = none;
+  __syncthreads();
+  float before = lane < warp ? sh.scratch[lane] : 0.f;      // of the warps in front
+  before = base + warp_sum(before);
+  const unsigned reached = __ballot_sync(0xffffffffu, tid < n && !(before + sum < target));
+  __syncthreads();
+  if (lane == 0) sh.scratch[warp] = reached ? 1.f : 0.f;
+  __syncthreads();
+  const unsigned warps = __ballot_sync(0xffffffffu, sh.scratch[lane] != 0.f);
+  if (warps && warp == __ffs(warps) - 1 && lane == __ffs(reached) - 1) sh.found = v;
+  __syncthreads();
+  return sh.found;
+}
 
 // COUNT values per CTA over the cluster: their sums in the order of the CTAs, or the largest. `turn` alternates from
 // call to call, so that one barrier of all CTAs a call is enough.
@@ -203,7 +266,7 @@ __device__ __forceinline__ const float* nucleus_exchange(NucleusShared& sh, int 
 
 // HELD: weights a thread keeps in registers, 0: they are read and raised again in every pass.
 template <int CTAS, int HELD>
-__device__ __forceinline__ float nucleus_threshold(const float* __restrict__ l, int begin, int end, float inv_t, float top_p,
+__device__ __forceinline__ float nucleus_threshold(const float* __restrict__ l, int vocab, int begin, int end, float inv_t, float top_p,
                                                    float& row_max, NucleusShared& sh) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float e[HELD ? HELD : 1];
@@ -234,12 +297,53 @@ __device__ __forceinline__ float nucleus_threshold(const float* __restrict__ l, 
     for (int i = begin + tid; i < end; i += SM_THREADS) z += weight_of(l[i], inv_t, mx);
   }
   z = block_sum(z, sh.scratch);
-  if (tid == 0) sh.mine[1][0] = z;
-  const float target = top_p * nucleus_exchange<CTAS, 1, false>(sh, 1)[0];
+  if (tid == 0) { sh.mine[1][0] = z; sh.listed[0] = sh.listed[1] = 0; }
+  const float all = nucleus_exchange<CTAS, 1, false>(sh, 1)[0], target = top_p * all;
+  if (!(target == target)) return 1.f;        // no threshold's sum is below it
 
   uint32_t lo = 0u, hi = 0x3f800000u;
+  // A threshold's sum is short of the whole by at most the threshold times the number of tokens, so it reaches the target at
+  // half of (1 - top_p) times their mean weight, unless 1 - top_p is a matter of rounding.
+  if (1.f - top_p > 1e-4f) lo = __float_as_uint(fminf(0.5f * (1.f - top_p) * all / (float)vocab, 1.f));
   int turn = 0;
   bool open = true;                     // whether a weight of this warp may lie between the bounds
+  float base = 0.f;                     // the sum above `hi`
+  auto list_between = [&](int which) {
+    if constexpr (HELD > 0) {
+      // weights at or below float(lo) count for no threshold left, those above float(hi) for each of them
+      const float low = __uint_as_float(lo), high = __uint_as_float(hi);
+      if (!open) return;
+      int between = 0;
+      float above = 0.f;
+#pragma unroll
+      for (int j = 0; j < HELD; ++j) {
+        between += e[j] > low && e[j] <= high ? 1 : 0;
+        if (e[j] > high) above += e[j];
+      }
+      const int of_warp = __reduce_add_sync(0xffffffffu, between);
+      open = of_warp != 0;
+      if (!open) {
+        above = warp_sum(above);
+        if (lane < NUCLEUS_WAYS - 1) sh.by_warp[lane][warp] = above;
+        return;
+      }
+      int at = 0;
+      if (lane == 0) at = atomicAdd(&sh.listed[which], of_warp);
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (at + of_warp > NUCLEUS_LIST) return;
+      int in_front = between;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int below = __shfl_up_sync(0xffffffffu, in_front, o);
+        if (lane >= o) in_front += below;
+      }
+      at += in_front - between;
+#pragma unroll
+      for (int j = 0; j < HELD; ++j)
+        if (e[j] > low && e[j] <= high) sh.list[at++] = e[j];
+    }
+  };
+  list_between(0);
   while (lo < hi) {
     if (open) {        // else the warp's sums, the same for every threshold left, are where it has put them
       float t[NUCLEUS_WAYS - 1], mass[NUCLEUS_WAYS - 1];
@@ -272,8 +376,13 @@ __device__ __forceinline__ float nucleus_threshold(const float* __restrict__ l, 
     if (warp < NUCLEUS_WAYS - 1) {
       const float v = warp_sum(sh.by_warp[warp][lane]);
       if (lane == 0) sh.mine[turn][warp] = v;
+    } else if (tid == SM_THREADS - 1) {
+      sh.mine[turn][NUCLEUS_WAYS - 1] = (float)sh.listed[turn];
+      sh.listed[turn ^ 1] = 0;
     }
-    const float* whole = nucleus_exchange<CTAS, NUCLEUS_WAYS - 1, false>(sh, turn);
+    const float* whole = nucleus_exchange<CTAS, NUCLEUS_WAYS, false>(sh, turn);
+    if (HELD && whole[NUCLEUS_WAYS - 1] <= (float)NUCLEUS_LIST)
+      return nucleus_from_lists<CTAS>(sh, turn, (int)whole[NUCLEUS_WAYS - 1], base, target, __uint_as_float(lo));
     // sums of the same terms in the same order grow as the threshold falls: the first one below the target ends the search
     uint32_t below = lo, next = hi;
     bool found = false;
@@ -281,29 +390,14 @@ __device__ __forceinline__ float nucleus_threshold(const float* __restrict__ l, 
     for (int q = 0; q < NUCLEUS_WAYS - 1; ++q) {
       const uint32_t mid = lo + (uint32_t)(((unsigned long long)(hi - lo) * (q + 1)) / NUCLEUS_WAYS);
       if (!found) {
-        if (whole[q] < target) { next = mid; found = true; }
+        if (whole[q] < target) { next = mid; base = whole[q]; found = true; }
         else below = mid + 1u;
       }
     }
     lo = below;
     hi = next;
     turn ^= 1;
-    if (HELD && open) {
-      // weights at or below float(lo) count for no threshold left, those above float(hi) for each of them
-      const float low = __uint_as_float(lo), high = __uint_as_float(hi);
-      bool between = false;
-      float above = 0.f;
-#pragma unroll
-      for (int j = 0; j < HELD; ++j) {
-        between = between || (e[j] > low && e[j] <= high);
-        if (e[j] > high) above += e[j];
-      }
-      open = __any_sync(0xffffffffu, between);
-      if (!open) {
-        above = warp_sum(above);
-        if (lane < NUCLEUS_WAYS - 1) sh.by_warp[lane][warp] = above;
-      }
-    }
+    list_between(turn);
   }
   return __uint_as_float(lo);
 }
@@ -339,7 +433,7 @@ __global__ void __launch_bounds__(SM_THREADS) sample_kernel(const float* __restr
   float mx = 0.f, threshold = 0.f;
   if constexpr (CTAS > 0) if (tp < 1.f) {
     __shared__ NucleusShared sh;
-    threshold = nucleus_threshold<CTAS, HELD>(l, begin, end, 1.f / temp, tp, mx, sh);
+    threshold = nucleus_threshold<CTAS, HELD>(l, vocab, begin, end, 1.f / temp, tp, mx, sh);
   }
 
   // ---- this CTA's chunk, then one CTA picks among the chunks
