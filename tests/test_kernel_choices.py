@@ -107,6 +107,20 @@ def test_one_head_or_two_a_cta_in_the_prompt_attention() -> None:
     assert choice([8192], [8192], heads=24) == 1          # three heads a group: no pairs
 
 
+def test_one_head_or_two_a_cta_by_the_head_size_and_a_recorded_portion_s_note_of_it() -> None:
+    """Heads of 64 and of 128 lie on different sides where the two forms were measured to; a step notes which of its layouts have
+    which, so that the note alone gives the choice again."""
+    from types import SimpleNamespace
+
+    assert ops.prefill_heads_per_cta([1024], [1024], 32, 8) == 1 and ops.prefill_heads_per_cta([1024], [1024], 32, 8, 0, 64) == 2
+    for d in (64, 128):
+        assert ops.prefill_heads_per_cta([512], [512], 16, 8, 0, d) == 1 and ops.prefill_heads_per_cta([4096], [4096], 16, 8, 0, d) == 2
+        ctx = SimpleNamespace(query_lens=[1024], context_lens=[1024], prompt_heads={})
+        heads = ops._prefill_heads_per_cta(ctx, 32, 8, 0, d)
+        (layout, noted), = ctx.prompt_heads.items()
+        assert noted == heads == ops.prefill_heads_per_cta([1024], [1024], *layout)
+
+
 def test_expert_products_of_a_few_tokens_by_their_ctas_per_k() -> None:
     """On either side of the line, shapes measured on both; never beyond the 16 rows that the form holds."""
     take = ops.moe_takes_few_rows

@@ -128,6 +128,10 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
   using L = FaLayout<D64, NQ, PAIR>;
   constexpr int D = L::D, BN = FA_BN, FA_KV_STAGES = L::STAGES, SPB = L::SPB, FA_SOFTMAX_WARPS = L::SOFTMAX_WARPS, HS = L::HS, PW = L::PW;
   constexpr int HC = BN / HS;                                  // score columns of one softmax thread
+  // One head of 128 a CTA: the probabilities ahead of the tile's maximum, the MMAs from the converged warp. Heads of 64, whose MMA
+  // warp has fewer instructions a tile, lose by that (100 tokens 7.9 -> 9.0 us, 256 behind 7,000 with a window of 512 20.6 -> 24.5, 2,048
+  // tokens 25.8 / 25.7) and keep the other way of both.
+  constexpr bool AHEAD = HS == 2 && D64 == 2, BY_LANE = NQ == 1 && D64 == 1;
   // instruction descriptors: D = f32, A = B = bf16, M = 128; S: N = BN, both operands K-major;
   // PV: N = D, B MN-major (bit 16)
   constexpr uint32_t IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(FA_BM >> 4) << 24);
@@ -140,7 +144,7 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
   __shared__ int failed_flag;
   __shared__ float pair_value[NQ][4][HS][32];      // what the warps of a row quarter tell one another: a row maximum, a row sum
   __shared__ int pair_ok[NQ][4][HS];
-  __shared__ uint2 pair_grown[2][4][2];             // (HS = 2) the rows whose maximum has grown, and whether the waits have held
+  __shared__ uint2 pair_grown[2][4][2];             // (AHEAD) the rows whose maximum has grown, and whether the waits have held
   volatile int* failed = &failed_flag;
 
   // ---- which rows and keys (uniform over the CTA); a CTA without rows leaves before any set-up
@@ -168,8 +172,8 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
 
   pdl_trigger();
   unsigned char* smem = (unsigned char*)(((uintptr_t)fa_raw + 1023) & ~(uintptr_t)1023);
-  // known to the compiler to be the same in the whole warp, so that the MMA warp's operands are (umma_bf16_by)
-  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  // unless BY_LANE known to the compiler to be the same in the whole warp, so that the MMA warp's operands are (umma_bf16_by)
+  const int warp = BY_LANE ? (int)(threadIdx.x >> 5) : __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < FA_KV_STAGES; ++s) {
       mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
@@ -247,7 +251,7 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
         return all_ok;
       }
     };
-    // (HS = 2) Whether a row of either warp has `grown`. One meeting: tiles take the two places in turn, so a place is written
+    // (AHEAD) Whether a row of either warp has `grown`. One meeting: tiles take the two places in turn, so a place is written
     // again behind the meeting of the tile between, which a warp reaches after it has read.
     auto any_grown = [&](int turn, bool grown, bool mine_ok, bool& any) -> bool {
       const unsigned mine = __ballot_sync(0xffffffffu, grown);
@@ -277,7 +281,7 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
       const int k0 = tile_of(j) * BN + half * HC;              // the first key of this thread's columns
       // Two threads a row: the probabilities of the thread's 64 columns as bf16, two keys per word, and their sum, in the scale
       // of the maximum so far; `look` finds the columns' own maximum on the way, beside the exponentials.
-      uint32_t packed[HS == 2 ? 32 : 1];
+      uint32_t packed[AHEAD ? 32 : 1];
       float part = 0.f;
       auto probabilities = [&](bool look) {
         const float m_sub = m_used == -INFINITY ? 0.f : m_used;
@@ -299,7 +303,7 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
         tmem_ld_wait();
         const bool edge = (k0 + HC - 1 > p_lo) || (CHUNKED ? k0 < first_visible(p_lo + FA_BM - 1, a)
                                                            : a.window > 0 && k0 < p_lo + FA_BM - a.window);
-        if constexpr (HS == 2) {
+        if constexpr (AHEAD) {
           if (edge) {
             const int first = CHUNKED ? first_visible(p_abs, a) : a.window > 0 ? p_abs - a.window + 1 : 0;
 #pragma unroll
@@ -338,7 +342,7 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
       }
       // every score of the tile has been read by both warps behind this, so the probabilities may overwrite them
       bool look_closer = true;
-      if constexpr (HS == 2) {
+      if constexpr (AHEAD) {
         if (j > 0 && !any_grown(j & 1, mx * a.scale_log2 > m_used + FA_RESCALE_STEP, ok, look_closer)) { stopped = true; break; }
       }
       if (look_closer) {
@@ -374,9 +378,9 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
             }
           }
         }
-        if constexpr (HS == 2) probabilities(false);
+        if constexpr (AHEAD) probabilities(false);
       }
-      if constexpr (HS == 2) {
+      if constexpr (AHEAD) {
         tmem_st_32_nowait(tmem_sp + half * (HC / 2), packed);
         l_part[0] += part;
       } else {
@@ -555,21 +559,30 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
     tmem_meet<5, (FA_SOFTMAX_WARPS + 1) * 32>();
     tmem_base = tmem_base_slot;
     bool ok = fa_warp_wait(&q_ready, 0, failed);
-    const uint32_t elected = elect_one();       // issued by the converged warp, not from a branch on the lane
+    const uint32_t elected = BY_LANE ? 1u : elect_one();
+    auto by_one = [&](auto&& issue) {
+      if constexpr (BY_LANE) {
+        if (lane == 0) issue();
+      } else {
+        issue();
+      }
+    };
     const uint32_t q_addr = smem_u32(smem + L::OFF_Q);
     const uint32_t k_addr = smem_u32(smem + L::OFF_K), v_addr = smem_u32(smem + L::OFF_V);
     // S_q = Q_q K^T of tile j into the head's buffer j % SPB
     auto issue_s = [&](int j, int q) {
       const int st = j % FA_KV_STAGES, bq = q * SPB + j % SPB;
+      by_one([&] {
 #pragma unroll
-      for (int i = 0; i < (PAIR ? 4 : D / 16); ++i) {
-        const int ks = PAIR ? 4 * q + i : i;
-        const uint64_t ad = sw128_desc(q_addr + (PAIR ? 0 : q) * L::Q_BYTES + (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32);
-        const uint64_t bd = sw128_desc(k_addr + st * L::KV_BYTES + (ks >> 2) * (BN * 128) + (ks & 3) * 32);
-        umma_bf16_by(elected, tmem_base + L::TMEM_SP + (uint32_t)(bq * BN), ad, bd, IDESC_S, i != 0);
-      }
-      umma_commit_by(elected, &s_full[q][j % SPB]);
-      if (q == NQ - 1) umma_commit_by(elected, &k_empty[st]);       // the K stage is free once the last head's S has read it
+        for (int i = 0; i < (PAIR ? 4 : D / 16); ++i) {
+          const int ks = PAIR ? 4 * q + i : i;
+          const uint64_t ad = sw128_desc(q_addr + (PAIR ? 0 : q) * L::Q_BYTES + (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32);
+          const uint64_t bd = sw128_desc(k_addr + st * L::KV_BYTES + (ks >> 2) * (BN * 128) + (ks & 3) * 32);
+          umma_bf16_by(elected, tmem_base + L::TMEM_SP + (uint32_t)(bq * BN), ad, bd, IDESC_S, i != 0);
+        }
+        umma_commit_by(elected, &s_full[q][j % SPB]);
+        if (q == NQ - 1) umma_commit_by(elected, &k_empty[st]);       // the K stage is free once the last head's S has read it
+      });
       __syncwarp();
     };
     // O_q += P_q V of tile j, P read from the head's buffer in tensor memory
@@ -577,14 +590,16 @@ __global__ void __launch_bounds__((4 * (NQ == 1 ? 2 : 1) * NQ + 2 * (NQ == 1 ? 2
       const int st = j % FA_KV_STAGES, b = j % SPB;
       if (!fa_warp_wait(&p_full[q][b], (j / SPB) & 1, failed)) return false;
       tc_fence_after();
+      by_one([&] {
 #pragma unroll
-      for (int ks = 0; ks < BN / 16; ++ks) {
-        const uint64_t bd = sw128_desc_mn(v_addr + st * L::KV_BYTES + ks * (16 * 128), BN * 128);
-        umma_bf16_ta_by(elected, tmem_base + L::TMEM_O + (uint32_t)(q * D),
-                     tmem_base + L::TMEM_SP + (uint32_t)((q * SPB + b) * BN + ks * 8), bd, IDESC_PV, (j | ks) != 0);
-      }
-      umma_commit_by(elected, &pv_done[q][b]);
-      if (q == NQ - 1) umma_commit_by(elected, &v_empty[st]);
+        for (int ks = 0; ks < BN / 16; ++ks) {
+          const uint64_t bd = sw128_desc_mn(v_addr + st * L::KV_BYTES + ks * (16 * 128), BN * 128);
+          umma_bf16_ta_by(elected, tmem_base + L::TMEM_O + (uint32_t)(q * D),
+                       tmem_base + L::TMEM_SP + (uint32_t)((q * SPB + b) * BN + ks * 8), bd, IDESC_PV, (j | ks) != 0);
+        }
+        umma_commit_by(elected, &pv_done[q][b]);
+        if (q == NQ - 1) umma_commit_by(elected, &v_empty[st]);
+      });
       __syncwarp();
       return true;
     };

@@ -222,7 +222,7 @@ class PrefillGraph:
             buf[st] = g.pad_page
         self.dev.copy_(self.host)
         self._arange = np.arange(t, dtype=np.int64)
-        self.layouts: dict[tuple[int, int, int], int] = {}                    # of the model's prompt attention
+        self.layouts: dict[tuple[int, ...], int] = {}                         # of the model's prompt attention
         self.graphs: dict[tuple[int, ...], torch.cuda.CUDAGraph] = {}         # heads a CTA of each layout -> recording
         self.logits: torch.Tensor | None = None
 

@@ -419,18 +419,19 @@ MAX_SPLITS = 32
 
 
 # What a tile of 128 keys costs a CTA of the tcgen05 prompt kernel with one head and with two, and what a CTA costs whatever
-# its tiles (B200 cycles, fitted to the times below; a tile of two heads takes 4,050, but portions of 2,048 tokens behind as
-# many, 67 us with one head a CTA and 76 with two, stay with two, which they are recorded with: 3,600 draws the line there).
-PREFILL_TILE_CYCLES = {1: 2330, 2: 3600}
-PREFILL_CTA_CYCLES = {1: 12000, 2: 15000}
+# its tiles, for heads of 128 and of 64 (B200 cycles, fitted to times like those below; a tile of two heads of 128 takes 4,050, but
+# portions of 2,048 tokens behind as many, 67 us with one head a CTA and 76 with two, stay with two, which they are recorded
+# with: 3,600 draws the line there).
+PREFILL_TILE_CYCLES = {128: {1: 2330, 2: 3600}, 64: {1: 2560, 2: 4050}}
+PREFILL_CTA_CYCLES = {128: {1: 12000, 2: 15000}, 64: {1: 15000, 2: 15000}}
 
 
-def _prefill_cycles(tiles: list[int], heads: int, heads_per_cta: int) -> float:
+def _prefill_cycles(tiles: list[int], heads: int, heads_per_cta: int, head_dim: int) -> float:
     """Estimated cycles of a launch whose query tiles see ``tiles`` (longest first) tiles of keys each, for ``heads`` heads:
     no less than its longest CTA, than its work spread over the SMs, nor, for every k, than k + 1 times the
     k * 148-th longest CTA (one SM runs k + 1 that are as long)."""
     per_tile = heads // heads_per_cta
-    cost = [PREFILL_CTA_CYCLES[heads_per_cta] + t * PREFILL_TILE_CYCLES[heads_per_cta] for t in tiles]
+    cost = [PREFILL_CTA_CYCLES[head_dim][heads_per_cta] + t * PREFILL_TILE_CYCLES[head_dim][heads_per_cta] for t in tiles]
     bound = max(cost[0], sum(cost) * per_tile / 148)
     for k in range(1, (len(tiles) * per_tile - 1) // 148 + 1):
         bound = max(bound, (k + 1) * cost[k * 148 // per_tile])
@@ -438,7 +439,8 @@ def _prefill_cycles(tiles: list[int], heads: int, heads_per_cta: int) -> float:
 
 
 @functools.lru_cache(maxsize=256)
-def _one_head_or_two(query_lens: tuple[int, ...], context_lens: tuple[int, ...], num_heads: int, window: int) -> int:
+def _one_head_or_two(query_lens: tuple[int, ...], context_lens: tuple[int, ...], num_heads: int, window: int,
+                     head_dim: int) -> int:
     tiles = []
     for n, total in zip(query_lens, context_lens):
         if n > 1:
@@ -447,32 +449,32 @@ def _one_head_or_two(query_lens: tuple[int, ...], context_lens: tuple[int, ...],
                 last = min(first + 128, total)
                 tiles.append((last + 127) // 128 - (max(0, first - window + 1) // 128 if window else 0))
     tiles.sort(reverse=True)
-    return 1 if not tiles or _prefill_cycles(tiles, num_heads, 1) <= _prefill_cycles(tiles, num_heads, 2) else 2
+    return 1 if not tiles or _prefill_cycles(tiles, num_heads, 1, head_dim) <= _prefill_cycles(tiles, num_heads, 2, head_dim) else 2
 
 
 def prefill_heads_per_cta(query_lens: Sequence[int], context_lens: Sequence[int], num_heads: int, num_kv_heads: int,
-                          window: int = 0) -> int:
+                          window: int = 0, head_dim: int = 128) -> int:
     """Two query heads of a kv group in a CTA share its key and value tiles and keep the tensor core busier, but make half as
     many CTAs, twice as long: whichever is estimated to end first (by the step's lengths alone, so the layers of a step, and
     steps alike, share the estimate). Measured on B200, 16 / 8 heads of 128, one head / two: 512 tokens 11 / 17 us, 2,048
     tokens 30 / 43, 2,048 at 4,096 positions 67 / 76, at 9,001 positions 153 / 156, 4,096 tokens 90 / 76, 8,192 tokens
-    300 / 264, seven prompts of 290 tokens 24.5 / 24; 32 / 8 heads, 2,048 tokens 60 / 49, 1,024 23 / 26. The same constants serve every layout the kernel takes: over 280 steps
-    with 16, 32 and 64 heads of 128 and 4 to 32 of 64, groups of 2, 4 and 8, windows or none, the choice took as long as
-    the faster form to within the noise for heads of 128 and 0.3 % longer on average (17 % at worst) for heads of 64."""
+    300 / 264, seven prompts of 290 tokens 24.5 / 24; 32 / 8 heads, 2,048 tokens 60 / 49, 1,024 23 / 26. Over 60 steps with 16, 32 and 64 heads, groups of 2, 4 and 8, windows or none, the choice took 0.5 %
+    longer than the faster form on average (13 % at worst, where the line is drawn for recorded portions). Heads of 64 (16 / 8): 512
+    tokens 12 / 14, 2,048 32 / 37, 4,096 93 / 67, seven prompts of 290 26 / 19."""
     if (num_heads // num_kv_heads) % 2:
         return 1
     if PREFILL_HEADS_PER_CTA:
         return PREFILL_HEADS_PER_CTA
-    return _one_head_or_two(tuple(query_lens), tuple(context_lens), num_heads, window)
+    return _one_head_or_two(tuple(query_lens), tuple(context_lens), num_heads, window, 64 if head_dim == 64 else 128)
 
 
-def _prefill_heads_per_cta(ctx: Any, num_heads: int, num_kv_heads: int, window: int = 0) -> int:
+def _prefill_heads_per_cta(ctx: Any, num_heads: int, num_kv_heads: int, window: int = 0, head_dim: int = 128) -> int:
     """:func:`prefill_heads_per_cta` of a step, noted in its ``prompt_heads`` if that is asked for."""
     contexts = getattr(ctx, "context_lens", None) or ctx.query_lens      # (a caller of the kernel alone may not know them here)
-    heads = prefill_heads_per_cta(ctx.query_lens, contexts, num_heads, num_kv_heads, window)
+    heads = prefill_heads_per_cta(ctx.query_lens, contexts, num_heads, num_kv_heads, window, head_dim)
     notes = getattr(ctx, "prompt_heads", None)
     if notes is not None:
-        notes[num_heads, num_kv_heads, window] = heads
+        notes[(num_heads, num_kv_heads, window) + ((head_dim,) if head_dim != 128 else ())] = heads
     return heads
 
 
@@ -592,7 +594,7 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
                 _dev(ctx.context_lens_dev, "context_lens", torch.int32),
                 _dev(ctx.prefill_seqs, "prefill_seqs", torch.int32), num_prefill, ctx.max_query_len,
                 hq, hkv, d, page_size, float(scale), int(window),
-                1 if chunk or maps == 2 else _prefill_heads_per_cta(ctx, hq, hkv, int(window)),       # (those have one form)
+                1 if chunk or maps == 2 else _prefill_heads_per_cta(ctx, hq, hkv, int(window), d),       # (those have one form)
                 _error_word(q.device).data_ptr(), _opt(sinks, "sinks", torch.float32), keep_first, int(chunk), maps,
                 factor.data_ptr() if maps == 2 else None, float(mult) if maps == 2 else 1.0, float(mix_eps) if maps == 2 else 0.0, _stream()),
                 "prefill_attention_tcgen05")

@@ -267,8 +267,9 @@ class StepContext:
     # pages brought into L2) costs the host some 50 us a layer in events and stream switches, paid once by a recording; a
     # step launched kernel by kernel waits for them (three requests, 28 dense layers, 32 bits: 6.0 against 4.5 ms a step).
     recorded: bool = False
-    # If given: the layouts of prompt attention that the step ran, (heads, kv heads, window), and how many heads a CTA took.
-    prompt_heads: dict[tuple[int, int, int], int] | None = None
+    # If given: the layouts of prompt attention that the step ran, (heads, kv heads, window), with the head size behind unless
+    # it is 128, and how many heads a CTA took.
+    prompt_heads: dict[tuple[int, ...], int] | None = None
     # Weights that the kernels after the current mixer will stream (set by the block): a mixer
     # with a long kernel that leaves memory bandwidth idle may have them fetched into L2 beside it.
     upcoming_weights: list[torch.Tensor] = field(default_factory=list)
