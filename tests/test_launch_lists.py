@@ -48,3 +48,43 @@ def test_a_part_that_does_not_say_so_is_launched_as_always() -> None:
     from guzovik_cases import CONFIG_A
 
     assert rows_of(CONFIG_A) == {}
+
+
+def with_kinds(config: dict, **kinds: str):
+    """The config's spec with other registered kinds in some roles; ``block`` and ``position`` name the layer's own."""
+    import dataclasses
+
+    from tinyserve_b200.config import PartSpec
+
+    spec = config_from_dict(config).to_spec()
+    layers = []
+    for layer in spec.layers:
+        parts = {role: PartSpec(kinds.get(role, p.kind), p.args) for role, p in layer.parts.items()}
+        layers.append(dataclasses.replace(layer, parts=parts, block=kinds.get("block", layer.block),
+                                          position=PartSpec(kinds.get("position", layer.position.kind), layer.position.args)))
+    return dataclasses.replace(spec, layers=tuple(layers))
+
+
+def test_a_derived_class_is_launched_as_always_unless_it_says_so_itself() -> None:
+    """A part, a block or a position encoding derived from one that may be listed does something of its own beside what it
+    inherits (here an operation that is no launch of the library), so nothing is taken for granted of it."""
+    from tinyserve_b200.parts import attention, base, block, mlp, norm, rope
+
+    class HalvedSwiGLU(mlp.SwiGLU):
+        def forward(self, x, ctx, stream=None):
+            return super().forward(x, ctx, stream=None) * 0.5
+
+    class SameSwiGLU(mlp.SwiGLU):
+        same_launches = True
+
+    derived = {
+        "feed_forward": (base.FEED_FORWARDS, HalvedSwiGLU), "mixer": (base.MIXERS, type("M", (attention.GQAAttention,), {})),
+        "mixer_norm": (base.NORMS, type("N", (norm.RMSNorm,), {})), "block": (base.BLOCKS, type("B", (block.PreNormBlock,), {})),
+        "position": (base.POSITION_ENCODINGS, type("R", (rope.RotaryEncoding,), {}))}
+    config = {**TINY_A, "num_hidden_layers": 9}
+    for role, (family, cls) in derived.items():
+        family.register(f"derived_{role}_of_this_test", cls)
+        assert ModelParts(with_kinds(config, **{role: f"derived_{role}_of_this_test"}))._rows_of_alike == {}
+    base.FEED_FORWARDS.register("same_swiglu_of_this_test", SameSwiGLU)
+    assert ModelParts(with_kinds(config, feed_forward="same_swiglu_of_this_test"))._rows_of_alike == {0: 9}
+    assert ModelParts(with_kinds(config))._rows_of_alike == {0: 9}

@@ -22,7 +22,7 @@ from .kernels import launch_list, ops
 from .config.base import LayerSpec, ModelConfig, ModelSpec
 from .parts.base import (
     BLOCKS, EMBEDDINGS, HEADS, NORMS, PART_FAMILIES, POSITION_ENCODINGS, STREAM_INPUTS,
-    Block, CacheNeed, KVCacheEntry, PagedNeed, PositionEncoding, ResidualStream, StepContext, StreamInput, TensorSpec,
+    Block, CacheNeed, KVCacheEntry, PagedNeed, PositionEncoding, ResidualStream, StepContext, StreamInput, TensorSpec, launches_alike,
 )
 from .weights.loader import load_tensors, merge_specs
 from .weights.random_init import random_bound_tensors
@@ -135,6 +135,11 @@ class ModelParts:
 
     def _find_alike(self) -> dict[int, int]:
         """Rows of calls of the order that differ in nothing but their tensors: first call -> the one after the last."""
+        def listable(n: int) -> bool:
+            layer = self.layers[self.spec.order[n].layer]
+            of = [layer.block, *layer.block.parts.values(), *layer.positions.values()]
+            return all(map(launches_alike, of if layer.position is None else [*of, layer.position]))
+
         def like_next(n: int) -> bool:
             a, b = self.spec.order[n], self.spec.order[n + 1]
             if a.layer == b.layer or self.stream_inputs[n] is not None or self.stream_inputs[n + 1] is not None:
@@ -147,10 +152,8 @@ class ModelParts:
         rows, n, calls = {}, 0, len(self.spec.order)
         while n < calls:
             end = n + 1
-            block = self.layers[self.spec.order[n].layer].block
-            if block.same_launches and all(p.same_launches for p in block.parts.values()):
-                while end < calls and like_next(end - 1):
-                    end += 1
+            while listable(n) and end < calls and listable(end) and like_next(end - 1):
+                end += 1
             if end - n >= self.MIN_ALIKE:
                 rows[n] = end
             n = end

@@ -414,7 +414,8 @@ class Part:
     # True if, in a step that is not being recorded, two parts of this class with equal arguments launch the same kernels
     # with the same arguments but for their own tensors (attributes of the part), their cache entries and the place of
     # what they take from the arena, and do nothing else: then the launches of one layer can stand for those of
-    # the next ones (``kernels.launch_list``).
+    # the next ones (``kernels.launch_list``). It is not inherited (``launches_alike``). Of a position encoding: its position
+    # data hands the same rotation to every layer of a step.
     same_launches: bool = False
 
     def tensor_specs(self, prefix: str) -> list[TensorSpec]:
@@ -518,6 +519,11 @@ class StreamInput(Part):
 
     def forward(self, stream: ResidualStream, ctx: StepContext) -> None:
         raise NotImplementedError
+
+
+def launches_alike(of: "Part | Block") -> bool:
+    """Whether the object's very class says ``same_launches``: a class derived from one that does may do more in any method."""
+    return bool(type(of).__dict__.get("same_launches", False))
 
 
 class Block:

@@ -55,6 +55,7 @@ def scale_yarn(freq: torch.Tensor, dims: int, base: float, factor: float, origin
 
 class RotaryEncoding(PositionEncoding):
     recordable = EVERY_STEP
+    same_launches = True
 
     def __init__(self, head_dim: int, rotary_dim: int, theta: float, pairing: str = "half",
                  scaling: "dict[str, float] | None" = None) -> None:
