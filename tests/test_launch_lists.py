@@ -4,6 +4,7 @@ the arguments of the entry points that lists may name. Needs no GPU."""
 from __future__ import annotations
 
 import ctypes
+import types
 
 import pytest
 
@@ -88,3 +89,43 @@ def test_a_derived_class_is_launched_as_always_unless_it_says_so_itself() -> Non
     base.FEED_FORWARDS.register("same_swiglu_of_this_test", SameSwiGLU)
     assert ModelParts(with_kinds(config, feed_forward="same_swiglu_of_this_test"))._rows_of_alike == {0: 9}
     assert ModelParts(with_kinds(config))._rows_of_alike == {0: 9}
+
+
+@pytest.mark.parametrize("layers", [6, 7, 8, 9])
+@pytest.mark.parametrize("hidden, inner", [(64, 16), (64, 200)])
+def test_the_arena_behind_a_list_stands_as_behind_the_layers(layers, hidden, inner, monkeypatch) -> None:
+    """Behind an even and an odd number of listed layers: what the last one left pending lies where it would, and so does
+    what a stream input takes before the next block turns to the other half, without an overlap of the two."""
+    import torch
+
+    from tinyserve_b200.engine.arena import Arena
+    from tinyserve_b200.model import DecoderModel
+    from tinyserve_b200.parts.base import ResidualStream
+
+    class Model:
+        """Layers without a feed-forward: a norm's output, two of a mixer's inner rows and its output, left pending."""
+
+        parts = types.SimpleNamespace(places_of_alike=lambda *a: ())
+        _run_alike = DecoderModel._run_alike
+
+        def _run_call(self, n, stream, ctx, caches):
+            ctx.arena.next_frame()
+            for width in (hidden, inner, inner):
+                ctx.arena.take((5, width), torch.bfloat16)
+            stream.delta = ctx.arena.take((5, hidden), torch.bfloat16)
+
+    def run(listed: bool):
+        stream, ctx, model = ResidualStream(torch.zeros(5, hidden)), types.SimpleNamespace(arena=arena), Model()
+        arena.begin_step()
+        monkeypatch.setattr(launch_list, "run", lambda noted, *at: listed)
+        model._run_alike(0, layers, stream, ctx, [])
+        beside = arena.take((5, 2 * hidden), torch.bfloat16)
+        return [(t.data_ptr(), t.data_ptr() + t.numel() * t.element_size()) for t in (stream.delta, beside)]
+
+    arena = Arena("cpu")
+    for _ in range(3):
+        want = run(False)
+    got = run(True)
+    assert got == want
+    (a, b), (c, d) = got
+    assert b <= c or d <= a

@@ -108,6 +108,17 @@ class Arena:
         self._current = self._frames[self._frame_index]
         self._current.reset()
 
+    def frame_state(self) -> tuple[int, int, int]:
+        """The current frame and how far it is used, for ``resume_frame``."""
+        return self._frame_index, self._current.used, self._current.demand
+
+    def resume_frame(self, state: tuple[int, int, int]) -> None:
+        """The frame of ``state`` again, used as far as it was then: what was taken from it stays whole. (``next_frame`` hands
+        a frame over empty.)"""
+        self._frame_index, used, demand = state
+        self._current = self._frames[self._frame_index]
+        self._current.used, self._current.demand = used, demand
+
     def step_region(self) -> None:
         """Later takes live until the end of the step (used after the last layer)."""
         self._current = self._step

@@ -361,12 +361,12 @@ class DecoderModel:
             with launch_list.Noting() as calls:
                 self._run_call(m, stream, ctx, caches)
             noted.append(calls)
-            left.append(stream.state())
+            left.append((ctx.arena.frame_state(), stream.state()))
         at = self.parts.places_of_alike(n, range(n + 1, end), caches) if ctx.arena.moves == moves else None
         if at is not None and launch_list.run(noted, *at):
             if (end - n - 3) % 2:           # the last layer worked where the first of the two did
-                ctx.arena.next_frame()
-                stream.set_state(left[0])
+                ctx.arena.resume_frame(left[0][0])       # as far as that one used it: its output still lies there
+                stream.set_state(left[0][1])
             return
         for m in range(n + 3, end):
             self._run_call(m, stream, ctx, caches)
