@@ -129,3 +129,67 @@ def test_the_arena_behind_a_list_stands_as_behind_the_layers(layers, hidden, inn
     assert got == want
     (a, b), (c, d) = got
     assert b <= c or d <= a
+
+
+def test_what_is_put_in_place_of_a_layer_s_tensors_or_attributes_is_seen() -> None:
+    """Another storage under a bound tensor, another tensor, a plain attribute, a method or a part of one layer, each
+    without ``bind``: the list follows where the layers are still alike, and there is none where they are not."""
+    import torch
+
+    from tinyserve_b200.model import DecoderModel
+    from tinyserve_b200.parts.base import KVCacheEntry
+
+    def fresh():
+        model = DecoderModel.from_config(config_from_dict({**TINY_A, "num_hidden_layers": 9}), 3, torch.float32, "cpu")
+        parts = [layer.block.parts for layer in model.parts.layers]
+        return model.parts, parts, [layer.block for layer in model.parts.layers]
+
+    def places(of):
+        caches = [KVCacheEntry(k=torch.zeros(2, 2, 4, 16), v=torch.zeros(2, 2, 4, 16), page_size=4, group=0) for _ in range(9)]
+        got = of.places_of_alike(0, range(1, 9), caches)
+        return None if got is None else list(got[0])
+
+    model, parts, _ = fresh()
+    names = [v.data_ptr() for part in parts[5].values() for v in vars(part).values() if isinstance(v, torch.Tensor)]
+    assert set(names) <= set(places(model))
+    down = parts[5]["feed_forward"].w_down
+    down.data = down.data.clone()                                     # another storage
+    assert down.data_ptr() not in names and down.data_ptr() in places(model)
+    old = down.data_ptr()
+    parts[5]["feed_forward"].w_down = down.clone()                    # another tensor; the old one may have gone
+    del down
+    assert parts[5]["feed_forward"].w_down.data_ptr() in places(model) and old not in places(model)
+    parts[5]["feed_forward"].w_down = parts[5]["feed_forward"].w_down.double()
+    assert places(model) is None and model.alike_from(0) == 0         # another form
+    for change in (lambda p, b: setattr(p["mixer"], "scale", 0.5), lambda p, b: setattr(p["mixer"], "forward", lambda *a: None),
+                   lambda p, b: setattr(p["feed_forward_norm"], "eps", 0.1), lambda p, b: setattr(b, "feed_forward", p["mixer"]),
+                   lambda p, b: setattr(p["mixer"], "q_norm_w", None), lambda p, b: setattr(p["mixer"], "extra", torch.zeros(2)),
+                   lambda p, b: setattr(b, "scale_b", torch.ones(3)), lambda p, b: setattr(b, "forward", lambda *a: None)):
+        for which in ([5], range(9)):
+            model, parts, blocks = fresh()
+            assert model.alike_from(0) == 9 and places(model) is not None
+            for n in which:
+                change(parts[n], blocks[n])
+            if len(which) == 1 or "forward" in {**vars(parts[5]["mixer"]), **vars(blocks[5])}:
+                assert places(model) is None and model.alike_from(0) == 0
+    model, parts, blocks = fresh()
+    model.layers[4] = model.layers[5]
+    got, each = places(model), len(names) + 2
+    assert got[3 * each: 3 * each + len(names)] == got[4 * each: 4 * each + len(names)]
+
+
+def test_a_copy_of_the_layers_looks_for_its_own_tensors() -> None:
+    import copy
+    import pickle
+
+    import torch
+
+    from tinyserve_b200.model import DecoderModel
+    from tinyserve_b200.parts.base import KVCacheEntry
+
+    model = DecoderModel.from_config(config_from_dict({**TINY_A, "num_hidden_layers": 9}), 3, torch.float32, "cpu").parts
+    caches = [KVCacheEntry(k=torch.zeros(2, 2, 4, 16), v=torch.zeros(2, 2, 4, 16), page_size=4, group=0) for _ in range(9)]
+    for other in (copy.deepcopy(model), pickle.loads(pickle.dumps(model))):
+        got, _ = other.places_of_alike(0, range(1, 9), caches)
+        assert other.alike_from(0) == 9 and other.weight_bytes(0) == model.weight_bytes(0)
+        assert other.layers[7].block.parts["mixer"].w_o.data_ptr() in got and model.layers[7].block.parts["mixer"].w_o.data_ptr() not in got

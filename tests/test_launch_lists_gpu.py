@@ -77,3 +77,27 @@ def test_a_layer_off_the_16_byte_grid_is_not_listed(monkeypatch) -> None:
         want, _ = logits_of(model, False, steps, 64)
         got, _ = logits_of(model, True, steps, 64)
         assert not any(ran) and torch.equal(got, want)
+
+
+def test_a_tensor_replaced_without_bind_is_followed(monkeypatch) -> None:
+    """Another storage under a tensor of a layer behind the third, and another tensor: the listed step reads them."""
+    from tinyserve_b200.config import config_from_dict
+    from tinyserve_b200.kernels import launch_list
+    from tinyserve_b200.model import DecoderModel
+
+    model = DecoderModel.from_config(config_from_dict(SIZES["tiny"]), 3, torch.float32, "cuda")
+    prompt = random_prompt(50, 256, 1)
+    steps = [[("a", prompt[:40], [39])], [("a", prompt[40:], [9])], [("b", prompt[:30], [29])]]
+    ran = []
+    run = launch_list.run
+    monkeypatch.setattr(launch_list, "run", lambda *args: ran.append(run(*args)) or ran[-1])
+    before, _ = logits_of(model, True, steps, 128)
+    mixer, mlp = (model.parts.layers[6].block.parts[role] for role in ("mixer", "feed_forward"))
+    mixer.w_o.data = mixer.w_o.data * 1.5
+    for change in ("storage", "tensor"):
+        want, _ = logits_of(model, False, steps, 128)
+        ran.clear()
+        got, _ = logits_of(model, True, steps, 128)
+        assert any(ran) and torch.equal(got, want) and not torch.equal(got, before)
+        mlp.w_down = mlp.w_down * 0.5
+        before = got

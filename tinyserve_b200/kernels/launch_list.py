@@ -3,8 +3,9 @@
 A step that is not replayed from a recording is launched kernel by kernel, 14 to 17 us of the host's time each, most of it
 spent in the interpreter on checks and choices that come out the same for every layer. So the model runs the first layers
 of such a row as always, writes down what two neighbouring ones launched, and hands that over for all further ones: the
-library makes the same calls with each pointer into one of the layer's own tensors moved to the next layer's. Nothing is
-kept from one step for the next.
+library makes the same calls with each pointer into one of the layer's own tensors moved to the next layer's. No list is
+kept from one step for the next; where the layers' tensors lie is known from when they were bound, and looked at again for
+every list.
 """
 
 from __future__ import annotations

@@ -10,8 +10,11 @@ wanted rows, apply the final norm to those rows only and multiply by the output 
 
 from __future__ import annotations
 
+import weakref
 from array import array
 from dataclasses import dataclass
+from itertools import chain
+from operator import itemgetter
 from pathlib import Path
 from typing import Any, Mapping
 
@@ -39,6 +42,42 @@ class Layer:
     block: Block
     position: PositionEncoding | None
     positions: dict[str, PositionEncoding]      # by mixer role, when the mixers have encodings of their own
+
+
+class _RowPlaces:
+    """Where the tensors of a row of layers lie, call by call, and the bytes of each of a call's; with it, all that this was
+    read from, so that whatever has been replaced since (a tensor, its storage, an attribute, a part) shows."""
+
+    def __init__(self, layers: "list[Layer]", watched: list[dict[str, Any]], places: list[int], sizes: list[int]) -> None:
+        self.places, self.sizes = places, sizes
+        self._watched, self._layers, self._gone = watched, layers, []
+        if not places:          # (a copy)
+            self._gone.append(None)
+            return
+        values = self._values()
+        tensors = [i for i, v in enumerate(values) if isinstance(v, torch.Tensor)]
+        self._tensors, self._others = itemgetter(*tensors), itemgetter(*sorted({*range(len(values))} - {*tensors}))
+        # tensors by their identity, which something new may have once one has gone: that is noted, so none is kept alive here
+        self._ids = list(map(id, self._tensors(values)))
+        self._alive = [weakref.ref(v, self._gone.append) for v in self._tensors(values)]
+        self._plain, self._count = self._others(values), len(values)
+
+    def _values(self) -> list[Any]:
+        return list(chain(self._layers, *map(dict.values, self._watched)))
+
+    def __reduce__(self) -> Any:      # a copy of the layers has them elsewhere: nothing holds for it, and it looks anew
+        return _RowPlaces, ([], [], [], self.sizes)
+
+    def hold(self) -> bool:
+        values = self._values()
+        if self._gone or len(values) != self._count:
+            return False
+        tensors = self._tensors(values)
+        try:
+            return (list(map(id, tensors)) == self._ids and self._others(values) == self._plain
+                    and list(map(torch.Tensor.data_ptr, tensors)) == self.places)
+        except RuntimeError:          # a tensor where none was does not compare
+            return False
 
 
 class ModelParts:
@@ -81,8 +120,7 @@ class ModelParts:
                 self._needs += several if call.reads_cache_of is None else (None,) * len(several)
         self._check_order()
         self._rows_of_alike = self._find_alike()
-        # of a row, once the parts hold their tensors: where those of each call lie, call by call, and the bytes of each
-        self._tensor_places: dict[int, tuple[list[int], list[int]]] = {}
+        self._row_places: "dict[int, _RowPlaces | None]" = {}      # of a row, once its parts hold their tensors
         self._cache_indices = []      # of a call: the cache entries that its mixers keep
         for n, call in enumerate(spec.order):
             of = [self._user_index[(n, role)] for role in self.layers[call.layer].block.mixers()]
@@ -133,13 +171,13 @@ class ModelParts:
     # ---- layers whose launches are the same but for their tensors
     MIN_ALIKE = 6      # one layer as it comes, two that are written down, and enough that follow them
 
+    def _listable(self, n: int) -> bool:
+        layer = self.layers[self.spec.order[n].layer]
+        of = [layer.block, *layer.block.parts.values(), *layer.positions.values()]
+        return all(map(launches_alike, of if layer.position is None else [*of, layer.position]))
+
     def _find_alike(self) -> dict[int, int]:
         """Rows of calls of the order that differ in nothing but their tensors: first call -> the one after the last."""
-        def listable(n: int) -> bool:
-            layer = self.layers[self.spec.order[n].layer]
-            of = [layer.block, *layer.block.parts.values(), *layer.positions.values()]
-            return all(map(launches_alike, of if layer.position is None else [*of, layer.position]))
-
         def like_next(n: int) -> bool:
             a, b = self.spec.order[n], self.spec.order[n + 1]
             if a.layer == b.layer or self.stream_inputs[n] is not None or self.stream_inputs[n + 1] is not None:
@@ -152,50 +190,66 @@ class ModelParts:
         rows, n, calls = {}, 0, len(self.spec.order)
         while n < calls:
             end = n + 1
-            while listable(n) and end < calls and listable(end) and like_next(end - 1):
+            while self._listable(n) and end < calls and self._listable(end) and like_next(end - 1):
                 end += 1
             if end - n >= self.MIN_ALIKE:
                 rows[n] = end
             n = end
         return rows
 
-    def _place_tensors(self) -> None:
-        """For each such row, where the tensors of its layers lie (the attributes of their parts, which change by ``bind``
-        alone). A row whose layers' tensors differ in their forms, or in how they lie to one another (a view of another
-        tensor in one layer and none in the next) is given up."""
-        self._tensor_places = {}
-        for n, end in self._rows_of_alike.items():
-            places, form, sizes = [], None, []
-            for call in range(n, end):
-                block = self.layers[self.spec.order[call].layer].block
-                named = [(role, name, t) for role, part in block.parts.items() for name, t in vars(part).items()
-                         if isinstance(t, torch.Tensor)]
-                storages = [t.untyped_storage().data_ptr() for _, _, t in named]
-                at = [t.data_ptr() for _, _, t in named]
-                first = [storages.index(s) for s in storages]          # the first tensor of the same memory
-                mine = [(role, name, t.shape, t.dtype, t.stride(), first[i], at[i] - at[first[i]])
-                        for i, (role, name, t) in enumerate(named)]
-                if form is None:
-                    form, sizes = mine, [t.numel() * t.element_size() for _, _, t in named]
-                if mine != form:
-                    break
-                places += at
-            else:
-                self._tensor_places[n] = places, sizes
+    def _place_row(self, n: int) -> "_RowPlaces | None":
+        """Where the tensors of the layers of the row that starts at ``n`` lie (attributes of their parts). ``None`` if the layers
+        differ in more: in the form of a tensor, in how the tensors lie to one another (a view of another tensor in one
+        layer and none in the next), in a plain attribute, or if an attribute is neither (a method put in place of
+        the class's, say)."""
+        places, form, sizes, watched = [], None, [], []
+        for call in range(n, self._rows_of_alike[n]):
+            if not self._listable(call):
+                return None
+            layer = self.layers[self.spec.order[call].layer]
+            roles = {id(part): role for role, part in layer.block.parts.items()}
+            of = [(role, vars(part)) for role, part in layer.block.parts.items()] + [("", vars(layer.block))]
+            watched += [vars(layer), layer.block.parts, *[attributes for _, attributes in of]]
+            now = [v for _, attributes in of for v in attributes.values() if isinstance(v, torch.Tensor)]
+            if len(now) < 2:
+                return None
+            storages, at = [t.untyped_storage().data_ptr() for t in now], [t.data_ptr() for t in now]
+            first = [storages.index(s) for s in storages]          # the first tensor of the same memory
+            mine: list[Any] = [(t.shape, t.dtype, t.stride(), first[i], at[i] - at[first[i]]) for i, t in enumerate(now)]
+            mine += [layer.position, *layer.positions.items()]
+            for role, attributes in of:
+                for name, v in attributes.items():
+                    if id(v) in roles:
+                        v = roles[id(v)]                           # the block's name for one of its parts
+                    elif isinstance(v, torch.Tensor):
+                        v = torch.Tensor
+                    elif not (v is None or isinstance(v, (bool, int, float, str)) or v is layer.block.parts):
+                        return None
+                    mine.append((role, name, None if v is layer.block.parts else v))
+            if form is None:
+                form, sizes = mine, [t.numel() * t.element_size() for t in now]
+            if mine != form:
+                return None
+            places += at
+        return _RowPlaces(self.layers, watched, places, sizes)
 
     def weight_bytes(self, row: int) -> int:
         """The bytes of the tensors of one layer of such a row."""
-        return sum(self._tensor_places[row][1])
+        return sum(self._row_places[row].sizes)
 
     def alike_from(self, n: int) -> int:
         """If a row of calls starts at ``n`` whose launches are the same but for their tensors, the call after its last
         one; else 0."""
-        return self._rows_of_alike[n] if n in self._tensor_places else 0
+        return self._rows_of_alike[n] if self._row_places.get(n) is not None else 0
 
     def places_of_alike(self, row: int, calls: range, caches: list[Any]) -> "tuple[array[int], list[int]] | None":
         """Where the tensors of these calls of the row that starts at ``row`` lie, weights and caches, call by call, and the
-        bytes of each of a call's; ``None`` if the caches are not alike."""
-        weights, sizes = self._tensor_places[row]
+        bytes of each of a call's; ``None`` if the layers, since their tensors were bound, or the caches are not alike."""
+        if not self._row_places[row].hold():
+            self._row_places[row] = self._place_row(row)
+            if self._row_places[row] is None:
+                return None
+        weights, sizes = self._row_places[row].places, self._row_places[row].sizes
         like = [caches[i] for i in self._cache_indices[calls[0]]]
         if any(type(e) is not KVCacheEntry for e in like):
             return None
@@ -237,7 +291,7 @@ class ModelParts:
     def bind(self, tensors: Mapping[str, torch.Tensor]) -> None:
         for prefix, part in self._each_part():
             part.bind(prefix, tensors)
-        self._place_tensors()
+        self._row_places = {n: self._place_row(n) for n in self._rows_of_alike}
 
     # ---- cache
     def cache_needs(self) -> list[CacheNeed | None]:

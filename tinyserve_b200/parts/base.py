@@ -414,7 +414,7 @@ class Part:
     # True if, in a step that is not being recorded, two parts of this class with equal arguments launch the same kernels
     # with the same arguments but for their own tensors (attributes of the part), their cache entries and the place of
     # what they take from the arena, and do nothing else: then the launches of one layer can stand for those of
-    # the next ones (``kernels.launch_list``). It is not inherited (``launches_alike``). Of a position encoding: its position
+    # the next ones (``kernels.launch_list``). Its attributes are tensors and plain values. It is not inherited (``launches_alike``). Of a position encoding: its position
     # data hands the same rotation to every layer of a step.
     same_launches: bool = False
 
