@@ -193,3 +193,48 @@ def test_a_copy_of_the_layers_looks_for_its_own_tensors() -> None:
         got, _ = other.places_of_alike(0, range(1, 9), caches)
         assert other.alike_from(0) == 9 and other.weight_bytes(0) == model.weight_bytes(0)
         assert other.layers[7].block.parts["mixer"].w_o.data_ptr() in got and model.layers[7].block.parts["mixer"].w_o.data_ptr() not in got
+
+
+def test_a_library_product_that_torch_was_asked_to_make_otherwise_is_in_no_list(monkeypatch) -> None:
+    """The flag for sums in 32 bits, another library, its tuning, a mode that sees torch's operations, or a library that is not
+    where torch's build says: the noted call is one that no list may name."""
+    import torch
+
+    monkeypatch.setattr(torch.cuda, "current_blas_handle", lambda: 7)
+    note = lambda: ops._library_gemm_call(16, 32, 48, 20, 64, 128, 1)
+    assert note() == ("ts_library_gemm", (16, 32, 48, 20, 64, 128, 1, ops._library_gemm_function(), 7)) and launch_list._entry(note()[0])
+    matmul = torch.backends.cuda.matmul
+    matmul.allow_bf16_reduced_precision_reduction = False
+    try:
+        assert launch_list._entry(note()[0]) is None
+    finally:
+        matmul.allow_bf16_reduced_precision_reduction = True
+    with monkeypatch.context() as m:
+        m.setattr(torch.backends.cuda, "preferred_blas_library", lambda: types.SimpleNamespace(name="Cublaslt"))
+        assert launch_list._entry(note()[0]) is None
+    with monkeypatch.context() as m:
+        m.setattr(torch.cuda.tunable, "is_enabled", lambda: True)
+        assert launch_list._entry(note()[0]) is None
+
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Sees(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types_, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    class SeesToo(TorchFunctionMode):
+        def __torch_function__(self, func, types_, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    for mode in (Sees, SeesToo):
+        with mode():
+            assert launch_list._entry(note()[0]) is None
+    assert launch_list._entry(note()[0]) is not None
+    ops._library_gemm_function.cache_clear()
+    try:
+        with monkeypatch.context() as m:
+            m.setattr(torch.version, "cuda", "99.0")
+            assert ops._library_gemm_function() == 0 and launch_list._entry(note()[0]) is None
+    finally:
+        ops._library_gemm_function.cache_clear()

@@ -101,3 +101,45 @@ def test_a_tensor_replaced_without_bind_is_followed(monkeypatch) -> None:
         assert any(ran) and torch.equal(got, want) and not torch.equal(got, before)
         mlp.w_down = mlp.w_down * 0.5
         before = got
+
+
+@pytest.mark.parametrize("how", ["flag", "mode"])
+def test_library_products_follow_what_torch_is_asked_for(how, monkeypatch) -> None:
+    """Products of 30 rows go to the vendor library: with sums in 32 bits asked for, or a mode that sees torch's operations, all
+    layers are launched call by call, and the mode sees a product in every layer."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from tinyserve_b200.config import config_from_dict
+    from tinyserve_b200.kernels import launch_list
+    from tinyserve_b200.model import DecoderModel
+
+    seen = []
+
+    class Sees(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    model = DecoderModel.from_config(config_from_dict(SIZES["wide"]), 3, torch.bfloat16, "cuda")
+    steps = [[("a", random_prompt(30, 2048, 1), [29])], [("b", random_prompt(30, 2048, 2), [29])]]
+    ran = []
+    run = launch_list.run
+    monkeypatch.setattr(launch_list, "run", lambda *args: ran.append(run(*args)) or ran[-1])
+    matmul = torch.backends.cuda.matmul
+    logits_of(model, True, steps, 128)
+    assert any(ran)
+    ran.clear()
+    try:
+        if how == "flag":
+            matmul.allow_bf16_reduced_precision_reduction = False
+            want, _ = logits_of(model, False, steps, 128)
+            got, _ = logits_of(model, True, steps, 128)
+            assert torch.equal(got, want)
+        else:
+            with Sees():
+                logits_of(model, True, steps, 128)
+            products = sum("mm" in name for name in seen)
+            assert products >= 2 * SIZES["wide"]["num_hidden_layers"]
+    finally:
+        matmul.allow_bf16_reduced_precision_reduction = True
+    assert ran and not any(ran)

@@ -810,8 +810,7 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
             return
     px, pw, po = _dev(x, "x"), _dev(w, "w"), _dev(out, "out")
     if notes.calls is not None:
-        notes.calls.append(("ts_library_gemm", (px, pw, po, m, n, k, _code(out.dtype), _library_gemm_function(),
-                                                torch.cuda.current_blas_handle())))
+        notes.calls.append(_library_gemm_call(px, pw, po, m, n, k, _code(out.dtype)))
     if out.dtype == torch.bfloat16:
         torch.mm(x, w.t(), out=out)                       # vendor library matrix product
     else:
@@ -820,8 +819,24 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
 
 @functools.lru_cache(maxsize=None)
 def _library_gemm_function() -> int:
-    """Where the vendor library that torch has loaded keeps the function that ``torch.mm`` calls."""
-    return ctypes.cast(ctypes.CDLL("libcublas.so.12").cublasGemmEx, _vp).value
+    """Where the vendor library that torch has loaded keeps the function that ``torch.mm`` calls; 0 if it is not found."""
+    try:
+        library = ctypes.CDLL(f"libcublas.so.{(torch.version.cuda or '').split('.')[0]}", mode=os.RTLD_NOLOAD | os.RTLD_LAZY)
+        return ctypes.cast(library.cublasGemmEx, _vp).value or 0
+    except (OSError, AttributeError):
+        return 0
+
+
+def _library_gemm_call(px: int, pw: int, po: int, m: int, n: int, k: int, dtype: int) -> tuple[str, tuple[Any, ...]]:
+    """``torch.mm`` of :func:`gemm` as a call for ``kernels.launch_list``, which makes torch's plain one: one that no list may name
+    where torch has been asked for another (another library, its tuning, sums that stay in 32 bits, a mode that sees
+    torch's operations) or the library is not found."""
+    plain = (torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction is True
+             and torch.backends.cuda.preferred_blas_library().name in ("Default", "Cublas") and not torch.cuda.tunable.is_enabled()
+             and not torch._C._len_torch_dispatch_stack() and not torch._C._len_torch_function_stack())
+    if not plain or not _library_gemm_function():
+        return "torch.mm", ()
+    return "ts_library_gemm", (px, pw, po, m, n, k, dtype, _library_gemm_function(), torch.cuda.current_blas_handle())
 
 
 # The 32-bit product's tiles hold 32 rows, a grid 65,535 of them (the general kernel twice as many).
