@@ -237,6 +237,31 @@ def test_mlstm_scan_over_chunks(dtype, heads, d, dv, lens, monkeypatch) -> None:
         assert over_chunks[1] <= 8 * token_by_token[1] + 2.0 ** -22, (key, over_chunks, token_by_token)
 
 
+@pytest.mark.parametrize("chunks", [True, False])
+def test_mlstm_scan_where_the_running_maximum_falls_below_what_its_exponential_holds(chunks, monkeypatch) -> None:
+    """Gates that a cap of 200 lets fall to -120 and -190: e^(-m) is more than 32 bits hold, and the read-outs go to zero (in
+    64 bits they are below 1e-30 of a token's values) in one head, while the other's gates are ordinary."""
+    from tinyserve_b200.kernels import ops
+
+    monkeypatch.setattr(ops, "MLSTM_CHUNKS", chunks)
+    heads, d, dv, cap = 2, 32, 32, 200.0
+    size, gb, offs = ops.mlstm_state_size(heads, d, dv), torch.zeros(2 * heads, device="cuda"), (0, heads * d, 2 * heads * d)
+    state = torch.zeros(2, size, device="cuda")
+    exact = state.double().cpu()
+    for i, n in enumerate((150, 1, 140)):
+        x, step = _rand(n, 2 * heads * d + heads * dv, seed=20 + i), FakeStep([n], [0], "cuda")
+        gates = _rand(n, 2 * heads, seed=30 + i)
+        gates[:, 0] = -140.0 + 3.0 * gates[:, 0]
+        gates[:, heads] = -400.0
+        out = torch.full((n, heads, dv), float("nan"), device="cuda")
+        ops.mlstm_scan(x, *offs, gates, gb, cap, d ** -0.5, state, step, heads, d, dv, out)
+        want = _mlstm_in_64_bits(x, offs, gates, gb, cap, d ** -0.5, exact, step, heads, d, dv)
+        assert want[:, 0].abs().max() < 1e-30 * x.abs().max()
+        assert torch.equal(out[:, 0], torch.zeros_like(out[:, 0]))
+        torch.testing.assert_close(out[:, 1].double().cpu(), want[:, 1], atol=2e-5, rtol=2e-4)
+        assert not state.isnan().any()
+
+
 def test_mlstm_scan_into_an_output_off_the_16_byte_grid() -> None:
     """A long portion whose read-outs go to a place that the chunks' wide stores do not take."""
     from tinyserve_b200.kernels import ops

@@ -6,7 +6,7 @@
 //   o_t     = S_t q_t / (max(|n_t . q_t|, e^(-m_t)) + 1e-6)
 //   S'      = e^(F_end + m_0 - m') S_0 + e^(F_end - m') sum_s e^(g_s) k_s v_s^T,   m' = F_end + R_end      (n' likewise)
 //
-// the recurrence's own stabiliser, so every exponent is at most zero.
+// the recurrence's own stabiliser, so every exponent but that of e^(-m_t) is at most zero.
 //  * leave kernel   : the last sums of a chunk, in the scale of its largest g, and F_end and that g;
 //  * combine kernel : walks a request's chunks in order, leaves each one's starting state in the place of those sums, and
 //                     stores the request's slot;
@@ -42,7 +42,8 @@ struct MlstmChunkArgs {
 // e^x of a difference of sums in 64-bit: rounded to 32 bits, an x in the tens would leave its last digits to the result.
 __device__ __forceinline__ float exp_of(double x) {
   const float hi = (float)x, e = expf(hi);
-  return hi > -100.f ? fmaf(e, (float)(x - (double)hi), e) : e;        // (below, both are zero, and x may be -inf)
+  // (below -100 both are zero, and x may be -inf; e^(-m) may be more than 32 bits hold)
+  return hi > -100.f && e < INFINITY ? fmaf(e, (float)(x - (double)hi), e) : e;
 }
 
 // By one warp: F and g of the chunk's tokens (two a lane; past the end F stays and g is -inf), and the largest g so far.
