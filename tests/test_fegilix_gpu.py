@@ -262,6 +262,30 @@ def test_mlstm_scan_where_the_running_maximum_falls_below_what_its_exponential_h
         assert not state.isnan().any()
 
 
+@pytest.mark.parametrize("at", [0, 1, 64, 127])
+@pytest.mark.parametrize("what", ["input gate", "forget gate", "value"])
+def test_mlstm_scan_of_a_token_that_is_no_number_leaves_those_before_it(at, what) -> None:
+    """A NaN in one token's gates or values: the tokens before it are the same bits as without it, itself and those behind it are
+    NaN (with a value: in the columns that have it), token by token and over chunks."""
+    from tinyserve_b200.kernels import ops
+
+    heads, d, dv, n = 2, 32, 32, 130
+    offs, gb = (0, heads * d, 2 * heads * d), _rand(2 * heads, seed=1)
+    outs = []
+    for bad in (False, True):
+        x, gates = _rand(n, 2 * heads * d + heads * dv, seed=2), _rand(n, 2 * heads, seed=3)
+        if bad and what == "value":
+            x[at, offs[2] + 5] = float("nan")
+        elif bad:
+            gates[at, 0 if what == "input gate" else heads] = float("nan")
+        state, out = torch.zeros(2, ops.mlstm_state_size(heads, d, dv), device="cuda"), torch.empty(n, heads, dv, device="cuda")
+        ops.mlstm_scan(x, *offs, gates, gb, 5.0, d ** -0.5, state, FakeStep([n], [0], "cuda"), heads, d, dv, out)
+        outs.append(out)
+    assert torch.equal(outs[1][:at], outs[0][:at]) and torch.equal(outs[1][:, 1], outs[0][:, 1])
+    behind = outs[1][at:, 0]
+    assert bool((behind[:, 5] if what == "value" else behind).isnan().all())
+
+
 def test_mlstm_scan_into_an_output_off_the_16_byte_grid() -> None:
     """A long portion whose read-outs go to a place that the chunks' wide stores do not take."""
     from tinyserve_b200.kernels import ops

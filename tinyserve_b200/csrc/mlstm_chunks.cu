@@ -69,7 +69,8 @@ __device__ __forceinline__ void mlstm_gates(const MlstmChunkArgs& a, int h, int 
     const double other = __shfl_up_sync(0xffffffffu, run, o);
     if (lane >= o) run += other;
   }
-  const double f0 = run - lf[1], f1 = run;
+  // (not run - lf[1]: a token whose gate is no number is not to be seen by the one before it)
+  const double in_front = __shfl_up_sync(0xffffffffu, run, 1), f0 = (lane ? in_front : 0.0) + lf[0], f1 = run;
   const double g0 = (double)li[0] - f0, g1 = (double)li[1] - f1;
   double top = fmax(g0, g1);
 #pragma unroll
