@@ -345,12 +345,56 @@ def test_decode_attention_cluster_merge_gives_the_same_bits(hq, hkv, d, page, sp
 @pytest.mark.parametrize("hq,hkv,d,page", [(16, 8, 128, 16), (8, 4, 64, 8)])
 @pytest.mark.parametrize("batch", [2, 16, 18, 19, 37, 38, 50])
 def test_decode_attention_with_an_sm_for_every_cta_or_several_ctas_an_sm(hq, hkv, d, page, batch) -> None:
-    """Up to 148 CTAs (requests x kv heads x key ranges) keep four tiles a warp in flight, more of them two."""
+    """From a few CTAs (requests x kv heads x key ranges) to several an SM, key ranges merged in clusters and none."""
     lens = [(1 + (i * 53) % 700, 1) for i in range(batch - 1)] + [(1500, 1)]
     out, want = _attention_case(torch.bfloat16, hq, hkv, d, page, lens, 0, seed=3, spike=(batch - 1, 1100))
     ops.check_device_errors()
     assert not out.isnan().any()
     torch.testing.assert_close(out.float(), want.float(), **tol(torch.bfloat16))
+
+
+@pytest.mark.parametrize("hq,hkv,d,page,lens,ctas", [
+    (16, 8, 128, 16, [17, 120, 1, 33, 90, 64, 16, 15, 2], 72), (16, 8, 128, 16, [17, 120, 1, 33, 90, 64, 16, 15, 2, 65], 80),
+    (16, 8, 128, 8, [1500], 64), (16, 8, 128, 16, [1500, 40], 128), (5, 5, 128, 16, [700, 30], 80), (3, 3, 128, 32, [1, 90, 700], 72),
+    (8, 4, 64, 8, [(i * 13) % 127 + 1 for i in range(18)], 72), (8, 4, 64, 16, [(i * 13) % 127 + 1 for i in range(19)], 76),
+    (16, 2, 64, 16, [2000, 3, 515, 900], 64), (16, 2, 64, 8, [2000, 3, 515, 900, 64], 80), (24, 1, 64, 16, [3000, 16], 32)])
+@pytest.mark.parametrize("window", [0, 100])
+def test_decode_attention_of_eight_warps_a_cta_and_of_four(hq, hkv, d, page, lens, ctas, window, monkeypatch) -> None:
+    """Up to 74 CTAs have eight warps, beyond they have four: both sides of that line, for ranges with fewer tiles of 16 keys than
+    warps, as many and more, merged in clusters, through memory (the same bits) or not at all, from separate kernels and in
+    the fused form."""
+    splits = ops.choose_splits(len(lens) * hkv * -(-(hq // hkv) // 16), ops._decode_slots(d, True), max(lens) // 64, cluster=True)
+    assert len(lens) * hkv * -(-(hq // hkv) // 16) * splits == ctas
+    monkeypatch.setattr(ops, "choose_splits", lambda *a, **kw: splits)
+    out, want = _attention_case(torch.bfloat16, hq, hkv, d, page, [(n, 1) for n in lens], window, seed=9)
+    ops.set_decode_cluster_merge(False)
+    try:
+        assert torch.equal(out, _attention_case(torch.bfloat16, hq, hkv, d, page, [(n, 1) for n in lens], window, seed=9)[0])
+    finally:
+        ops.set_decode_cluster_merge(True)
+    ops.check_device_errors()
+    assert not out.isnan().any()
+    torch.testing.assert_close(out.float(), want.float(), **tol(torch.bfloat16))
+
+    b, width = len(lens), -(-max(lens) // page)
+    tables = torch.randperm(b * width, generator=torch.Generator().manual_seed(2)).int().view(b, width).cuda()
+    k, v = (rnd(b * width, hkv, page, d, dtype=torch.bfloat16, seed=s) for s in (3, 4))
+    at = torch.tensor(lens, device="cuda") - 1
+    slots = (tables[torch.arange(b, device="cuda"), at // page] * page + at % page).int()
+    qkv = rnd(b, (hq + 2 * hkv) * d, dtype=torch.bfloat16, seed=5)
+    ctx = SimpleNamespace(
+        num_seqs=b, query_lens=[1] * b, cu_query_lens=torch.arange(b + 1, dtype=torch.int32, device="cuda"),
+        context_lens_dev=torch.tensor(lens, dtype=torch.int32, device="cuda"), decode_seqs=torch.arange(b, dtype=torch.int32, device="cuda"),
+        prefill_seqs=torch.zeros(b, dtype=torch.int32, device="cuda"), num_decode=b, num_prefill=0, max_query_len=1, max_context_len=max(lens),
+        arena=Arena("cuda"))
+    fused, two = (torch.empty(b, hq * d, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    q, kv = torch.empty(b, hq, d, dtype=torch.bfloat16, device="cuda"), (k.clone(), v.clone())
+    ops.decode_attention_fused(qkv, None, None, 1e-6, None, None, slots, k, v, page, tables, ctx, d ** -0.5, window, hq, fused)
+    ops.qk_norm_rope_write(qkv, q, None, None, 1e-6, None, None, 0, False, slots, *kv, page, hq, hkv, d, True)
+    ref.paged_attention(q, *kv, page, tables, ctx, d ** -0.5, window, two)
+    ops.check_device_errors()
+    torch.testing.assert_close(fused.float(), two.float(), **tol(torch.bfloat16))
+    assert torch.equal(k, kv[0]) and torch.equal(v, kv[1])
 
 
 @pytest.mark.parametrize("dtype", DTYPES)

@@ -14,12 +14,12 @@
 // range hold whatever the page holds there; their scores are masked and their values zeroed
 // before use. Every warp runs its own two-stage pipeline of tiles;
 // S = Q K^T and O += P V are mma.sync m16n8k16 with 32-bit accumulators; the softmax is
-// online, 32-bit, base 2. A CTA is one (request, kv group, key range); its four warps take
-// tiles in turn and merge at the end; the CTA that finishes a request's last range merges the
+// online, 32-bit, base 2. A CTA is one (request, kv group, key range); its warps (four, eight
+// where every CTA has an SM to itself, three in one layout) take tiles in turn and merge at the end; the CTA that finishes a request's last range merges the
 // ranges (arrival counter), so there is no second kernel.
 // Every mbarrier wait is bounded; a wait that runs out sets *error_flag and the CTA leaves.
 #define TS_PDL_CLASS PDL_ATTENTION
-
+#include <type_traits>
 
 #include "attention.cuh"
 #include "bounded_wait.cuh"
@@ -192,7 +192,7 @@ __device__ __forceinline__ void fused_head_row(const bf16* src, const HeadWeight
 // D64 = head_dim / 64 (1 or 2). BR = rows of a tensor box: 16 (page size a multiple of 16) or 8.
 // blockIdx = (request in the list, kv head * passes + pass, key range); a pass covers up to 16
 // query heads of the group.
-// WARPS: warps per CTA (4; 3 where one more CTA per SM lets a grid run as a single wave).
+// WARPS: warps per CTA (4; 8 up to DM_FEW_CTAS; 3 where one more CTA per SM lets a grid run as a single wave).
 // CLUSTER: the CTAs of the key ranges of one (request, kv head, pass) form a thread-block cluster
 // (1, 1, num_splits) and merge their results through distributed shared memory instead of through
 // global memory and an arrival counter: the tail of the kernel, where no key is in flight any
@@ -253,8 +253,11 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attn_tma_kernel(const __gri
   const int* table = a.block_tables + (size_t)seq * a.table_width;
 
   // One lane fetches a tile: the 16 positions from k0 lie in one page (BR = 16) or in two pages
-  // of 8. Row of the cache matrix = (page * kv_heads + kvh) * page_size + offset in the page. The pages are looked up apart
-  // from the copies and earlier: the look-up is a trip to L2 of its own.
+  // of 8. Row of the cache matrix = (page * kv_heads + kvh) * page_size + offset in the page. With eight warps the pages are
+  // looked up apart from the copies and earlier (AHEAD): the look-up is a trip to L2 of its own. With fewer warps they are
+  // not: several CTAs an SM hide that trip, and to hold the pages costs 2 to 4 % with heads of 128, 10 to 40 % with heads of
+  // 64 (16 requests of 16 / 2 heads and 4,000 keys 12.9 / 16.0 us).
+  constexpr bool AHEAD = WARPS == 8;
   constexpr int BOXES = DM_TK / BR;
   auto box_pos = [&](int tile, int part) {
     const int k0 = lo_al + tile * DM_TK, kpos = k0 + part * BR;
@@ -268,7 +271,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attn_tma_kernel(const __gri
       page[part] = table[a.page_shift >= 0 ? kpos >> a.page_shift : kpos / a.page_size];
     }
   };
-  auto load_tile = [&](int tile, int stage, const int (&page)[BOXES]) {
+  auto load_tile = [&](int tile, int stage, const int* pages) {      // (AHEAD) `pages`: of the tile's boxes
     if (lane != 0 || wait_test_unarmed()) return;
     unsigned char* kd = my + (size_t)stage * 2 * TILE_BYTES;
     unsigned char* vd = kd + TILE_BYTES;
@@ -277,8 +280,15 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attn_tma_kernel(const __gri
 #pragma unroll
     for (int part = 0; part < BOXES; ++part) {
       const int kpos = box_pos(tile, part);
-      const int off = a.page_shift >= 0 ? kpos & (a.page_size - 1) : kpos % a.page_size;
-      const int y = (page[part] * a.num_kv_heads + kvh) * a.page_size + off;
+      int page, off;
+      if constexpr (AHEAD) {
+        page = pages[part];
+        off = a.page_shift >= 0 ? kpos & (a.page_size - 1) : kpos % a.page_size;
+      } else {
+        if (a.page_shift >= 0) { page = table[kpos >> a.page_shift]; off = kpos & (a.page_size - 1); }
+        else { const int idx = kpos / a.page_size; page = table[idx]; off = kpos - idx * a.page_size; }
+      }
+      const int y = (page * a.num_kv_heads + kvh) * a.page_size + off;
 #pragma unroll
       for (int h = 0; h < D64; ++h) {
         dm_tensor_copy(kd + h * 2048 + part * BR * 128, &map_k, h * 64, y, bar);
@@ -297,11 +307,14 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attn_tma_kernel(const __gri
 
   // this warp's tiles: tile_begin + warp, + WARPS, ...
   const int first = tile_begin + warp;
+  // Of eight warps the second four have no tile in a range of up to four: they fetch no queries and leave nothing to merge.
+  const int working = AHEAD && tile_end - tile_begin <= DM_WARPS ? DM_WARPS : WARPS;
   int pages[DM_STAGES][BOXES];
+  if constexpr (AHEAD) {
 #pragma unroll
-  for (int s = 0; s < DM_STAGES; ++s)
-    if (first + s * WARPS < tile_end) look_up(first + s * WARPS, pages[s]);
-#pragma unroll
+    for (int s = 0; s < DM_STAGES; ++s)
+      if (first + s * WARPS < tile_end) look_up(first + s * WARPS, pages[s]);
+  }
   for (int s = 0; s < DM_STAGES; ++s) {
     const int tile = first + s * WARPS;
     if (tile < tile_end && (FUSED || tile < ntiles_all - 1)) load_tile(tile, s, pages[s]);
@@ -319,7 +332,6 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attn_tma_kernel(const __gri
   }
   pdl_wait();
   if constexpr (!FUSED) {
-#pragma unroll
     for (int s = 0; s < DM_STAGES; ++s) {
       const int tile = first + s * WARPS;
       if (tile < tile_end && tile == ntiles_all - 1) load_tile(tile, s, pages[s]);
@@ -372,7 +384,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attn_tma_kernel(const __gri
         if constexpr (FUSED) {
           lo_w = *reinterpret_cast<const uint32_t*>(q_stage + (size_t)r * QS + kk * 16 + 2 * t);
           hi_w = *reinterpret_cast<const uint32_t*>(q_stage + (size_t)r * QS + kk * 16 + 8 + 2 * t);
-        } else if (r < ng) {
+        } else if (r < ng && warp < working) {
           const int pair = kvh * G + g0 + r;
           const bf16* qr = (const bf16*)a.q + q_row_of(qrow, pair, a) * D;
           if (q_col_lives(pair, kk * 16, D, a)) lo_w = *reinterpret_cast<const uint32_t*>(qr + kk * 16 + 2 * t);
@@ -388,9 +400,10 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attn_tma_kernel(const __gri
   for (int tile = first; tile < tile_end; tile += WARPS, ++n) {
     const int stage = n % DM_STAGES;
     const uint32_t parity = (n / DM_STAGES) & 1;
-    const int nxt = tile + DM_STAGES * WARPS;      // takes this tile's place
     int next_page[BOXES];
-    if (nxt < tile_end) look_up(nxt, next_page);
+    if constexpr (AHEAD) {
+      if (tile + DM_STAGES * WARPS < tile_end) look_up(tile + DM_STAGES * WARPS, next_page);
+    }
     if (!dm_bar_wait(&bars[warp][stage], parity)) { failed = true; break; }
     unsigned char* kt = my + (size_t)stage * 2 * TILE_BYTES;
     unsigned char* vt = kt + TILE_BYTES;
@@ -491,6 +504,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attn_tma_kernel(const __gri
     // order this warp's accesses to the stage (reads, and the zeroing above) before the copy
     // engine's next write into it
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    const int nxt = tile + DM_STAGES * WARPS;      // takes this tile's place
     if (nxt < tile_end) load_tile(nxt, stage, next_page);
   }
   if (failed && lane == 0) atomicExch(error_flag, WAIT_FAILED_DECODE_TMA);
@@ -510,7 +524,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attn_tma_kernel(const __gri
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int r = g + 8 * h;
-    if (r < ng) {
+    if (r < ng && warp < working) {
       float* w = red + ((size_t)warp * 16 + r) * WS;
 #pragma unroll
       for (int i = 0; i < 2 * D16; ++i) {
@@ -520,19 +534,23 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attn_tma_kernel(const __gri
     }
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < ng * D; idx += (WARPS * 32)) {
-    const int r = idx / D, d = idx - r * D;
-    float mm = -INFINITY;
+  // the sums of the first N warps for one output
+  auto add_up = [&](auto N, int r, int d, float& mm, float& num, float& den) {
 #pragma unroll
-    for (int w = 0; w < WARPS; ++w) mm = fmaxf(mm, red[((size_t)w * 16 + r) * WS + D]);
-    float num = 0.f, den = 0.f;
+    for (int w = 0; w < decltype(N)::value; ++w) mm = fmaxf(mm, red[((size_t)w * 16 + r) * WS + D]);
 #pragma unroll
-    for (int w = 0; w < WARPS; ++w) {
+    for (int w = 0; w < decltype(N)::value; ++w) {
       const float* ws = red + ((size_t)w * 16 + r) * WS;
       const float c = (ws[D] == -INFINITY) ? 0.f : exp2f(ws[D] - mm);
       num += ws[d] * c;
       den += ws[D + 1] * c;
     }
+  };
+  for (int idx = threadIdx.x; idx < ng * D; idx += (WARPS * 32)) {
+    const int r = idx / D, d = idx - r * D;
+    float mm = -INFINITY, num = 0.f, den = 0.f;
+    if (AHEAD && working != WARPS) add_up(std::integral_constant<int, DM_WARPS>(), r, d, mm, num, den);
+    else add_up(std::integral_constant<int, WARPS>(), r, d, mm, num, den);
     const int head = kvh * G + g0 + r;
     if (a.num_splits == 1) {
       ((bf16*)a.out)[((size_t)qrow * a.num_heads + head) * D + d] = __float2bfloat16_rn(finish_row(num, den, mm, a.sinks, head));
