@@ -74,7 +74,8 @@ def test_norms_around_a_sub_layer_kernel(dtype, rows, hidden) -> None:
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("rows, hidden", [(1, 4), (3, 2048), (7, 2052), (2, 4096), (2, 4100), (511, 256), (512, 256)])
+@pytest.mark.parametrize("rows, hidden", [(1, 4), (3, 2048), (7, 2052), (2, 4096), (2, 4100), (511, 256), (512, 256), (511, 1536), (296, 1540),
+                                          (297, 1540), (296, 2560), (297, 2560), (148, 2564), (149, 2564), (148, 4096), (149, 4096)])
 def test_norms_around_a_sub_layer_in_registers_and_in_shared_memory(dtype, rows, hidden) -> None:
     """Rows on the 16-byte grid (few of them: a CTA a row, in registers) against the same values a single element off it, which
     go the general way, with every optional operand: sums of squares in another order, 2^-21 of them at most, which may move

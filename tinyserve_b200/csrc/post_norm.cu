@@ -45,8 +45,10 @@ struct PostNormArgs {
 // (the weights) is asked for in front of the wait, all that belongs to the row at once behind it, and each of the two sums
 // meets at one barrier. Needs hidden % 4 == 0 and hidden <= 4,096 (beyond, the registers do not hold a row). The kernel below /
 // this one, rows of 1,024, bf16, both norms, back to back: 1 row 2.54 / 2.03 us, 64 2.84 / 2.11, 190 4.44 / 2.62, 500 5.15 / 3.04; from 1,000
-// rows on equal.
-constexpr int POST_ROW_ROWS = 512;       // from this many rows on bound by throughput
+// rows on equal. So it takes up to 511 rows of up to 1,024 values; longer ones as many as run at once, two CTAs an SM up to 2,560
+// values, one beyond (registers): 4,096 values, 148 rows 4.1 / 3.7 us, 149 4.5 / 6.1, 511 7.0 / 11.6; 2,560 values, 296 rows 4.3 / 3.7, 297
+// 5.3 / 5.8, 511 5.7 / 6.7.
+static int post_row_most(int hidden) { return hidden <= 1024 ? 511 : hidden <= 2560 ? 2 * 148 : hidden <= 4096 ? 148 : 0; }
 template <typename T, int NV>
 __global__ void __launch_bounds__(512) post_norm_row_kernel(PostNormArgs a) {
   __shared__ float parts[2][32];
@@ -255,7 +257,7 @@ extern "C" int ts_post_norm_add_rms_norm(float* resid, const void* delta, const 
   const bool aligned = hidden % 4 == 0 &&
       (((uintptr_t)resid | (uintptr_t)delta | (uintptr_t)post_weight | (uintptr_t)layer_scale | (uintptr_t)delta_bias | (uintptr_t)weight | (uintptr_t)out |
         (uintptr_t)second | (uintptr_t)add_rows | (uintptr_t)add_vec) & 15) == 0;
-  if (aligned && hidden <= 4096 && num_rows < POST_ROW_ROWS) {
+  if (aligned && num_rows <= post_row_most(hidden)) {
     const int quads = hidden / 4, threads = ((quads <= 512 ? quads : (quads + 1) / 2) + 31) / 32 * 32;
 #define TS_PN_ROW(T_)                                                                          \
   return quads <= 512 ? launch(post_norm_row_kernel<T_, 1>, num_rows, threads, 0, stream, a)  \
