@@ -181,8 +181,23 @@ def test_latent_attention_of_single_tokens_over_any_number_of_ranges(heads, rank
     it, so a sum of values of at most about 5 is off by 5 x 2^-9 and rounded once more."""
     from tinyserve_b200.kernels import ops
 
+    monkeypatch.setattr(ops, "LATENT_FORM", "rows16")
     monkeypatch.setattr(ops, "latent_splits", lambda *args: splits)
     lens = [1, 15, 16, 17, 64, 65, 127, 128, 129, 256, 257, 1000]
+    for sinks in (None, _rand(heads, seed=9, scale=2.0)):
+        got, want, *_ = _sink_case(torch.bfloat16, heads, rank, rot, 16, lens, [1] * len(lens), sinks)
+        torch.testing.assert_close(got, want, **_tol(torch.bfloat16))
+
+
+@pytest.mark.parametrize("splits", [1, 2, 16])
+@pytest.mark.parametrize("heads, rank, rot", [(1, 16, 0), (64, 512, 64), (65, 128, 64), (128, 272, 32)])
+def test_latent_attention_of_single_tokens_64_heads_a_cta(heads, rank, rot, splits, monkeypatch) -> None:
+    """Keys around the 32 of a tile, fewer of them than ranges, heads around the 64 of a CTA, with and without sinks."""
+    from tinyserve_b200.kernels import ops
+
+    monkeypatch.setattr(ops, "LATENT_FORM", "rows64")
+    monkeypatch.setattr(ops, "latent_splits_rows64", lambda *args: splits)
+    lens = [1, 31, 32, 33, 64, 65, 1000]
     for sinks in (None, _rand(heads, seed=9, scale=2.0)):
         got, want, *_ = _sink_case(torch.bfloat16, heads, rank, rot, 16, lens, [1] * len(lens), sinks)
         torch.testing.assert_close(got, want, **_tol(torch.bfloat16))

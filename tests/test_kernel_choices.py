@@ -148,3 +148,22 @@ def test_few_rows_of_large_matrices_by_the_shape_of_the_matrix() -> None:
     assert not take(1, 4096, 4088) and not take(1, 4096, 4100) and not take(1, 4096, 4096, dtype=torch.float32)
     assert take(1, 12288, 4096, True) and take(16, 1024, 8192, True) and take(1, 16384, 512, True)
     assert not take(1, 512, 16384, True) and not take(1, 32768, 256, True) and not take(17, 12288, 4096, True)
+
+
+def test_latent_attention_of_single_tokens_by_16_heads_a_cta_or_64() -> None:
+    """Shapes measured on both sides (the comment at ``latent_form``): few heads, few requests or few keys take 16 heads a CTA."""
+    for requests, heads, keys, rank, d, rows64 in [(1, 16, 4000, 512, 576, False), (64, 32, 4000, 512, 576, False), (1, 64, 60000, 512, 576, False),
+                                                   (4, 64, 500, 512, 576, False), (1, 128, 16000, 512, 576, False), (16, 8, 500, 128, 144, False),
+                                                   (4, 64, 16000, 512, 576, True), (64, 64, 4000, 512, 576, True), (64, 128, 200, 512, 576, True),
+                                                   (256, 128, 2000, 512, 576, True), (16, 64, 4000, 128, 192, True)]:
+        form, splits = ops.latent_form(requests, heads, keys, rank, d)
+        assert form == rows64, (requests, heads, keys)
+        if rows64:
+            assert splits == ops.latent_splits_rows64(requests, heads, keys) <= 16 and splits * 64 <= max(64, keys)
+        else:
+            assert splits == ops.latent_splits(requests, heads, keys) <= 8
+    for requests in range(1, 300, 7):
+        for heads in (1, 16, 17, 64, 65, 128):
+            for keys in (1, 63, 64, 129, 5000):
+                form, splits = ops.latent_form(requests, heads, keys, 512, 576)
+                assert 1 <= splits <= (16 if form else 8) and splits * requests * -(-heads // (64 if form else 16)) <= max(148, requests * -(-heads // (64 if form else 16)))

@@ -328,6 +328,8 @@ static int launch_latent(const LatentAttnArgs& a, int max_query_len, cudaStream_
 // P V to its columns, V being the first R elements of the very same rows in shared memory (read
 // transposed by ldmatrix). Both warps of a row group form the same S; that costs a third of the
 // multiply-adds again and saves exchanging P through shared memory.
+// With `splits` > 1 (steps of single tokens, see ts_latent_attention) a CTA takes one range of the keys and leaves an
+// unnormalised partial result; latent_merge_kernel adds the ranges up.
 constexpr int LM_THREADS = 256, LM_ROWS = 64, LM_TK = 32;
 
 __device__ __forceinline__ void lm_cp_async16(void* smem, const void* gmem, bool valid) {
@@ -356,9 +358,15 @@ __device__ __forceinline__ uint32_t lm_pack(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
+struct LatentSplit {
+  int splits;
+  float* part_acc;   // [T, H, splits, R]
+  float* part_ml;    // [T, H, splits, 2]
+};
+
 // NB: blocks of 8 output columns a warp owns at most (its half of R is 8 NB columns or fewer).
 template <int NB>
-__global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(LatentAttnArgs a, int ld) {
+__global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(LatentAttnArgs a, LatentSplit sp, int ld) {
   extern __shared__ __align__(16) unsigned char lm_raw[];
   bf16* Qs = (bf16*)lm_raw;                        // [LM_ROWS][ld]
   bf16* Ks = Qs + (size_t)LM_ROWS * ld;            // [2][LM_TK][ld]
@@ -371,7 +379,8 @@ __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(Lat
   const int t0 = blockIdx.x * a.tokens_per_cta;
   if (t0 >= n) return;
   const int nt = min(a.tokens_per_cta, n - t0);
-  const int h0 = blockIdx.z * a.heads_per_cta;
+  const int chunk = blockIdx.z / sp.splits, split = blockIdx.z - chunk * sp.splits;
+  const int h0 = chunk * a.heads_per_cta;
   const int nh = min(a.heads_per_cta, a.heads - h0);
   const int nrows = nt * nh;
   const int ctx = a.ctx_lens[seq];
@@ -384,7 +393,13 @@ __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(Lat
   const int chunks = D >> 3;                       // 16-byte pieces of a row
 
   const int qpos_first = first_pos + t0, qpos_last = first_pos + t0 + nt - 1;
-  const int k_lo = a.window > 0 ? max(0, qpos_first - a.window + 1) : 0, k_hi = qpos_last + 1;
+  int k_lo = a.window > 0 ? max(0, qpos_first - a.window + 1) : 0;
+  int k_hi = qpos_last + 1;
+  if (sp.splits > 1) {
+    const int per = (((k_hi - k_lo) + sp.splits - 1) / sp.splits + LM_TK - 1) / LM_TK * LM_TK;
+    k_lo = k_lo + split * per;
+    k_hi = min(k_hi, k_lo + per);
+  }
   const int k_begin = (k_lo / LM_TK) * LM_TK;
   const int tiles = k_hi > k_begin ? (k_hi - k_begin + LM_TK - 1) / LM_TK : 0;
 
@@ -554,20 +569,59 @@ __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(Lat
     const int tt = r / nh, hh = r - tt * nh;
     const size_t orow = (size_t)(row0 + t0 + tt) * a.heads + h0 + hh;
     const float l = half ? l_b : l_a, m = half ? m_b : m_a;
-    float den = l, keep = 1.f;
-    if (a.sinks) {
-      const float sk = a.sinks[h0 + hh] * 1.4426950408889634f;
-      const float m_new = fmaxf(m, sk);
-      keep = exp2f(m - m_new);                        // m = -inf gives 0
-      den = den * keep + exp2f(sk - m_new);
-    }
-    const float inv = den > 0.f ? keep / den : 0.f;
-    bf16* out = (bf16*)a.out + orow * R;
+    if (sp.splits == 1) {
+      float den = l, keep = 1.f;
+      if (a.sinks) {
+        const float sk = a.sinks[h0 + hh] * 1.4426950408889634f;
+        const float m_new = fmaxf(m, sk);
+        keep = exp2f(m - m_new);                      // m = -inf gives 0
+        den = den * keep + exp2f(sk - m_new);
+      }
+      const float inv = den > 0.f ? keep / den : 0.f;
+      bf16* out = (bf16*)a.out + orow * R;
 #pragma unroll
-    for (int j = 0; j < NB; ++j) {
-      const int col = col_base + j * 8 + (lane & 3) * 2;
-      if (col < R) *reinterpret_cast<__nv_bfloat162*>(out + col) = __floats2bfloat162_rn(o[j][half * 2] * inv, o[j][half * 2 + 1] * inv);
+      for (int j = 0; j < NB; ++j) {
+        const int col = col_base + j * 8 + (lane & 3) * 2;
+        if (col < R) *reinterpret_cast<__nv_bfloat162*>(out + col) = __floats2bfloat162_rn(o[j][half * 2] * inv, o[j][half * 2 + 1] * inv);
+      }
+    } else {
+      float* acc = sp.part_acc + (orow * sp.splits + split) * R;
+#pragma unroll
+      for (int j = 0; j < NB; ++j) {
+        const int col = col_base + j * 8 + (lane & 3) * 2;
+        if (col < R) *reinterpret_cast<float2*>(acc + col) = make_float2(o[j][half * 2], o[j][half * 2 + 1]);
+      }
+      if (ch == 0 && (lane & 3) == 0) {
+        sp.part_ml[(orow * sp.splits + split) * 2] = m;
+        sp.part_ml[(orow * sp.splits + split) * 2 + 1] = l;
+      }
     }
+  }
+}
+
+// out[row, :] = sum_s 2^(m_s - M) acc_s / sum_s 2^(m_s - M) l_s over the key ranges of a row.
+// With sinks, head (row % heads) adds 2^(sink log2(e) - M) to the denominator.
+__global__ void latent_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, bf16* __restrict__ out,
+                                    int splits, int R, const float* __restrict__ sinks, int heads) {
+  pdl_trigger();
+  pdl_wait();
+  const size_t row = blockIdx.x;
+  const float* ml = part_ml + row * splits * 2;
+  float mm = -INFINITY;
+  for (int s = 0; s < splits; ++s) mm = fmaxf(mm, ml[2 * s]);
+  float den = 0.f;
+  if (sinks) {
+    const float sk = sinks[row % heads] * 1.4426950408889634f;
+    mm = fmaxf(mm, sk);
+    den = exp2f(sk - mm);
+  }
+  for (int s = 0; s < splits; ++s) den += ml[2 * s] == -INFINITY ? 0.f : ml[2 * s + 1] * exp2f(ml[2 * s] - mm);
+  const float inv = den > 0.f ? 1.f / den : 0.f;
+  for (int c = threadIdx.x; c < R; c += blockDim.x) {
+    float num = 0.f;
+    for (int s = 0; s < splits; ++s)
+      if (ml[2 * s] != -INFINITY) num += part_acc[(row * splits + s) * R + c] * exp2f(ml[2 * s] - mm);
+    out[row * R + c] = from_float<bf16>(num * inv);
   }
 }
 
@@ -839,15 +893,16 @@ static int launch_latent_single(const LatentAttnArgs& a, int ld, int splits, cud
 static int latent_row_length(int D) { return ((D + 8) >> 3) & 1 ? D + 8 : D + 16; }
 
 template <int NB>
-static int launch_latent_mma(const LatentAttnArgs& a, int max_query_len, cudaStream_t stream) {
+static int launch_latent_mma(const LatentAttnArgs& a, const LatentSplit& sp, int max_query_len, cudaStream_t stream) {
   const int ld = latent_row_length(a.rank + a.rot);
   const size_t smem = sizeof(bf16) * (size_t)(LM_ROWS + 2 * LM_TK) * ld;
   if (smem > 220 * 1024) return TS_ERR_UNSUPPORTED;
   auto kern = latent_attention_mma_kernel<NB>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  dim3 grid((max_query_len + a.tokens_per_cta - 1) / a.tokens_per_cta, a.num_seqs, (a.heads + a.heads_per_cta - 1) / a.heads_per_cta);
-  return launch(kern, grid, LM_THREADS, smem, stream, a, ld);
+  const int chunks = (a.heads + a.heads_per_cta - 1) / a.heads_per_cta;
+  dim3 grid((max_query_len + a.tokens_per_cta - 1) / a.tokens_per_cta, a.num_seqs, chunks * sp.splits);
+  return launch(kern, grid, LM_THREADS, smem, stream, a, sp, ld);
 }
 
 }  // namespace ts
@@ -892,11 +947,14 @@ extern "C" int ts_latent_attention_mma_takes(int rank, int rot) {
   return rank % 16 == 0 && D % 16 == 0 && rank <= 512 && sizeof(bf16) * (size_t)(LM_ROWS + 2 * LM_TK) * latent_row_length(D) <= 220 * 1024;
 }
 
-// `splits`: key ranges per request, 1 to 8 (more than one: steps of single tokens, tensor-core form only).
+// `splits`: key ranges per request (more than one: steps of single tokens, tensor-core forms only). rows64: single tokens by
+// the kernel of 64 rows, up to 64 heads a CTA, with scratch part_acc [T, heads, splits, rank] and part_ml [T, heads, splits, 2]
+// floats where there is more than one range; else by the kernel of 16 heads a CTA, up to 8 ranges (ops.latent_form chooses).
 extern "C" int ts_latent_attention(const void* q, void* out, const void* cache, const int* block_tables, int table_width,
                                    const int* cu_q, const int* ctx_lens, int num_seqs, int max_query_len, int heads,
                                    int rank, int rot, int page_size, float scale, int window, int dtype, int use_mma,
-                                   int splits, const float* sinks, cudaStream_t stream) {
+                                   int splits, int rows64, float* part_acc, float* part_ml, int num_tokens, const float* sinks,
+                                   cudaStream_t stream) {
   if (num_seqs <= 0 || max_query_len <= 0) return 0;
   if (heads <= 0 || rank <= 0 || rank > 512 || rot < 0 || page_size <= 0 || window < 0) return TS_ERR_BAD_ARGUMENT;
   LatentAttnArgs a;
@@ -906,21 +964,29 @@ extern "C" int ts_latent_attention(const void* q, void* out, const void* cache, 
   a.sinks = sinks;
   if (dtype == TS_DTYPE_BF16 && use_mma && ts_latent_attention_mma_takes(rank, rot) &&
       (((uintptr_t)q | (uintptr_t)cache | (uintptr_t)out) & 15) == 0) {
-    if (splits < 1 || splits > LD_MAX_SPLITS || (splits > 1 && max_query_len != 1)) return TS_ERR_BAD_ARGUMENT;
-    if (max_query_len == 1) {
+    if (splits < 1 || (splits > 1 && max_query_len != 1)) return TS_ERR_BAD_ARGUMENT;
+    if (max_query_len == 1 && !rows64) {
+      if (splits > LD_MAX_SPLITS) return TS_ERR_BAD_ARGUMENT;
       const int ld = latent_row_length(rank + rot);
       const int nb = (rank + 127) / 128 * 2;        // blocks of 8 columns per warp, an even number
       if (nb <= 2) return launch_latent_single<2>(a, ld, splits, stream);
       if (nb <= 4) return launch_latent_single<4>(a, ld, splits, stream);
       return launch_latent_single<8>(a, ld, splits, stream);
     }
+    if (splits > 1 && (part_acc == nullptr || part_ml == nullptr)) return TS_ERR_BAD_ARGUMENT;
     // 64 rows a CTA where the step has them: up to 64 heads of as many tokens as fit
     a.heads_per_cta = heads < LM_ROWS ? heads : LM_ROWS;
-    a.tokens_per_cta = LM_ROWS / a.heads_per_cta;
+    a.tokens_per_cta = max_query_len == 1 ? 1 : (LM_ROWS / a.heads_per_cta);
+    LatentSplit sp;
+    sp.splits = splits; sp.part_acc = part_acc; sp.part_ml = part_ml;
     const int nb = (rank / 2 + 15) / 16 * 2;        // blocks of 8 columns per half, an even number
-    if (nb <= 8) return launch_latent_mma<8>(a, max_query_len, stream);
-    if (nb <= 16) return launch_latent_mma<16>(a, max_query_len, stream);
-    return launch_latent_mma<32>(a, max_query_len, stream);
+    int st;
+    if (nb <= 8) st = launch_latent_mma<8>(a, sp, max_query_len, stream);
+    else if (nb <= 16) st = launch_latent_mma<16>(a, sp, max_query_len, stream);
+    else st = launch_latent_mma<32>(a, sp, max_query_len, stream);
+    if (st != 0 || splits == 1) return st;
+    return launch(latent_merge_kernel, num_tokens * heads, 128, 0, stream, (const float*)part_acc, (const float*)part_ml,
+                  (bf16*)out, splits, rank, sinks, heads);
   }
   // 32 rows a CTA where the step has them: 8 heads of 4 tokens (a single token: 8 heads)
   a.heads_per_cta = heads < 8 ? heads : 8;

@@ -104,7 +104,7 @@ _SIGNATURES: dict[str, list[Any]] = {
     "ts_gemm_skinny_gated": [_vp, _vp, _vp, _i, _i, _i, _i, _f, _vp],
     "ts_latent_prepare": [_vp, _c.c_longlong, _vp, _vp, _c.c_longlong, _vp, _f, _vp, _vp, _i, _i, _vp, _vp, _vp, _i, _i, _i,
                           _i, _i, _i, _vp],
-    "ts_latent_attention": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _i, _i, _vp, _vp],
+    "ts_latent_attention": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _i, _i, _i, _vp, _vp, _i, _vp, _vp],
     "ts_latent_attention_mma_takes": [_i, _i],
     "ts_moe_route": [_vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _i,
                      _vp],
@@ -2001,15 +2001,48 @@ def talking_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
 # ------------------------------------------------------------- latent attention
 LATENT_MAX_RANK = 512
 LATENT_TENSOR_CORES = True        # bf16 at sizes the mma.sync form takes; False: CUDA cores always
-LATENT_MAX_SPLITS = 8              # the CTAs of a cluster
-LATENT_KEYS_PER_SPLIT = 128        # what a CTA takes at a time
+# Steps of single tokens have two forms on the tensor cores. 16 heads a CTA: rounds of 128 keys, up to eight ranges, the CTAs of a
+# cluster, in one kernel. 64 heads a CTA (fewer leave its rows empty): tiles of 32 keys, up to 16 ranges of 64 keys at least,
+# which a second kernel merges.
+LATENT_MAX_SPLITS = 8
+LATENT_KEYS_PER_SPLIT = 128
+LATENT_ROWS64_MAX_SPLITS = 16
+LATENT_ROWS64_KEYS_PER_SPLIT = 64
+LATENT_FORM = ""                   # "rows16" or "rows64": that form always
 
 
 def latent_splits(num_seqs: int, heads: int, keys: int) -> int:
-    """Key ranges per request for a step of single tokens: as many CTAs (one per request, 16 heads and range) as the SMs hold
-    one each, no range shorter than what a CTA takes at a time. Depends only on the step's shape."""
+    """Key ranges per request for a step of single tokens, 16 heads a CTA: as many CTAs (one per request, 16 heads and range)
+    as the SMs hold one each, no range shorter than what a CTA takes at a time. Depends only on the step's shape."""
     ctas = max(1, num_seqs * -(-heads // 16))
     return max(1, min(SM_COUNT // ctas, -(-keys // LATENT_KEYS_PER_SPLIT), LATENT_MAX_SPLITS))
+
+
+def latent_splits_rows64(num_seqs: int, heads: int, keys: int) -> int:
+    """The same, 64 heads a CTA."""
+    ctas = max(1, num_seqs * -(-heads // 64))
+    return max(1, min(SM_COUNT // ctas, keys // LATENT_ROWS64_KEYS_PER_SPLIT, LATENT_ROWS64_MAX_SPLITS))
+
+
+def latent_form(num_seqs: int, heads: int, keys: int, rank: int, d: int) -> tuple[bool, int]:
+    """For a step of single tokens, whether it takes the form of 64 heads a CTA, and its key ranges: whichever is estimated to
+    end first. A round of 128 keys takes a CTA of 16 heads some 4.7 us with rows of 192 elements, 6.7 with 576; a tile of 32
+    keys one of 64 heads 2.6 and 4.7 us. Latents of up to 256 elements leave room for two CTAs of 16 heads an SM, and clusters
+    need some SMs free to find room. Measured on B200, 16 heads a CTA / 64, 512 + 64 elements: one request of 64 heads, 500 keys
+    10.7 / 27.4 us, 60,000 400 / 559; 4 of them, 500 keys 10.9 / 27.8, 16,000 222 / 168; 64, 200 keys 34 / 36, 4,000 438 /
+    311; 64 of 128 heads, 200 keys 67 / 40, 4,000 871 / 585; 64 of 32 heads, 4,000 keys 221 / 305; 128 + 64 elements, 16 of 64
+    heads, 4,000 keys 91 / 48. Over 84 shapes (8 to 128 heads, 1 to 256 requests, 60 to 60,000 keys) the choice took no longer
+    than the faster form but for two where it is 5 and 10 % longer."""
+    splits, splits64 = latent_splits(num_seqs, heads, keys), latent_splits_rows64(num_seqs, heads, keys)
+    if LATENT_FORM:
+        return LATENT_FORM == "rows64", splits64 if LATENT_FORM == "rows64" else splits
+    ctas, ctas64 = num_seqs * -(-heads // 16) * splits, num_seqs * -(-heads // 64) * splits64
+    an_sm = 2 if rank <= 256 else 1
+    waves = -(-ctas // (an_sm * (SM_COUNT - (4 * splits if splits > 1 else 0))))
+    rounds = -(-(-(-keys // splits)) // LATENT_KEYS_PER_SPLIT)
+    us = 7.0 + waves * rounds * (3.7 + 0.0052 * d) * (1.2 if an_sm == 2 and ctas > SM_COUNT else 1.0)
+    us64 = (14.0 if splits64 > 1 else 8.0) + -(-ctas64 // SM_COUNT) * -(-(-(-keys // splits64)) // 32) * (1.55 + 0.0055 * d)
+    return (True, splits64) if us64 < us else (False, splits)
 
 
 def latent_prepare(q_in: torch.Tensor, q_folded: torch.Tensor, ckr: torch.Tensor | None, norm_weight: torch.Tensor | None,
@@ -2063,15 +2096,19 @@ def latent_attention(q: torch.Tensor, cache: torch.Tensor, page_size: int, block
         raise KernelError("latent_attention: sinks must be float32, one per head")
     _check_indices("latent_attention", block_tables, ctx, page_size, cache.shape[0] // page_size)
     mma = bool(LATENT_TENSOR_CORES and dt == torch.bfloat16 and _fn("ts_latent_attention_mma_takes")(rank, d - rank))
-    splits = 1
+    splits, rows64, part_acc, part_ml = 1, False, None, None
     if mma and ctx.max_query_len == 1:
-        splits = latent_splits(ctx.num_seqs, heads, min(ctx.max_context_len, window) if window else ctx.max_context_len)
+        rows64, splits = latent_form(ctx.num_seqs, heads, min(ctx.max_context_len, window) if window else ctx.max_context_len, rank, d)
+        if rows64 and splits > 1:
+            part_acc = ctx.arena.take((t, heads, splits, rank), torch.float32)
+            part_ml = ctx.arena.take((t, heads, splits, 2), torch.float32)
     _check(_fn("ts_latent_attention")(
         _dev(q, "q"), _dev(out, "out"), _dev(cache, "cache"), _dev(block_tables, "block_tables", torch.int32),
         block_tables.shape[1], _dev(ctx.cu_query_lens, "cu_query_lens", torch.int32),
         _dev(ctx.context_lens_dev, "context_lens", torch.int32), ctx.num_seqs, ctx.max_query_len, heads, rank, d - rank,
-        page_size, float(scale), int(window), _code(dt), int(mma), splits, _opt(sinks, "sinks", torch.float32), _stream()),
-        "latent_attention")
+        page_size, float(scale), int(window), _code(dt), int(mma), splits, int(rows64), _opt(part_acc, "part_acc"),
+        _opt(part_ml, "part_ml"), t, _opt(sinks, "sinks", torch.float32), _stream()), "latent_attention",
+        kernels=2 if part_acc is not None else 1)
 
 
 def bmm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
