@@ -214,6 +214,7 @@ def test_mlstm_scan_over_chunks(dtype, heads, d, dv, lens, monkeypatch) -> None:
 
     slots, size, gb = list(range(len(lens))), ops.mlstm_state_size(heads, d, dv), _rand(2 * heads, seed=1)
     offs = (8, 8 + heads * d, 8 + 2 * heads * d)
+    assert ops.mlstm_chunk_heads(sum(lens), len(lens), max(lens), heads, d, dv) == heads
     errors = {}
     for chunks in (True, False):
         monkeypatch.setattr(ops, "MLSTM_CHUNKS", chunks)

@@ -167,3 +167,16 @@ def test_latent_attention_of_single_tokens_by_16_heads_a_cta_or_64() -> None:
             for keys in (1, 63, 64, 129, 5000):
                 form, splits = ops.latent_form(requests, heads, keys, 512, 576)
                 assert 1 <= splits <= (16 if form else 8) and splits * requests * -(-heads // (64 if form else 16)) <= max(148, requests * -(-heads // (64 if form else 16)))
+
+
+def test_mlstm_over_chunks_by_the_step() -> None:
+    """Steps measured on both sides (the comment at ``mlstm_chunk_heads``): many short portions beside one of 128 go token by token."""
+    def some(lens, heads=8, d=128, dv=128):
+        return ops.mlstm_chunk_heads(sum(lens), len(lens), max(lens), heads, d, dv)
+
+    for lens in ([128], [256], [2048], [128] * 16, [800] * 8, [1] * 64 + [400], [100, 370, 650]):
+        assert some(lens) == 8
+    for lens in ([127], [1] * 64, [1] * 64 + [128], [1] * 256 + [128], [4] * 255 + [150]):
+        assert some(lens) == 0
+    assert some([1] * 64 + [400], heads=16) == 0 and some([256], d=129) == 0
+    assert some([1] * 256 + [128], 4, 64, 64) and not some([1] * 256 + [128], 2, 64, 512) and some([1] * 64 + [128], 2, 64, 512)

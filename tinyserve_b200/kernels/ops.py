@@ -1498,15 +1498,31 @@ def mlstm_state_size(heads: int, d: int, dv: int) -> int:
     return heads * (d * dv + -(-dv // 32) * (d + 1))
 
 
-# Long portions as products over chunks; False: token by token always. Measured on B200, 8 heads of 128 x 128, token by token / over
-# chunks: 129 tokens 54.7 / 54.8 us, 256 102 / 57, 650 252 / 63, 2,048 780 / 114; portions of 100, 370 and 650 265 / 89, eight of 800
-# 392 / 325. The kernel's tiles hold keys of up to 128; its scratch is a chunk's sums per head, and a step that would need more
-# than this of it goes token by token.
+# Long portions as products over chunks; False: token by token always. The kernel's tiles hold keys of up to 128; its scratch is a
+# chunk's sums per head, and a step that would need more than this of it goes token by token.
 MLSTM_CHUNKS = True
 MLSTM_CHUNK = 64                  # tokens of a chunk, as the kernel is built
 MLSTM_CHUNKS_MIN_TOKENS = 128
 MLSTM_CHUNKS_MAX_KEY_DIM = 128
 MLSTM_CHUNKS_SCRATCH_BYTES = 1 << 30
+
+
+def mlstm_chunk_heads(num_tokens: int, num_seqs: int, longest: int, heads: int, d: int, dv: int) -> int:
+    """``heads`` if a step's mLSTM runs over chunks; 0: token by token. Over chunks where some portion is of 128
+    tokens and that is estimated to end first: the chain of the longest portion takes 0.39 us a token, all others 1 / 560 us a
+    token and block of 32 value columns, and a state 8.5 tokens' time to come and go; a chunk, however short, moves and
+    multiplies whole states. Measured on B200, 8 heads of 128 x 128, token by token / over chunks: one portion of 128 tokens
+    53 / 47 us, 256 101 / 46, 2,048 773 / 100; 16 of 128 130 / 106, 64 of 128 457 / 407, eight of 800 386 / 288; 64 single tokens and 128 83 /
+    133, and 400 205 / 153; 256 single tokens and 128 181 / 528; 255 portions of 4 and one of 150 234 / 576."""
+    if longest < MLSTM_CHUNKS_MIN_TOKENS or d > MLSTM_CHUNKS_MAX_KEY_DIM:
+        return 0
+    blocks = heads * -(-dv // 32)
+    by_token = 4.0 + 0.39 * longest + (num_tokens - longest + 8.5 * (num_seqs - 1)) * blocks / 560.0
+    chunks, wide = num_tokens // MLSTM_CHUNK + num_seqs, d > 64
+    states = heads * (2 if wide else 1) * -(-dv // 64) / 4.0         # in states of 128 x 128
+    if 4 * chunks * heads * d * dv > MLSTM_CHUNKS_SCRATCH_BYTES:
+        return 0
+    return heads if (40.0 if wide else 25.0) + states * (0.21 * (chunks - 1) + 0.0022 * num_tokens) <= by_token else 0
 
 
 def mlstm_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: torch.Tensor, gate_bias: torch.Tensor,
@@ -1526,10 +1542,9 @@ def mlstm_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: tor
     common = (_dev(qkv, "qkv"), qkv.shape[1], q_off, k_off, v_off, _dev(gates, "gates", torch.float32),
               _dev(gate_bias, "gate_bias", torch.float32), float(cap), float(q_scale), state_ptr, state_stride,
               _dev(ctx.cu_query_lens, "cu_query_lens", torch.int32), _dev(ctx.state_slots, "state_slots", torch.int32), ctx.num_seqs)
-    chunks = t // MLSTM_CHUNK + ctx.num_seqs
-    if (MLSTM_CHUNKS and ctx.max_query_len >= MLSTM_CHUNKS_MIN_TOKENS and d <= MLSTM_CHUNKS_MAX_KEY_DIM
-            and 4 * chunks * heads * d * dv <= MLSTM_CHUNKS_SCRATCH_BYTES and out.data_ptr() % 16 == 0):
+    if MLSTM_CHUNKS and out.data_ptr() % 16 == 0 and mlstm_chunk_heads(t, ctx.num_seqs, ctx.max_query_len, heads, d, dv):
         # long portions: 32-bit products over chunks of 64 tokens (``csrc/mlstm_chunks.cu``)
+        chunks = t // MLSTM_CHUNK + ctx.num_seqs
         left, left_n = ctx.arena.take((chunks, heads, d, dv), torch.float32), ctx.arena.take((chunks, heads, d), torch.float32)
         ends, starts = ctx.arena.take((chunks, heads, 2), torch.float64), ctx.arena.take((chunks, heads), torch.float32)
         _check(_fn("ts_mlstm_chunks")(*common, t, heads, d, dv, left.data_ptr(), left_n.data_ptr(), ends.data_ptr(), starts.data_ptr(),
