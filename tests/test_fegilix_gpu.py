@@ -287,6 +287,42 @@ def test_mlstm_scan_of_a_token_that_is_no_number_leaves_those_before_it(at, what
     assert bool((behind[:, 5] if what == "value" else behind).isnan().all())
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_mlstm_scan_over_chunks_some_heads_at_a_time(dtype, monkeypatch) -> None:
+    """Scratch for one, two (a pass that is not full behind) and all three heads: the same bits, states among them. Without
+    memory for it the step goes token by token."""
+    from tinyserve_b200.kernels import ops
+
+    heads, d, dv, lens = 3, 64, 96, [200, 1, 129]
+    t, chunks, offs = sum(lens), sum(lens) // 64 + 3, (0, heads * d, 2 * heads * d)
+    assert ops.mlstm_chunk_heads(t, 3, 200, heads, d, dv) == heads
+    x, gates, gb = _rand(t, 2 * heads * d + heads * dv, seed=1, dtype=dtype), _rand(t, 2 * heads, seed=2, scale=3.0), _rand(2 * heads, seed=3)
+
+    def run(arena=None):
+        step = FakeStep(lens, [2, 0, 1], "cuda")
+        step.arena = arena or step.arena
+        state, out = _rand(4, ops.mlstm_state_size(heads, d, dv), seed=4, scale=0.1), torch.full((t, heads, dv), float("nan"), device="cuda")
+        ops.mlstm_scan(x, *offs, gates, gb, 5.0, d ** -0.5, state, step, heads, d, dv, out)
+        return out, state
+
+    want = run()
+    for some in (1, 2):
+        monkeypatch.setattr(ops, "MLSTM_CHUNKS_SCRATCH_BYTES", some * 4 * chunks * d * dv)
+        assert ops.mlstm_chunk_heads(t, 3, 200, heads, d, dv) == some
+        for got, ref in zip(run(), want):
+            assert torch.equal(got, ref)
+    monkeypatch.undo()
+
+    class Full:
+        def take(self, shape, dtype):
+            raise torch.cuda.OutOfMemoryError("no memory")
+
+    got = run(Full())
+    monkeypatch.setattr(ops, "MLSTM_CHUNKS", False)
+    for a, b in zip(got, run()):
+        assert torch.equal(a, b)
+
+
 def test_mlstm_scan_into_an_output_off_the_16_byte_grid() -> None:
     """A long portion whose read-outs go to a place that the chunks' wide stores do not take."""
     from tinyserve_b200.kernels import ops

@@ -169,14 +169,20 @@ def test_latent_attention_of_single_tokens_by_16_heads_a_cta_or_64() -> None:
                 assert 1 <= splits <= (16 if form else 8) and splits * requests * -(-heads // (64 if form else 16)) <= max(148, requests * -(-heads // (64 if form else 16)))
 
 
-def test_mlstm_over_chunks_by_the_step() -> None:
-    """Steps measured on both sides (the comment at ``mlstm_chunk_heads``): many short portions beside one of 128 go token by token."""
+def test_mlstm_over_chunks_by_the_step_and_its_scratch() -> None:
+    """Steps measured on both sides (the comment at ``mlstm_chunk_heads``): many short portions beside one of 128 go token by token.
+    The scratch stays within its limit, whatever the step."""
     def some(lens, heads=8, d=128, dv=128):
         return ops.mlstm_chunk_heads(sum(lens), len(lens), max(lens), heads, d, dv)
 
     for lens in ([128], [256], [2048], [128] * 16, [800] * 8, [1] * 64 + [400], [100, 370, 650]):
         assert some(lens) == 8
-    for lens in ([127], [1] * 64, [1] * 64 + [128], [1] * 256 + [128], [4] * 255 + [150]):
+    for lens in ([127], [1] * 64, [1] * 64 + [128], [1] * 256 + [128], [4] * 255 + [150], [100] * 63 + [130]):
         assert some(lens) == 0
     assert some([1] * 64 + [400], heads=16) == 0 and some([256], d=129) == 0
     assert some([1] * 256 + [128], 4, 64, 64) and not some([1] * 256 + [128], 2, 64, 512) and some([1] * 64 + [128], 2, 64, 512)
+    for lens in ([2048], [800] * 8, [128] * 64, [8192] * 4, [300000]):
+        for heads, d, dv in ((8, 128, 128), (64, 128, 512), (16, 64, 64), (3, 1, 1)):
+            n = some(lens, heads, d, dv)
+            assert 0 <= n <= heads and 4 * (sum(lens) // 64 + len(lens)) * n * d * dv <= 1 << 26
+    assert 0 < some([800] * 8, 64) < 64 and some([1 << 21]) == 0

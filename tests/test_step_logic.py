@@ -88,3 +88,27 @@ def test_a_recorded_portion_replays_the_form_of_its_own_context() -> None:
     g.replay(9001)
     g.replay(2048)
     assert replayed[4] == "b" and replayed[5] in "ab"
+
+
+def test_an_arena_that_finds_no_memory_asks_for_none_of_it_later(monkeypatch) -> None:
+    """Who can do without (the mLSTM's scratch) catches the error and goes on: neither this step's other takes nor the buffer that
+    holds the next whole step are to be as large as what failed."""
+    from tinyserve_b200.engine import arena as module
+
+    arena, empty = module.Arena("cpu"), torch.empty
+
+    def limited(*shape, **kw):
+        if kw.get("dtype") is torch.uint8 and shape[0] > 1 << 20:
+            raise torch.cuda.OutOfMemoryError("no memory")
+        return empty(*shape, **kw)
+
+    monkeypatch.setattr(module.torch, "empty", limited)
+    for _ in range(3):
+        arena.begin_step()
+        arena.next_frame()
+        a = arena.take((1000,), torch.float32)
+        with pytest.raises(torch.cuda.OutOfMemoryError):
+            arena.take((1 << 21,), torch.uint8)
+        b = arena.take((1000,), torch.float32)
+        assert a.data_ptr() + 4000 <= b.data_ptr() or b.data_ptr() + 4000 <= a.data_ptr()
+    assert arena.reserved_bytes < 1 << 20

@@ -32,11 +32,12 @@ struct MlstmChunkArgs {
   float* state; int state_stride;     // per head: S [d][dv], then a copy of (n [d], m) per block of 32 value columns
   const int* cu_q; const int* state_slots;
   int num_seqs, H, d, dv;
+  int h0, some;                       // the heads of this pass: h0 .. h0 + some (all, where the scratch holds all)
   float* out;                         // [T, H, dv]
-  float* left;                        // [chunks, H, d, dv]: what a chunk leaves, then its starting state
-  float* left_n;                      // [chunks, H, d]: the same of the normaliser
-  double* ends;                       // [chunks, H, 2]: F_end and the largest g
-  float* starts;                      // [chunks, H]: m_0
+  float* left;                        // [chunks, some, d, dv]: what a chunk leaves, then its starting state
+  float* left_n;                      // [chunks, some, d]: the same of the normaliser
+  double* ends;                       // [chunks, some, 2]: F_end and the largest g
+  float* starts;                      // [chunks, some]: m_0
 };
 
 // e^x of a difference of sums in 64-bit: rounded to 32 bits, an x in the tens would leave its last digits to the result.
@@ -99,7 +100,7 @@ __global__ void __launch_bounds__(2 * NP) mlstm_leave_kernel(MlstmChunkArgs a) {
   pdl_trigger();
   pdl_wait();
   int t0, nt;
-  const int g = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * SC_V;
+  const int g = blockIdx.x, h = a.h0 + blockIdx.y, v0 = blockIdx.z * SC_V;
   if (!find_chunk(a.cu_q, a.num_seqs, g, t0, nt)) return;
   const int tid = threadIdx.x, lane = tid & 31;
   if (tid < 32) mlstm_gates(a, h, t0, nt, lane, cum_s, g_s, top_s);
@@ -118,7 +119,7 @@ __global__ void __launch_bounds__(2 * NP) mlstm_leave_kernel(MlstmChunkArgs a) {
     v.x *= w; v.y *= w; v.z *= w; v.w *= w;
     *p = v;
   }
-  const size_t at = (size_t)g * a.H + h;
+  const size_t at = (size_t)g * a.some + blockIdx.y;
   if (blockIdx.z == 0) {
     if (tid == 0) {
       a.ends[2 * at] = cum_s[SC_Q - 1];
@@ -156,7 +157,7 @@ template <int VEC>
 __global__ void __launch_bounds__(128) mlstm_combine_kernel(MlstmChunkArgs a) {
   pdl_trigger();
   pdl_wait();
-  const int b = blockIdx.x, h = blockIdx.y;
+  const int b = blockIdx.x, h = a.h0 + blockIdx.y;
   const int start = a.cu_q[b], n = a.cu_q[b + 1] - start;
   if (n <= 0) return;
   const int copies = (a.dv + 31) / 32, per_head = a.d * a.dv;
@@ -167,10 +168,10 @@ __global__ void __launch_bounds__(128) mlstm_combine_kernel(MlstmChunkArgs a) {
   const int idx = (normaliser ? threadIdx.x : blockIdx.z * blockDim.x + threadIdx.x) * VEC;
   const int size = normaliser ? a.d : per_head;
   const bool mine = idx < size;
-  float* p0 = (normaliser ? a.left_n : a.left) + ((size_t)first * a.H + h) * size + idx;
-  const size_t step = (size_t)a.H * size;
-  double* e0 = a.ends + ((size_t)first * a.H + h) * 2;
-  const size_t estep = (size_t)a.H * 2;
+  float* p0 = (normaliser ? a.left_n : a.left) + ((size_t)first * a.some + blockIdx.y) * size + idx;
+  const size_t step = (size_t)a.some * size;
+  double* e0 = a.ends + ((size_t)first * a.some + blockIdx.y) * 2;
+  const size_t estep = (size_t)a.some * 2;
   float s[VEC], m = of_n[a.d];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) s[e] = mine && idx + e < size ? (normaliser ? of_n : head)[idx + e] : 0.f;
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(128) mlstm_combine_kernel(MlstmChunkArgs a) {
       // (S and n carry e^(-m) with m as it is stored, rounded to 32 bits)
       const float m_new = (float)(fall[j] + fmax((double)m, top[j]));
       const float keep = exp_of(fall[j] + (double)m - (double)m_new), take = exp_of(fall[j] + top[j] - (double)m_new);
-      if (normaliser && threadIdx.x == 0) a.starts[(size_t)(first + c0 + j) * a.H + h] = m;
+      if (normaliser && threadIdx.x == 0) a.starts[(size_t)(first + c0 + j) * a.some + blockIdx.y] = m;
 #pragma unroll
       for (int e = 0; e < VEC; ++e) s[e] = fmaf(keep, s[e], take * left[j][e]);
       m = m_new;
@@ -232,10 +233,10 @@ __global__ void __launch_bounds__(MC_THREADS, 2) mlstm_read_kernel(MlstmChunkArg
   pdl_trigger();
   pdl_wait();
   int t0, nt, seq;
-  const int g = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * SC_V, d = a.d;
+  const int g = blockIdx.x, h = a.h0 + blockIdx.y, v0 = blockIdx.z * SC_V, d = a.d;
   if (!find_chunk(a.cu_q, a.num_seqs, g, t0, nt, &seq)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const size_t at = (size_t)g * a.H + h;
+  const size_t at = (size_t)g * a.some + blockIdx.y;
   const T* row = (const T*)a.qkv + (size_t)t0 * a.stride;
   load_transposed(row + a.q_off + h * d, a.stride, nt, d, NP, q_s, warp, MC_THREADS / 32, lane, a.q_scale);
   load_transposed(row + a.k_off + h * d, a.stride, nt, d, NP, s_s, warp, MC_THREADS / 32, lane);
@@ -336,7 +337,7 @@ __global__ void __launch_bounds__(MC_THREADS, 2) mlstm_read_kernel(MlstmChunkArg
 }
 
 template <typename T, int NP>
-static int launch_mlstm_chunks(const MlstmChunkArgs& a, int chunks, cudaStream_t stream) {
+static int launch_mlstm_chunks(MlstmChunkArgs a, int chunks, cudaStream_t stream) {
   const int vblocks = (a.dv + SC_V - 1) / SC_V, per_head = a.d * a.dv;
   const size_t leave = sizeof(float) * SC_Q * (NP + SC_V);
   const size_t read = sizeof(float) * (2 * (size_t)NP * SC_LD + SC_Q * SC_V + SC_Q * SC_LD);
@@ -344,31 +345,35 @@ static int launch_mlstm_chunks(const MlstmChunkArgs& a, int chunks, cudaStream_t
   auto rk = mlstm_read_kernel<T, NP>;
   if (int e = (int)cudaFuncSetAttribute(lk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)leave)) return e;
   if (int e = (int)cudaFuncSetAttribute(rk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)read)) return e;
-  if (int e = launch(lk, dim3(chunks, a.H, vblocks), 2 * NP, leave, stream, a)) return e;
-  const int vec = a.d % 4 == 0 ? 4 : 1;
-  const dim3 cgrid(a.num_seqs, a.H, (per_head / vec + 127) / 128 + 1);
-  if (int e = vec == 4 ? launch(mlstm_combine_kernel<4>, cgrid, 128, 0, stream, a) : launch(mlstm_combine_kernel<1>, cgrid, 128, 0, stream, a)) return e;
-  return launch(rk, dim3(chunks, a.H, vblocks), MC_THREADS, read, stream, a);
+  const int vec = a.d % 4 == 0 ? 4 : 1, most = a.some;
+  for (; a.h0 < a.H; a.h0 += most) {       // (each kernel waits for the pass before, whose scratch it takes over)
+    a.some = a.H - a.h0 < most ? a.H - a.h0 : most;
+    if (int e = launch(lk, dim3(chunks, a.some, vblocks), 2 * NP, leave, stream, a)) return e;
+    const dim3 cgrid(a.num_seqs, a.some, (per_head / vec + 127) / 128 + 1);
+    if (int e = vec == 4 ? launch(mlstm_combine_kernel<4>, cgrid, 128, 0, stream, a) : launch(mlstm_combine_kernel<1>, cgrid, 128, 0, stream, a)) return e;
+    if (int e = launch(rk, dim3(chunks, a.some, vblocks), MC_THREADS, read, stream, a)) return e;
+  }
+  return 0;
 }
 
 }  // namespace ts
 
 using namespace ts;
 
-// As ts_mlstm_scan, d up to 128; left [chunks, heads, d, dv], left_n [chunks, heads, d], ends [chunks, heads, 2] doubles and
-// starts [chunks, heads] are scratch with chunks = num_tokens / 64 + num_seqs.
+// As ts_mlstm_scan, d up to 128, `some` heads at a time; left [chunks, some, d, dv], left_n [chunks, some, d], ends
+// [chunks, some, 2] doubles and starts [chunks, some] are scratch with chunks = num_tokens / 64 + num_seqs.
 extern "C" int ts_mlstm_chunks(const void* qkv, int stride, int q_off, int k_off, int v_off, const float* gates, const float* gate_bias,
                                float cap, float q_scale, float* state, int state_stride, const int* cu_q, const int* state_slots,
-                               int num_seqs, int num_tokens, int heads, int d, int dv, float* left, float* left_n, double* ends,
+                               int num_seqs, int num_tokens, int heads, int some, int d, int dv, float* left, float* left_n, double* ends,
                                float* starts, float* out, int dtype, cudaStream_t stream) {
   if (num_seqs <= 0 || num_tokens <= 0) return 0;
-  if (heads <= 0 || d <= 0 || dv <= 0 || !(cap > 0.f) || !left || !left_n || !ends || !starts || !state || !out) return TS_ERR_BAD_ARGUMENT;
+  if (heads <= 0 || some <= 0 || some > heads || d <= 0 || dv <= 0 || !(cap > 0.f) || !left || !left_n || !ends || !starts || !state || !out) return TS_ERR_BAD_ARGUMENT;
   if (d > SC_MAX_STATE || (((uintptr_t)left | (uintptr_t)left_n | (uintptr_t)ends | (uintptr_t)out) & 15)) return TS_ERR_UNSUPPORTED;
   MlstmChunkArgs a;
   a.qkv = qkv; a.stride = stride; a.q_off = q_off; a.k_off = k_off; a.v_off = v_off;
   a.gates = gates; a.gate_bias = gate_bias; a.cap = cap; a.q_scale = q_scale; a.state = state; a.state_stride = state_stride;
   a.cu_q = cu_q; a.state_slots = state_slots; a.num_seqs = num_seqs; a.H = heads; a.d = d; a.dv = dv;
-  a.out = out; a.left = left; a.left_n = left_n; a.ends = ends; a.starts = starts;
+  a.h0 = 0; a.some = some; a.out = out; a.left = left; a.left_n = left_n; a.ends = ends; a.starts = starts;
   const int chunks = num_tokens / SC_Q + num_seqs;
   if (dtype == TS_DTYPE_F32) return d <= 64 ? launch_mlstm_chunks<float, 64>(a, chunks, stream) : launch_mlstm_chunks<float, 128>(a, chunks, stream);
   if (dtype == TS_DTYPE_BF16) return d <= 64 ? launch_mlstm_chunks<bf16, 64>(a, chunks, stream) : launch_mlstm_chunks<bf16, 128>(a, chunks, stream);

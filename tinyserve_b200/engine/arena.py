@@ -66,13 +66,18 @@ class _Region:
             numel *= int(s)
         size = _element_size(dtype)
         nbytes = numel * size
+        before = self.demand, self.high_water
         self.demand = (self.demand + _ALIGN - 1) // _ALIGN * _ALIGN + nbytes
         self.high_water = max(self.high_water, self.demand)
         end = start + nbytes
         if end > self.buf.numel():
             # Grow: views handed out earlier keep the old buffer alive until they die.
             grow = max(nbytes, 2 * self.buf.numel(), 1 << 16)
-            self.buf = torch.empty((grow + _ALIGN - 1) // _ALIGN * _ALIGN, dtype=torch.uint8, device=self.device)
+            try:
+                self.buf = torch.empty((grow + _ALIGN - 1) // _ALIGN * _ALIGN, dtype=torch.uint8, device=self.device)
+            except torch.cuda.OutOfMemoryError:
+                self.demand, self.high_water = before        # who can do without it goes on; no later step is to hold it
+                raise
             self.moves += 1
             self._typed = {}
             self._views = {}

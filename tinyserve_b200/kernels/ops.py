@@ -61,7 +61,7 @@ _SIGNATURES: dict[str, list[Any]] = {
     "ts_head_norm_gate": [_vp, _i, _vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _f, _i, _i, _i, _i, _vp],
     "ts_post_norm_add_rms_norm": [_vp, _vp, _vp, _vp, _f, _i, _f, _vp, _i, _f, _vp, _vp, _i, _i, _vp, _vp, _f, _vp, _vp, _i, _vp],
     "ts_mlstm_scan": [_vp, _i, _i, _i, _i, _vp, _vp, _f, _f, _vp, _i, _vp, _vp, _i, _i, _i, _i, _vp, _i, _vp],
-    "ts_mlstm_chunks": [_vp, _i, _i, _i, _i, _vp, _vp, _f, _f, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp],
+    "ts_mlstm_chunks": [_vp, _i, _i, _i, _i, _vp, _vp, _f, _f, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp],
     "ts_delta_scan": [_vp, _i, _i, _i, _i, _vp, _i, _i, _vp, _vp, _vp, _i, _f, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp],
     "ts_causal_conv_silu": [_vp, _i, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _vp, _i, _i, _vp],
     "ts_qkv_prepare": [_vp, _i, _vp, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp, _f, _vp, _vp, _i, _vp, _vp, _vp, _i, _i, _i, _i,
@@ -1498,17 +1498,18 @@ def mlstm_state_size(heads: int, d: int, dv: int) -> int:
     return heads * (d * dv + -(-dv // 32) * (d + 1))
 
 
-# Long portions as products over chunks; False: token by token always. The kernel's tiles hold keys of up to 128; its scratch is a
-# chunk's sums per head, and a step that would need more than this of it goes token by token.
+# Long portions as products over chunks; False: token by token always. The kernel's tiles hold keys of up to 128. Its scratch
+# is a chunk's sums per head, as many heads at a time as keep it within this size; a step whose one head does not fit goes
+# token by token, and so does one that finds no memory for it.
 MLSTM_CHUNKS = True
 MLSTM_CHUNK = 64                  # tokens of a chunk, as the kernel is built
 MLSTM_CHUNKS_MIN_TOKENS = 128
 MLSTM_CHUNKS_MAX_KEY_DIM = 128
-MLSTM_CHUNKS_SCRATCH_BYTES = 1 << 30
+MLSTM_CHUNKS_SCRATCH_BYTES = 1 << 26
 
 
 def mlstm_chunk_heads(num_tokens: int, num_seqs: int, longest: int, heads: int, d: int, dv: int) -> int:
-    """``heads`` if a step's mLSTM runs over chunks; 0: token by token. Over chunks where some portion is of 128
+    """How many heads at a time a step's mLSTM runs over chunks; 0: token by token. Over chunks where some portion is of 128
     tokens and that is estimated to end first: the chain of the longest portion takes 0.39 us a token, all others 1 / 560 us a
     token and block of 32 value columns, and a state 8.5 tokens' time to come and go; a chunk, however short, moves and
     multiplies whole states. Measured on B200, 8 heads of 128 x 128, token by token / over chunks: one portion of 128 tokens
@@ -1520,9 +1521,11 @@ def mlstm_chunk_heads(num_tokens: int, num_seqs: int, longest: int, heads: int, 
     by_token = 4.0 + 0.39 * longest + (num_tokens - longest + 8.5 * (num_seqs - 1)) * blocks / 560.0
     chunks, wide = num_tokens // MLSTM_CHUNK + num_seqs, d > 64
     states = heads * (2 if wide else 1) * -(-dv // 64) / 4.0         # in states of 128 x 128
-    if 4 * chunks * heads * d * dv > MLSTM_CHUNKS_SCRATCH_BYTES:
+    some = min(heads, MLSTM_CHUNKS_SCRATCH_BYTES // (4 * chunks * d * dv))
+    if not some:
         return 0
-    return heads if (40.0 if wide else 25.0) + states * (0.21 * (chunks - 1) + 0.0022 * num_tokens) <= by_token else 0
+    fixed = (40.0 if wide else 25.0) + 25.0 * ((heads - 1) // some)         # a further pass over heads starts and ends anew
+    return some if fixed + states * (0.21 * (chunks - 1) + 0.0022 * num_tokens) <= by_token else 0
 
 
 def mlstm_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: torch.Tensor, gate_bias: torch.Tensor,
@@ -1542,13 +1545,18 @@ def mlstm_scan(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, gates: tor
     common = (_dev(qkv, "qkv"), qkv.shape[1], q_off, k_off, v_off, _dev(gates, "gates", torch.float32),
               _dev(gate_bias, "gate_bias", torch.float32), float(cap), float(q_scale), state_ptr, state_stride,
               _dev(ctx.cu_query_lens, "cu_query_lens", torch.int32), _dev(ctx.state_slots, "state_slots", torch.int32), ctx.num_seqs)
-    if MLSTM_CHUNKS and out.data_ptr() % 16 == 0 and mlstm_chunk_heads(t, ctx.num_seqs, ctx.max_query_len, heads, d, dv):
+    some = mlstm_chunk_heads(t, ctx.num_seqs, ctx.max_query_len, heads, d, dv) if MLSTM_CHUNKS and out.data_ptr() % 16 == 0 else 0
+    if some:
         # long portions: 32-bit products over chunks of 64 tokens (``csrc/mlstm_chunks.cu``)
         chunks = t // MLSTM_CHUNK + ctx.num_seqs
-        left, left_n = ctx.arena.take((chunks, heads, d, dv), torch.float32), ctx.arena.take((chunks, heads, d), torch.float32)
-        ends, starts = ctx.arena.take((chunks, heads, 2), torch.float64), ctx.arena.take((chunks, heads), torch.float32)
-        _check(_fn("ts_mlstm_chunks")(*common, t, heads, d, dv, left.data_ptr(), left_n.data_ptr(), ends.data_ptr(), starts.data_ptr(),
-                                      _dev(out, "out", torch.float32), _code(qkv.dtype), _stream()), "mlstm_scan", kernels=3)
+        try:
+            left, left_n = ctx.arena.take((chunks, some, d, dv), torch.float32), ctx.arena.take((chunks, some, d), torch.float32)
+            ends, starts = ctx.arena.take((chunks, some, 2), torch.float64), ctx.arena.take((chunks, some), torch.float32)
+        except torch.cuda.OutOfMemoryError:
+            some = 0
+    if some:
+        _check(_fn("ts_mlstm_chunks")(*common, t, heads, some, d, dv, left.data_ptr(), left_n.data_ptr(), ends.data_ptr(), starts.data_ptr(),
+                                      _dev(out, "out", torch.float32), _code(qkv.dtype), _stream()), "mlstm_scan", kernels=3 * -(-heads // some))
         return
     _check(_fn("ts_mlstm_scan")(
         *common, heads, d, dv, _dev(out, "out", torch.float32), _code(qkv.dtype), _stream()), "mlstm_scan")
