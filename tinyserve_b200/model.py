@@ -25,7 +25,7 @@ from .kernels import launch_list, ops
 from .config.base import LayerSpec, ModelConfig, ModelSpec
 from .parts.base import (
     BLOCKS, EMBEDDINGS, HEADS, NORMS, PART_FAMILIES, POSITION_ENCODINGS, STREAM_INPUTS,
-    Block, CacheNeed, KVCacheEntry, PagedNeed, PositionEncoding, ResidualStream, StepContext, StreamInput, TensorSpec, launches_alike,
+    Block, CacheNeed, KVCacheEntry, PagedNeed, PositionEncoding, ResidualStream, StepContext, StreamInput, TensorSpec, Watched, launches_alike,
 )
 from .weights.loader import load_tensors, merge_specs
 from .weights.random_init import random_bound_tensors
@@ -37,7 +37,7 @@ BYTE_TOKENS_PER_US = {torch.bfloat16: 1.4e9, torch.float32: 7.4e7}
 
 
 @dataclass
-class Layer:
+class Layer(Watched):
     spec: LayerSpec
     block: Block
     position: PositionEncoding | None
@@ -50,7 +50,7 @@ class _RowPlaces:
 
     def __init__(self, layers: "list[Layer]", watched: list[dict[str, Any]], places: list[int], sizes: list[int]) -> None:
         self.places, self.sizes = places, sizes
-        self._watched, self._layers, self._gone = watched, layers, []
+        self._watched, self._layers, self._gone, self._seen, self._layer_ids = watched, layers, [], -1, list(map(id, layers))
         if not places:          # (a copy)
             self._gone.append(None)
             return
@@ -69,15 +69,18 @@ class _RowPlaces:
         return _RowPlaces, ([], [], [], self.sizes)
 
     def hold(self) -> bool:
-        values = self._values()
-        if self._gone or len(values) != self._count:
-            return False
-        tensors = self._tensors(values)
-        try:
-            return (list(map(id, tensors)) == self._ids and self._others(values) == self._plain
-                    and list(map(torch.Tensor.data_ptr, tensors)) == self.places)
-        except RuntimeError:          # a tensor where none was does not compare
-            return False
+        changes = Watched.changes()
+        if self._seen != changes or list(map(id, self._layers)) != self._layer_ids:
+            values = self._values()
+            if self._gone or len(values) != self._count:
+                return False
+            try:
+                if list(map(id, self._tensors(values))) != self._ids or self._others(values) != self._plain:
+                    return False
+            except RuntimeError:          # a tensor where none was does not compare
+                return False
+            self._seen = changes
+        return list(map(torch.Tensor.data_ptr, [t() for t in self._alive])) == self.places
 
 
 class ModelParts:
@@ -171,10 +174,10 @@ class ModelParts:
     # ---- layers whose launches are the same but for their tensors
     MIN_ALIKE = 6      # one layer as it comes, two that are written down, and enough that follow them
 
-    def _listable(self, n: int) -> bool:
-        layer = self.layers[self.spec.order[n].layer]
-        of = [layer.block, *layer.block.parts.values(), *layer.positions.values()]
-        return all(map(launches_alike, of if layer.position is None else [*of, layer.position]))
+    @staticmethod
+    def _listable(layer: Layer) -> bool:
+        return all(map(launches_alike, (layer.block, *layer.block.parts.values(), *layer.positions.values(),
+                                        *(() if layer.position is None else (layer.position,)))))
 
     def _find_alike(self) -> dict[int, int]:
         """Rows of calls of the order that differ in nothing but their tensors: first call -> the one after the last."""
@@ -187,10 +190,12 @@ class ModelParts:
             one, two = self.layers[a.layer], self.layers[b.layer]
             return {**vars(one.spec), "prefix": None} == {**vars(two.spec), "prefix": None}
 
+        of_layer = list(map(self._listable, self.layers))
+        listable = [of_layer[call.layer] for call in self.spec.order]
         rows, n, calls = {}, 0, len(self.spec.order)
         while n < calls:
             end = n + 1
-            while self._listable(n) and end < calls and self._listable(end) and like_next(end - 1):
+            while listable[n] and end < calls and listable[end] and like_next(end - 1):
                 end += 1
             if end - n >= self.MIN_ALIKE:
                 rows[n] = end
@@ -204,32 +209,34 @@ class ModelParts:
         the class's, say)."""
         places, form, sizes, watched = [], None, [], []
         for call in range(n, self._rows_of_alike[n]):
-            if not self._listable(call):
-                return None
             layer = self.layers[self.spec.order[call].layer]
-            roles = {id(part): role for role, part in layer.block.parts.items()}
-            of = [(role, vars(part)) for role, part in layer.block.parts.items()] + [("", vars(layer.block))]
-            watched += [vars(layer), layer.block.parts, *[attributes for _, attributes in of]]
-            now = [v for _, attributes in of for v in attributes.values() if isinstance(v, torch.Tensor)]
-            if len(now) < 2:
+            block, parts = layer.block, layer.block.parts
+            if not self._listable(layer):
                 return None
-            storages, at = [t.untyped_storage().data_ptr() for t in now], [t.data_ptr() for t in now]
-            first = [storages.index(s) for s in storages]          # the first tensor of the same memory
-            mine: list[Any] = [(t.shape, t.dtype, t.stride(), first[i], at[i] - at[first[i]]) for i, t in enumerate(now)]
-            mine += [layer.position, *layer.positions.items()]
-            for role, attributes in of:
+            of, now, plain = [vars(part) for part in parts.values()], [], []
+            for attributes in of:
                 for name, v in attributes.items():
-                    if id(v) in roles:
-                        v = roles[id(v)]                           # the block's name for one of its parts
-                    elif isinstance(v, torch.Tensor):
+                    if isinstance(v, torch.Tensor):
+                        now.append(v)
                         v = torch.Tensor
-                    elif not (v is None or isinstance(v, (bool, int, float, str)) or v is layer.block.parts):
-                        return None
-                    mine.append((role, name, None if v is layer.block.parts else v))
-            if form is None:
-                form, sizes = mine, [t.numel() * t.element_size() for t in now]
-            if mine != form:
+                    plain.append((name, v))
+            roles = {id(part): role for role, part in parts.items()}           # (the block's names for its parts)
+            own = [(name, roles.get(id(v), v)) for name, v in vars(block).items() if v is not parts]
+            if any(isinstance(v, torch.Tensor) for _, v in own):
                 return None
+            at = [t.data_ptr() for t in now]
+            starts = [p - t.storage_offset() * t.element_size() for p, t in zip(at, now)]
+            first = [starts.index(p) for p in starts]          # the first tensor of the same memory
+            mine = (list(parts), plain, own, layer.position, layer.positions,
+                    [(t.shape, t.dtype, t.stride(), f, p - at[f]) for t, f, p in zip(now, first, at)])
+            if form is None:
+                allowed = (bool, int, float, str, type(None))
+                if len(now) < 2 or not all(v is torch.Tensor or isinstance(v, allowed) for _, v in plain + own):
+                    return None
+                form, sizes = mine, [t.numel() * t.element_size() for t in now]
+            elif mine != form:
+                return None
+            watched += [vars(layer), parts, *of, vars(block)]
             places += at
         return _RowPlaces(self.layers, watched, places, sizes)
 

@@ -401,7 +401,27 @@ def project_to_stream(x: torch.Tensor, w: torch.Tensor, stream: ResidualStream |
 EVERY_STEP = frozenset({"decode", "prefill"})
 
 
-class Part:
+_attribute_changes = [0]
+
+
+class Watched:
+    """Counts, over all objects, the attributes that are set or deleted: what was read from attributes holds as long as the count
+    stays, without another look at them."""
+
+    def __setattr__(self, name: str, value: Any) -> None:
+        _attribute_changes[0] += 1
+        object.__setattr__(self, name, value)
+
+    def __delattr__(self, name: str) -> None:
+        _attribute_changes[0] += 1
+        object.__delattr__(self, name)
+
+    @staticmethod
+    def changes() -> int:
+        return _attribute_changes[0]
+
+
+class Part(Watched):
     # The kinds of step in which the part reads nothing of the step on the host (no lengths, no
     # slot lists, no result of a device computation) and launches the same work whatever the step's
     # values: "decode" (every request brings one token) and/or "prefill" (one request brings a
@@ -526,7 +546,7 @@ def launches_alike(of: "Part | Block") -> bool:
     return bool(type(of).__dict__.get("same_launches", False))
 
 
-class Block:
+class Block(Watched):
     """Arranges the parts of one layer around the residual stream. A block class names the roles
     it wants filled: ``roles`` maps a role (a name of the block's own choosing, the key under which
     ``LayerSpec.parts`` gives the part) to the family the part comes from ("mixer",
