@@ -531,6 +531,21 @@ def test_gemm_f32_forms_agree_bit_for_bit(m, n, k) -> None:
     assert torch.equal(row[0], out[m - 1])
 
 
+@pytest.mark.parametrize("m,n,k", [(17, 65, 196), (600, 1000, 288), (600, 1000, 448), (250, 1000, 320), (96, 2050, 576), (200, 1000, 224), (1030, 512, 256)])
+def test_gemm_f32_tiles_of_a_cta_where_parts_are_no_whole_steps(m, n, k) -> None:
+    """Parts of 16 to 36 k, whole steps of a warp's tiles and not, of a last group that K does not fill: the four forms give the
+    same bits, within the bound of their order of summation, and so does what is chosen on either side of its lines."""
+    x, w = rnd(m, k, seed=1), rnd(n, k, seed=2)
+    wide = x.double() @ w.double().T
+    bound = (k / 16 + 4 + 15 + 1) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    outs = []
+    for form in (0, 3, 4, 5, 6):
+        outs.append(torch.full((m, n), float("nan"), device="cuda"))
+        ops._check(ops._fn("ts_gemm_f32")(x.data_ptr(), w.data_ptr(), outs[-1].data_ptr(), m, n, k, form, ops._stream()), "gemm")
+        assert torch.equal(outs[0], outs[-1]), form
+    assert bool(((outs[0].double() - wide).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("m,n,k", [(33, 64, 1024), (40, 132, 68), (130, 1000, 132), (5, 24, 64)])
 def test_gemm_f32_stores_to_an_output_off_the_16_byte_grid(m, n, k) -> None:
     x, w = rnd(m, k, seed=1), rnd(n, k, seed=2)

@@ -21,7 +21,8 @@
 // copies its own rows of x and w, in steps of 16 k and three cp.async stages, and none waits for another before the sums
 // meet in shared memory. Where the tiles are too few for the machine, a CTA takes one of the four groups, a warp one of its
 // parts, and the groups' CTAs are a cluster that adds up through distributed shared memory; else a warp takes a group and
-// keeps its parts' sums in shared memory. Parts shorter than a step (K up to 192) go to a kernel of thread tiles of 4 x 4
+// keeps its parts' sums in shared memory. Parts shorter than a step (K up to 192), and many tiles whose parts are no whole steps
+// (ts_gemm_f32), go to a kernel of thread tiles of 4 x 4
 // whose steps hold several parts (600 rows of 10,000 x 100 50 us, in steps of their own 73). Measured, 4 x 4 tiles for all / now: 64 rows of
 // 1,024 x 2,048 15.1 / 12.3 us, of 1,024 x 3,072 21.1 / 16.7, 128 rows of 4,096 x 1,024 39.9 / 32.7, of 1,024 x 3,072 32.8 / 24.6,
 // 190 rows of 6,144 x 1,024 70.8 / 64.5, 600 rows 216 / 203 (37 TFLOP/s: two or three warps a scheduler, which issue 72 % of
@@ -359,7 +360,7 @@ __global__ void __launch_bounds__(FT_THREADS, CTAS) gemm_f32_tile_kernel(const f
   }
 }
 
-// ----------------------------------------------------------------------------------- more rows, parts of 4 to 12 k
+// ----------------------------------------------------------------------- more rows, parts that are no whole steps
 constexpr int FS_OWN = 4, FS_K = 32, FS_STRIDE = FS_K + 4, FS_STAGES = 3;
 constexpr int FS_THREADS = (FT_M / FS_OWN) * (FT_N / FS_OWN), FS_STAGE = (FT_M + FT_N) * FS_STRIDE;     // floats
 
@@ -460,7 +461,12 @@ __global__ void __launch_bounds__(FS_THREADS, 4) gemm_f32_short_kernel(const flo
     ahead -= fours;
     for (int done = 0; done < fours;) {
       const int run = left < fours - done ? left : fours - done;
-      for (int q = 0; q < run; ++q) four(4 * (done + q));
+      if (run == WORDS) {
+#pragma unroll
+        for (int q = 0; q < WORDS; ++q) four(4 * q);
+      } else {
+        for (int q = 0; q < run; ++q) four(4 * (done + q));
+      }
       done += run;
       forward(run);
     }
@@ -511,10 +517,10 @@ static int launch_spread(Kernel kernel, dim3 grid, int threads, int own, int clu
 static long long f32_rounds(long long ctas, int per) { return (ctas + 148 * per - 1) / (148 * per) * per; }
 
 template <int SPLIT>
-static int launch_tile(const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
+static int launch_tile(bool fine, const float* x, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
   if ((M + FT_M - 1) / FT_M > 65535) return TS_ERR_BAD_ARGUMENT;
   const dim3 grid((N + FT_N - 1) / FT_N, (M + FT_M - 1) / FT_M, SPLIT);
-  if (f32_part_length(K) < FT_K) {
+  if (fine) {
     constexpr int own = (FS_STAGES * FS_STAGE + (SPLIT == 1 ? 0 : FT_M * FT_N)) * (int)sizeof(float);      // the ring, and the CTA's sums
     return launch_spread(gemm_f32_short_kernel<SPLIT>, grid, FS_THREADS, own, SPLIT, x, w, out, M, N, K, stream);
   }
@@ -532,20 +538,31 @@ static int launch_tile(const float* x, const float* w, float* out, int M, int N,
 
 using namespace ts;
 
-// `form`: 0 = chosen here; 1, 2 = a few rows, one or two weight rows a thread; 3, 4 = tiles, K over 1, 4 CTAs.
+// `form`: 0 = chosen here; 1, 2 = a few rows, one or two weight rows a thread; 3, 4 = tiles of a warp, K over 1, 4 CTAs; 5, 6 =
+// tiles of a CTA, likewise.
 extern "C" int ts_gemm_f32(const float* x, const float* w, float* out, int M, int N, int K, int form, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
-  if (K <= 0 || form < 0 || form > 4) return TS_ERR_BAD_ARGUMENT;
+  if (K <= 0 || form < 0 || form > 6) return TS_ERR_BAD_ARGUMENT;
   if (K % 4 != 0 || (((uintptr_t)x | (uintptr_t)w) & 15) != 0) return TS_ERR_UNSUPPORTED;
   if (form == 0) {
     const long long tiles = (long long)((M + FT_M - 1) / FT_M) * ((N + FT_N - 1) / FT_N);
-    // K over four CTAs where an SM is then given less than a quarter as many CTAs' worth, the cluster's meeting counted as 384 k;
-    // many tiles, or a few hundred of a short K, fill the machine as they are (640 tiles of K = 1,024 81 / 88 us with one / four)
+    // K over four CTAs where an SM is then given less than a quarter as many CTAs' worth, the cluster's meeting counted as 384 k
+    // (192 of a short K); many tiles, or a few hundred of a short K, fill the machine as they are (640 tiles of K = 1,024 81 / 88
+    // us with one / four; 96 of K = 320 11.2 / 8.8).
     const long long four = f32_rounds(4 * tiles, 2) < f32_rounds(4 * tiles, 3) ? f32_rounds(4 * tiles, 2) : f32_rounds(4 * tiles, 3);
-    const bool split = f32_part_length(K) < FT_K ? tiles <= 400 && tiles <= 100 + K / 2
-                                                 : tiles <= (K < 512 ? 100 : 320) && four + 384.0 / K < 4.0 * f32_rounds(tiles, 1);
+    const int part = f32_part_length(K);
+    const bool split = part < FT_K ? tiles <= 400 && tiles <= 100 + K / 2
+                                   : tiles <= (K < 512 ? 110 : 320) && four + (K < 512 ? 192.0 : 384.0) / K < 4.0 * f32_rounds(tiles, 1);
+    // A warp's own steps end with each part, so parts that are no whole steps, or of which K is short, leave steps half empty. With
+    // more tiles than run at once a CTA's tiles then are ahead (a warp's / a CTA's: 1,000 rows of 4,096 x 196 72 / 57 us, x 288
+    // 95 / 79, x 448 128 / 118, x 512, whole steps, 119 / 127; 190 rows of 4,096 x 1,040 76 / 67), and with a tile for nearly every SM they are with K over four
+    // CTAs (256 rows of 1,000 x 320 11.2 / 10.4).
+    const bool ragged = (part <= 68 && part % 8 == 4) || part == 24;
     if (M <= 16) form = M > 2 && N >= 2048 ? 2 : 1;
-    else form = split ? 4 : 3;
+    else if (part < FT_K) form = split ? 6 : 5;
+    else if (split) form = 4;
+    else if (tiles > 256 && (ragged || K <= 256)) form = 5;
+    else form = ragged && tiles > 110 && tiles <= 148 ? 6 : 3;
   }
   if (form <= 2) {
     if ((M + 7) / 8 > 65535) return TS_ERR_BAD_ARGUMENT;
@@ -557,6 +574,7 @@ extern "C" int ts_gemm_f32(const float* x, const float* w, float* out, int M, in
     }
     return M <= 4 ? launch_rows<4, 2>(x, w, out, M, N, K, stream) : launch_rows<8, 2>(x, w, out, M, N, K, stream);
   }
-  return form == 3 ? launch_tile<1>(x, w, out, M, N, K, stream) : launch_tile<4>(x, w, out, M, N, K, stream);
+  const bool fine = form > 4 || f32_part_length(K) < FT_K;
+  return form & 1 ? launch_tile<1>(fine, x, w, out, M, N, K, stream) : launch_tile<4>(fine, x, w, out, M, N, K, stream);
 }
 TS_LIST_ENTRY(ts_gemm_f32);
