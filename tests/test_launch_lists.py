@@ -238,3 +238,23 @@ def test_a_library_product_that_torch_was_asked_to_make_otherwise_is_in_no_list(
             assert ops._library_gemm_function() == 0 and launch_list._entry(note()[0]) is None
     finally:
         ops._library_gemm_function.cache_clear()
+
+
+def test_a_part_that_is_a_torch_module_as_well_keeps_its_parameters() -> None:
+    """Parts count what is set on them and leave the setting to the other classes that they are of."""
+    import torch
+
+    from tinyserve_b200.parts import FeedForward
+    from tinyserve_b200.parts.base import Watched
+
+    class Module(FeedForward, torch.nn.Module):
+        def __init__(self):
+            torch.nn.Module.__init__(self)
+            self.weight = torch.nn.Parameter(torch.zeros(3))
+
+    before = Watched.changes()
+    part = Module()
+    assert [name for name, _ in part.named_parameters()] == ["weight"] and Watched.changes() > before
+    before = Watched.changes()
+    del part.weight
+    assert not list(part.parameters()) and Watched.changes() == before + 1

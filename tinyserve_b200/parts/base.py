@@ -410,11 +410,11 @@ class Watched:
 
     def __setattr__(self, name: str, value: Any) -> None:
         _attribute_changes[0] += 1
-        object.__setattr__(self, name, value)
+        super().__setattr__(name, value)
 
     def __delattr__(self, name: str) -> None:
         _attribute_changes[0] += 1
-        object.__delattr__(self, name)
+        super().__delattr__(name)
 
     @staticmethod
     def changes() -> int:
