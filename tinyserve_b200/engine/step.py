@@ -182,8 +182,8 @@ class PrefillGraph:
     logits of the portion's last token are always computed (a mid-prompt portion ignores them).
 
     The prompt attention has two forms, one head a CTA or two, with the same results; which is faster
-    depends on the context (2,048 tokens of 16 / 8 heads: one head without context, 36 against 45 us a
-    layer; two at 9,001 positions, 183 against 160). So the step is recorded once for every choice that
+    depends on the portion and its context (2,048 tokens of 16 / 8 heads: one head without context, 30 against
+    43 us a layer, level at 9,001 positions, 153 and 156; 4,096 tokens: two, 76 against 90). So the step is recorded once for every choice that
     some context up to ``max_context`` makes, and a step replays the one that its own context makes."""
 
     MOST_FORMS = 4        # recordings; layouts whose choices change at many contexts share the nearest

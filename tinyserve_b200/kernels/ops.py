@@ -419,9 +419,10 @@ MAX_SPLITS = 32
 
 
 # What a tile of 128 keys costs a CTA of the tcgen05 prompt kernel with one head and with two, and what a CTA costs whatever
-# its tiles, for heads of 128 and of 64 (B200 cycles, fitted to times like those below; a tile of two heads of 128 takes 4,050, but
-# portions of 2,048 tokens behind as many, 67 us with one head a CTA and 76 with two, stay with two, which they are recorded
-# with: 3,600 draws the line there).
+# its tiles, for heads of 128 and of 64 (B200 cycles, fitted to times like those below but for one: a tile of two heads of 128 takes
+# 4,050. The 3,600 keeps portions of 2,048 tokens behind as many with two, 76 us against 67 with one, as they were chosen and
+# recorded before a tile of one head became faster and as tests/test_recorded_steps_gpu.py has them; one in twenty of random
+# steps lies between the two values).
 PREFILL_TILE_CYCLES = {128: {1: 2330, 2: 3600}, 64: {1: 2560, 2: 4050}}
 PREFILL_CTA_CYCLES = {128: {1: 12000, 2: 15000}, 64: {1: 15000, 2: 15000}}
 
