@@ -134,6 +134,7 @@ def test_the_arena_behind_a_list_stands_as_behind_the_layers(layers, hidden, inn
 def test_what_is_put_in_place_of_a_layer_s_tensors_or_attributes_is_seen() -> None:
     """Another storage under a bound tensor, another tensor, a plain attribute, a method or a part of one layer, each
     without ``bind``: the list follows where the layers are still alike, and there is none where they are not."""
+    import numpy
     import torch
 
     from tinyserve_b200.model import DecoderModel
@@ -164,13 +165,13 @@ def test_what_is_put_in_place_of_a_layer_s_tensors_or_attributes_is_seen() -> No
     for change in (lambda p, b: setattr(p["mixer"], "scale", 0.5), lambda p, b: setattr(p["mixer"], "forward", lambda *a: None),
                    lambda p, b: setattr(p["feed_forward_norm"], "eps", 0.1), lambda p, b: setattr(b, "feed_forward", p["mixer"]),
                    lambda p, b: setattr(p["mixer"], "q_norm_w", None), lambda p, b: setattr(p["mixer"], "extra", torch.zeros(2)),
-                   lambda p, b: setattr(b, "scale_b", torch.ones(3)), lambda p, b: setattr(b, "forward", lambda *a: None)):
+                   lambda p, b: setattr(b, "scale_b", torch.ones(3)), lambda p, b: setattr(p["mixer"], "scale", numpy.ones(3)), lambda p, b: setattr(b, "forward", lambda *a: None)):
         for which in ([5], range(9)):
             model, parts, blocks = fresh()
             assert model.alike_from(0) == 9 and places(model) is not None
             for n in which:
                 change(parts[n], blocks[n])
-            if len(which) == 1 or "forward" in {**vars(parts[5]["mixer"]), **vars(blocks[5])}:
+            if len(which) == 1 or isinstance(parts[5]["mixer"].scale, numpy.ndarray) or "forward" in {**vars(parts[5]["mixer"]), **vars(blocks[5])}:
                 assert places(model) is None and model.alike_from(0) == 0
     model, parts, blocks = fresh()
     model.layers[4] = model.layers[5]

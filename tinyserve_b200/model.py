@@ -44,6 +44,10 @@ class Layer(Watched):
     positions: dict[str, PositionEncoding]      # by mixer role, when the mixers have encodings of their own
 
 
+_TENSORS = frozenset({torch.Tensor, torch.nn.Parameter})      # (other classes of tensors are in no list)
+_PLAIN = frozenset({bool, int, float, str, type(None)})
+
+
 class _RowPlaces:
     """Where the tensors of a row of layers lie, call by call, and the bytes of each of a call's; with it, all that this was
     read from, so that whatever has been replaced since (a tensor, its storage, an attribute, a part) shows."""
@@ -55,8 +59,9 @@ class _RowPlaces:
             self._gone.append(None)
             return
         values = self._values()
-        tensors = [i for i, v in enumerate(values) if isinstance(v, torch.Tensor)]
-        self._tensors, self._others = itemgetter(*tensors), itemgetter(*sorted({*range(len(values))} - {*tensors}))
+        types = list(map(type, values))
+        tensors = [i for i, t in enumerate(types) if t in _TENSORS]
+        self._tensors, self._others = itemgetter(*tensors), itemgetter(*[i for i, t in enumerate(types) if t not in _TENSORS])
         # tensors by their identity, which something new may have once one has gone: that is noted, so none is kept alive here
         self._ids = list(map(id, self._tensors(values)))
         self._alive = [weakref.ref(v, self._gone.append) for v in self._tensors(values)]
@@ -213,26 +218,21 @@ class ModelParts:
             block, parts = layer.block, layer.block.parts
             if not self._listable(layer):
                 return None
-            of, now, plain = [vars(part) for part in parts.values()], [], []
-            for attributes in of:
-                for name, v in attributes.items():
-                    if isinstance(v, torch.Tensor):
-                        now.append(v)
-                        v = torch.Tensor
-                    plain.append((name, v))
+            of = [vars(part) for part in parts.values()]
             roles = {id(part): role for role, part in parts.items()}           # (the block's names for its parts)
-            own = [(name, roles.get(id(v), v)) for name, v in vars(block).items() if v is not parts]
-            if any(isinstance(v, torch.Tensor) for _, v in own):
+            own = [roles.get(id(v), v) for v in vars(block).values() if v is not parts]
+            values = list(chain(own, *map(dict.values, of)))
+            types = list(map(type, values))
+            now = [v for v, t in zip(values, types) if t in _TENSORS]
+            plain = [v for v, t in zip(values, types) if t in _PLAIN]
+            if len(now) < 2 or len(now) + len(plain) != len(values) or any(type(v) in _TENSORS for v in own):
                 return None
             at = [t.data_ptr() for t in now]
             starts = [p - t.storage_offset() * t.element_size() for p, t in zip(at, now)]
             first = [starts.index(p) for p in starts]          # the first tensor of the same memory
-            mine = (list(parts), plain, own, layer.position, layer.positions,
+            mine = (list(parts), list(chain(vars(block), *of)), types, plain, layer.position, layer.positions,
                     [(t.shape, t.dtype, t.stride(), f, p - at[f]) for t, f, p in zip(now, first, at)])
             if form is None:
-                allowed = (bool, int, float, str, type(None))
-                if len(now) < 2 or not all(v is torch.Tensor or isinstance(v, allowed) for _, v in plain + own):
-                    return None
                 form, sizes = mine, [t.numel() * t.element_size() for t in now]
             elif mine != form:
                 return None
