@@ -82,7 +82,7 @@ class _RowPlaces:
             try:
                 if list(map(id, self._tensors(values))) != self._ids or self._others(values) != self._plain:
                     return False
-            except RuntimeError:          # a tensor where none was does not compare
+            except (RuntimeError, ValueError):          # a tensor or an array where none was does not compare
                 return False
             self._seen = changes
         return list(map(torch.Tensor.data_ptr, [t() for t in self._alive])) == self.places
