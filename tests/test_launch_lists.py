@@ -165,7 +165,8 @@ def test_what_is_put_in_place_of_a_layer_s_tensors_or_attributes_is_seen() -> No
     for change in (lambda p, b: setattr(p["mixer"], "scale", 0.5), lambda p, b: setattr(p["mixer"], "forward", lambda *a: None),
                    lambda p, b: setattr(p["feed_forward_norm"], "eps", 0.1), lambda p, b: setattr(b, "feed_forward", p["mixer"]),
                    lambda p, b: setattr(p["mixer"], "q_norm_w", None), lambda p, b: setattr(p["mixer"], "extra", torch.zeros(2)),
-                   lambda p, b: setattr(b, "scale_b", torch.ones(3)), lambda p, b: setattr(p["mixer"], "scale", numpy.ones(3)), lambda p, b: setattr(b, "forward", lambda *a: None)):
+                   lambda p, b: setattr(b, "scale_b", torch.ones(3)), lambda p, b: setattr(p["mixer"], "scale", numpy.ones(3)),
+                   lambda p, b: vars(p["feed_forward"]).pop("w_down"), lambda p, b: setattr(b, "forward", lambda *a: None)):
         for which in ([5], range(9)):
             model, parts, blocks = fresh()
             assert model.alike_from(0) == 9 and places(model) is not None

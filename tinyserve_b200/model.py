@@ -74,10 +74,12 @@ class _RowPlaces:
         return _RowPlaces, ([], [], [], self.sizes)
 
     def hold(self) -> bool:
+        if self._gone:
+            return False
         changes = Watched.changes()
         if self._seen != changes or list(map(id, self._layers)) != self._layer_ids:
             values = self._values()
-            if self._gone or len(values) != self._count:
+            if len(values) != self._count:
                 return False
             try:
                 if list(map(id, self._tensors(values))) != self._ids or self._others(values) != self._plain:
